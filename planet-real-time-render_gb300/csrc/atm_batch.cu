@@ -7,10 +7,9 @@
 // (aerial).  A grid of blocks_per_sm x SM-count blocks stays resident; each
 // warp takes the next work item from an atomic ticket, finds its job by
 // binary search over the item prefix sums, copies the job's parameters into
-// its shared-memory slot and evaluates the texels/columns with the same
-// warp-level functions as the single-LUT kernels.  Warps never wait on each
-// other (the ticket is a plain atomicAdd), so uneven job sizes balance
-// without barriers.
+// its shared-memory slot and evaluates the texels or columns, one a lane.
+// Warps never wait on each other (the ticket is a plain atomicAdd), so uneven
+// job sizes balance without barriers.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -26,15 +25,13 @@
 namespace atm {
 
 struct BatchJobDev {
-  DevParams P;  // the job's parameter set with its own LUT size
+  DevParams P;   // the job's parameter set with its own LUT size
+  Frame F;       // with the job's sun
+  AerialView V;  // sky-view jobs: the camera altitude alone
   float4* out;
-  const float4* tlut;
-  const float4* mslut;
   int kind;      // ATM_LUT_SKY_VIEW or ATM_LUT_AERIAL
   int units;     // texels (sky-view) or columns (aerial)
   int per_item;  // units per work item
-  float bottom, cam_alt, sun_cos, ar, aspect, tanfov;
-  f3 sun, E, right, up, fwd;
 };
 
 namespace {
@@ -45,7 +42,9 @@ __global__ void __launch_bounds__(256, 3) k_batch(const BatchJobDev* __restrict_
                                                const long long* __restrict__ prefix, int n_jobs, long long n_items,
                                                unsigned long long* __restrict__ ticket,
                                                unsigned long long* __restrict__ samples_counter) {
-  __shared__ DevParams s_params[kBatchWarps];
+  __shared__ BatchJobDev s_job[kBatchWarps];
+  __shared__ float s_sky[kBatchWarps][kMaxSkySteps + 1];
+  __shared__ float s_aerial[kBatchWarps][kMaxAerialSteps + 1];
   const int lane = threadIdx.x & 31;
   const int warp = threadIdx.x >> 5;
   uint32_t samples = 0;
@@ -62,29 +61,29 @@ __global__ void __launch_bounds__(256, 3) k_batch(const BatchJobDev* __restrict_
       if (prefix[mid] <= static_cast<long long>(item)) lo = mid;
       else hi = mid;
     }
-    const BatchJobDev* J = jobs + lo;
-    if (lo != loaded) {  // stage the job's parameters in this warp's slot
+    const BatchJobDev& J = s_job[warp];
+    if (lo != loaded) {  // stage the job in this warp's slot
       __syncwarp();
-      const int* src = reinterpret_cast<const int*>(&J->P);
-      int* dst = reinterpret_cast<int*>(&s_params[warp]);
-      for (int k = lane; k < int(sizeof(DevParams) / sizeof(int)); k += 32) dst[k] = src[k];
+      const int* src = reinterpret_cast<const int*>(jobs + lo);
+      int* dst = reinterpret_cast<int*>(&s_job[warp]);
+      for (int k = lane; k < int(sizeof(BatchJobDev) / sizeof(int)); k += 32) dst[k] = src[k];
+      __syncwarp();
+      if (J.kind == ATM_LUT_SKY_VIEW)
+        fill_fractions(s_sky[warp], J.P.sv_steps, lane, 32);
+      else
+        fill_fractions(s_aerial[warp], J.P.ap_steps, lane, 32);
       __syncwarp();
       loaded = lo;
     }
-    const DevParams& P = s_params[warp];
     const long long local = static_cast<long long>(item) - prefix[lo];
-    const int per = J->per_item;
-    const int u0 = static_cast<int>(local * per);
-    const int u1 = min(u0 + per, J->units);
-    if (J->kind == ATM_LUT_SKY_VIEW) {
-      const float sc = J->sun_cos;
-      const float ss = sqrtf(mx(1.0f - sc * sc, 0.0f));
-      const Frame F = make_frame(P, J->tlut, J->mslut, J->bottom, J->ar, mk(ss, sc, 0.0f), J->E);
-      for (int u = u0; u < u1; ++u) samples += sky_view_texel(P, F, J->cam_alt, u % P.sv_w, u / P.sv_w, J->out);
+    const int u0 = static_cast<int>(local * J.per_item);
+    const int u1 = min(u0 + J.per_item, J.units);
+    if (J.kind == ATM_LUT_SKY_VIEW) {
+      for (int u = u0 + lane; u < u1; u += 32)
+        samples += sky_view_texel<1>(J.P, J.F, J.V.cam_alt, u % J.P.sv_w, u / J.P.sv_w, true, {s_sky[warp]}, J.out);
     } else {
-      const Frame F = make_frame(P, J->tlut, J->mslut, J->bottom, J->ar, J->sun, J->E);
-      const AerialView V{J->aspect, J->cam_alt, J->right, J->up, J->fwd, J->tanfov};
-      for (int u = u0; u < u1; ++u) samples += aerial_column(P, F, V, u % P.ap_w, u / P.ap_w, J->out);
+      for (int u = u0 + lane; u < u1; u += 32)
+        samples += aerial_column_lane(J.P, J.F, J.V, u % J.P.ap_w, u / J.P.ap_w, {s_aerial[warp]}, J.out);
     }
   }
   warp_count(samples, samples_counter);
@@ -110,30 +109,25 @@ void fill_batch_job(BatchJobDev& d, const DevParams& set_params, const AtmBatchJ
   d.P = set_params;
   d.kind = j.kind;
   d.out = arena + j.output_offset;
-  d.tlut = tlut;
-  d.mslut = mslut;
-  d.bottom = float(radius);
-  d.cam_alt = float(j.camera_altitude_m);
-  d.ar = float(ar_rad);
-  d.E = {float(E[0]), float(E[1]), float(E[2])};
   d.per_item = per_item;
+  d.units = j.width * j.height;
+  f3 sun;
   if (j.kind == ATM_LUT_SKY_VIEW) {
     d.P.sv_w = j.width;
     d.P.sv_h = j.height;
-    d.units = j.width * j.height;
-    d.sun_cos = float(j.sun_zenith_cosine);
+    sun = sky_view_sun(float(j.sun_zenith_cosine));
+    d.V.cam_alt = float(j.camera_altitude_m);
   } else {
     d.P.ap_w = j.width;
     d.P.ap_h = j.height;
     d.P.ap_d = j.depth;
-    d.units = j.width * j.height;
-    d.sun = {float(j.sun_local[0]), float(j.sun_local[1]), float(j.sun_local[2])};
-    d.right = {float(j.view_basis[0]), float(j.view_basis[1]), float(j.view_basis[2])};
-    d.up = {float(j.view_basis[3]), float(j.view_basis[4]), float(j.view_basis[5])};
-    d.fwd = {float(j.view_basis[6]), float(j.view_basis[7]), float(j.view_basis[8])};
-    d.tanfov = float(j.tangent_half_fov);
-    d.aspect = float(j.frame_width) / float(j.frame_height);
+    sun = {float(j.sun_local[0]), float(j.sun_local[1]), float(j.sun_local[2])};
+    float b[9];
+    for (int k = 0; k < 9; ++k) b[k] = float(j.view_basis[k]);
+    d.V = aerial_view(float(j.frame_width) / float(j.frame_height), float(j.camera_altitude_m), b, b + 3, b + 6,
+                      float(j.tangent_half_fov));
   }
+  d.F = make_frame(set_params, tlut, mslut, float(radius), float(ar_rad), sun, {float(E[0]), float(E[1]), float(E[2])});
 }
 
 }  // namespace atm

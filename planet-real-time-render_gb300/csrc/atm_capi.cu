@@ -125,8 +125,8 @@ DevParams make_dev_params(const AtmParams& p) {
   d.mie_k1 = float(3.0 * (1.0 - g * g));
   d.mie_k2 = float(8.0 * kPi * (2.0 + g * g));
   d.ray_k = float(16.0 * kPi);
-  d.inv_h_r = float(1.0 / p.rayleigh_scale_height_m);
-  d.inv_h_m = float(1.0 / p.mie_scale_height_m);
+  d.exp2_r = float(-M_LOG2E / p.rayleigh_scale_height_m);
+  d.exp2_m = float(-M_LOG2E / p.mie_scale_height_m);
   d.inv_oz_half = float(1.0 / p.absorption_half_width_m);
   d.inv_top = float(1.0 / p.top_altitude_m);
   d.t_w = p.transmittance_lut_width;
@@ -145,6 +145,9 @@ DevParams make_dev_params(const AtmParams& p) {
   d.ap_steps = p.aerial_steps_per_slice;
   d.limb_steps = p.aerial_horizon_raymarch_steps;
   d.substeps = p.aerial_terminator_substeps;
+  d.t_lut = lut_dims(d.t_w, d.t_h);
+  d.ms_lut = lut_dims(d.ms_w, d.ms_h);
+  d.sv_lut = lut_dims(d.sv_w, d.sv_h);
   return d;
 }
 
@@ -632,10 +635,13 @@ ATM_API int atm_batch_create(const AtmParams* sets, const double* planet_radius_
 ATM_API int atm_batch_build(AtmBatch* b, const AtmBatchJob* jobs, int32_t n_jobs, void* arena, int64_t arena_texels,
                             const AtmBatchTuning* tuning, void* stream) {
   if (!b || !jobs || !arena || !tuning || n_jobs < 1) return fail(ATM_E_INVALID, "null argument to atm_batch_build");
-  const int sv_item = tuning->sky_view_texels_per_item, ap_item = tuning->aerial_columns_per_item;
+  int sv_item = tuning->sky_view_texels_per_item, ap_item = tuning->aerial_columns_per_item;
   if (sv_item < 1 || sv_item > 4096 || ap_item < 1 || ap_item > 4096 || tuning->blocks_per_sm < 1 ||
       tuning->blocks_per_sm > 8)
     return fail(ATM_E_INVALID, "tuning out of range");
+  // a lane takes a texel or a column: items are whole warps
+  sv_item = (sv_item + 31) / 32 * 32;
+  ap_item = (ap_item + 31) / 32 * 32;
   const size_t jsz = atm::batch_job_size();
   b->h_jobs.assign(size_t(n_jobs) * jsz, 0);
   b->h_prefix.assign(size_t(n_jobs) + 1, 0);
@@ -980,9 +986,8 @@ ATM_API int atm_surrogate_samples(AtmBatch* b, int32_t kind, int64_t n, uint64_t
         p.mie_scale_height_m > r[3])
       return fail(ATM_E_INVALID, "set %d has scale heights outside the feature range", i);
     sets[i].P = b->dev[i];
-    sets[i].tlut = b->tlut[i];
-    sets[i].mslut = b->mslut[i];
-    sets[i].bottom = float(b->radius[i]);
+    sets[i].F = atm::make_frame(b->dev[i], b->tlut[i], b->mslut[i], float(b->radius[i]), float(b->ar_rad),
+                                {0.0f, 1.0f, 0.0f}, {float(b->E[0]), float(b->E[1]), float(b->E[2])});
     sets[i].lhr_n = log_feature(p.rayleigh_scale_height_m, r[0], r[1]);
     sets[i].lhm_n = log_feature(p.mie_scale_height_m, r[2], r[3]);
   }
@@ -990,10 +995,7 @@ ATM_API int atm_surrogate_samples(AtmBatch* b, int32_t kind, int64_t n, uint64_t
   if (!b->d_sets) ATM_CUDA(cudaMalloc(&b->d_sets, sizeof(atm::SurrogateSetDev) * 1024), "sample set table");
   ATM_CUDA(cudaMemcpyAsync(b->d_sets, sets.data(), sizeof(atm::SurrogateSetDev) * n_sets, cudaMemcpyHostToDevice, s),
            "sample set upload");
-  float ef[3];
-  to_f32(b->E, ef, 3);
-  ATM_CUDA(atm::launch_gen_samples(b->d_sets, n_sets, kind, n, seed, shaping, ef, float(b->ar_rad), features,
-                                   targets, b->d_samples, s),
+  ATM_CUDA(atm::launch_gen_samples(b->d_sets, n_sets, kind, n, seed, shaping, features, targets, b->d_samples, s),
            "surrogate samples");
   // the table is read by the launch: keep the host copy alive until it ran
   ATM_CUDA(cudaStreamSynchronize(s), "surrogate samples");

@@ -4,9 +4,11 @@
 // The composite is the per-frame hot loop: every surface pixel integrates
 // the real camera-to-G-buffer path over `aerial_horizon_raymarch_steps` warped
 // base intervals, each refined into `aerial_terminator_substeps` children
-// where the terminator weight is non-zero.  One thread per pixel; a warp
-// covers an 8x4 pixel tile so that the data-dependent paths (sky vs surface,
-// refined intervals) diverge as little as neighbouring pixels do.  The
+// where the terminator weight is non-zero.  One thread per pixel (several
+// lanes in small frames, launch_split); a warp covers an 8x4 pixel tile so
+// that the data-dependent paths (sky vs surface, refined intervals) diverge as
+// little as neighbouring pixels do.  Bound by instruction issue (88% active,
+// about 290 instructions a sample).  The
 // terminator weight reuses the disk visibility of the interval's coarse
 // sample, which the reference computes twice from identical inputs.
 #include <cuda_runtime.h>
@@ -20,20 +22,16 @@
 namespace atm {
 namespace {
 
-constexpr unsigned kFull = 0xffffffffu;
-
 // _prepare_surface_lighting :1422-1472
-__global__ void __launch_bounds__(256) k_prepare_surface(DevParams P, ImageLayout L, const float* __restrict__ pos,
-                                                         const int32_t* __restrict__ sid, float bottom, float cam_alt,
-                                                         f3 sun, float ar, f3 right, f3 up, f3 fwd,
-                                                         const float4* __restrict__ tlut,
-                                                         const float4* __restrict__ mslut, float* __restrict__ out_t,
+__global__ void __launch_bounds__(256) k_prepare_surface(DevParams P, Frame F, ImageLayout L,
+                                                         const float* __restrict__ pos,
+                                                         const int32_t* __restrict__ sid, float cam_alt, f3 right,
+                                                         f3 up, f3 fwd, float* __restrict__ out_t,
                                                          float* __restrict__ out_sky) {
   int x, y;
   if (!linear_pixel(L, x, y)) return;
   const size_t e = pix_offset(L, x, y);
   const size_t o = e * L.channels;
-  Frame F = make_frame(P, tlut, mslut, bottom, ar, sun, splat(0.0f));
   f3 st = splat(1.0f), sky = splat(0.0f);
   if (sid[e] >= 0) surface_lighting(P, F, cam_alt, right, up, fwd, ld3(pos + o), st, sky);
   out_t[o + 0] = st.x;
@@ -44,55 +42,68 @@ __global__ void __launch_bounds__(256) k_prepare_surface(DevParams P, ImageLayou
   out_sky[o + 2] = sky.z;
 }
 
-// One pixel of the COMPOSITE view (:1860-1940) given its surface colour
-// (scene_hdr) and surface id: writes hdr and adds the pixel's radiance
-// samples to `samples`.  Shared by the composite, its no-allocation variant
-// and the fused frame so that they cannot drift apart.
+// One pixel of the COMPOSITE view (:1860-1940) given its surface id and, as a
+// function, its surface colour (scene_hdr): writes hdr and adds the pixel's
+// radiance samples to `samples`.  Shared by the composite, its no-allocation
+// variant and the fused frame so that they cannot drift apart.  kLanes
+// consecutive lanes share the pixel's march, the first does the rest; every
+// lane of the warp must call when kLanes > 1 (`inside`: the pixel exists).
+template <int kLanes, class Scene>
 __device__ __forceinline__ void composite_pixel_with(const DevParams& P, const ImageLayout& L, const CompositeScalars& A,
-                                                     const Frame& F, f3 color, int32_t sidv,
+                                                     const Frame& F, Scene scene, int32_t sidv,
                                                      const float* __restrict__ space, const float* __restrict__ pos,
                                                      const float4* __restrict__ svlut, float* __restrict__ hdr, int x,
-                                                     int y, uint32_t& samples) {
+                                                     int y, bool inside, const TableFractions& fractions,
+                                                     uint32_t& samples) {
   const size_t o = pix_offset(L, x, y) * L.channels;
   PixelRay pr = pixel_ray(L, A, x, y);
-  if (sidv >= 0) {
+  const bool first = kLanes == 1 || (threadIdx.x & (kLanes - 1)) == 0;
+  f3 color = splat(0.0f);
+  if (kLanes > 1 || sidv >= 0) {
     const RayGeom G = camera_ray_geom(P, A.bottom, A.cam_alt, pr.ray);
-    float sd = norm(ld3(pos + o));
-    float start, end;
-    if (surface_interval(P, G, A.bottom, sd, start, end)) {
-      f3 scat = integrate_surface(P, F, G, pr.ray, start, end, samples);
-      f3 tr = surface_segment_t(P, F, G, pr.ray, start, end);
-      color = scat + color * tr;
+    float start = 0.0f, end = 0.0f;
+    const bool clipped =
+        inside && sidv >= 0 && surface_interval(P, G, A.bottom, norm(ld3(pos + o)), start, end);
+    const f3 scat = integrate_surface_split<kLanes>(P, F, G, pr.ray, start, end, clipped, fractions, samples);
+    if (first && sidv >= 0) {
+      color = scene();
+      if (clipped) color = scat + color * surface_segment_t(P, F, G, start, end);
     }
-  } else {
-    color = composite_sky(P, F, A, svlut, pr.ray, color, ld3(space + o), float(L.height));
   }
+  if (!first || !inside) return;
+  if (sidv < 0) color = composite_sky(P, F, A, svlut, pr.ray, scene(), ld3(space + o), float(L.height));
   color = vmax(color, 0.0f);
   hdr[o + 0] = color.x;
   hdr[o + 1] = color.y;
   hdr[o + 2] = color.z;
 }
-__device__ __forceinline__ void composite_pixel(const DevParams& P, const ImageLayout& L, const CompositeScalars& A,
-                                                const float* __restrict__ scene, const float* __restrict__ space,
-                                                const int32_t* __restrict__ sid, const float* __restrict__ pos,
-                                                const float4* __restrict__ tlut, const float4* __restrict__ mslut,
-                                                const float4* __restrict__ svlut, float* __restrict__ hdr, int x,
-                                                int y, uint32_t& samples) {
+template <int kLanes>
+__device__ __forceinline__ void composite_pixel(const DevParams& P, const Frame& F, const ImageLayout& L,
+                                                const CompositeScalars& A, const float* __restrict__ scene,
+                                                const float* __restrict__ space, const int32_t* __restrict__ sid,
+                                                const float* __restrict__ pos, const float4* __restrict__ svlut,
+                                                float* __restrict__ hdr, int x, int y, bool inside,
+                                                const TableFractions& fractions, uint32_t& samples) {
   const size_t e = pix_offset(L, x, y);
-  const Frame F = make_frame(P, tlut, mslut, A.bottom, A.ar, arr3(A.sun), arr3(A.E));
-  composite_pixel_with(P, L, A, F, ld3(scene + e * L.channels), sid[e], space, pos, svlut, hdr, x, y, samples);
+  composite_pixel_with<kLanes>(
+      P, L, A, F, [&] { return ld3(scene + e * L.channels); }, sid[e], space, pos, svlut, hdr, x, y, inside, fractions,
+      samples);
 }
 
 // COMPOSITE view (:1860-1940): the per-frame path.
-__global__ void __launch_bounds__(256, 3) k_composite(DevParams P, ImageLayout L, CompositeScalars A,
+template <int kLanes>
+__global__ void __launch_bounds__(256, 3) k_composite(DevParams P, Frame F, ImageLayout L, CompositeScalars A,
                                                    const float* __restrict__ scene, const float* __restrict__ space,
                                                    const int32_t* __restrict__ sid, const float* __restrict__ pos,
-                                                   const float4* __restrict__ tlut, const float4* __restrict__ mslut,
                                                    const float4* __restrict__ svlut, float* __restrict__ hdr,
                                                    unsigned long long* counter) {
+  __shared__ float s_fractions[kFractionTable];
+  const TableFractions fractions = table_fractions(P, s_fractions);
   int x, y;
   uint32_t samples = 0;
-  if (tile_pixel(L, x, y)) composite_pixel(P, L, A, scene, space, sid, pos, tlut, mslut, svlut, hdr, x, y, samples);
+  const bool inside = split_pixel<kLanes>(L, x, y);
+  if (kLanes > 1 || inside)
+    composite_pixel<kLanes>(P, F, L, A, scene, space, sid, pos, svlut, hdr, x, y, inside, fractions, samples);
   warp_count(samples, counter);
 }
 
@@ -101,19 +112,22 @@ __global__ void __launch_bounds__(256, 3) k_composite(DevParams P, ImageLayout L
 // (:1860-1940), with the lighting and the shaded colour in registers instead
 // of the three full-resolution images that the separate calls write and
 // read back.
-__global__ void __launch_bounds__(256, 3) k_frame(DevParams P, ImageLayout L, CompositeScalars A, ShadeParams S,
-                                               ShadeImages I, const float* __restrict__ space,
-                                               const float4* __restrict__ tlut, const float4* __restrict__ mslut,
+template <int kLanes>
+__global__ void __launch_bounds__(256, 3) k_frame(DevParams P, Frame F, ImageLayout L, CompositeScalars A,
+                                               ShadeParams S, ShadeImages I, const float* __restrict__ space,
                                                const float4* __restrict__ svlut, float* __restrict__ hdr,
                                                unsigned long long* counter) {
+  __shared__ float s_fractions[kFractionTable];
+  const TableFractions fractions = table_fractions(P, s_fractions);
   int x, y;
   uint32_t samples = 0;
-  if (tile_pixel(L, x, y)) {
+  const bool inside = split_pixel<kLanes>(L, x, y);
+  if (kLanes > 1 || inside) {
     const size_t e = pix_offset(L, x, y);
     const int32_t sidv = I.surface_id[e];
-    const Frame F = make_frame(P, tlut, mslut, A.bottom, A.ar, arr3(A.sun), arr3(A.E));
-    const f3 scene = shaded_scene(P, F, A, S, L, I, x, y, e, sidv);
-    composite_pixel_with(P, L, A, F, scene, sidv, space, I.position, svlut, hdr, x, y, samples);
+    composite_pixel_with<kLanes>(
+        P, L, A, F, [&] { return shaded_scene(P, F, A, S, L, I, x, y, e, sidv); }, sidv, space, I.position, svlut, hdr,
+        x, y, inside, fractions, samples);
   }
   warp_count(samples, counter);
 }
@@ -138,23 +152,22 @@ __device__ __forceinline__ f3 sample_aerial_field(const DevParams& P, const floa
 }
 
 // Diagnostic views (:1941-2052); not on the per-frame path.
-__global__ void __launch_bounds__(256, 3) k_composite_views(DevParams P, ImageLayout L, CompositeScalars A,
+__global__ void __launch_bounds__(256, 3) k_composite_views(DevParams P, Frame F, ImageLayout L, CompositeScalars A,
                                                          const float* __restrict__ scene,
                                                          const float* __restrict__ space,
                                                          const int32_t* __restrict__ sid,
                                                          const float* __restrict__ pos,
-                                                         const float4* __restrict__ tlut,
-                                                         const float4* __restrict__ mslut,
                                                          const float4* __restrict__ svlut,
                                                          const float4* __restrict__ aplut, float* __restrict__ hdr,
                                                          unsigned long long* counter) {
+  __shared__ float s_fractions[kFractionTable];
+  const TableFractions fractions = table_fractions(P, s_fractions);
   int x, y;
   const bool inside = tile_pixel(L, x, y);
   uint32_t samples = 0;
   if (inside) {
     const size_t e = pix_offset(L, x, y);
     const size_t o = e * L.channels;
-    Frame F = make_frame(P, tlut, mslut, A.bottom, A.ar, arr3(A.sun), arr3(A.E));
     PixelRay pr = pixel_ray(L, A, x, y);
     const RayGeom G = camera_ray_geom(P, A.bottom, A.cam_alt, pr.ray);
     const bool surface = sid[e] >= 0;
@@ -164,18 +177,18 @@ __global__ void __launch_bounds__(256, 3) k_composite_views(DevParams P, ImageLa
         color = sample_sky_view(P, svlut, pr.ray, F.sun, A.sky_alt, A.bottom);
         break;
       case ATM_VIEW_CAMERA_TRANSMITTANCE:
-        color = camera_t(P, F, G, pr.ray);
+        color = camera_t(P, F, G);
         break;
       case ATM_VIEW_TRANSMITTANCE_LUT: {
         int lx = min(int(pr.su * float(P.t_w)), P.t_w - 1);
         int ly = min(int(pr.sv * float(P.t_h)), P.t_h - 1);
-        color = from4(tlut[ly * P.t_w + lx]);
+        color = from4(F.tlut[ly * P.t_w + lx]);
         break;
       }
       case ATM_VIEW_MULTI_SCATTERING_LUT: {
         int lx = min(int(pr.su * float(P.ms_w)), P.ms_w - 1);
         int ly = min(int(pr.sv * float(P.ms_h)), P.ms_h - 1);
-        color = from4(mslut[ly * P.ms_w + lx]);
+        color = from4(F.mslut[ly * P.ms_w + lx]);
         break;
       }
       case ATM_VIEW_AERIAL_SCATTERING:
@@ -183,7 +196,7 @@ __global__ void __launch_bounds__(256, 3) k_composite_views(DevParams P, ImageLa
         color = splat(0.0f);
         float start, end;
         if (surface && surface_interval(P, G, A.bottom, norm(ld3(pos + o)), start, end))
-          color = integrate_surface(P, F, G, pr.ray, start, end, samples);
+          color = integrate_surface(P, F, G, pr.ray, start, end, fractions, samples);
         break;
       }
       case ATM_VIEW_AERIAL_FROXEL_ONLY: {
@@ -207,7 +220,7 @@ __global__ void __launch_bounds__(256, 3) k_composite_views(DevParams P, ImageLa
           float start, end;
           color = splat(1.0f);
           if (surface_interval(P, G, A.bottom, norm(ld3(pos + o)), start, end))
-            color = surface_segment_t(P, F, G, pr.ray, start, end);
+            color = surface_segment_t(P, F, G, start, end);
         }
         break;
       }
@@ -234,15 +247,17 @@ cudaError_t launch_prepare_surface(const DevParams& P, const ImageLayout& L, con
                                    const float up[3], const float fwd[3], const float4* tlut, const float4* mslut,
                                    float* out_sun_t, float* out_sky, cudaStream_t s) {
   const unsigned blocks = unsigned((static_cast<long long>(L.width) * L.height + 255) / 256);
-  k_prepare_surface<<<blocks, 256, 0, s>>>(P, L, pos, sid, bottom, cam_alt, host3(sun), ar, host3(right),
-                                                 host3(up), host3(fwd), tlut, mslut, out_sun_t, out_sky);
+  const Frame F = make_frame(P, tlut, mslut, bottom, ar, host3(sun), {0.0f, 0.0f, 0.0f});
+  k_prepare_surface<<<blocks, 256, 0, s>>>(P, F, L, pos, sid, cam_alt, host3(right), host3(up), host3(fwd), out_sun_t,
+                                           out_sky);
   return cudaGetLastError();
 }
 
 cudaError_t launch_frame(const DevParams& P, const ImageLayout& L, const CompositeScalars& A, const ShadeParams& S,
                          const ShadeImages& I, const float* space, const float4* tlut, const float4* mslut,
                          const float4* svlut, float* hdr, unsigned long long* sample_counter, cudaStream_t s) {
-  k_frame<<<tile_grid(L), 256, 0, s>>>(P, L, A, S, I, space, tlut, mslut, svlut, hdr, sample_counter);
+  const Frame F = frame_of(P, A, tlut, mslut);
+  k_frame<1><<<tile_grid(L), 256, 0, s>>>(P, F, L, with_image(A, L), S, I, space, svlut, hdr, sample_counter);
   return cudaGetLastError();
 }
 
@@ -250,12 +265,13 @@ cudaError_t launch_composite(const DevParams& P, const ImageLayout& L, const Com
                              const float* scene, const float* space, const int32_t* sid, const float* pos,
                              const float4* tlut, const float4* mslut, const float4* svlut, const float4* aplut,
                              float* hdr, unsigned long long* sample_counter, cudaStream_t s) {
+  const Frame F = frame_of(P, A, tlut, mslut);
   if (A.view == ATM_VIEW_COMPOSITE)
-    k_composite<<<tile_grid(L), 256, 0, s>>>(P, L, A, scene, space, sid, pos, tlut, mslut, svlut, hdr,
-                                             sample_counter);
+    k_composite<1><<<tile_grid(L), 256, 0, s>>>(P, F, L, with_image(A, L), scene, space, sid, pos, svlut, hdr,
+                                                sample_counter);
   else
-    k_composite_views<<<tile_grid(L), 256, 0, s>>>(P, L, A, scene, space, sid, pos, tlut, mslut, svlut, aplut, hdr,
-                                                   sample_counter);
+    k_composite_views<<<tile_grid(L), 256, 0, s>>>(P, F, L, with_image(A, L), scene, space, sid, pos, svlut, aplut, hdr,
+                                                 sample_counter);
   return cudaGetLastError();
 }
 
@@ -275,19 +291,20 @@ namespace {
 // COMPOSITE view of k_composite (the same composite_pixel); the block's
 // sample count goes to its tile slot instead of an atomic counter (every
 // launched block writes its slot).
-__global__ void __launch_bounds__(256, 3) k_composite_tiles(DevParams P, ImageLayout L, CompositeScalars A,
+__global__ void __launch_bounds__(256, 3) k_composite_tiles(DevParams P, Frame F, ImageLayout L, CompositeScalars A,
                                                          const float* __restrict__ scene,
                                                          const float* __restrict__ space,
                                                          const int32_t* __restrict__ sid,
                                                          const float* __restrict__ pos,
-                                                         const float4* __restrict__ tlut,
-                                                         const float4* __restrict__ mslut,
                                                          const float4* __restrict__ svlut, float* __restrict__ hdr,
                                                          uint32_t* __restrict__ tile_samples) {
   __shared__ uint32_t s_warp[8];
+  __shared__ float s_fractions[kFractionTable];
+  const TableFractions fractions = table_fractions(P, s_fractions);
   int x, y;
   uint32_t samples = 0;
-  if (tile_pixel(L, x, y)) composite_pixel(P, L, A, scene, space, sid, pos, tlut, mslut, svlut, hdr, x, y, samples);
+  if (tile_pixel(L, x, y))
+    composite_pixel<1>(P, F, L, A, scene, space, sid, pos, svlut, hdr, x, y, true, fractions, samples);
   __syncwarp();
 #pragma unroll
   for (int k = 16; k > 0; k >>= 1) samples += __shfl_xor_sync(kFull, samples, k);
@@ -352,7 +369,8 @@ cudaError_t launch_composite_noalloc(const DevParams& P, const ImageLayout& L, c
                                      const float4* tlut, const float4* mslut, const float4* svlut, float* hdr,
                                      uint32_t* tile_scratch, unsigned long long* samples_out, cudaStream_t s) {
   const dim3 grid = tile_grid(L);
-  k_composite_tiles<<<grid, 256, 0, s>>>(P, L, A, scene, space, sid, pos, tlut, mslut, svlut, hdr, tile_scratch);
+  k_composite_tiles<<<grid, 256, 0, s>>>(P, frame_of(P, A, tlut, mslut), L, with_image(A, L), scene, space, sid, pos,
+                                         svlut, hdr, tile_scratch);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess || samples_out == nullptr) return e;
   k_sum_tiles<<<1, 1024, 0, s>>>(tile_scratch, int(grid.x * grid.y), samples_out);

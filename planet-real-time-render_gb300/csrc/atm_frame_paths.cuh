@@ -6,6 +6,7 @@
 
 #include "atm_device.cuh"
 #include "atm_kernels.h"
+#include "atm_lut_warp.cuh"
 #include "atm_shade.cuh"
 
 namespace atm {
@@ -24,6 +25,19 @@ __device__ __forceinline__ bool tile_pixel_at(const ImageLayout& L, int bx, int 
 }
 __device__ __forceinline__ bool tile_pixel(const ImageLayout& L, int& x, int& y) {
   return tile_pixel_at(L, blockIdx.x, blockIdx.y, x, y);
+}
+
+// Pixel of a thread when kLanes consecutive lanes share a pixel: 256 / kLanes
+// pixels a block, 8 (one lane a pixel: 16) wide.  Lanes outside the frame
+// still belong to a group: false, with x and y clamped into the frame.
+template <int kLanes>
+__device__ __forceinline__ bool split_pixel(const ImageLayout& L, int& x, int& y) {
+  if (kLanes == 1) return tile_pixel(L, x, y);
+  const int p = threadIdx.x / kLanes;
+  const int px = blockIdx.x * 8 + (p & 7), py = blockIdx.y * (32 / kLanes) + (p >> 3);
+  x = min(px, L.width - 1);
+  y = min(py, L.height - 1);
+  return px < L.width && py < L.height;
 }
 
 // Pixel of a thread for memory-bound per-pixel kernels: consecutive threads
@@ -47,12 +61,11 @@ struct PixelRay {
 };
 __device__ __forceinline__ PixelRay pixel_ray(const ImageLayout& L, const CompositeScalars& A, int x, int y) {
   PixelRay r;
-  const float aspect = float(L.width) / float(L.height);
   r.su = (float(x) + 0.5f) / float(L.width);
   r.sv = (float(y) + 0.5f) / float(L.height);
-  float sx = (r.su * 2.0f - 1.0f) * aspect;
+  float sx = (r.su * 2.0f - 1.0f) * A.aspect;
   float sy = r.sv * 2.0f - 1.0f;
-  f3 rv = (arr3(A.right) * sx + arr3(A.up) * sy) + arr3(A.fwd) / A.tanfov;
+  f3 rv = (arr3(A.right) * sx + arr3(A.up) * sy) + arr3(A.fwd_t);
   r.ray = rv * (1.0f / norm(rv));
   return r;
 }
@@ -163,15 +176,45 @@ __device__ __forceinline__ SurfaceMarch make_surface_march(const DevParams& P, c
     shadow_roots_far(G.h0, ray, F.sun, F.bottom, M.sr0, M.sr1, M.sv0, M.sv1);
   else
     shadow_roots(mk(0.0f, F.bottom + G.h0, 0.0f), ray, F.sun, F.bottom, M.sr0, M.sr1, M.sv0, M.sv1);
+  // a root further than two interval lengths from the whole march leaves
+  // every interval's proximity at 0: the march does not look at it
+  const float reach = 2.001f * mx(end - start, 1.0e-4f);
+  M.sv0 = M.sv0 && M.sr0 > start - reach && M.sr0 < end + reach;
+  M.sv1 = M.sv1 && M.sr1 > start - reach && M.sr1 < end + reach;
   M.rs = make_ray_source(P, F, G, ray);
   M.rw = make_warp(G.tc, start, end);
   return M;
 }
+// Fractions of a surface march's boundaries: of the base intervals and of a
+// refined interval's children.
+template <class Limb, class Sub>
+struct MarchFractions {
+  Limb limb;
+  Sub sub;
+};
+constexpr int kMaxLimbSteps = 64, kMaxSubsteps = 16;  // atm_create's ranges
+// The tables of a block (every thread must call), s of kFractionTable floats.
+constexpr int kFractionTable = kMaxLimbSteps + 1 + kMaxSubsteps + 1;
+using TableFractions = MarchFractions<TableFraction, TableFraction>;
+__device__ __forceinline__ TableFractions table_fractions(const DevParams& P, float* s) {
+  for (int i = threadIdx.x; i < kFractionTable; i += blockDim.x) {
+    const bool limb = i <= kMaxLimbSteps;
+    s[i] = float(limb ? i : i - kMaxLimbSteps - 1) / float(limb ? P.limb_steps : P.substeps);
+  }
+  __syncthreads();
+  return {{s}, {s + kMaxLimbSteps + 1}};
+}
+using DivideFractions = MarchFractions<DivideFraction, DivideFraction>;
+__device__ __forceinline__ DivideFractions divide_fractions(const DevParams& P) {
+  return {{float(P.limb_steps)}, {float(P.substeps)}};
+}
+
 // One base interval [d0, d1] with its terminator refinement (:901-1031).
+template <class Fractions>
 __device__ __forceinline__ Seg surface_interval_seg(const DevParams& P, const Frame& F, const SurfaceMarch& M, float d0,
-                                                    float d1, uint32_t& samples) {
+                                                    float d1, const Fractions& fractions, uint32_t& samples) {
   float vis;
-  Seg coarse = source_segment<true>(P, F, M.rs, d0, d1, vis);
+  Seg coarse = source_segment(P, F, M.rs, d0, d1, vis);
   ++samples;
   // _terminator_refinement_weight :901-966; zero unless a shadow-cylinder
   // root exists or the disk is partly hidden at the midpoint
@@ -191,11 +234,11 @@ __device__ __forceinline__ Seg surface_interval_seg(const DevParams& P, const Fr
     // _integrate_adaptive_scattering_interval :998-1031
     const int nsub = P.substeps;
     Seg fine = {splat(0.0f), splat(1.0f)};
-    float c0 = d0 + (d1 - d0) * 0.0f;
+    float c0 = d0;
     for (int k = 0; k < nsub; ++k) {
-      float c1 = d0 + (d1 - d0) * (float(k + 1) / float(nsub));
+      float c1 = fmaf(d1 - d0, fractions.sub(k + 1), d0);
       float cvis;
-      fine = seg_then(fine, source_segment<true>(P, F, M.rs, c0, c1, cvis));
+      fine = seg_then(fine, source_segment(P, F, M.rs, c0, c1, cvis));
       c0 = c1;
     }
     samples += nsub;
@@ -205,61 +248,80 @@ __device__ __forceinline__ Seg surface_interval_seg(const DevParams& P, const Fr
   return interval;
 }
 
-// _integrate_surface_scattering :1667-1755 (with :901-1032).  `start`/`end`
-// are the shell-clipped interval; the caller has checked it is non-empty.
-__device__ __forceinline__ f3 integrate_surface(const DevParams& P, const Frame& F, const RayGeom& G, f3 ray,
-                                                float start, float end, uint32_t& samples) {
-  const SurfaceMarch M = make_surface_march(P, F, G, ray, start, end);
+// The base intervals [i0, i1) of a surface march, in ray order.
+template <class Fractions>
+__device__ __forceinline__ Seg surface_march(const DevParams& P, const Frame& F, const SurfaceMarch& M, int i0, int i1,
+                                             const Fractions& fractions, uint32_t& samples) {
   const int n = P.limb_steps;
   Seg acc = {splat(0.0f), splat(1.0f)};
-  float d0 = warp_at(M.rw, 0.0f);
-  for (int i = 0; i < n; ++i) {
-    float d1 = warp_at(M.rw, float(i + 1) / float(n));
-    acc = seg_then(acc, surface_interval_seg(P, F, M, d0, d1, samples));
+  bool second = warp_second(i0, n);
+  WarpHalf half = warp_half(M.rw, second);
+  float d0 = warp_at(half, fractions.limb(i0));
+  for (int i = i0; i < i1; ++i) {
+    if (!second && warp_second(i + 1, n)) {
+      second = true;
+      half = warp_half(M.rw, true);
+    }
+    const float d1 = warp_at(half, fractions.limb(i + 1));
+    acc = seg_then(acc, surface_interval_seg(P, F, M, d0, d1, fractions, samples));
     d0 = d1;
   }
-  return vmax(acc.L, 0.0f);
+  return acc;
+}
+// _integrate_surface_scattering :1667-1755 (with :901-1032).  `start`/`end`
+// are the shell-clipped interval; the caller has checked it is non-empty.
+template <class Fractions>
+__device__ __forceinline__ f3 integrate_surface(const DevParams& P, const Frame& F, const RayGeom& G, f3 ray,
+                                                float start, float end, const Fractions& fractions, uint32_t& samples) {
+  const SurfaceMarch M = make_surface_march(P, F, G, ray, start, end);
+  return vmax(surface_march(P, F, M, 0, P.limb_steps, fractions, samples).L, 0.0f);
+}
+// The same by kLanes consecutive lanes, each a run of the base intervals; the
+// group's first lane receives the result.  Every lane of the warp must call
+// when kLanes > 1; a group that is not `active` marches nothing.
+template <int kLanes, class Fractions>
+__device__ __forceinline__ f3 integrate_surface_split(const DevParams& P, const Frame& F, const RayGeom& G, f3 ray,
+                                                      float start, float end, bool active, const Fractions& fractions,
+                                                      uint32_t& samples) {
+  Seg acc = seg_identity();
+  if (active) {
+    const SurfaceMarch M = make_surface_march(P, F, G, ray, start, end);
+    const int n = P.limb_steps, per = (n + kLanes - 1) / kLanes;
+    const int i0 = min(int(threadIdx.x & (kLanes - 1)) * per, n);
+    acc = surface_march(P, F, M, i0, min(i0 + per, n), fractions, samples);
+  }
+  return vmax(group_compose<kLanes>(acc).L, 0.0f);
+}
+
+// The transmittance LUT at distance t along a camera ray, in the direction of
+// the ray (sign 1) or back toward the camera (sign -1): the local vertical's
+// cosine is (t - t_c) / r, so neither the point nor its normal is formed.
+__device__ __forceinline__ f3 ray_t(const DevParams& P, const Frame& F, const RayGeom& G, float t, float sign) {
+  const float u = t - G.t0;
+  const float delta = fmaf(u, u, fmaf(G.q1, u, G.q0));
+  const float r2 = mx(fmaf(F.bottom, F.bottom, delta), 1.0f);
+  const float inv_r = frsqrt(r2);
+  const float h = clampf(delta * frcp(r2 * inv_r + F.bottom), 0.0f, P.top);
+  const float rho2 = clampf(delta, 0.0f, F.shell2);
+  // clamped with the radius that the clamped altitude has
+  return sample_t_at(P, F, h, rho2, fsqrt(rho2), sign * (t - G.tc) * (inv_r * (F.bottom + h)));
 }
 
 // _surface_segment_transmittance :1603-1665 on an already clipped interval.
-__device__ __forceinline__ f3 surface_segment_t(const DevParams& P, const Frame& F, const RayGeom& G, f3 ray,
-                                                float start, float end) {
-  f3 s2t, n2t;
-  if (!G.far) {
-    const float cam_alt = G.h0;
-    const f3 origin = mk(0.0f, F.bottom + cam_alt, 0.0f);
-    f3 np = origin + ray * start;
-    f3 sp = origin + ray * end;
-    f3 rr = -ray;
-    f3 nrad = np / mx(norm(np), 1.0f);
-    f3 srad = sp / mx(norm(sp), 1.0f);
-    float na = altitude_on_ray(cam_alt, ray.y, start, F.bottom);
-    float sa = altitude_on_ray(cam_alt, ray.y, end, F.bottom);
-    s2t = sample_t(P, F, sa, dot(srad, rr));
-    n2t = sample_t(P, F, na, dot(nrad, rr));
-  } else {  // radial . (-ray) = -(t - t_c) / r
-    const float na = altitude_at(G, start, F.bottom), sa = altitude_at(G, end, F.bottom);
-    s2t = sample_t(P, F, sa, -vertical_cosine_at(G, end, F.bottom + sa));
-    n2t = sample_t(P, F, na, -vertical_cosine_at(G, start, F.bottom + na));
-  }
-  return vclamp(s2t / vmax(n2t, 1.0e-6f), 0.0f, 1.0f);
+__device__ __forceinline__ f3 surface_segment_t(const DevParams& P, const Frame& F, const RayGeom& G, float start,
+                                                float end) {
+  const f3 s2t = ray_t(P, F, G, end, -1.0f), n2t = vmax(ray_t(P, F, G, start, -1.0f), 1.0e-6f);
+  return vclamp(mk(fdiv(s2t.x, n2t.x), fdiv(s2t.y, n2t.y), fdiv(s2t.z, n2t.z)), 0.0f, 1.0f);
 }
 
 // _camera_transmittance :1788-1825
-__device__ __forceinline__ f3 camera_t(const DevParams& P, const Frame& F, const RayGeom& G, f3 ray) {
+__device__ __forceinline__ f3 camera_t(const DevParams& P, const Frame& F, const RayGeom& G) {
   float s, e;
   bool valid, ground;
   segment_of(P, G, F.bottom, s, e, valid, ground);
   if (!valid) return splat(1.0f);
   if (ground) return splat(0.0f);
-  if (G.far) {
-    const float ea = altitude_at(G, s, F.bottom);
-    return sample_t(P, F, ea, vertical_cosine_at(G, s, F.bottom + ea));
-  }
-  f3 entry = mk(0.0f, F.bottom + G.h0, 0.0f) + ray * s;
-  f3 radial = entry / mx(norm(entry), 1.0f);
-  float ea = altitude_on_ray(G.h0, ray.y, s, F.bottom);
-  return sample_t(P, F, ea, dot(radial, ray));
+  return ray_t(P, F, G, s, 1.0f);
 }
 
 // _sample_sky_view :1474-1525
@@ -272,7 +334,7 @@ __device__ __forceinline__ f3 sample_sky_view(const DevParams& P, const float4* 
   if (vl > 1.0e-6f && sl > 1.0e-6f) ra = acosf(clampf((ray.x * sun.x + ray.z * sun.z) / (vl * sl), -1.0f, 1.0f));
   float u = ra / kPiF;
   float v = sky_zenith_to_v(zen, sky_horizon_zenith(sky_alt, bottom));
-  return bilinear(svlut, P.sv_w, P.sv_h, u, v);
+  return bilinear(svlut, P.sv_lut, u, v);
 }
 
 // Shell clip shared by the scattering integral and the transmittance ratio.
@@ -289,7 +351,7 @@ __device__ __forceinline__ bool surface_interval(const DevParams& P, const RayGe
 // Sky branch of the COMPOSITE view (:1883-1940) given the sky radiance.
 __device__ __forceinline__ f3 composite_sky_with(const DevParams& P, const Frame& F, const CompositeScalars& A, f3 sky,
                                                  f3 ray, f3 color, f3 space, float height) {
-  f3 tr = camera_t(P, F, camera_ray_geom(P, F.bottom, A.cam_alt, ray), ray);
+  f3 tr = camera_t(P, F, camera_ray_geom(P, F.bottom, A.cam_alt, ray));
   f3 star = space * tr;
   const f3 lw = mk(0.2126f, 0.7152f, 0.0722f);
   float contrast = dot(star, lw) / mx(dot(sky, lw), 1.0e-5f);

@@ -24,7 +24,17 @@ struct CompositeScalars {
   float bottom, cam_alt, sky_alt, ar, tanfov, star_start, star_end;
   float sun[3], E[3], disk[3], right[3], up[3], fwd[3];
   int32_t view;
+  // set by the launch: width / height and fwd / tanfov, of every pixel's ray
+  float aspect, fwd_t[3];
 };
+inline Frame frame_of(const DevParams& P, const CompositeScalars& A, const float4* tlut, const float4* mslut) {
+  return make_frame(P, tlut, mslut, A.bottom, A.ar, {A.sun[0], A.sun[1], A.sun[2]}, {A.E[0], A.E[1], A.E[2]});
+}
+inline CompositeScalars with_image(CompositeScalars A, const ImageLayout& L) {
+  A.aspect = float(L.width) / float(L.height);
+  for (int k = 0; k < 3; ++k) A.fwd_t[k] = A.fwd[k] / A.tanfov;
+  return A;
+}
 
 cudaError_t launch_transmittance(const DevParams& P, float bottom, float4* out, cudaStream_t s);
 // The LUT builds and the composite add the radiance samples they evaluate to
@@ -97,9 +107,7 @@ constexpr int kSurrogateApIn = 11, kSurrogateApOut = 6, kSurrogateApHidden = 4;
 constexpr int kSurrogateSkyIn = 10, kSurrogateSkyOut = 3, kSurrogateSkyHidden = 3;
 struct SurrogateSetDev {
   DevParams P;
-  const float4* tlut;
-  const float4* mslut;
-  float bottom;
+  Frame F;  // the sample puts its own sun in
   float lhr_n, lhm_n;  // normalised log scale heights (features 4, 5)
 };
 // Bound of a tensor-core completion wait, in mbarrier polls (each try_wait
@@ -163,8 +171,8 @@ struct SampleShaping {
   float sun_angle_max;       // radians
 };
 cudaError_t launch_gen_samples(const SurrogateSetDev* sets, int n_sets, int kind, long long n, unsigned long long seed,
-                               const SampleShaping& shaping, const float E[3], float ar, float* features,
-                               float* targets, unsigned long long* counter, cudaStream_t s);
+                               const SampleShaping& shaping, float* features, float* targets,
+                               unsigned long long* counter, cudaStream_t s);
 size_t surrogate_smem_bytes(const SurrogateNets& nets);
 // Sky radiance of every pixel: mode 0 the plain integrator per pixel, 1 the
 // sky network (plain where a gate trips; status bit 0 set on a tensor-core

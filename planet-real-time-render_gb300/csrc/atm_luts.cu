@@ -5,11 +5,11 @@
 // marching its ray sequentially):
 //  - transmittance: 8 lanes per texel split the 40 optical-depth steps and
 //    sum with xor shuffles;
-//  - multi-scattering: one thread per (texel, direction); a block holds one
-//    texel; the direction sums are added in the reference's order;
-//  - sky-view: one warp per texel, lanes over march steps; the per-step
-//    (radiance, transmittance) segments are composed in ray order by a
-//    shuffle tree ((L1,T1) then (L2,T2) = (L1 + T1 L2, T1 T2));
+//  - multi-scattering: a block per texel, a few lanes per direction which
+//    split its march; the directions are summed by shuffles;
+//  - sky-view: a few lanes per texel over its march steps; the per-step
+//    (radiance, transmittance) segments are composed in ray order by
+//    shuffles ((L1,T1) then (L2,T2) = (L1 + T1 L2, T1 T2));
 //  - aerial perspective: one warp per froxel column, lanes over depth
 //    slices; an ordered inclusive shuffle scan of the slice segments gives
 //    each slice's cumulative in-scattering.
@@ -28,6 +28,7 @@ namespace {
 
 // ---- transmittance (:1034-1063, :570-607) ----------------------------------
 constexpr int kTLanes = 8;
+constexpr long long kWaveThreads = 152LL * 2048;  // resident threads of the whole chip
 
 __global__ void __launch_bounds__(256) k_transmittance(DevParams P, float bottom, float4* __restrict__ out) {
   const int gid = blockIdx.x * blockDim.x + threadIdx.x;
@@ -62,27 +63,38 @@ __global__ void __launch_bounds__(256) k_transmittance(DevParams P, float bottom
 }
 
 // ---- multi-scattering (:1065-1206) ------------------------------------------
-constexpr int kMaxDirs = 128;
+constexpr int kMaxDirs = 128, kMaxDirectionSteps = 128;  // atm_create's ranges
 
-__global__ void __launch_bounds__(kMaxDirs) k_multi_scattering(DevParams P, float bottom, f3 E, float ar,
-                                                               const float4* __restrict__ tlut,
-                                                               float4* __restrict__ out,
-                                                               unsigned long long* counter) {
-  __shared__ f3 s_l[kMaxDirs];
-  __shared__ f3 s_f[kMaxDirs];
+// kLanes consecutive lanes share a direction's march; kLanes ms_dirs threads
+// (rounded up to whole warps) a texel.  Latency-bound: 32x32 texels of 64
+// directions are 13 warps an SM at one lane a direction (44 us), 54 at four
+// (30 us).
+template <int kLanes>
+__global__ void __launch_bounds__(kMaxDirs* kLanes) k_multi_scattering(DevParams P, Frame F,
+                                                                       float4* __restrict__ out,
+                                                                       unsigned long long* counter) {
+  __shared__ float s_fraction[kMaxDirectionSteps + 1];
+  __shared__ f3 s_l[kMaxDirs * kLanes / 32];
+  __shared__ f3 s_f[kMaxDirs * kLanes / 32];
+  const float bottom = F.bottom;
+  fill_fractions(s_fraction, P.ms_steps, threadIdx.x, blockDim.x);
+  __syncthreads();
   const int texel = blockIdx.x;
   const int x = texel % P.ms_w, y = texel / P.ms_w;
-  const int di = threadIdx.x;
+  const int di = threadIdx.x / kLanes, sub = threadIdx.x % kLanes;
   float u = (float(x) + 0.5f) / float(P.ms_w);
   float v = (float(y) + 0.5f) / float(P.ms_h);
   float h0 = v * v * P.top;
   float radius = bottom + h0;
   float sc = sun_u_to_cosine(u, h0, bottom);
   float ss = sqrtf(mx(1.0f - sc * sc, 0.0f));
-  Frame F = make_frame(P, tlut, nullptr, bottom, ar, mk(ss, sc, 0.0f), E);
+  F.sun = mk(ss, sc, 0.0f);
   f3 o = mk(0.0f, radius, 0.0f);
-  f3 dL = splat(0.0f), dF = splat(0.0f);
+  f3 dL = splat(0.0f), dF = splat(0.0f), pT = splat(1.0f);
   uint32_t samples = 0;
+  bool ground = false;
+  float end = 0.0f;
+  f3 ray = splat(0.0f);
   if (di < P.ms_dirs) {
     const int ndir = P.ms_dirs;
     float si = float(di) + 0.5f;
@@ -91,87 +103,105 @@ __global__ void __launch_bounds__(kMaxDirs) k_multi_scattering(DevParams P, floa
     float az = float(di) * 2.39996323f;
     float saz, caz;
     sincosf(az, &saz, &caz);
-    f3 ray = mk(ds * caz, dc, ds * saz);
-    float start, end;
-    bool valid, ground;
+    ray = mk(ds * caz, dc, ds * saz);
+    float start;
+    bool valid;
     segment_vec(P, o, ray, bottom, start, end, valid, ground);
+    ground = ground && valid;
     if (valid) {
-      const float phase_r = rayleigh_phase(P, clampf(dot(ray, F.sun), -1.0f, 1.0f));
-      const float phase_m = mie_phase(P, clampf(dot(ray, F.sun), -1.0f, 1.0f));
+      const float orad = bottom + h0;
       const float closest_raw = -dot(o, ray);
-      f3 pT = splat(1.0f);
+      const RaySource R = make_ray_source(P, F, RayGeom{h0, dc, 0.0f, h0 * (2.0f * bottom + h0), 2.0f * orad * dc}, ray);
+      const RayWarp w = make_warp(closest_raw, start, end);
       const int n = P.ms_steps;
-      float d0 = warp_boundary(closest_raw, start, end, 0.0f);
-      for (int pi = 0; pi < n; ++pi) {
-        float d1 = warp_boundary(closest_raw, start, end, float(pi + 1) / float(n));
-        float dist = (d0 + d1) * 0.5f;
-        float step = d1 - d0;
-        f3 point = o + ray * dist;
-        float hh = altitude_on_ray(h0, dc, dist, bottom);
-        Density d = density(P, hh);
-        f3 sT, sI;
-        segment_integral(extinction_of(P, d), step, sT, sI);
-        float rr = norm(point);
-        f3 radial = point / mx(rr, 1.0f);
-        float psc = dot(radial, F.sun);
-        float vis;
-        f3 st = sample_solar_t(P, F, hh, psc, horizon_at(hh, bottom), vis);
-        f3 src = (F.E * st) * (arr3(P.beta_r) * d.r * phase_r + arr3(P.beta_ms) * d.m * phase_m);
-        dL = dL + pT * src * sI;
-        dF = dF + pT * scattering_of(P, d) * sI;
-        pT = pT * sT;
+      const int per = (n + kLanes - 1) / kLanes;
+      const int i0 = min(sub * per, n), i1 = min(i0 + per, n);
+      bool second = warp_second(i0, n);
+      WarpHalf half = warp_half(w, second);
+      float d0 = warp_at(half, s_fraction[i0]);
+      for (int i = i0; i < i1; ++i) {
+        if (!second && warp_second(i + 1, n)) {
+          second = true;
+          half = warp_half(w, true);
+        }
+        const float d1 = warp_at(half, s_fraction[i + 1]);
+        const MarchSample m = march_sample(P, F, R, d0, d1);
+        const f3 t = pT * m.weight;
+        dL = dL + t * (m.st * (R.ER * m.d.r + R.EM * m.d.m));
+        dF = dF + t * scattering_of(P, m.d);
+        pT = pT * m.T;
         d0 = d1;
       }
-      samples = uint32_t(n);
-      if (ground) {
-        f3 gp = o + ray * end;
-        f3 gn = gp * (1.0f / norm(gp));  // Taichi normalized(): v * (1/|v|)
-        float gsc = dot(gn, F.sun);
-        float vis;
-        f3 gT = sample_solar_t(P, F, 0.0f, gsc, horizon_at(0.0f, bottom), vis);
-        f3 gL = arr3(P.albedo) * F.E * gT * mx(gsc, 0.0f) / kPiF;
-        dL = dL + pT * gL;
-      }
+      samples = uint32_t(i1 - i0);
     }
   }
   warp_count(samples, counter);
-  s_l[di] = dL;
-  s_f[di] = dF;
-  __syncthreads();
-  if (di == 0) {
-    f3 lsum = splat(0.0f), fsum = splat(0.0f);
-    for (int k = 0; k < P.ms_dirs; ++k) {
-      lsum = lsum + s_l[k];
-      fsum = fsum + s_f[k];
+  // the lanes' parts in ray order: the direction's first lane gets the whole
+#pragma unroll
+  for (int k = 1; k < kLanes; k <<= 1) {
+    const Seg l = shfl_down_seg({dL, pT}, k);
+    const f3 f = shfl_down3(dF, k);
+    if (sub + k < kLanes) {
+      dL = dL + pT * l.L;
+      dF = dF + pT * f;
+      pT = pT * l.T;
     }
-    f3 avg_l = lsum / float(P.ms_dirs);
-    f3 avg_f = vclamp(fsum / float(P.ms_dirs), 0.0f, 0.95f);
+  }
+  if (sub != 0) dL = dF = splat(0.0f);
+  if (ground && sub == 0) {
+    f3 gp = o + ray * end;
+    f3 gn = gp * (1.0f / norm(gp));  // Taichi normalized(): v * (1/|v|)
+    float gsc = dot(gn, F.sun);
+    float vis;
+    f3 gT = sample_solar_t(P, F, 0.0f, gsc, horizon_at(0.0f, bottom), vis);
+    f3 gL = arr3(P.albedo) * F.E * gT * mx(gsc, 0.0f) / kPiF;
+    dL = dL + pT * gL;
+  }
+  // sum over the directions
+#pragma unroll
+  for (int k = 16; k >= kLanes; k >>= 1) {
+    dL = dL + shfl_xor3(dL, k);
+    dF = dF + shfl_xor3(dF, k);
+  }
+  if ((threadIdx.x & 31) == 0) {
+    s_l[threadIdx.x >> 5] = dL;
+    s_f[threadIdx.x >> 5] = dF;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int k = 1; k < int(blockDim.x >> 5); ++k) {
+      dL = dL + s_l[k];
+      dF = dF + s_f[k];
+    }
+    f3 avg_l = dL / float(P.ms_dirs);
+    f3 avg_f = vclamp(dF / float(P.ms_dirs), 0.0f, 0.95f);
     out[y * P.ms_w + x] = to4(vmax(avg_l / (splat(1.0f) - avg_f), 0.0f));
   }
 }
 
 // ---- sky-view (:1208-1302) and aerial perspective (:1304-1420) -----------------
-__global__ void __launch_bounds__(256) k_sky_view(DevParams P, float bottom, float cam_alt, float sun_cos, f3 E,
-                                                  float ar, const float4* __restrict__ tlut,
-                                                  const float4* __restrict__ mslut, float4* __restrict__ out,
+template <int kLanes>
+__global__ void __launch_bounds__(256) k_sky_view(DevParams P, Frame F, float cam_alt, float4* __restrict__ out,
                                                   unsigned long long* counter) {
-  const int warp_id = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  if (warp_id >= P.sv_w * P.sv_h) return;  // warp-uniform
-  float ss = sqrtf(mx(1.0f - sun_cos * sun_cos, 0.0f));
-  Frame F = make_frame(P, tlut, mslut, bottom, ar, mk(ss, sun_cos, 0.0f), E);
-  uint32_t samples = sky_view_texel(P, F, cam_alt, warp_id % P.sv_w, warp_id / P.sv_w, out);
+  __shared__ float s_fraction[kMaxSkySteps + 1];
+  fill_fractions(s_fraction, P.sv_steps, threadIdx.x, blockDim.x);
+  __syncthreads();
+  const int texels = P.sv_w * P.sv_h;
+  const int texel = (blockIdx.x * blockDim.x + threadIdx.x) / kLanes;
+  const int t = min(texel, texels - 1);  // every lane takes part in the group's shuffles
+  uint32_t samples =
+      sky_view_texel<kLanes>(P, F, cam_alt, t % P.sv_w, t / P.sv_w, texel < texels, {s_fraction}, out);
   warp_count(samples, counter);
 }
 
-__global__ void __launch_bounds__(256) k_aerial(DevParams P, float aspect, float bottom, float cam_alt, f3 sun, f3 E,
-                                                float ar, f3 right, f3 up, f3 fwd, float tanfov,
-                                                const float4* __restrict__ tlut, const float4* __restrict__ mslut,
-                                                float4* __restrict__ out, unsigned long long* counter) {
+__global__ void __launch_bounds__(256) k_aerial(DevParams P, Frame F, AerialView V, float4* __restrict__ out,
+                                                unsigned long long* counter) {
+  __shared__ float s_fraction[kMaxAerialSteps + 1];
+  fill_fractions(s_fraction, P.ap_steps, threadIdx.x, blockDim.x);
+  __syncthreads();
   const int warp_id = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   if (warp_id >= P.ap_w * P.ap_h) return;  // warp-uniform
-  Frame F = make_frame(P, tlut, mslut, bottom, ar, sun, E);
-  AerialView V{aspect, cam_alt, right, up, fwd, tanfov};
-  uint32_t samples = aerial_column(P, F, V, warp_id % P.ap_w, warp_id / P.ap_w, out);
+  uint32_t samples = aerial_column_warp(P, F, V, warp_id % P.ap_w, warp_id / P.ap_w, {s_fraction}, out);
   warp_count(samples, counter);
 }
 
@@ -208,19 +238,40 @@ cudaError_t launch_transmittance(const DevParams& P, float bottom, float4* out, 
 
 cudaError_t launch_multi_scattering(const DevParams& P, float bottom, const float E[3], float ar,
                                     const float4* tlut, float4* out, unsigned long long* counter, cudaStream_t s) {
-  if (P.ms_dirs > kMaxDirs) return cudaErrorInvalidValue;
-  const int threads = ((P.ms_dirs + 31) / 32) * 32;
-  k_multi_scattering<<<P.ms_w * P.ms_h, threads, 0, s>>>(P, bottom, host3(E), ar, tlut, out, counter);
+  if (P.ms_dirs > kMaxDirs || P.ms_steps > kMaxDirectionSteps) return cudaErrorInvalidValue;
+  // Four lanes a direction while that leaves the launch within one resident
+  // wave of threads, else one: the set-up is then repeated for nothing.
+  const int lanes = 4LL * P.ms_w * P.ms_h * P.ms_dirs <= kWaveThreads ? 4 : 1;
+  const int threads = ((lanes * P.ms_dirs + 31) / 32) * 32;
+  const int blocks = P.ms_w * P.ms_h;
+  const Frame F = make_frame(P, tlut, nullptr, bottom, ar, {0.0f, 1.0f, 0.0f}, host3(E));  // the texel's own sun in it
+  if (lanes == 4)
+    k_multi_scattering<4><<<blocks, threads, 0, s>>>(P, F, out, counter);
+  else
+    k_multi_scattering<1><<<blocks, threads, 0, s>>>(P, F, out, counter);
   return cudaGetLastError();
 }
 
 cudaError_t launch_sky_view(const DevParams& P, float bottom, float cam_alt, float sun_cos, const float E[3],
                             float ar, const float4* tlut, const float4* mslut, float4* out,
                             unsigned long long* counter, cudaStream_t s) {
+  if (P.sv_steps > kMaxSkySteps) return cudaErrorInvalidValue;
   const int threads = 256;
-  const long long total = 32LL * P.sv_w * P.sv_h;
-  k_sky_view<<<unsigned((total + threads - 1) / threads), threads, 0, s>>>(P, bottom, cam_alt, sun_cos, host3(E), ar,
-                                                                          tlut, mslut, out, counter);
+  const long long texels = (long long)P.sv_w * P.sv_h;
+  const auto go = [&](auto kernel, int lanes) {
+    kernel<<<unsigned((lanes * texels + threads - 1) / threads), threads, 0, s>>>(
+        P, make_frame(P, tlut, mslut, bottom, ar, sky_view_sun(sun_cos), host3(E)), cam_alt, out, counter);
+  };
+  // The most lanes a texel that keep the launch within half a resident wave:
+  // beyond that the warps only repeat the set-up.
+  if (8 * texels <= kWaveThreads / 2)
+    go(k_sky_view<8>, 8);
+  else if (4 * texels <= kWaveThreads / 2)
+    go(k_sky_view<4>, 4);
+  else if (2 * texels <= kWaveThreads / 2)
+    go(k_sky_view<2>, 2);
+  else
+    go(k_sky_view<1>, 1);
   return cudaGetLastError();
 }
 
@@ -228,12 +279,13 @@ cudaError_t launch_aerial(const DevParams& P, int width, int height, float botto
                           const float E[3], float ar, const float right[3], const float up[3], const float fwd[3],
                           float tanfov, const float4* tlut, const float4* mslut, float4* out,
                           unsigned long long* counter, cudaStream_t s) {
+  if (P.ap_steps > kMaxAerialSteps) return cudaErrorInvalidValue;
   const int threads = 256;
   const long long total = 32LL * P.ap_w * P.ap_h;
   const float aspect = float(width) / float(height);
   k_aerial<<<unsigned((total + threads - 1) / threads), threads, 0, s>>>(
-      P, aspect, bottom, cam_alt, host3(sun), host3(E), ar, host3(right), host3(up), host3(fwd), tanfov, tlut, mslut,
-      out, counter);
+      P, make_frame(P, tlut, mslut, bottom, ar, host3(sun), host3(E)),
+      aerial_view(aspect, cam_alt, right, up, fwd, tanfov), out, counter);
   return cudaGetLastError();
 }
 

@@ -338,22 +338,26 @@ __global__ void k_pack_tc(MlpShape m, const float* __restrict__ params, unsigned
   int off = 0;
   for (int l = 0; l < m.n_layers; ++l) {
     const int in = m.in_dim[l], out = m.out_dim[l];
-    const int kp = tc_k_pad(in), np = tc_n_pad(out);
+    const int kp = tc_k_pad(in), np = tc_n_pad(out), bk = tc_bias_k(in);
     const float scale = l + 1 < m.n_layers ? 0.5f : 1.0f;
     for (int i = threadIdx.x; i < kp * np; i += blockDim.x) {
       const int n = i / kp, k = i % kp;
-      const float v = (n < out && k < in) ? params[m.off_w[l] + n * in + k] * scale : 0.0f;
+      float v = 0.0f;
+      if (n < out && k < in) {
+        v = params[m.off_w[l] + n * in + k] * scale;
+      } else if (n < out && k >= bk && k < bk + 3) {  // the bias in three BF16 parts
+        v = params[m.off_b[l] + n] * scale;
+        for (int part = bk; part < k; ++part) v -= __bfloat162float(__float2bfloat16_rn(v));
+      }
       *reinterpret_cast<__nv_bfloat16*>(packed + off + tc_w_offset(n, k, np)) = __float2bfloat16_rn(v);
     }
-    float* b = reinterpret_cast<float*>(packed + off + kp * np * 2);
-    for (int j = threadIdx.x; j < np; j += blockDim.x) b[j] = j < out ? params[m.off_b[l] + j] * scale : 0.0f;
     off += tc_layer_bytes(in, out);
   }
 }
 
 // Forward of n samples on the tcgen05 path: one tile of 128 samples per
 // block at a time (grid-stride); TMEM: accumulators at column 0, activations
-// at column 128 of a 256-column allocation.  *error is set when an MMA did
+// at column 128 and the bias's ones at 192 of a 256-column allocation.  *error is set when an MMA did
 // not complete in time.
 template <int kHidden>
 __global__ void __launch_bounds__(128) k_mlp_forward_tc(MlpShape m, const unsigned char* __restrict__ packed,
@@ -374,14 +378,17 @@ __global__ void __launch_bounds__(128) k_mlp_forward_tc(MlpShape m, const unsign
   tc::fence_before_sync();
   __syncthreads();
   tc::fence_after_sync();
-  TcTile T{s_tmem, s_tmem + 128, &s_mbar, 0u, 0, int(threadIdx.x)};
+  TcTile T{s_tmem, s_tmem + 128, s_tmem + 192, &s_mbar, 0u, 0, int(threadIdx.x)};
+  store_ones(T.tmem_ones, T.row);
   bool ok = true;
   for (long long base = blockIdx.x * 128LL; base < n; base += gridDim.x * 128LL) {
     const long long r = base + threadIdx.x;
     float x[16] = {}, y[8];
     if (r < n)
       for (int k = 0; k < m.n_in; ++k) x[k] = inputs[r * m.n_in + k];
-    ok = mlp_tile_tc<kHidden>(smw, m.n_in, T, x, y);
+    uint32_t xp[8];
+    pack_inputs(x, m.n_in, xp);
+    ok = mlp_tile_tc<kHidden>(smw, m.n_in, T, xp, y);
     if (!ok) break;  // block-uniform (one tile per block); no MMA is issued after it
     if (r < n)
       for (int k = 0; k < m.n_out; ++k) outputs[r * m.n_out + k] = y[k];

@@ -41,6 +41,17 @@ __device__ __forceinline__ float silu_half(float h) {
 __device__ __forceinline__ uint32_t silu_half_bf16x2(float h_lo, float h_hi) {
   return pack_bf16(silu_half(h_lo), silu_half(h_hi));
 }
+// The same with the two FMAs as one packed instruction (the same roundings).
+__device__ __forceinline__ uint32_t silu_half_pair(float h_lo, float h_hi) {
+  float t_lo, t_hi, r_lo, r_hi;
+  asm("tanh.approx.f32 %0, %1;" : "=f"(t_lo) : "f"(h_lo));
+  asm("tanh.approx.f32 %0, %1;" : "=f"(t_hi) : "f"(h_hi));
+  asm("{\n\t.reg .b64 h, t, r;\n\tmov.b64 h, {%2, %3};\n\tmov.b64 t, {%4, %5};\n\t"
+      "fma.rn.f32x2 r, h, t, h;\n\tmov.b64 {%0, %1}, r;\n\t}"
+      : "=f"(r_lo), "=f"(r_hi)
+      : "f"(h_lo), "f"(h_hi), "f"(t_lo), "f"(t_hi));
+  return pack_bf16(r_lo, r_hi);
+}
 
 
 constexpr int kMlpH = 64;

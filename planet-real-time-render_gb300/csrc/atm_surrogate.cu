@@ -20,6 +20,7 @@
 // terminator get the same resolution the LUTs give them.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdint>
 
 #include "atm_device.cuh"
@@ -33,12 +34,31 @@ namespace {
 
 constexpr unsigned kAll = 0xffffffffu;
 
+// The features are rounded to BF16, and what they cost is most of what a
+// network pixel executes beside its network: they take the hardware's square
+// root, reciprocal and rsqrt (1-2 ulp).  The sun cosines do not: gates
+// compare them, and a pixel's path hangs on their last bit.
+//
+// Sky-view v of a zenith angle whose cosine is mu, at altitude h
+// (sky_zenith_to_v of sky_horizon_zenith).
+__device__ __forceinline__ float view_feature(float mu, float h, float bottom) {
+  const float z = acosf(clampf(mu, -1.0f, 1.0f));
+  const float a = mx(h, 0.0f);
+  const float hz = kPiF - acosf(clampf(shell_rho(a, bottom) * frcp(mx(bottom + a, 1.0f)), 0.0f, 1.0f));
+  const bool above = z < hz;
+  const float n = __saturatef(fdiv(above ? z : z - hz, mx(above ? hz : kPiF - hz, 1.0e-6f)));
+  return above ? 0.5f * (1.0f - fsqrt(1.0f - n)) : 0.5f + 0.5f * fsqrt(n);
+}
+// Cosine of the azimuth between two horizontal vectors, from their dot
+// product and squared lengths; 1 where one is shorter than 1e-6.
+__device__ __forceinline__ float azimuth_cosine(float ab, float aa, float bb) {
+  return aa > 1.0e-12f && bb > 1.0e-12f ? ab * frsqrt(aa * bb) : 1.0f;
+}
 // x[0..3]: altitude, view, sun, relative azimuth at the segment's first point.
 __device__ __forceinline__ void geometry_features(const DevParams& P, float bottom, float h, float mu_v, float mu_s,
                                                   float cos_dphi, float* x) {
-  const float hn = clampf(h * P.inv_top, 0.0f, 1.0f);
-  x[0] = 2.0f * sqrtf(hn) - 1.0f;
-  x[1] = 2.0f * sky_zenith_to_v(acosf(clampf(mu_v, -1.0f, 1.0f)), sky_horizon_zenith(h, bottom)) - 1.0f;
+  x[0] = 2.0f * fsqrt(__saturatef(h * P.inv_top)) - 1.0f;
+  x[1] = 2.0f * view_feature(mu_v, h, bottom) - 1.0f;
   x[2] = 2.0f * sun_cosine_to_u(clampf(mu_s, -1.0f, 1.0f), horizon_cosine(h, bottom)) - 1.0f;
   x[3] = clampf(cos_dphi, -1.0f, 1.0f);
 }
@@ -55,7 +75,7 @@ __device__ __forceinline__ float point_features(const DevParams& P, float bottom
   const float mu = clampf(dot(sun, pt) / mx(norm(pt), 1.0f), -1.0f, 1.0f);
   const float h = altitude_at(G, t, bottom);
   x[0] = 2.0f * sun_cosine_to_u(mu, horizon_cosine(h, bottom)) - 1.0f;
-  x[1] = 2.0f * sqrtf(clampf(h * P.inv_top, 0.0f, 1.0f)) - 1.0f;
+  x[1] = 2.0f * fsqrt(__saturatef(h * P.inv_top)) - 1.0f;
   return mu;
 }
 // Aerial x[7..10]: the segment's end, then its middle.  Returns the smaller
@@ -96,20 +116,10 @@ __device__ f3 sky_radiance(const DevParams& P, const Frame& F, float h, f3 ray) 
   bool valid, ground;
   const RayGeom G = camera_ray_geom(P, F.bottom, h, ray);
   segment_of(P, G, F.bottom, start, end, valid, ground);
-  Seg acc = {splat(0.0f), splat(1.0f)};
-  if (valid) {
-    const RaySource rs = make_ray_source(P, F, G, ray);
-    const RayWarp rw = make_warp(G.tc, start, end);
-    const int n = P.sv_steps;
-    float d0 = warp_at(rw, 0.0f);
-    for (int i = 0; i < n; ++i) {
-      const float d1 = warp_at(rw, float(i + 1) / float(n));
-      float vis;
-      acc = seg_then(acc, source_segment<true>(P, F, rs, d0, d1, vis));
-      d0 = d1;
-    }
-  }
-  return vmax(acc.L, 0.0f);
+  if (!valid) return splat(0.0f);
+  const RaySource rs = make_ray_source(P, F, G, ray);
+  const int n = P.sv_steps;
+  return vmax(march(P, F, rs, make_warp(G.tc, start, end), 0, n, n, DivideFraction{float(n)}).L, 0.0f);
 }
 
 // Aerial samples may be shaped toward camera-to-surface segments: a share
@@ -118,15 +128,14 @@ __device__ f3 sky_radiance(const DevParams& P, const Frame& F, float h, f3 ray) 
 // reaches it (the segment's length then follows from the geometry).
 __global__ void __launch_bounds__(128) k_gen_samples(const SurrogateSetDev* __restrict__ sets, int n_sets, int kind,
                                                      long long n, unsigned long long seed, SampleShaping shaping,
-                                                     f3 E, float ar, float* __restrict__ features,
-                                                     float* __restrict__ targets,
+                                                     float* __restrict__ features, float* __restrict__ targets,
                                                      unsigned long long* __restrict__ counter) {
   const long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
   uint32_t samples = 0;
   if (i < n) {
     const SurrogateSetDev& S = sets[min(int(uniform01(seed, i, 0) * n_sets), n_sets - 1)];
     const DevParams& P = S.P;
-    const float R = S.bottom;
+    const float R = S.F.bottom;
     float x[16];
     for (int k = 0; k < 4; ++k) x[k] = 2.0f * uniform01(seed, i, k + 1) - 1.0f;
     if (shaping.x0_lo < shaping.x0_hi) x[0] = shaping.x0_lo + (shaping.x0_hi - shaping.x0_lo) * uniform01(seed, i, 9);
@@ -148,8 +157,9 @@ __global__ void __launch_bounds__(128) k_gen_samples(const SurrogateSetDev* __re
     geometry_features(P, R, h, mu_v, mu_s, cphi, x);  // rounding-consistent features
     x[4] = S.lhr_n;
     x[5] = S.lhm_n;
-    const Frame F = make_frame(P, S.tlut, S.mslut, R, ar, sun, E);
-    const f3 inv_e = mk(1.0f / E.x, 1.0f / E.y, 1.0f / E.z);
+    Frame F = S.F;
+    F.sun = sun;
+    const f3 inv_e = mk(1.0f / F.E.x, 1.0f / F.E.y, 1.0f / F.E.z);
     if (kind == 0) {  // sky: 10 features -> log(L/E + floor)
       const f3 L = sky_radiance(P, F, h, ray) * inv_e;
       samples = uint32_t(P.sv_steps);
@@ -177,8 +187,8 @@ __global__ void __launch_bounds__(128) k_gen_samples(const SurrogateSetDev* __re
       float start, end;
       const RayGeom G = ray_geom(P, R, h, mu_v, sv);
       if (surface_interval(P, G, R, len, start, end)) {
-        L = integrate_surface(P, F, G, ray, start, end, samples) * inv_e;
-        T = surface_segment_t(P, F, G, ray, start, end);
+        L = integrate_surface(P, F, G, ray, start, end, divide_fractions(P), samples) * inv_e;
+        T = surface_segment_t(P, F, G, start, end);
       } else {
         start = end = 0.0f;
       }
@@ -224,289 +234,384 @@ __device__ __forceinline__ f3 net_radiance(const float (&y)[8], const float* E, 
 
 enum PixelKind : int { kNone = 0, kSurfMlp, kSurfPlain, kSurfEmpty, kSkyMlp, kSkyLut };
 
-// 256 threads = two tiles of 128 pixels (warps 0-3, 4-7); a pixel is one
-// tensor-memory lane of its tile.  Tensor memory (256 columns): tile t holds
-// its accumulators at column 128 t and its activations at 128 t + 64.
-constexpr uint32_t kSurrogateTmemCols = 256;
+// The network kernels: one block an SM stays for the launch and its kWorkers
+// tiles of 128 threads each run 128-pixel tiles of the frame one after
+// another, every tile on its own barriers - while one waits for its MMAs the
+// others have features and activations to compute.  The weights and the
+// tensor memory are taken once a block.  What bounds them is the activations'
+// tanh (XU) and the issue of features and outputs around them, at the
+// latency of the five serial layers; five tiles are what 512 tensor-memory
+// columns hold (64 accumulator and 32 activation columns a tile, the bias's 8
+// shared).  A 4K frame takes 0.83 ms, against 0.99 ms with two tiles a block,
+// three blocks an SM and the weights copied by each block.
+constexpr int kWorkers = 5;
+constexpr uint32_t kWorkerCols = 96, kOnesCol = kWorkers * kWorkerCols, kSurrogateTmemCols = 512;
+
+struct NetBlock {
+  uint64_t mbar[kWorkers + 1];  // the tiles' MMA completions, the weights' arrival
+  uint32_t tmem;
+  float horizon;  // the camera's horizon zenith
+};
+// Sets a block up (every thread calls): the weights into smem by bulk copies,
+// tensor memory, barriers.  Returns this thread's tile; `weights` false if the
+// weights did not arrive in time.
+__device__ __forceinline__ TcTile net_block_begin(NetBlock& B, unsigned char* smem, const unsigned char* w0, int n0,
+                                                  const unsigned char* w1, int n1, float horizon_altitude, float bottom,
+                                                  bool& weights) {
+  if (threadIdx.x == 0) {
+    for (int k = 0; k <= kWorkers; ++k) tc::mbar_init(&B.mbar[k], 1);
+    tc::mbar_init_fence();
+    tc::mbar_arrive_expect_tx(&B.mbar[kWorkers], uint32_t(n0 + n1));
+    if (n0 > 0) tc::bulk_g2s(smem, w0, uint32_t(n0), &B.mbar[kWorkers]);
+    if (n1 > 0) tc::bulk_g2s(smem + n0, w1, uint32_t(n1), &B.mbar[kWorkers]);
+    B.horizon = sky_horizon_zenith(horizon_altitude, bottom);
+  }
+  if (threadIdx.x >> 5 == 1) tc::alloc(&B.tmem, kSurrogateTmemCols);
+  tc::fence_before_sync();
+  __syncthreads();
+  tc::fence_after_sync();
+  const int tile = threadIdx.x >> 7, row = threadIdx.x & 127;
+  if (tile == 0) store_ones(B.tmem + kOnesCol, row);
+  // each thread observes the weights' mbarrier before any MMA of its tile reads them
+  const bool arrived = tc::mbar_wait(&B.mbar[kWorkers], 0u, kTcWaitTries);
+  tc::fence_before_sync();
+  weights = __syncthreads_and(arrived);
+  tc::fence_after_sync();
+  return TcTile{B.tmem + kWorkerCols * tile, B.tmem + kWorkerCols * tile + 64u, B.tmem + kOnesCol, &B.mbar[tile], 0u,
+                tile, row};
+}
+// Frees the tensor memory (every thread calls; no MMA of its tile in flight).
+__device__ __forceinline__ void net_block_end(NetBlock& B) {
+  tc::fence_before_sync();
+  __syncthreads();
+  tc::fence_after_sync();
+  if (threadIdx.x >> 5 == 1) tc::dealloc(B.tmem, kSurrogateTmemCols);
+}
+// After a network run that gave up: waits, with the library's full bound
+// whatever the frame's own bound was, for the one commit in flight.  False in
+// every thread of the tile if that does not come either: no more networks.
+__device__ __forceinline__ bool tile_recover(TcTile& T) {
+  return tc::tile_all(T.tile, tc::mbar_wait(T.mbar, T.phase ^ 1u, kTcWaitTries));
+}
+
+// A frame's 128-pixel tiles: 16 pixels along the image's contiguous axis by 8,
+// a warp 16 x 2 of them (whole sectors of every image).
+struct PixelTiles {
+  int across, count;  // tiles along y (y contiguous) or x, tiles in all
+};
+__host__ __device__ inline bool y_contiguous(const ImageLayout& L) { return L.sy <= L.sx; }
+inline PixelTiles pixel_tiles(const ImageLayout& L) {
+  const int fast = y_contiguous(L) ? L.height : L.width, slow = y_contiguous(L) ? L.width : L.height;
+  const int across = (fast + 15) / 16;
+  return {across, across * ((slow + 7) / 8)};
+}
+__device__ __forceinline__ bool tile_pixel_of(const ImageLayout& L, const PixelTiles& N, int tile, int row, int& x,
+                                              int& y) {
+  const int slow = (tile / N.across) * 8 + (row >> 4), fast = (tile % N.across) * 16 + (row & 15);
+  x = y_contiguous(L) ? slow : fast;
+  y = y_contiguous(L) ? fast : slow;
+  return x < L.width && y < L.height;
+}
 
 // kShade: the surface colour comes from the fused surface lighting and
 // shading (shaded_scene) instead of the scene image.
 template <bool kShade>
-__global__ void __launch_bounds__(256, 3) k_composite_surrogate(
-    DevParams P, ImageLayout L, CompositeScalars A, const float* __restrict__ scene, const float* __restrict__ space,
-    const int32_t* __restrict__ sid, const float* __restrict__ pos, const float4* __restrict__ tlut,
-    const float4* __restrict__ mslut, const float4* __restrict__ svlut, SurrogateNets nets, SurrogateQueue Q,
-    float* __restrict__ hdr, ShadeParams S, ShadeImages I) {
+__global__ void __launch_bounds__(128 * kWorkers, 1) k_composite_surrogate(
+    DevParams P, Frame F, ImageLayout L, PixelTiles N, CompositeScalars A, const float* __restrict__ scene,
+    const float* __restrict__ space, const int32_t* __restrict__ sid, const float* __restrict__ pos,
+    const float4* __restrict__ svlut, SurrogateNets nets, SurrogateQueue Q, float* __restrict__ hdr, ShadeParams S,
+    ShadeImages I) {
   extern __shared__ __align__(128) unsigned char smem[];  // the aerial network, then the sky network
-  __shared__ __align__(8) uint64_t s_mbar[3];  // the two tiles' MMA completions, the weights' arrival
-  __shared__ uint32_t s_tmem;
-  const int wbytes = nets.ap_bytes + nets.sky_bytes;
-  if (threadIdx.x == 0) {
-    tc::mbar_init(&s_mbar[0], 1);
-    tc::mbar_init(&s_mbar[1], 1);
-    tc::mbar_init(&s_mbar[2], 1);
-    tc::mbar_init_fence();
-  }
-  __syncthreads();
-  // the weights arrive by bulk copy while the block computes its features
-  if (threadIdx.x == 0) {
-    tc::mbar_arrive_expect_tx(&s_mbar[2], uint32_t(wbytes));
-    if (nets.ap_bytes > 0) tc::bulk_g2s(smem, nets.ap, uint32_t(nets.ap_bytes), &s_mbar[2]);
-    if (nets.sky_bytes > 0) tc::bulk_g2s(smem + nets.ap_bytes, nets.sky, uint32_t(nets.sky_bytes), &s_mbar[2]);
-  }
-  const int tile = threadIdx.x >> 7;
+  __shared__ NetBlock B;
+  bool nets_ok;  // tile-uniform: the networks may run
+  TcTile T = net_block_begin(B, smem, nets.ap, nets.ap_bytes, nets.sky, nets.sky_bytes, A.cam_alt, A.bottom, nets_ok);
+  const int lane = threadIdx.x & 31;
+  for (int t = T.tile * gridDim.x + blockIdx.x; t < N.count; t += kWorkers * gridDim.x) {
+    int x, y;
+    const bool inside = tile_pixel_of(L, N, t, T.row, x, y);
+    const int cx = inside ? x : 0, cy = inside ? y : 0;
+    const size_t e = pix_offset(L, cx, cy);
+    const size_t o = e * L.channels;
+    const f3 ray = pixel_ray(L, A, cx, cy).ray;
+    const bool near_limb = fabsf(acosf(clampf(ray.y, -1.0f, 1.0f)) - B.horizon) < nets.limb_rad;
 
-  int x, y;
-  const bool inside = tile_pixel(L, x, y);
-  const int cx = inside ? x : 0, cy = inside ? y : 0;
-  const size_t e = pix_offset(L, cx, cy);
-  const size_t o = e * L.channels;
-  const Frame F = make_frame(P, tlut, mslut, A.bottom, A.ar, arr3(A.sun), arr3(A.E));
-  const f3 ray = pixel_ray(L, A, cx, cy).ray;
-  const bool near_limb =
-      fabsf(acosf(clampf(ray.y, -1.0f, 1.0f)) - sky_horizon_zenith(A.cam_alt, A.bottom)) < nets.limb_rad;
-
-  int kind = kNone;
-  float fx[16] = {};
-  float start = 0.0f, end = 0.0f;
-  if (inside) {
-    if (sid[e] >= 0) {
-      const RayGeom G = camera_ray_geom(P, A.bottom, A.cam_alt, ray);
-      if (!surface_interval(P, G, A.bottom, norm(ld3(pos + o)), start, end)) {
-        kind = kSurfEmpty;
-      } else if (nets.ap == nullptr || near_limb) {
-        kind = kSurfPlain;
-      } else {
-        // features at the segment's first point inside the shell
-        const float o_y = A.bottom + A.cam_alt;
-        const float hs = altitude_at(G, start, A.bottom);
-        const f3 ps = mk(ray.x * start, o_y + ray.y * start, ray.z * start);
-        const f3 up = ps * (1.0f / mx(norm(ps), 1.0f));
-        const float mu_v = dot(ray, up), mu_s = dot(F.sun, up);
-        const f3 tv = ray - up * mu_v, ts = F.sun - up * mu_s;
-        const float nv = norm(tv), ns = norm(ts);
-        const float cphi = (nv > 1e-6f && ns > 1e-6f) ? dot(tv, ts) / (nv * ns) : 1.0f;
-        geometry_features(P, A.bottom, hs, mu_v, mu_s, cphi, fx);
+    int kind = kNone;
+    uint32_t xp[8] = {};
+    float start = 0.0f, end = 0.0f;
+    if (inside) {
+      float fx[16] = {};
+      if (sid[e] >= 0) {
+        const RayGeom G = camera_ray_geom(P, A.bottom, A.cam_alt, ray);
+        if (!surface_interval(P, G, A.bottom, norm(ld3(pos + o)), start, end)) {
+          kind = kSurfEmpty;
+        } else if (nets.ap == nullptr || near_limb) {
+          kind = kSurfPlain;
+        } else {
+          // features at the segment's first point inside the shell
+          const float o_y = A.bottom + A.cam_alt;
+          const float hs = altitude_at(G, start, A.bottom);
+          const f3 ps = mk(ray.x * start, o_y + ray.y * start, ray.z * start);
+          const f3 up = ps * (1.0f / mx(norm(ps), 1.0f));
+          const float mu_v = dot(ray, up), mu_s = dot(F.sun, up);
+          const f3 tv = ray - up * mu_v, ts = F.sun - up * mu_s;
+          const float cphi = azimuth_cosine(dot(tv, ts), dot(tv, tv), dot(ts, ts));
+          geometry_features(P, A.bottom, hs, mu_v, mu_s, cphi, fx);
+          fx[4] = nets.lhr_n;
+          fx[5] = nets.lhm_n;
+          fx[6] = 2.0f * __logf(clampf(end - start, 1.0f, kSurrogateMaxLength)) / logf(kSurrogateMaxLength) - 1.0f;
+          // twilight gate: the sun cosine small at the start, middle or end, or
+          // of different signs there (the segment crosses the terminator)
+          float mu_end, mu_mid;
+          const float mu_min =
+              mn(fabsf(mu_s), segment_features(P, A.bottom, G, ray, o_y, F.sun, start, end, fx, mu_end, mu_mid));
+          const bool crosses =
+              nets.gate_crossing && ((mu_s > 0.0f) != (mu_end > 0.0f) || (mu_s > 0.0f) != (mu_mid > 0.0f));
+          kind = (mu_min < nets.twilight_cos || crosses) ? kSurfPlain : kSurfMlp;
+          pack_inputs(fx, kSurrogateApIn, xp);
+        }
+      } else if (nets.sky != nullptr && A.cam_alt <= P.top && fabsf(F.sun.y) >= nets.sky_twilight_cos && !near_limb) {
+        kind = kSkyMlp;
+        const float cphi = azimuth_cosine(ray.x * F.sun.x + ray.z * F.sun.z, ray.x * ray.x + ray.z * ray.z,
+                                          F.sun.x * F.sun.x + F.sun.z * F.sun.z);
+        geometry_features(P, A.bottom, A.cam_alt, ray.y, F.sun.y, cphi, fx);
         fx[4] = nets.lhr_n;
         fx[5] = nets.lhm_n;
-        fx[6] = 2.0f * __logf(clampf(end - start, 1.0f, kSurrogateMaxLength)) / logf(kSurrogateMaxLength) - 1.0f;
-        // twilight gate: the sun cosine small at the start, middle or end, or
-        // of different signs there (the segment crosses the terminator)
-        float mu_end, mu_mid;
-        const float mu_min =
-            mn(fabsf(mu_s), segment_features(P, A.bottom, G, ray, o_y, F.sun, start, end, fx, mu_end, mu_mid));
-        const bool crosses = nets.gate_crossing && ((mu_s > 0.0f) != (mu_end > 0.0f) || (mu_s > 0.0f) != (mu_mid > 0.0f));
-        kind = (mu_min < nets.twilight_cos || crosses) ? kSurfPlain : kSurfMlp;
+        sky_ray_features(P, A.bottom, A.cam_alt, ray, F.sun, fx);
+        pack_inputs(fx, kSurrogateSkyIn, xp);
+      } else {
+        kind = kSkyLut;
       }
-    } else if (nets.sky != nullptr && A.cam_alt <= P.top && fabsf(F.sun.y) >= nets.sky_twilight_cos && !near_limb) {
-      kind = kSkyMlp;
-      const float vl = sqrtf(ray.x * ray.x + ray.z * ray.z), sl = sqrtf(F.sun.x * F.sun.x + F.sun.z * F.sun.z);
-      const float cphi = (vl > 1e-6f && sl > 1e-6f) ? (ray.x * F.sun.x + ray.z * F.sun.z) / (vl * sl) : 1.0f;
-      geometry_features(P, A.bottom, A.cam_alt, ray.y, F.sun.y, cphi, fx);
-      fx[4] = nets.lhr_n;
-      fx[5] = nets.lhm_n;
-      sky_ray_features(P, A.bottom, A.cam_alt, ray, F.sun, fx);
-    } else {
-      kind = kSkyLut;
     }
-  }
 
-  // the networks on the tensor cores, each run by the whole block when any
-  // of its pixels needs it (block-uniform: every barrier stays convergent).
-  // Tensor memory is taken only now, so that a block waiting for columns
-  // has its features done, and not at all by a block without MLP pixels.
-  // tc_ok is uniform over a tile; a tile whose wait timed out issues nothing
-  // more and its MLP pixels take the plain path below.
-  float yv[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-  bool tc_ok = true;
-  const bool need_ap = __syncthreads_or(kind == kSurfMlp);
-  const bool need_sky = __syncthreads_or(kind == kSkyMlp);
-  // the weights have arrived (each thread observes the mbarrier before any
-  // MMA of its tile reads them)
-  const bool weights_ok = __syncthreads_and(tc::mbar_wait(&s_mbar[2], 0u, kTcWaitTries));
-  if ((need_ap || need_sky) && weights_ok) {
-    if (threadIdx.x < 32) tc::alloc(&s_tmem, kSurrogateTmemCols);
-    tc::fence_before_sync();
-    __syncthreads();
-    tc::fence_after_sync();
-    TcTile T{s_tmem + 128u * tile, s_tmem + 128u * tile + 64u, &s_mbar[tile], 0u, tile, int(threadIdx.x & 127)};
-    if (need_ap) {
-      float t[8];
-      tc_ok = mlp_tile_tc<kSurrogateApHidden>(smem, kSurrogateApIn, T, fx, t, nets.wait_tries);
+    // the networks on the tensor cores, each run by the whole tile when any of
+    // its pixels needs it (tile-uniform: every barrier stays convergent).  A
+    // tile whose wait timed out issues nothing more and its MLP pixels take
+    // the plain path below.
+    float yv[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+    const bool need_ap = nets.ap != nullptr && tc::tile_any(T.tile, kind == kSurfMlp);
+    const bool need_sky = nets.sky != nullptr && tc::tile_any(T.tile, kind == kSkyMlp);
+    bool tc_ok = nets_ok;
+    if (need_ap && tc_ok) {
+      float v[8];
+      tc_ok = mlp_tile_tc<kSurrogateApHidden>(smem, kSurrogateApIn, T, xp, v, nets.wait_tries);
       if (kind == kSurfMlp)
-        for (int k = 0; k < 8; ++k) yv[k] = t[k];
+        for (int k = 0; k < 8; ++k) yv[k] = v[k];
     }
     if (need_sky && tc_ok) {
-      float t[8];
-      tc_ok = mlp_tile_tc<kSurrogateSkyHidden>(smem + nets.ap_bytes, kSurrogateSkyIn, T, fx, t, nets.wait_tries);
+      float v[8];
+      tc_ok = mlp_tile_tc<kSurrogateSkyHidden>(smem + nets.ap_bytes, kSurrogateSkyIn, T, xp, v, nets.wait_tries);
       if (kind == kSkyMlp)
-        for (int k = 0; k < 8; ++k) yv[k] = t[k];
+        for (int k = 0; k < 8; ++k) yv[k] = v[k];
     }
-    // tensor memory is freed once no MMA is in flight: a tile that timed out
-    // has exactly one commit outstanding, waited for here with the library's
-    // full bound whatever the frame's own bound was
-    tc::fence_before_sync();
-    if (!tc_ok) tc::mbar_wait(T.mbar, T.phase ^ 1u, kTcWaitTries);
-    __syncthreads();
-    tc::fence_after_sync();
-    if (threadIdx.x < 32) tc::dealloc(s_tmem, kSurrogateTmemCols);
-  } else if (need_ap || need_sky) {
-    tc_ok = false;  // the weights did not arrive in time
-  }
-  if (!tc_ok) {
-    // the networks' outputs are not valid: the plain path for these pixels
-    if (kind == kSurfMlp) kind = kSurfPlain;
-    if (kind == kSkyMlp) kind = kSkyLut;
-    if ((threadIdx.x & 127) == 0) atomicOr(Q.status, 1u);
-  }
+    tc_ok = tc_ok || !(need_ap || need_sky);
+    if (!tc_ok) {
+      // the networks' outputs are not valid: the plain path for these pixels
+      if (kind == kSurfMlp) kind = kSurfPlain;
+      if (kind == kSkyMlp) kind = kSkyLut;
+      if (T.row == 0) atomicOr(Q.status, 1u);
+      if (nets_ok) nets_ok = tile_recover(T);
+    }
 
-  bool queued = false;
-  uint32_t qkind = kQueueSurface;
-  f3 Lnet = mk(-1.0f, 0.0f, 0.0f);  // the network's in-scattering (x < 0: none)
-  if (inside && kind != kSurfPlain) {
-    f3 color = kShade ? shaded_scene(P, F, A, S, L, I, x, y, e, sid[e]) : ld3(scene + o);
-    if (kind == kSurfMlp) {
-      // transmittance: the plain path's own two-tap LUT ratio (:1603-1665);
-      // in-scattering: the network, ln(L / E + floor + floor_t T)
-      const f3 Tm = surface_segment_t(P, F, camera_ray_geom(P, A.bottom, A.cam_alt, ray), ray, start, end);
-      const f3 Lm = net_radiance(yv, A.E, splat(nets.floor) + Tm * nets.floor_t);
-      color = Lm + color * Tm;
-      Lnet = Lm;
-      if (check_pixel(x, y, Q.seed, Q.check_fraction)) {
-        queued = true;
-        qkind = kQueueSurfaceCheck;
+    bool queued = false;
+    uint32_t qkind = kQueueSurface;
+    f3 Lnet = mk(-1.0f, 0.0f, 0.0f);  // the network's in-scattering (x < 0: none)
+    if (inside && kind != kSurfPlain) {
+      f3 color = kShade ? shaded_scene(P, F, A, S, L, I, x, y, e, sid[e]) : ld3(scene + o);
+      if (kind == kSurfMlp) {
+        // transmittance: the plain path's own two-tap LUT ratio (:1603-1665);
+        // in-scattering: the network, ln(L / E + floor + floor_t T)
+        const f3 Tm = surface_segment_t(P, F, camera_ray_geom(P, A.bottom, A.cam_alt, ray), start, end);
+        const f3 Lm = net_radiance(yv, A.E, splat(nets.floor) + Tm * nets.floor_t);
+        color = Lm + color * Tm;
+        Lnet = Lm;
+        if (check_pixel(x, y, Q.seed, Q.check_fraction)) {
+          queued = true;
+          qkind = kQueueSurfaceCheck;
+        }
+      } else if (kind == kSkyMlp) {
+        const f3 sky = net_radiance(yv, A.E, splat(nets.sky_floor));
+        color = composite_sky_with(P, F, A, sky, ray, color, ld3(space + o), float(L.height));
+        if (check_pixel(x, y, Q.seed, Q.check_fraction)) {
+          queued = true;
+          qkind = kQueueSkyCheck;
+        }
+      } else if (kind == kSkyLut) {
+        color = composite_sky(P, F, A, svlut, ray, color, ld3(space + o), float(L.height));
       }
-    } else if (kind == kSkyMlp) {
-      const f3 sky = net_radiance(yv, A.E, splat(nets.sky_floor));
-      color = composite_sky_with(P, F, A, sky, ray, color, ld3(space + o), float(L.height));
-      if (check_pixel(x, y, Q.seed, Q.check_fraction)) {
-        queued = true;
-        qkind = kQueueSkyCheck;
+      color = vmax(color, 0.0f);
+      hdr[o + 0] = color.x;
+      hdr[o + 1] = color.y;
+      hdr[o + 2] = color.z;
+    } else if (kind == kSurfPlain) {
+      queued = true;
+    }
+    if (inside && Q.lm != nullptr) {  // the calibration's scratch: every pixel, each frame
+      float* lm = Q.lm + 3 * storage_index(L, x, y);
+      lm[0] = Lnet.x;
+      if (Lnet.x >= 0.0f) {
+        lm[1] = Lnet.y;
+        lm[2] = Lnet.z;
       }
-    } else if (kind == kSkyLut) {
-      color = composite_sky(P, F, A, svlut, ray, color, ld3(space + o), float(L.height));
     }
-    color = vmax(color, 0.0f);
-    hdr[o + 0] = color.x;
-    hdr[o + 1] = color.y;
-    hdr[o + 2] = color.z;
-  } else if (kind == kSurfPlain) {
-    queued = true;
-  }
-  if (inside && Q.lm != nullptr) {  // the calibration's scratch: every pixel, each frame
-    float* lm = Q.lm + 3 * storage_index(L, x, y);
-    lm[0] = Lnet.x;
-    if (Lnet.x >= 0.0f) {
-      lm[1] = Lnet.y;
-      lm[2] = Lnet.z;
-    }
-  }
 
-  // warp-aggregated append to the fallback queue
-  const int lane = threadIdx.x & 31;
-  const unsigned qm = __ballot_sync(kAll, queued);
-  if (qm) {
-    const int leader = __ffs(qm) - 1;
-    uint32_t base = 0;
-    if (lane == leader) base = atomicAdd(Q.count, uint32_t(__popc(qm)));
-    base = __shfl_sync(kAll, base, leader);
-    if (queued)
-      Q.items[base + __popc(qm & ((1u << lane) - 1u))] = (qkind << 30) | uint32_t(cy * L.width + cx);
-  }
-  if (Q.stats != nullptr) {
-    if (!tc_ok && (threadIdx.x & 127) == 0) atomicAdd(Q.stats + 7, 1.0f);  // tiles whose MMA timed out
-    const unsigned gs = __ballot_sync(kAll, kind == kSurfPlain), ms = __ballot_sync(kAll, kind == kSurfMlp);
-    const unsigned mk_ = __ballot_sync(kAll, kind == kSkyMlp), ls = __ballot_sync(kAll, kind == kSkyLut);
-    if (lane == 0) {
-      if (gs) atomicAdd(Q.stats + 3, float(__popc(gs)));
-      if (ms) atomicAdd(Q.stats + 4, float(__popc(ms)));
-      if (mk_) atomicAdd(Q.stats + 5, float(__popc(mk_)));
-      if (ls) atomicAdd(Q.stats + 6, float(__popc(ls)));
+    // warp-aggregated append to the fallback queue
+    const unsigned qm = __ballot_sync(kAll, queued);
+    if (qm) {
+      const int leader = __ffs(qm) - 1;
+      uint32_t base = 0;
+      if (lane == leader) base = atomicAdd(Q.count, uint32_t(__popc(qm)));
+      base = __shfl_sync(kAll, base, leader);
+      if (queued)
+        Q.items[base + __popc(qm & ((1u << lane) - 1u))] = (qkind << 30) | uint32_t(cy * L.width + cx);
+    }
+    if (Q.stats != nullptr) {
+      if (!tc_ok && T.row == 0) atomicAdd(Q.stats + 7, 1.0f);  // tiles whose MMA timed out
+      const unsigned gs = __ballot_sync(kAll, kind == kSurfPlain), ms = __ballot_sync(kAll, kind == kSurfMlp);
+      const unsigned mk_ = __ballot_sync(kAll, kind == kSkyMlp), ls = __ballot_sync(kAll, kind == kSkyLut);
+      if (lane == 0) {
+        if (gs) atomicAdd(Q.stats + 3, float(__popc(gs)));
+        if (ms) atomicAdd(Q.stats + 4, float(__popc(ms)));
+        if (mk_) atomicAdd(Q.stats + 5, float(__popc(mk_)));
+        if (ls) atomicAdd(Q.stats + 6, float(__popc(ls)));
+      }
     }
   }
+  net_block_end(B);
+}
+
+// Lanes that share a queued pixel's march: a short queue (the checked 1% of a
+// frame is about one pixel a resident thread) would run as one or two whole
+// marches a thread on part of the warps; a long one would only repeat each
+// pixel's set-up.  4K, 1% checked: 77 us against 111 us at one lane a pixel.
+constexpr int kQueueLanes = 4;
+__device__ __forceinline__ bool split_queue(uint32_t n) { return n <= 8u * gridDim.x * blockDim.x; }
+
+// Sky radiance along `ray` by kLanes consecutive lanes, as sky_radiance; the
+// group's first lane receives it.  Every lane of the warp must call.
+template <int kLanes>
+__device__ __forceinline__ f3 sky_radiance_split(const DevParams& P, const Frame& F, float h, f3 ray, bool active) {
+  Seg acc = seg_identity();
+  float start, end;
+  bool valid, ground;
+  const RayGeom G = camera_ray_geom(P, F.bottom, h, ray);
+  segment_of(P, G, F.bottom, start, end, valid, ground);
+  if (active && valid) {
+    const int n = P.sv_steps, per = (n + kLanes - 1) / kLanes;
+    const int i0 = min(int(threadIdx.x & (kLanes - 1)) * per, n);
+    acc = march(P, F, make_ray_source(P, F, G, ray), make_warp(G.tc, start, end), i0, min(i0 + per, n), n,
+                DivideFraction{float(n)});
+  }
+  return vmax(group_compose<kLanes>(acc).L, 0.0f);
 }
 
 // The plain integrator over the queued pixels: gated surface pixels get it
 // as their result; checked pixels compare the MLP's color (in hdr) with it,
-// then keep the plain result.  Warps take 32 entries per ticket.
-template <bool kShade>
-__global__ void __launch_bounds__(256, 2) k_surrogate_fallback(
-    DevParams P, ImageLayout L, CompositeScalars A, const float* __restrict__ scene, const float* __restrict__ space,
-    const float* __restrict__ pos, const float4* __restrict__ tlut, const float4* __restrict__ mslut,
-    SurrogateQueue Q, float* __restrict__ hdr, unsigned long long* counter, ShadeParams S, ShadeImages I) {
-  const Frame F = make_frame(P, tlut, mslut, A.bottom, A.ar, arr3(A.sun), arr3(A.E));
-  const int lane = threadIdx.x & 31;
-  const uint32_t n = *Q.count;
+// then keep the plain result.  Warps take 32 / kLanes entries per ticket.
+struct CheckSums {
   uint32_t samples = 0, checked = 0;
   float err_sum = 0.0f, err_max = 0.0f;
+};
+template <int kLanes, bool kShade>
+__device__ __forceinline__ void fallback_queue(const DevParams& P, const Frame& F, const ImageLayout& L,
+                                               const CompositeScalars& A, const float* __restrict__ scene,
+                                               const float* __restrict__ space, const float* __restrict__ pos,
+                                               const SurrogateQueue& Q, float* __restrict__ hdr, const ShadeParams& S,
+                                               const ShadeImages& I, uint32_t n, const TableFractions& fractions,
+                                               CheckSums& sums) {
+  const int lane = threadIdx.x & 31;
+  const bool first = (lane & (kLanes - 1)) == 0;
   for (;;) {
     uint32_t base = 0;
-    if (lane == 0) base = atomicAdd(Q.count + 1, 32u);
+    if (lane == 0) base = atomicAdd(Q.count + 1, 32u / kLanes);
     base = __shfl_sync(kAll, base, 0);
     if (base >= n) break;
-    const uint32_t i = base + uint32_t(lane);
-    if (i < n) {
-      const uint32_t entry = Q.items[i];
-      const uint32_t kind = entry >> 30, p = entry & 0x3fffffffu;
-      const int x = int(p % uint32_t(L.width)), y = int(p / uint32_t(L.width));
-      const size_t e = pix_offset(L, x, y);
-      const size_t o = e * L.channels;
-      const f3 ray = pixel_ray(L, A, x, y).ray;
-      f3 color = kShade ? shaded_scene(P, F, A, S, L, I, x, y, e, I.surface_id[e]) : ld3(scene + o);
-      if (kind == kQueueSkyCheck) {
-        const f3 sky = sky_radiance(P, F, A.cam_alt, ray);
-        samples += uint32_t(P.sv_steps);
+    const uint32_t i = base + uint32_t(lane / kLanes);
+    const bool has = i < n;
+    const uint32_t entry = has ? Q.items[i] : 0;
+    const uint32_t kind = entry >> 30, p = entry & 0x3fffffffu;
+    const int x = int(p % uint32_t(L.width)), y = int(p / uint32_t(L.width));
+    const size_t e = pix_offset(L, x, y);
+    const size_t o = e * L.channels;
+    const f3 ray = pixel_ray(L, A, x, y).ray;
+    const bool sky_check = has && kind == kQueueSkyCheck;
+    f3 color = splat(0.0f);
+    if (__any_sync(kAll, sky_check)) {
+      const f3 sky = sky_radiance_split<kLanes>(P, F, A.cam_alt, ray, sky_check);
+      if (sky_check && first) {
+        sums.samples += uint32_t(P.sv_steps);
+        color = kShade ? shaded_scene(P, F, A, S, L, I, x, y, e, I.surface_id[e]) : ld3(scene + o);
         color = composite_sky_with(P, F, A, sky, ray, color, ld3(space + o), float(L.height));
-      } else {
-        float start, end;
-        const RayGeom G = camera_ray_geom(P, A.bottom, A.cam_alt, ray);
-        if (surface_interval(P, G, A.bottom, norm(ld3(pos + o)), start, end)) {
-          const f3 Ls = integrate_surface(P, F, G, ray, start, end, samples);
-          color = Ls + color * surface_segment_t(P, F, G, ray, start, end);
-          if (kind == kQueueSurfaceCheck && Q.lm != nullptr) {
-            // the calibration: this tile's log ratio of the plain in-scattering
-            // to the network's; the pixel itself keeps the plain result
-            float* lm = Q.lm + 3 * storage_index(L, x, y);
-            const f3 Ln = ld3(lm);
-            if (Ln.x >= 0.0f) {
-              float* t = Q.tiles + 4 * ((y >> Q.tile_shift) * Q.tiles_x + (x >> Q.tile_shift));
-              atomicAdd(t + 0, clampf(__logf(mx(Ls.x, 1e-12f) / mx(Ln.x, 1e-12f)), -kCalibrationClamp,
-                                      kCalibrationClamp));
-              atomicAdd(t + 1, clampf(__logf(mx(Ls.y, 1e-12f) / mx(Ln.y, 1e-12f)), -kCalibrationClamp,
-                                      kCalibrationClamp));
-              atomicAdd(t + 2, clampf(__logf(mx(Ls.z, 1e-12f) / mx(Ln.z, 1e-12f)), -kCalibrationClamp,
-                                      kCalibrationClamp));
-              atomicAdd(t + 3, 1.0f);
-            }
-            lm[0] = -1.0f;
+      }
+    }
+    const bool surface = has && !sky_check;
+    const RayGeom G = camera_ray_geom(P, A.bottom, A.cam_alt, ray);
+    float start = 0.0f, end = 0.0f;
+    const bool clipped = surface && surface_interval(P, G, A.bottom, norm(ld3(pos + o)), start, end);
+    const f3 Ls = integrate_surface_split<kLanes>(P, F, G, ray, start, end, clipped, fractions, sums.samples);
+    if (surface && first) {
+      color = kShade ? shaded_scene(P, F, A, S, L, I, x, y, e, I.surface_id[e]) : ld3(scene + o);
+      if (clipped) {
+        color = Ls + color * surface_segment_t(P, F, G, start, end);
+        if (kind == kQueueSurfaceCheck && Q.lm != nullptr) {
+          // the calibration: this tile's log ratio of the plain in-scattering
+          // to the network's; the pixel itself keeps the plain result
+          float* lm = Q.lm + 3 * storage_index(L, x, y);
+          const f3 Ln = ld3(lm);
+          if (Ln.x >= 0.0f) {
+            float* t = Q.tiles + 4 * ((y >> Q.tile_shift) * Q.tiles_x + (x >> Q.tile_shift));
+            atomicAdd(t + 0, clampf(__logf(mx(Ls.x, 1e-12f) / mx(Ln.x, 1e-12f)), -kCalibrationClamp,
+                                    kCalibrationClamp));
+            atomicAdd(t + 1, clampf(__logf(mx(Ls.y, 1e-12f) / mx(Ln.y, 1e-12f)), -kCalibrationClamp,
+                                    kCalibrationClamp));
+            atomicAdd(t + 2, clampf(__logf(mx(Ls.z, 1e-12f) / mx(Ln.z, 1e-12f)), -kCalibrationClamp,
+                                    kCalibrationClamp));
+            atomicAdd(t + 3, 1.0f);
           }
+          lm[0] = -1.0f;
         }
       }
+    }
+    if (has && first) {
       color = vmax(color, 0.0f);
       if (kind != kQueueSurface) {
         const float err = color_error(ld3(hdr + o), color, F.E);
-        ++checked;
-        err_sum += err;
-        err_max = mx(err_max, err);
+        ++sums.checked;
+        sums.err_sum += err;
+        sums.err_max = mx(sums.err_max, err);
       }
       hdr[o + 0] = color.x;
       hdr[o + 1] = color.y;
       hdr[o + 2] = color.z;
     }
   }
-  warp_count(samples, counter);
+}
+template <bool kShade>
+__global__ void __launch_bounds__(256, 2) k_surrogate_fallback(
+    DevParams P, Frame F, ImageLayout L, CompositeScalars A, const float* __restrict__ scene,
+    const float* __restrict__ space, const float* __restrict__ pos, SurrogateQueue Q, float* __restrict__ hdr,
+    unsigned long long* counter, ShadeParams S, ShadeImages I) {
+  __shared__ float s_fractions[kFractionTable];
+  const TableFractions fractions = table_fractions(P, s_fractions);
+  const int lane = threadIdx.x & 31;
+  const uint32_t n = *Q.count;
+  CheckSums sums;
+  if (split_queue(n))
+    fallback_queue<kQueueLanes, kShade>(P, F, L, A, scene, space, pos, Q, hdr, S, I, n, fractions, sums);
+  else
+    fallback_queue<1, kShade>(P, F, L, A, scene, space, pos, Q, hdr, S, I, n, fractions, sums);
+  warp_count(sums.samples, counter);
   if (Q.stats != nullptr) {
-    float c = float(checked);
+    float c = float(sums.checked);
 #pragma unroll
     for (int k = 16; k > 0; k >>= 1) {
       c += __shfl_xor_sync(kAll, c, k);
-      err_sum += __shfl_xor_sync(kAll, err_sum, k);
-      err_max = mx(err_max, __shfl_xor_sync(kAll, err_max, k));
+      sums.err_sum += __shfl_xor_sync(kAll, sums.err_sum, k);
+      sums.err_max = mx(sums.err_max, __shfl_xor_sync(kAll, sums.err_max, k));
     }
     if (lane == 0 && c > 0.0f) {
       atomicAdd(Q.stats + 0, c);
-      atomicAdd(Q.stats + 1, err_sum);
-      atomicMax(reinterpret_cast<int*>(Q.stats + 2), __float_as_int(err_max));  // non-negative floats
+      atomicAdd(Q.stats + 1, sums.err_sum);
+      atomicMax(reinterpret_cast<int*>(Q.stats + 2), __float_as_int(sums.err_max));  // non-negative floats
     }
   }
 }
@@ -541,88 +646,25 @@ __global__ void __launch_bounds__(256) k_surrogate_calibrate(ImageLayout L, Surr
 // camera (the learned sky-view workload; the G-buffer is not read):
 //  * kSkyPixelsPlain: the plain integrator per pixel - the sky-view march of
 //    :1208-1302 (sv_steps warped segments) along the pixel's ray;
-//  * kSkyPixelsNet: the sky network on the tensor cores; where a gate trips
-//    (|sun cosine| at the camera below sky_twilight_cos, the view ray within
-//    limb_rad of the limb, the camera above the shell) the plain integrator;
+//  * kSkyPixelsNet: the sky network on the tensor cores (k_sky_pixels_net);
+//    where a gate trips (|sun cosine| at the camera below sky_twilight_cos,
+//    the view ray within limb_rad of the limb, the camera above the shell)
+//    the plain integrator;
 //  * kSkyPixelsLut: the reference's own path, a bilinear tap of the sky-view
 //    LUT (:1474-1525).
-// 256 threads = two 128-pixel tiles, as in k_composite_surrogate.
 enum : int { kSkyPixelsPlain = 0, kSkyPixelsNet = 1, kSkyPixelsLut = 2 };
 template <int kMode>
-__global__ void __launch_bounds__(256, 2) k_sky_pixels(DevParams P, ImageLayout L, CompositeScalars A,
-                                                       const float4* __restrict__ tlut,
-                                                       const float4* __restrict__ mslut,
-                                                       const float4* __restrict__ svlut, SurrogateNets nets,
-                                                       uint32_t* __restrict__ status, float* __restrict__ out,
-                                                       unsigned long long* counter, SurrogateQueue Q) {
-  extern __shared__ __align__(128) unsigned char smem[];  // the sky network (kSkyPixelsNet)
-  __shared__ __align__(8) uint64_t s_mbar[3];
-  __shared__ uint32_t s_tmem;
-  if (kMode == kSkyPixelsNet) {
-    if (threadIdx.x == 0) {
-      tc::mbar_init(&s_mbar[0], 1);
-      tc::mbar_init(&s_mbar[1], 1);
-      tc::mbar_init(&s_mbar[2], 1);
-      tc::mbar_init_fence();
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      tc::mbar_arrive_expect_tx(&s_mbar[2], uint32_t(nets.sky_bytes));
-      tc::bulk_g2s(smem, nets.sky, uint32_t(nets.sky_bytes), &s_mbar[2]);
-    }
-  }
+__global__ void __launch_bounds__(256, 2) k_sky_pixels(DevParams P, Frame F, ImageLayout L, CompositeScalars A,
+                                                       const float4* __restrict__ svlut, float* __restrict__ out,
+                                                       unsigned long long* counter) {
   int x, y;
-  const bool inside = tile_pixel(L, x, y);
-  const int cx = inside ? x : 0, cy = inside ? y : 0;
-  const Frame F = make_frame(P, tlut, mslut, A.bottom, A.ar, arr3(A.sun), arr3(A.E));
-  const f3 ray = pixel_ray(L, A, cx, cy).ray;
   uint32_t samples = 0;
-  f3 sky = splat(0.0f);
-  bool plain = kMode == kSkyPixelsPlain;
-  bool checked = false;
-  if (kMode == kSkyPixelsLut) sky = sample_sky_view(P, svlut, ray, F.sun, A.sky_alt, A.bottom);
-  if (kMode == kSkyPixelsNet) {
-    const bool near_limb =
-        fabsf(acosf(clampf(ray.y, -1.0f, 1.0f)) - sky_horizon_zenith(A.cam_alt, A.bottom)) < nets.limb_rad;
-    const bool net = inside && A.cam_alt <= P.top && fabsf(F.sun.y) >= nets.sky_twilight_cos && !near_limb;
-    plain = !net;
-    float fx[16] = {};
-    if (net) {
-      const float vl = sqrtf(ray.x * ray.x + ray.z * ray.z), sl = sqrtf(F.sun.x * F.sun.x + F.sun.z * F.sun.z);
-      const float cphi = (vl > 1e-6f && sl > 1e-6f) ? (ray.x * F.sun.x + ray.z * F.sun.z) / (vl * sl) : 1.0f;
-      geometry_features(P, A.bottom, A.cam_alt, ray.y, F.sun.y, cphi, fx);
-      fx[4] = nets.lhr_n;
-      fx[5] = nets.lhm_n;
-      sky_ray_features(P, A.bottom, A.cam_alt, ray, F.sun, fx);
-    }
-    const bool need = __syncthreads_or(net);
-    const bool weights_ok = __syncthreads_and(tc::mbar_wait(&s_mbar[2], 0u, kTcWaitTries));
-    bool tc_ok = weights_ok;
-    float yv[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    if (need && weights_ok) {
-      if (threadIdx.x < 32) tc::alloc(&s_tmem, kSurrogateTmemCols);
-      tc::fence_before_sync();
-      __syncthreads();
-      tc::fence_after_sync();
-      const int tile = threadIdx.x >> 7;
-      TcTile T{s_tmem + 128u * tile, s_tmem + 128u * tile + 64u, &s_mbar[tile], 0u, tile, int(threadIdx.x & 127)};
-      tc_ok = mlp_tile_tc<kSurrogateSkyHidden>(smem, kSurrogateSkyIn, T, fx, yv, nets.wait_tries);
-      tc::fence_before_sync();
-      if (!tc_ok) tc::mbar_wait(T.mbar, T.phase ^ 1u, kTcWaitTries);
-      __syncthreads();
-      tc::fence_after_sync();
-      if (threadIdx.x < 32) tc::dealloc(s_tmem, kSurrogateTmemCols);
-    }
-    if (need && !tc_ok) {
-      plain = true;  // the network's outputs are not valid: the plain integrator
-      if ((threadIdx.x & 127) == 0) atomicOr(status, 1u);
-    } else if (net) {
-      sky = net_radiance(yv, A.E, splat(nets.sky_floor));
-      checked = Q.net_mask != nullptr && check_pixel(x, y, Q.seed, Q.check_fraction);
-    }
-  }
-  if (inside) {
-    if (plain) {
+  if (tile_pixel(L, x, y)) {
+    const f3 ray = pixel_ray(L, A, x, y).ray;
+    f3 sky;
+    if (kMode == kSkyPixelsLut) {
+      sky = sample_sky_view(P, svlut, ray, F.sun, A.sky_alt, A.bottom);
+    } else {
       sky = sky_radiance(P, F, A.cam_alt, ray);
       samples = uint32_t(P.sv_steps);
     }
@@ -630,11 +672,65 @@ __global__ void __launch_bounds__(256, 2) k_sky_pixels(DevParams P, ImageLayout 
     out[o + 0] = sky.x;
     out[o + 1] = sky.y;
     out[o + 2] = sky.z;
-    if (kMode == kSkyPixelsNet && Q.net_mask != nullptr)  // the calibration: which pixels are the network's
-      Q.net_mask[storage_index(L, x, y)] = plain ? 0 : 1;
   }
-  if (kMode == kSkyPixelsNet) {  // checked network pixels to the queue (warp-aggregated)
-    const int lane = threadIdx.x & 31;
+  warp_count(samples, counter);
+}
+__global__ void __launch_bounds__(128 * kWorkers, 1) k_sky_pixels_net(DevParams P, Frame F, ImageLayout L, PixelTiles N,
+                                                                      CompositeScalars A, SurrogateNets nets,
+                                                                      uint32_t* __restrict__ status,
+                                                                      float* __restrict__ out,
+                                                                      unsigned long long* counter, SurrogateQueue Q) {
+  extern __shared__ __align__(128) unsigned char smem[];  // the sky network
+  __shared__ NetBlock B;
+  bool nets_ok;
+  TcTile T = net_block_begin(B, smem, nets.sky, nets.sky_bytes, nullptr, 0, A.cam_alt, A.bottom, nets_ok);
+  const int lane = threadIdx.x & 31;
+  uint32_t samples = 0;
+  for (int t = T.tile * gridDim.x + blockIdx.x; t < N.count; t += kWorkers * gridDim.x) {
+    int x, y;
+    const bool inside = tile_pixel_of(L, N, t, T.row, x, y);
+    const int cx = inside ? x : 0, cy = inside ? y : 0;
+    const f3 ray = pixel_ray(L, A, cx, cy).ray;
+    const bool near_limb = fabsf(acosf(clampf(ray.y, -1.0f, 1.0f)) - B.horizon) < nets.limb_rad;
+    const bool net = inside && A.cam_alt <= P.top && fabsf(F.sun.y) >= nets.sky_twilight_cos && !near_limb;
+    bool plain = !net, checked = false;
+    uint32_t xp[8] = {};
+    if (net) {
+      float fx[16] = {};
+      const float cphi = azimuth_cosine(ray.x * F.sun.x + ray.z * F.sun.z, ray.x * ray.x + ray.z * ray.z,
+                                        F.sun.x * F.sun.x + F.sun.z * F.sun.z);
+      geometry_features(P, A.bottom, A.cam_alt, ray.y, F.sun.y, cphi, fx);
+      fx[4] = nets.lhr_n;
+      fx[5] = nets.lhm_n;
+      sky_ray_features(P, A.bottom, A.cam_alt, ray, F.sun, fx);
+      pack_inputs(fx, kSurrogateSkyIn, xp);
+    }
+    const bool need = tc::tile_any(T.tile, net);
+    bool tc_ok = nets_ok;
+    float yv[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+    if (need && tc_ok) tc_ok = mlp_tile_tc<kSurrogateSkyHidden>(smem, kSurrogateSkyIn, T, xp, yv, nets.wait_tries);
+    f3 sky = splat(0.0f);
+    if (need && !tc_ok) {
+      plain = true;  // the network's outputs are not valid: the plain integrator
+      if (T.row == 0) atomicOr(status, 1u);
+      if (nets_ok) nets_ok = tile_recover(T);
+    } else if (net) {
+      sky = net_radiance(yv, A.E, splat(nets.sky_floor));
+      checked = Q.net_mask != nullptr && check_pixel(x, y, Q.seed, Q.check_fraction);
+    }
+    if (inside) {
+      if (plain) {
+        sky = sky_radiance(P, F, A.cam_alt, ray);
+        samples += uint32_t(P.sv_steps);
+      }
+      const size_t o = pix_offset(L, x, y) * L.channels;
+      out[o + 0] = sky.x;
+      out[o + 1] = sky.y;
+      out[o + 2] = sky.z;
+      if (Q.net_mask != nullptr)  // the calibration: which pixels are the network's
+        Q.net_mask[storage_index(L, x, y)] = plain ? 0 : 1;
+    }
+    // checked network pixels to the queue (warp-aggregated)
     const unsigned qm = __ballot_sync(kAll, checked);
     if (qm) {
       const int leader = __ffs(qm) - 1;
@@ -646,6 +742,7 @@ __global__ void __launch_bounds__(256, 2) k_sky_pixels(DevParams P, ImageLayout 
     }
   }
   warp_count(samples, counter);
+  net_block_end(B);
 }
 
 // The sky-pixel calibration pass: every network pixel of a tile holding
@@ -673,26 +770,25 @@ __global__ void __launch_bounds__(256) k_sky_pixels_calibrate(ImageLayout L, Sur
 
 // The sky-pixel calibration's checks: each queued network pixel gets the
 // plain march, adds its tile's log ratio of plain to network radiance, and
-// keeps the plain result.  Warps take 32 entries per ticket.
-__global__ void __launch_bounds__(256) k_sky_pixels_check(DevParams P, ImageLayout L, CompositeScalars A,
-                                                          const float4* __restrict__ tlut,
-                                                          const float4* __restrict__ mslut, SurrogateQueue Q,
-                                                          float* __restrict__ out, unsigned long long* counter) {
-  const Frame F = make_frame(P, tlut, mslut, A.bottom, A.ar, arr3(A.sun), arr3(A.E));
+// keeps the plain result.  Warps take 32 / kLanes entries per ticket.
+template <int kLanes>
+__device__ __forceinline__ uint32_t check_queue(const DevParams& P, const Frame& F, const ImageLayout& L,
+                                                const CompositeScalars& A, const SurrogateQueue& Q,
+                                                float* __restrict__ out, uint32_t n) {
   const int lane = threadIdx.x & 31;
-  const uint32_t n = *Q.count;
+  const bool first = (lane & (kLanes - 1)) == 0;
   uint32_t samples = 0;
   for (;;) {
     uint32_t base = 0;
-    if (lane == 0) base = atomicAdd(Q.count + 1, 32u);
+    if (lane == 0) base = atomicAdd(Q.count + 1, 32u / kLanes);
     base = __shfl_sync(kAll, base, 0);
     if (base >= n) break;
-    const uint32_t i = base + uint32_t(lane);
-    if (i < n) {
-      const uint32_t p = Q.items[i] & 0x3fffffffu;
-      const int x = int(p % uint32_t(L.width)), y = int(p / uint32_t(L.width));
-      const f3 ray = pixel_ray(L, A, x, y).ray;
-      const f3 sky = sky_radiance(P, F, A.cam_alt, ray);
+    const uint32_t i = base + uint32_t(lane / kLanes);
+    const bool has = i < n;
+    const uint32_t p = has ? Q.items[i] & 0x3fffffffu : 0;
+    const int x = int(p % uint32_t(L.width)), y = int(p / uint32_t(L.width));
+    const f3 sky = sky_radiance_split<kLanes>(P, F, A.cam_alt, pixel_ray(L, A, x, y).ray, has);
+    if (has && first) {
       samples += uint32_t(P.sv_steps);
       const size_t o = pix_offset(L, x, y) * L.channels;
       const f3 Ln = ld3(out + o);  // the network's radiance
@@ -707,57 +803,66 @@ __global__ void __launch_bounds__(256) k_sky_pixels_check(DevParams P, ImageLayo
       out[o + 2] = sky.z;
     }
   }
-  warp_count(samples, counter);
+  return samples;
+}
+__global__ void __launch_bounds__(256) k_sky_pixels_check(DevParams P, Frame F, ImageLayout L, CompositeScalars A,
+                                                          SurrogateQueue Q, float* __restrict__ out,
+                                                          unsigned long long* counter) {
+  const uint32_t n = *Q.count;
+  warp_count(split_queue(n) ? check_queue<kQueueLanes>(P, F, L, A, Q, out, n) : check_queue<1>(P, F, L, A, Q, out, n),
+             counter);
 }
 
 }  // namespace
 
-cudaError_t launch_sky_pixels(int mode, const DevParams& P, const ImageLayout& L, const CompositeScalars& A,
+cudaError_t launch_sky_pixels(int mode, const DevParams& P, const ImageLayout& L, const CompositeScalars& scalars,
                               const float4* tlut, const float4* mslut, const float4* svlut, const SurrogateNets& nets,
                               uint32_t* status, float* out, unsigned long long* counter, int sm_count, cudaStream_t s,
                               const SurrogateQueue* calibration) {
-  const dim3 grid((L.width + 15) / 16, (L.height + 15) / 16);
-  SurrogateQueue Q{};
-  if (mode == kSkyPixelsNet && calibration != nullptr && calibration->net_mask != nullptr) Q = *calibration;
-  if (mode == kSkyPixelsNet) {
-    cudaError_t e = cudaFuncSetAttribute(k_sky_pixels<kSkyPixelsNet>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         nets.sky_bytes);
-    if (e != cudaSuccess) return e;
-    if (Q.net_mask != nullptr) {
-      const int tiles_y = (L.height + (1 << Q.tile_shift) - 1) >> Q.tile_shift;
-      e = cudaMemsetAsync(Q.count, 0, 2 * sizeof(uint32_t), s);
-      if (e == cudaSuccess) e = cudaMemsetAsync(Q.tiles, 0, sizeof(float) * 4 * size_t(Q.tiles_x) * tiles_y, s);
-      if (e != cudaSuccess) return e;
-    }
-    k_sky_pixels<kSkyPixelsNet><<<grid, 256, nets.sky_bytes, s>>>(P, L, A, tlut, mslut, svlut, nets, status, out,
-                                                                  counter, Q);
-    e = cudaGetLastError();
-    if (e != cudaSuccess || Q.net_mask == nullptr) return e;
-    k_sky_pixels_check<<<2 * sm_count, 256, 0, s>>>(P, L, A, tlut, mslut, Q, out, counter);
-    e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-    const size_t pixels = size_t(L.width) * L.height;
-    k_sky_pixels_calibrate<<<unsigned((pixels + 255) / 256), 256, 0, s>>>(L, Q, out);
-  } else if (mode == kSkyPixelsLut) {
-    k_sky_pixels<kSkyPixelsLut><<<grid, 256, 0, s>>>(P, L, A, tlut, mslut, svlut, nets, status, out, counter, Q);
-  } else {
-    k_sky_pixels<kSkyPixelsPlain><<<grid, 256, 0, s>>>(P, L, A, tlut, mslut, svlut, nets, status, out, counter, Q);
+  const CompositeScalars A = with_image(scalars, L);
+  const Frame F = frame_of(P, A, tlut, mslut);
+  if (mode != kSkyPixelsNet) {
+    const dim3 grid((L.width + 15) / 16, (L.height + 15) / 16);
+    if (mode == kSkyPixelsLut)
+      k_sky_pixels<kSkyPixelsLut><<<grid, 256, 0, s>>>(P, F, L, A, svlut, out, counter);
+    else
+      k_sky_pixels<kSkyPixelsPlain><<<grid, 256, 0, s>>>(P, F, L, A, svlut, out, counter);
+    return cudaGetLastError();
   }
+  SurrogateQueue Q{};
+  if (calibration != nullptr && calibration->net_mask != nullptr) Q = *calibration;
+  cudaError_t e = cudaFuncSetAttribute(k_sky_pixels_net, cudaFuncAttributeMaxDynamicSharedMemorySize, nets.sky_bytes);
+  if (e != cudaSuccess) return e;
+  if (Q.net_mask != nullptr) {
+    const int tiles_y = (L.height + (1 << Q.tile_shift) - 1) >> Q.tile_shift;
+    e = cudaMemsetAsync(Q.count, 0, 2 * sizeof(uint32_t), s);
+    if (e == cudaSuccess) e = cudaMemsetAsync(Q.tiles, 0, sizeof(float) * 4 * size_t(Q.tiles_x) * tiles_y, s);
+    if (e != cudaSuccess) return e;
+  }
+  const PixelTiles N = pixel_tiles(L);
+  k_sky_pixels_net<<<std::min(sm_count, N.count), 128 * kWorkers, nets.sky_bytes, s>>>(P, F, L, N, A, nets, status, out,
+                                                                                     counter, Q);
+  e = cudaGetLastError();
+  if (e != cudaSuccess || Q.net_mask == nullptr) return e;
+  k_sky_pixels_check<<<2 * sm_count, 256, 0, s>>>(P, F, L, A, Q, out, counter);
+  e = cudaGetLastError();
+  if (e != cudaSuccess) return e;
+  const size_t pixels = size_t(L.width) * L.height;
+  k_sky_pixels_calibrate<<<unsigned((pixels + 255) / 256), 256, 0, s>>>(L, Q, out);
   return cudaGetLastError();
 }
 
 cudaError_t launch_gen_samples(const SurrogateSetDev* sets, int n_sets, int kind, long long n, unsigned long long seed,
-                               const SampleShaping& shaping, const float E[3], float ar, float* features,
-                               float* targets, unsigned long long* counter, cudaStream_t s) {
-  const f3 e3 = {E[0], E[1], E[2]};
-  k_gen_samples<<<unsigned((n + 127) / 128), 128, 0, s>>>(sets, n_sets, kind, n, seed, shaping, e3, ar, features,
-                                                         targets, counter);
+                               const SampleShaping& shaping, float* features, float* targets,
+                               unsigned long long* counter, cudaStream_t s) {
+  k_gen_samples<<<unsigned((n + 127) / 128), 128, 0, s>>>(sets, n_sets, kind, n, seed, shaping, features, targets,
+                                                         counter);
   return cudaGetLastError();
 }
 
 size_t surrogate_smem_bytes(const SurrogateNets& nets) { return size_t(nets.ap_bytes) + size_t(nets.sky_bytes); }
 
-cudaError_t launch_composite_surrogate(const DevParams& P, const ImageLayout& L, const CompositeScalars& A,
+cudaError_t launch_composite_surrogate(const DevParams& P, const ImageLayout& L, const CompositeScalars& scalars,
                                        const float* scene, const float* space, const int32_t* sid, const float* pos,
                                        const float4* tlut, const float4* mslut, const float4* svlut,
                                        const SurrogateNets& nets, const SurrogateQueue& Q, float* hdr,
@@ -770,28 +875,29 @@ cudaError_t launch_composite_surrogate(const DevParams& P, const ImageLayout& L,
     e = cudaMemsetAsync(Q.tiles, 0, sizeof(float) * 4 * size_t(Q.tiles_x) * tiles_y, s);
     if (e != cudaSuccess) return e;
   }
+  const CompositeScalars A = with_image(scalars, L);
+  const Frame F = frame_of(P, A, tlut, mslut);
   const int smem = int(surrogate_smem_bytes(nets));
-  const dim3 grid((L.width + 15) / 16, (L.height + 15) / 16);
+  const PixelTiles N = pixel_tiles(L);
+  const int grid = std::min(sm_count, N.count);
   const ShadeParams S = shade ? *shade : ShadeParams{};
   const ShadeImages I = shade_images ? *shade_images : ShadeImages{};
   if (shade) {
     e = cudaFuncSetAttribute(k_composite_surrogate<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return e;
-    k_composite_surrogate<true><<<grid, 256, smem, s>>>(P, L, A, scene, space, sid, pos, tlut, mslut, svlut, nets, Q,
+    k_composite_surrogate<true><<<grid, 128 * kWorkers, smem, s>>>(P, F, L, N, A, scene, space, sid, pos, svlut, nets, Q,
                                                         hdr, S, I);
     e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    k_surrogate_fallback<true><<<2 * sm_count, 256, 0, s>>>(P, L, A, scene, space, pos, tlut, mslut, Q, hdr, counter,
-                                                            S, I);
+    k_surrogate_fallback<true><<<2 * sm_count, 256, 0, s>>>(P, F, L, A, scene, space, pos, Q, hdr, counter, S, I);
   } else {
     e = cudaFuncSetAttribute(k_composite_surrogate<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return e;
-    k_composite_surrogate<false><<<grid, 256, smem, s>>>(P, L, A, scene, space, sid, pos, tlut, mslut, svlut, nets,
+    k_composite_surrogate<false><<<grid, 128 * kWorkers, smem, s>>>(P, F, L, N, A, scene, space, sid, pos, svlut, nets,
                                                          Q, hdr, S, I);
     e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    k_surrogate_fallback<false><<<2 * sm_count, 256, 0, s>>>(P, L, A, scene, space, pos, tlut, mslut, Q, hdr,
-                                                             counter, S, I);
+    k_surrogate_fallback<false><<<2 * sm_count, 256, 0, s>>>(P, F, L, A, scene, space, pos, Q, hdr, counter, S, I);
   }
   e = cudaGetLastError();
   if (e != cudaSuccess || Q.lm == nullptr) return e;

@@ -145,8 +145,21 @@ __device__ __forceinline__ void tile_sync(int tile) {
 // tile must take one path afterwards (its barriers stay matched).
 __device__ __forceinline__ bool tile_all(int tile, bool v) {
   uint32_t r;
+  __syncwarp();  // the barrier takes whole warps
   asm volatile(
       "{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %1, 0;\n\tbar.red.and.pred q, %2, 128, p;\n\t"
+      "selp.u32 %0, 1, 0, q;\n\t}"
+      : "=r"(r)
+      : "r"(uint32_t(v)), "r"(tile + 1)
+      : "memory");
+  return r != 0;
+}
+// The same barrier, returning whether v holds in any thread of the tile.
+__device__ __forceinline__ bool tile_any(int tile, bool v) {
+  uint32_t r;
+  __syncwarp();
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %1, 0;\n\tbar.red.or.pred q, %2, 128, p;\n\t"
       "selp.u32 %0, 1, 0, q;\n\t}"
       : "=r"(r)
       : "r"(uint32_t(v)), "r"(tile + 1)
