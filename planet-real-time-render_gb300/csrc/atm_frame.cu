@@ -14,6 +14,7 @@
 #include <cuda_runtime.h>
 
 #include <mutex>
+#include <type_traits>
 
 #include "atm_device.cuh"
 #include "atm_frame_paths.cuh"
@@ -240,6 +241,29 @@ inline f3 host3(const float* v) { return {v[0], v[1], v[2]}; }
 
 inline dim3 tile_grid(const ImageLayout& L) { return dim3((L.width + 15) / 16, (L.height + 15) / 16); }
 
+// Lanes a pixel: the most that keep a frame's threads within the chip's
+// resident ones (three blocks of 256 an SM).  A pixel's march is a serial
+// chain of 48 and more samples; a frame that leaves warps free runs it on
+// several lanes, a larger one would only repeat each pixel's set-up.  A 96x54
+// composite takes 15-17 us on 16 lanes a pixel, 38-53 us on one.
+constexpr long long kResidentThreads = 152LL * 3 * 256;
+template <class Launch>
+inline cudaError_t launch_split(const ImageLayout& L, Launch launch) {
+  const long long pixels = (long long)L.width * L.height;
+  const auto grid = [&](int lanes) { return dim3((L.width + 7) / 8, (L.height * lanes + 31) / 32); };
+  if (16 * pixels <= kResidentThreads)
+    launch(std::integral_constant<int, 16>{}, grid(16));
+  else if (8 * pixels <= kResidentThreads)
+    launch(std::integral_constant<int, 8>{}, grid(8));
+  else if (4 * pixels <= kResidentThreads)
+    launch(std::integral_constant<int, 4>{}, grid(4));
+  else if (2 * pixels <= kResidentThreads)
+    launch(std::integral_constant<int, 2>{}, grid(2));
+  else
+    launch(std::integral_constant<int, 1>{}, tile_grid(L));
+  return cudaGetLastError();
+}
+
 }  // namespace
 
 cudaError_t launch_prepare_surface(const DevParams& P, const ImageLayout& L, const float* pos, const int32_t* sid,
@@ -257,8 +281,9 @@ cudaError_t launch_frame(const DevParams& P, const ImageLayout& L, const Composi
                          const ShadeImages& I, const float* space, const float4* tlut, const float4* mslut,
                          const float4* svlut, float* hdr, unsigned long long* sample_counter, cudaStream_t s) {
   const Frame F = frame_of(P, A, tlut, mslut);
-  k_frame<1><<<tile_grid(L), 256, 0, s>>>(P, F, L, with_image(A, L), S, I, space, svlut, hdr, sample_counter);
-  return cudaGetLastError();
+  return launch_split(L, [&](auto lanes, dim3 grid) {
+    k_frame<lanes.value><<<grid, 256, 0, s>>>(P, F, L, with_image(A, L), S, I, space, svlut, hdr, sample_counter);
+  });
 }
 
 cudaError_t launch_composite(const DevParams& P, const ImageLayout& L, const CompositeScalars& A,
@@ -267,10 +292,11 @@ cudaError_t launch_composite(const DevParams& P, const ImageLayout& L, const Com
                              float* hdr, unsigned long long* sample_counter, cudaStream_t s) {
   const Frame F = frame_of(P, A, tlut, mslut);
   if (A.view == ATM_VIEW_COMPOSITE)
-    k_composite<1><<<tile_grid(L), 256, 0, s>>>(P, F, L, with_image(A, L), scene, space, sid, pos, svlut, hdr,
-                                                sample_counter);
-  else
-    k_composite_views<<<tile_grid(L), 256, 0, s>>>(P, F, L, with_image(A, L), scene, space, sid, pos, svlut, aplut, hdr,
+    return launch_split(L, [&](auto lanes, dim3 grid) {
+      k_composite<lanes.value><<<grid, 256, 0, s>>>(P, F, L, with_image(A, L), scene, space, sid, pos, svlut, hdr,
+                                                    sample_counter);
+    });
+  k_composite_views<<<tile_grid(L), 256, 0, s>>>(P, F, L, with_image(A, L), scene, space, sid, pos, svlut, aplut, hdr,
                                                  sample_counter);
   return cudaGetLastError();
 }
