@@ -20,6 +20,24 @@ struct ImageLayout {
   int32_t channels;
 };
 
+// Memory-bound per-pixel kernels: blocks of 32 pixels along the image's
+// contiguous axis by 8 across it, a warp a run of 32.  No index is divided:
+// a flat 64-bit pixel index costs its kernel two long divisions a pixel.
+constexpr int kRunPixels = 32, kRunRows = 8;
+inline dim3 run_block() { return dim3(kRunPixels, kRunRows); }
+inline dim3 run_grid(const ImageLayout& L) {
+  const bool y_fast = L.sy <= L.sx;
+  const int fast = y_fast ? L.height : L.width, slow = y_fast ? L.width : L.height;
+  return dim3((fast + kRunPixels - 1) / kRunPixels, (slow + kRunRows - 1) / kRunRows);
+}
+__device__ __forceinline__ bool run_pixel(const ImageLayout& L, int& x, int& y) {
+  const int fast = blockIdx.x * kRunPixels + threadIdx.x, slow = blockIdx.y * kRunRows + threadIdx.y;
+  const bool y_fast = L.sy <= L.sx;  // the reference's (W, H, 3) layout
+  x = y_fast ? slow : fast;
+  y = y_fast ? fast : slow;
+  return x < L.width && y < L.height;
+}
+
 struct CompositeScalars {
   float bottom, cam_alt, sky_alt, ar, tanfov, star_start, star_end;
   float sun[3], E[3], disk[3], right[3], up[3], fwd[3];
@@ -342,6 +360,7 @@ struct OceanFrame {
   float offsets[kOceanCascades][2];
   float variances[kOceanCascades];
   int geometry_cascades, enabled, debug_mode;
+  float aspect, inv_tf;  // set by the launch: width / height, 1 / tf
 };
 // The G-buffer images it reads and overwrites, at the layout's element
 // strides: position, normal, albedo, seabed albedo and normal with

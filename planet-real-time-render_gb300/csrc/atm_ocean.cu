@@ -90,26 +90,61 @@ __global__ void __launch_bounds__(256) k_ocean_spectrum(OceanSpectrum S, float t
 
 __device__ __forceinline__ float lerp_ref(float a, float b, float f) { return add(mul(a, sub(1.0f, f)), mul(b, f)); }
 
-// _sample_spectrum_texture :383-425: periodic bilinear taps of one cascade.
+// The wind's cosine and sine, formed once a block: the cascades' sampling axes
+// are the global ones rotated by it (_cascade_axes :364-381).  Each axis has
+// one component that is 0: a dot product with it takes the other two.
+struct OceanAxes {
+  float cw, sw;
+};
+// rdot(v, au) and rdot(v, av) of cascade kC
+template <int kC>
+__device__ __forceinline__ void axis_dots(r3 v, OceanAxes A, float& u, float& w) {
+  if (kC == 0) {  // au = (cw, 0, sw), av = (-sw, 0, cw)
+    u = add(mul(v.x, A.cw), mul(v.z, A.sw));
+    w = add(mul(v.x, -A.sw), mul(v.z, A.cw));
+  } else if (kC == 1) {  // au = (sw, cw, 0), av = (cw, -sw, 0)
+    u = add(mul(v.x, A.sw), mul(v.y, A.cw));
+    w = add(mul(v.x, A.cw), mul(v.y, -A.sw));
+  } else {  // au = (0, sw, cw), av = (0, cw, -sw)
+    u = add(mul(v.y, A.sw), mul(v.z, A.cw));
+    w = add(mul(v.y, A.cw), mul(v.z, -A.sw));
+  }
+}
+template <int kC>
+__device__ __forceinline__ void cascade_axes(OceanAxes A, r3& au, r3& av) {
+  au = kC == 0 ? R3(A.cw, 0.0f, A.sw) : kC == 1 ? R3(A.sw, A.cw, 0.0f) : R3(0.0f, A.sw, A.cw);
+  av = kC == 0 ? R3(-A.sw, 0.0f, A.cw) : kC == 1 ? R3(A.cw, -A.sw, 0.0f) : R3(0.0f, A.cw, -A.sw);
+}
+__device__ constexpr float period_of(int c) { return c == 0 ? 2048.0f : c == 1 ? 256.0f : 32.0f; }
+
+// _sample_spectrum_texture :383-425: periodic bilinear taps of one cascade of
+// 2^kLog2N texels a side.  The size and the periods are powers of two, so the
+// scalings are exact, the wrap is a mask and nothing is divided: integer
+// remainders by a run-time size were most of this kernel (4K G-buffer over a
+// coast, 128 texels: 1016 us with them and flat pixel indices, 498 us without;
+// bound by issue, 1700 instructions a warp).  kTapMagic adds an integer below 2^22 into the low mantissa
+// bits; the mask keeps every index in range whatever the input.
 struct Taps {
   int i00, i10, i01, i11;
   float fx, fy;
 };
-__device__ __forceinline__ Taps spectrum_taps(int n, int cascade, float u, float v) {
+constexpr float kTapMagic = 12582912.0f;  // 1.5 x 2^23
+template <int kLog2N, int kC>
+__device__ __forceinline__ Taps spectrum_taps(float u, float v) {
+  constexpr int kN = 1 << kLog2N, kMask = kN - 1, kBase = kC << (2 * kLog2N);
   const float wu = sub(u, floorf(u)), wv = sub(v, floorf(v));
-  const float tu = sub(mul(wu, float(n)), 0.5f), tv = sub(mul(wv, float(n)), 0.5f);
+  const float tu = fmaf(wu, float(kN), -0.5f), tv = fmaf(wv, float(kN), -0.5f);  // the products are exact
   const float bu = floorf(tu), bv = floorf(tv);
-  const int bx = int(bu), by = int(bv);  // NaN converts to 0; the wrap keeps every index in range
   Taps t;
-  t.fx = sub(tu, float(bx));
-  t.fy = sub(tv, float(by));
-  const int x0 = ((bx % n) + n) % n, y0 = ((by % n) + n) % n;
-  const int x1 = (x0 + 1) % n, y1 = (y0 + 1) % n;
-  const int base = cascade * n * n;
-  t.i00 = base + x0 * n + y0;
-  t.i10 = base + x1 * n + y0;
-  t.i01 = base + x0 * n + y1;
-  t.i11 = base + x1 * n + y1;
+  t.fx = sub(tu, bu);
+  t.fy = sub(tv, bv);
+  const int bx = __float_as_int(add(bu, kTapMagic)), by = __float_as_int(add(bv, kTapMagic));
+  const int x0 = (bx & kMask) << kLog2N, x1 = ((bx + 1) & kMask) << kLog2N;
+  const int y0 = (by & kMask) + kBase, y1 = ((by + 1) & kMask) + kBase;
+  t.i00 = x0 + y0;
+  t.i10 = x1 + y0;
+  t.i01 = x0 + y1;
+  t.i11 = x1 + y1;
   return t;
 }
 __device__ __forceinline__ float2 taps_disp(const OceanSpectrum& S, const Taps& t) {
@@ -126,70 +161,69 @@ __device__ __forceinline__ float4 lerp4(const float4* p, const Taps& t) {
                      lerp_ref(lerp_ref(a.w, b.w, t.fx), lerp_ref(c.w, d.w, t.fx), t.fy));
 }
 
-// _cascade_axes :364-381 (global sampling axes rotated by the wind)
-__device__ __forceinline__ void cascade_axes(int c, float cw, float sw, r3& au, r3& av) {
-  const r3 bu = c == 0 ? R3(1.0f, 0.0f, 0.0f) : (c == 1 ? R3(0.0f, 1.0f, 0.0f) : R3(0.0f, 0.0f, 1.0f));
-  const r3 bv = c == 0 ? R3(0.0f, 0.0f, 1.0f) : (c == 1 ? R3(1.0f, 0.0f, 0.0f) : R3(0.0f, 1.0f, 0.0f));
-  au = radd(rscale(bu, cw), rscale(bv, sw));
-  av = radd(rscale(R3(-bu.x, -bu.y, -bu.z), sw), rscale(bv, cw));
-}
-
-// The undisturbed coordinate of cascade c under the displaced point: the
+// The undisturbed coordinate of cascade kC under the displaced point: the
 // Gerstner map inverted by two fixed-point steps (:448-468).
-__device__ __forceinline__ Taps inverted_taps(const OceanSpectrum& S, const OceanFrame& F, int c, r3 goff, r3 au,
-                                              r3 av) {
-  const float period = kPeriods[c];
-  const float bu = add(F.offsets[c][0], dv(rdot(goff, au), period));
-  const float bv = add(F.offsets[c][1], dv(rdot(goff, av), period));
+template <int kLog2N, int kC>
+__device__ __forceinline__ Taps inverted_taps(const OceanSpectrum& S, const OceanFrame& F, r3 goff, OceanAxes A) {
+  constexpr float kInv = 1.0f / period_of(kC);  // exact
+  float du, dw;
+  axis_dots<kC>(goff, A, du, dw);
+  const float bu = add(F.offsets[kC][0], mul(du, kInv));
+  const float bv = add(F.offsets[kC][1], mul(dw, kInv));
   float u = bu, v = bv;
 #pragma unroll
   for (int it = 0; it < 2; ++it) {
-    const float2 d = taps_disp(S, spectrum_taps(S.n, c, u, v));
-    u = sub(bu, dv(d.x, period));
-    v = sub(bv, dv(d.y, period));
+    const float2 d = taps_disp(S, spectrum_taps<kLog2N, kC>(u, v));
+    u = sub(bu, mul(d.x, kInv));
+    v = sub(bv, mul(d.y, kInv));
   }
-  return spectrum_taps(S.n, c, u, v);
+  return spectrum_taps<kLog2N, kC>(u, v);
 }
 
 // _sample_spectrum(geometry_only=True): summed height of the geometry cascades
-__device__ float wave_height(const OceanSpectrum& S, const OceanFrame& F, r3 goff, float cw, float sw) {
+template <int kLog2N>
+__device__ float wave_height(const OceanSpectrum& S, const OceanFrame& F, r3 goff, OceanAxes A) {
   float height = 0.0f;
-  for (int c = 0; c < kOceanCascades; ++c) {
-    if (c >= F.geometry_cascades) break;
-    r3 au, av;
-    cascade_axes(c, cw, sw, au, av);
-    const Taps t = inverted_taps(S, F, c, goff, au, av);
-    height = add(height, lerp4(S.height_gradient, t).x);
-  }
+  if (F.geometry_cascades > 0) height = add(height, lerp4(S.height_gradient, inverted_taps<kLog2N, 0>(S, F, goff, A)).x);
+  if (F.geometry_cascades > 1) height = add(height, lerp4(S.height_gradient, inverted_taps<kLog2N, 1>(S, F, goff, A)).x);
+  if (F.geometry_cascades > 2) height = add(height, lerp4(S.height_gradient, inverted_taps<kLog2N, 2>(S, F, goff, A)).x);
   return height;
 }
 
-// _sample_spectrum(geometry_only=False): the footprint-resolved slope and the
-// unresolved slope variance of all cascades
-__device__ void wave_slope(const OceanSpectrum& S, const OceanFrame& F, r3 goff, r3 radial, float footprint, float cw,
-                           float sw, r3& slope, float& unresolved) {
+// _sample_spectrum(geometry_only=False): one cascade's part of the
+// footprint-resolved slope and of the unresolved slope variance
+template <int kLog2N, int kC>
+__device__ __forceinline__ void cascade_slope(const OceanSpectrum& S, const OceanFrame& F, r3 goff, r3 radial,
+                                              float footprint, OceanAxes A, r3& slope, float& unresolved) {
+  r3 au, av;
+  cascade_axes<kC>(A, au, av);
+  const Taps t = inverted_taps<kLog2N, kC>(S, F, goff, A);
+  const float4 hg = lerp4(S.height_gradient, t);
+  const float4 j = lerp4(S.jacobian, t);
+  constexpr float kMinWavelength = period_of(kC) / 5.5f;
+  const float spw = dv(kMinWavelength, fmx(footprint, 0.01f));
+  float resolved = fmn(fmx(mul(sub(spw, 2.0f), 0.25f), 0.0f), 1.0f);
+  resolved = mul(mul(resolved, resolved), sub(3.0f, mul(2.0f, resolved)));
+  const float m00 = add(1.0f, j.x), m01 = j.y, m10 = j.z, m11 = add(1.0f, j.w);
+  const float det = sub(mul(m00, m11), mul(m01, m10));
+  const float safe = fabsf(det) < 0.15f ? (det >= 0.0f ? 0.15f : -0.15f) : det;
+  const float mg0 = dv(sub(mul(m11, hg.y), mul(m10, hg.z)), safe);
+  const float mg1 = dv(add(mul(-m01, hg.y), mul(m00, hg.z)), safe);
+  float ru, rw;
+  axis_dots<kC>(radial, A, ru, rw);
+  const r3 tu = rsub(au, rscale(radial, ru));
+  const r3 tv = rsub(av, rscale(radial, rw));
+  slope = radd(slope, rscale(radd(rscale(tu, mg0), rscale(tv, mg1)), resolved));
+  unresolved = add(unresolved, mul(F.variances[kC], sub(1.0f, mul(resolved, resolved))));
+}
+template <int kLog2N>
+__device__ void wave_slope(const OceanSpectrum& S, const OceanFrame& F, r3 goff, r3 radial, float footprint,
+                           OceanAxes A, r3& slope, float& unresolved) {
   slope = R3(0.0f, 0.0f, 0.0f);
   unresolved = 0.0f;
-  for (int c = 0; c < kOceanCascades; ++c) {
-    r3 au, av;
-    cascade_axes(c, cw, sw, au, av);
-    const Taps t = inverted_taps(S, F, c, goff, au, av);
-    const float4 hg = lerp4(S.height_gradient, t);
-    const float4 j = lerp4(S.jacobian, t);
-    const float min_wavelength = dv(kPeriods[c], 5.5f);
-    const float spw = dv(min_wavelength, fmx(footprint, 0.01f));
-    float resolved = fmn(fmx(dv(sub(spw, 2.0f), 4.0f), 0.0f), 1.0f);
-    resolved = mul(mul(resolved, resolved), sub(3.0f, mul(2.0f, resolved)));
-    const float m00 = add(1.0f, j.x), m01 = j.y, m10 = j.z, m11 = add(1.0f, j.w);
-    const float det = sub(mul(m00, m11), mul(m01, m10));
-    const float safe = fabsf(det) < 0.15f ? (det >= 0.0f ? 0.15f : -0.15f) : det;
-    const float mg0 = dv(sub(mul(m11, hg.y), mul(m10, hg.z)), safe);
-    const float mg1 = dv(add(mul(-m01, hg.y), mul(m00, hg.z)), safe);
-    const r3 tu = rsub(au, rscale(radial, rdot(radial, au)));
-    const r3 tv = rsub(av, rscale(radial, rdot(radial, av)));
-    slope = radd(slope, rscale(radd(rscale(tu, mg0), rscale(tv, mg1)), resolved));
-    unresolved = add(unresolved, mul(F.variances[c], sub(1.0f, mul(resolved, resolved))));
-  }
+  cascade_slope<kLog2N, 0>(S, F, goff, radial, footprint, A, slope, unresolved);
+  cascade_slope<kLog2N, 1>(S, F, goff, radial, footprint, A, slope, unresolved);
+  cascade_slope<kLog2N, 2>(S, F, goff, radial, footprint, A, slope, unresolved);
 }
 
 // _near_sphere_distance :339-362
@@ -226,24 +260,19 @@ __device__ __forceinline__ void st3(float* p, r3 v) {
 }
 
 // _rasterize :517-684
+template <int kLog2N>
 __global__ void __launch_bounds__(256) k_ocean_coverage(OceanSpectrum S, OceanFrame F, ImageLayout L,
                                                         OceanImages G) {
-  const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (i >= (long long)L.width * L.height) return;
+  __shared__ OceanAxes s_axes;
+  if (threadIdx.x == 0 && threadIdx.y == 0) s_axes = {cosf(F.wind), sinf(F.wind)};
+  __syncthreads();
   int x, y;
-  if (L.sy <= L.sx) {
-    x = int(i / L.height);
-    y = int(i % L.height);
-  } else {
-    y = int(i / L.width);
-    x = int(i % L.width);
-  }
+  if (!run_pixel(L, x, y)) return;
   const r3 east = R3(F.east[0], F.east[1], F.east[2]), up = R3(F.up[0], F.up[1], F.up[2]),
            north = R3(F.north[0], F.north[1], F.north[2]);
-  const float aspect = dv(float(L.width), float(L.height));
   const float su = dv(add(float(x), 0.5f), float(L.width)), sv = dv(add(float(y), 0.5f), float(L.height));
-  const float sx = mul(sub(mul(su, 2.0f), 1.0f), aspect), sy = sub(mul(sv, 2.0f), 1.0f);
-  const r3 ray_view = rnormalized(R3(sx, sy, dv(1.0f, F.tf)));
+  const float sx = mul(sub(mul(su, 2.0f), 1.0f), F.aspect), sy = sub(mul(sv, 2.0f), 1.0f);
+  const r3 ray_view = rnormalized(R3(sx, sy, F.inv_tf));
   const r3 ray_local = radd(radd(rscale(R3(F.right[0], F.right[1], F.right[2]), ray_view.x),
                                  rscale(R3(F.vup[0], F.vup[1], F.vup[2]), ray_view.y)),
                             rscale(R3(F.fwd[0], F.fwd[1], F.fwd[2]), ray_view.z));
@@ -252,7 +281,7 @@ __global__ void __launch_bounds__(256) k_ocean_coverage(OceanSpectrum S, OceanFr
   if (distance <= 0.1f && F.max_displacement > 0.0f && alt > F.max_displacement)
     distance = near_sphere_distance(sub(alt, F.max_displacement), ray_local.y, add(R, F.max_displacement));
   const r3 origin = R3(0.0f, add(R, alt), 0.0f);
-  const float cw = cosf(F.wind), sw = sinf(F.wind);
+  const OceanAxes A = s_axes;
   auto to_global = [&](r3 v) { return radd(radd(rscale(east, v.x), rscale(up, v.y)), rscale(north, v.z)); };
   auto offset_global = [&](r3 v) {
     return radd(radd(rscale(east, v.x), rscale(up, sub(v.y, R))), rscale(north, v.z));
@@ -260,7 +289,7 @@ __global__ void __launch_bounds__(256) k_ocean_coverage(OceanSpectrum S, OceanFr
   if (distance > 0.1f && distance <= F.geometry_max_distance) {
     for (int it = 0; it < 3; ++it) {
       const r3 cand = radd(origin, rscale(ray_local, distance));
-      const float h = wave_height(S, F, offset_global(cand), cw, sw);
+      const float h = wave_height<kLog2N>(S, F, offset_global(cand), A);
       const float displaced = near_sphere_distance(sub(alt, h), ray_local.y, add(R, h));
       if (displaced > 0.1f) distance = displaced;
     }
@@ -289,7 +318,7 @@ __global__ void __launch_bounds__(256) k_ocean_coverage(OceanSpectrum S, OceanFr
   const float footprint = dv(mul(mul(distance, 2.0f), F.tf), float(L.height));
   r3 slope = R3(0.0f, 0.0f, 0.0f);
   float unresolved = 0.0f;
-  if (F.enabled) wave_slope(S, F, offset_global(ocean_local), radial_global, footprint, cw, sw, slope, unresolved);
+  if (F.enabled) wave_slope<kLog2N>(S, F, offset_global(ocean_local), radial_global, footprint, A, slope, unresolved);
   const r3 water_normal = rnormalized(rsub(radial_global, rscale(slope, F.normal_strength)));
   r3 color = R3(F.albedo[0], F.albedo[1], F.albedo[2]);
   if (F.debug_mode == 1)
@@ -321,10 +350,19 @@ cudaError_t launch_ocean_spectrum(const OceanSpectrum& S, float time_s, float am
   return cudaGetLastError();
 }
 
-cudaError_t launch_ocean_coverage(const OceanSpectrum& S, const OceanFrame& F, const ImageLayout& L,
+cudaError_t launch_ocean_coverage(const OceanSpectrum& S, const OceanFrame& frame, const ImageLayout& L,
                                   const OceanImages& G, cudaStream_t s) {
-  const long long pixels = (long long)L.width * L.height;
-  k_ocean_coverage<<<unsigned((pixels + 255) / 256), 256, 0, s>>>(S, F, L, G);
+  OceanFrame F = frame;
+  F.aspect = float(L.width) / float(L.height);
+  F.inv_tf = 1.0f / F.tf;
+  const dim3 grid = run_grid(L), block = run_block();
+  switch (S.n) {
+    case 32: k_ocean_coverage<5><<<grid, block, 0, s>>>(S, F, L, G); break;
+    case 64: k_ocean_coverage<6><<<grid, block, 0, s>>>(S, F, L, G); break;
+    case 128: k_ocean_coverage<7><<<grid, block, 0, s>>>(S, F, L, G); break;
+    case 256: k_ocean_coverage<8><<<grid, block, 0, s>>>(S, F, L, G); break;
+    default: return cudaErrorInvalidValue;
+  }
   return cudaGetLastError();
 }
 
