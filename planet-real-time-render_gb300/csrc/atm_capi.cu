@@ -844,10 +844,12 @@ ATM_API int atm_mlp_reset_optimizer(AtmMlp* m, void* stream) {
 }
 
 namespace {
-int mlp_gradient(AtmMlp* m, const float* inputs, const float* targets, const float* weights, int64_t n,
-                 float* loss_out, cudaStream_t s) {
+// The batch's partial gradients and losses into the network's workspace;
+// `rows` receives their count.
+int mlp_partials(AtmMlp* m, const float* inputs, const float* targets, const float* weights, int64_t n, int* rows,
+                 cudaStream_t s) {
   if (!m || !inputs || !targets || n < 1) return fail(ATM_E_INVALID, "invalid MLP gradient arguments");
-  const size_t ctas = size_t(atm::mlp_train_ctas(n));
+  const size_t ctas = size_t(atm::mlp_train_ctas(n, m->sm_count));
   const size_t need = ctas * size_t(m->shape.n_params);
   if (m->partial_floats < need) {
     if (m->partial) cudaFree(m->partial);
@@ -864,11 +866,9 @@ int mlp_gradient(AtmMlp* m, const float* inputs, const float* targets, const flo
     m->loss_floats = ctas;
   }
   ATM_CUDA(atm::launch_mlp_grad(m->shape, m->params, inputs, targets, weights, n, m->partial, m->loss_partial,
-                                m->grad, s),
+                                m->sm_count, s),
            "MLP forward/backward");
-  if (loss_out) {
-    ATM_CUDA(atm::launch_reduce_partials(m->loss_partial, int(ctas), 1, loss_out, s), "loss reduction");
-  }
+  *rows = int(ctas);
   return ATM_OK;
 }
 }  // namespace
@@ -876,12 +876,12 @@ int mlp_gradient(AtmMlp* m, const float* inputs, const float* targets, const flo
 ATM_API int atm_mlp_gradient(AtmMlp* m, const float* inputs, const float* targets, const float* weights, int64_t n,
                              float* grad_out, float* loss_out, void* stream) {
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  int rc = mlp_gradient(m, inputs, targets, weights, n, loss_out, s);
+  int rows = 0;
+  int rc = mlp_partials(m, inputs, targets, weights, n, &rows, s);
   if (rc) return rc;
-  if (grad_out)
-    ATM_CUDA(cudaMemcpyAsync(grad_out, m->grad, size_t(m->shape.n_params) * sizeof(float), cudaMemcpyDeviceToDevice,
-                             s),
-             "gradient copy");
+  ATM_CUDA(atm::launch_mlp_reduce(m->shape, m->partial, rows, grad_out ? grad_out : m->grad, m->loss_partial, loss_out,
+                                  s),
+           "gradient reduction");
   return ATM_OK;
 }
 
@@ -890,11 +890,13 @@ ATM_API int atm_mlp_train_step(AtmMlp* m, const float* inputs, const float* targ
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   if (!(lr > 0.0f) || !(beta1 >= 0.0f && beta1 < 1.0f) || !(beta2 >= 0.0f && beta2 < 1.0f) || !(eps > 0.0f))
     return fail(ATM_E_INVALID, "invalid Adam hyper-parameters");
-  int rc = mlp_gradient(m, inputs, targets, weights, n, loss_out, s);
+  int rows = 0;
+  int rc = mlp_partials(m, inputs, targets, weights, n, &rows, s);
   if (rc) return rc;
   m->step += 1;
   m->packed_current = false;
-  ATM_CUDA(atm::launch_adam(m->params, m->grad, m->m1, m->m2, m->shape.n_params, lr, beta1, beta2, eps, m->step, s),
+  ATM_CUDA(atm::launch_mlp_adam(m->shape, m->partial, rows, m->grad, m->loss_partial, loss_out, m->params, m->m1,
+                                m->m2, lr, beta1, beta2, eps, m->step, s),
            "Adam update");
   return ATM_OK;
 }
@@ -914,7 +916,7 @@ ATM_API int atm_mlp_forward(const AtmMlp* m, const float* inputs, float* outputs
   if (!m || !inputs || !outputs || n < 1) return fail(ATM_E_INVALID, "invalid MLP forward arguments");
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   if (precision == 0)
-    ATM_CUDA(atm::launch_mlp_forward_f32(m->shape, m->params, inputs, outputs, n, s), "MLP forward (FP32)");
+    ATM_CUDA(atm::launch_mlp_forward_f32(m->shape, m->params, inputs, outputs, n, m->sm_count, s), "MLP forward (FP32)");
   else if (precision == 1)
     ATM_CUDA(atm::launch_mlp_forward_bf16(m->shape, m->packed, inputs, outputs, n, m->sm_count, s),
              "MLP forward (BF16 tensor cores)");

@@ -95,18 +95,22 @@ struct MlpShape {
   int in_dim[kMaxMlpLayers], out_dim[kMaxMlpLayers], off_w[kMaxMlpLayers], off_b[kMaxMlpLayers];
 };
 MlpShape make_mlp_shape(int n_in, int n_hidden, int n_out);
-int mlp_train_ctas(long long n);
-size_t mlp_train_smem_bytes(const MlpShape& m);
 size_t mlp_bf16_bytes(const MlpShape& m);
-// weights: per (sample, output) factors of the squared error, or null
+// A gradient: launch_mlp_grad writes mlp_train_ctas rows of partial gradients
+// and losses, then launch_mlp_reduce sums them, or launch_mlp_adam sums them
+// and takes the optimiser's step.  weights: per (sample, output) factors of
+// the squared error, or null; loss: null or the summed squared error.
+int mlp_train_ctas(long long n, int sm_count);
 cudaError_t launch_mlp_grad(const MlpShape& m, const float* params, const float* inputs, const float* targets,
-                            const float* weights, long long n, float* grad_partial, float* loss_partial, float* grad,
+                            const float* weights, long long n, float* grad_partial, float* loss_partial, int sm_count,
                             cudaStream_t s);
-cudaError_t launch_reduce_partials(const float* partial, int rows, int cols, float* out, cudaStream_t s);
-cudaError_t launch_adam(float* params, const float* grad, float* m1, float* m2, int n, float lr, float b1, float b2,
-                        float eps, long long step, cudaStream_t s);
+cudaError_t launch_mlp_reduce(const MlpShape& m, const float* grad_partial, int rows, float* grad,
+                              const float* loss_partial, float* loss, cudaStream_t s);
+cudaError_t launch_mlp_adam(const MlpShape& m, const float* grad_partial, int rows, float* grad,
+                            const float* loss_partial, float* loss, float* params, float* m1, float* m2, float lr,
+                            float b1, float b2, float eps, long long step, cudaStream_t s);
 cudaError_t launch_mlp_forward_f32(const MlpShape& m, const float* params, const float* inputs, float* outputs,
-                                   long long n, cudaStream_t s);
+                                   long long n, int sm_count, cudaStream_t s);
 cudaError_t launch_mlp_pack_bf16(const MlpShape& m, const float* params, void* packed, cudaStream_t s);
 // tcgen05 path: packed layout of atm_mlp_tc.cuh; *error set if an MMA timed out
 size_t mlp_tc_bytes(const MlpShape& m);

@@ -12,6 +12,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstdint>
+#include <type_traits>
 
 #include "atm_kernels.h"
 #include "atm_mlp_tc.cuh"
@@ -21,223 +22,320 @@ namespace atm {
 
 namespace {
 
-constexpr int kH = 64;          // hidden width
-constexpr int kS = 64;          // samples per training CTA
+constexpr int kH = 64;        // hidden width
+constexpr int kS = 64;        // samples of a tile
 constexpr int kThreads = 256;
-constexpr int kStride = kH + 1; // padded smem row of a 64-wide activation
 
 __device__ __forceinline__ float sigmoid(float z) { return 1.0f / (1.0f + expf(-z)); }
 // The training kernel's sigmoid: the hardware exponential and reciprocal
 // (a few ulp; the gradients are checked against the FP64 oracle at 1e-4).
 __device__ __forceinline__ float sigmoid_fast(float z) { return __fdividef(1.0f, 1.0f + __expf(-z)); }
 
-// Shared-memory layout of the training kernel (float offsets).
-struct TrainSmem {
-  int w[kMaxMlpLayers], b[kMaxMlpLayers];  // weights [out][in+1], biases
-  int x;                                   // inputs [kS][n_in+1]
-  int z[kMaxMlpLayers], a[kMaxMlpLayers];  // hidden pre-/post-activations [kS][65]
-  int y;                                   // outputs / output gradients [kS][n_out+1]
-  int total;
+// ---- FP32 tiles -----------------------------------------------------------------
+// A tile is 64 samples.  Its activations and their gradients lie feature-major
+// in shared memory, [feature][sample], weights row-major, [neuron][input], both
+// with 4 floats of padding a row, so that a thread's 4 x 4 products read
+// nothing but float4s, without bank conflicts, and two FMAs are fed by each
+// float read.  Shared memory is still what bounds them (32 floats a cycle
+// against 128 FMAs): 4 x 2 products by twice the threads are slower (78 us a
+// training step against 65), larger ones do not fit the registers beside the
+// weight gradients.
+constexpr int kRow = kH + 4;       // row of a 64-wide weight matrix or of 64 samples
+constexpr int kInRow = 16 + 4;     // row of the first layer's weights (n_in <= 16)
+constexpr int kOutPad = 8;         // output rows (n_out <= 8)
+
+struct Vec4 {
+  float v[4];
 };
-
-__host__ __device__ inline TrainSmem train_smem(const MlpShape& m) {
-  TrainSmem t{};
-  int o = 0;
-  for (int l = 0; l < m.n_layers; ++l) {
-    t.w[l] = o;
-    o += m.out_dim[l] * (m.in_dim[l] + 1);
-    t.b[l] = o;
-    o += m.out_dim[l];
-  }
-  t.x = o;
-  o += kS * (m.n_in + 1);
-  for (int l = 0; l + 1 < m.n_layers; ++l) {
-    t.z[l] = o;
-    o += kS * kStride;
-    t.a[l] = o;
-    o += kS * kStride;
-  }
-  t.y = o;
-  o += kS * (m.n_out + 1);
-  t.total = o;
-  return t;
+__device__ __forceinline__ Vec4 lds4(const float* p) {
+  const float4 f = *reinterpret_cast<const float4*>(p);
+  return {f.x, f.y, f.z, f.w};
 }
+__device__ __forceinline__ void sts4(float* p, const float (&v)[4]) {
+  *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], v[3]);
+}
+// A warp's threads are 8 sample (or input) groups by 4 neuron groups.
+__device__ __forceinline__ int group_wide() { return ((threadIdx.x >> 5) & 1) * 8 + (threadIdx.x & 7); }    // 0..15
+__device__ __forceinline__ int group_tall() { return (threadIdx.x >> 6) * 4 + ((threadIdx.x & 31) >> 3); }  // 0..15
 
-// out[s][j] = b[j] + sum_k in[s][k] W[j][k] for s < kS, j < out_dim.
-// 64-wide outputs: a thread holds 4 samples x 4 columns j0 + 16c (columns
-// interleaved so that a warp's weight reads hit distinct banks).
-__device__ void dense_forward(const float* __restrict__ in, int in_stride, int in_dim, const float* __restrict__ W,
-                              const float* __restrict__ b, int out_dim, float* __restrict__ out, int out_stride) {
-  const int t = threadIdx.x;
-  if (out_dim == kH) {
-    const int s0 = (t >> 4) * 4, j0 = t & 15;
-    float acc[4][4];
+// acc[r][c] += sum_k W[j + 16 r][k] in[k][4 s + c], k < 4 quads, in the order of k.
+__device__ __forceinline__ void product_forward(const float* __restrict__ W, int w_row, const float* __restrict__ in,
+                                                int quads, float (&acc)[4][4]) {
+  const int s = group_wide(), j = group_tall();
+#pragma unroll 4
+  for (int q = 0; q < quads; ++q) {
+    Vec4 w[4], a[4];
 #pragma unroll
-    for (int r = 0; r < 4; ++r)
+    for (int r = 0; r < 4; ++r) w[r] = lds4(W + (j + 16 * r) * w_row + 4 * q);
 #pragma unroll
-      for (int c = 0; c < 4; ++c) acc[r][c] = b[j0 + 16 * c];
-    for (int k = 0; k < in_dim; ++k) {
-      float av[4], wv[4];
+    for (int i = 0; i < 4; ++i) a[i] = lds4(in + (4 * q + i) * kRow + 4 * s);
 #pragma unroll
-      for (int r = 0; r < 4; ++r) av[r] = in[(s0 + r) * in_stride + k];
-#pragma unroll
-      for (int c = 0; c < 4; ++c) wv[c] = W[(j0 + 16 * c) * (in_dim + 1) + k];
+    for (int i = 0; i < 4; ++i)
 #pragma unroll
       for (int r = 0; r < 4; ++r)
 #pragma unroll
-        for (int c = 0; c < 4; ++c) acc[r][c] = fmaf(av[r], wv[c], acc[r][c]);
-    }
+        for (int c = 0; c < 4; ++c) acc[r][c] = fmaf(w[r].v[i], a[i].v[c], acc[r][c]);
+  }
+}
+// acc[r][c] += sum_j W[j][4 k + r] dz[j][4 s + c], j < n.
+__device__ __forceinline__ void product_data(const float* __restrict__ W, const float* __restrict__ dz, int n,
+                                             float (&acc)[4][4]) {
+  const int s = group_wide(), k = group_tall();
+#pragma unroll 8
+  for (int j = 0; j < n; ++j) {
+    const Vec4 w = lds4(W + j * kRow + 4 * k), d = lds4(dz + j * kRow + 4 * s);
 #pragma unroll
     for (int r = 0; r < 4; ++r)
 #pragma unroll
-      for (int c = 0; c < 4; ++c) out[(s0 + r) * out_stride + j0 + 16 * c] = acc[r][c];
-  } else {
-    for (int idx = t; idx < kS * out_dim; idx += kThreads) {
-      const int s = idx / out_dim, j = idx % out_dim;
-      float acc = b[j];
-      for (int k = 0; k < in_dim; ++k) acc = fmaf(in[s * in_stride + k], W[j * (in_dim + 1) + k], acc);
-      out[s * out_stride + j] = acc;
+      for (int c = 0; c < 4; ++c) acc[r][c] = fmaf(w.v[r], d.v[c], acc[r][c]);
+  }
+}
+// acc[r][c] += sum_s dz[j + 16 r][s] in[k + 16 c][s] over the tile's samples.
+__device__ __forceinline__ void product_weights(const float* __restrict__ dz, const float* __restrict__ in,
+                                                float (&acc)[4][4]) {
+  const int k = group_wide(), j = group_tall();
+#pragma unroll 4
+  for (int q = 0; q < kS / 4; ++q) {
+    Vec4 d[4], a[4];
+#pragma unroll
+    for (int r = 0; r < 4; ++r) d[r] = lds4(dz + (j + 16 * r) * kRow + 4 * q);
+#pragma unroll
+    for (int c = 0; c < 4; ++c) a[c] = lds4(in + (k + 16 * c) * kRow + 4 * q);
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int r = 0; r < 4; ++r)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) acc[r][c] = fmaf(d[r].v[i], a[c].v[i], acc[r][c]);
+  }
+}
+__device__ __forceinline__ float sum4(Vec4 a) { return (a.v[0] + a.v[1]) + (a.v[2] + a.v[3]); }
+__device__ __forceinline__ float dot4(Vec4 a, Vec4 b, float acc) {
+#pragma unroll
+  for (int i = 0; i < 4; ++i) acc = fmaf(a.v[i], b.v[i], acc);
+  return acc;
+}
+
+// Shared-memory layout of a network's FP32 weights (float offsets): rows
+// padded, missing inputs and outputs zero.
+template <int kHidden>
+struct TileWeights {
+  static constexpr int kFirst = 0;                                        // [64][kInRow]
+  static constexpr int kMiddle = kFirst + kH * kInRow;                    // [kHidden - 1][64][kRow]
+  static constexpr int kLast = kMiddle + (kHidden - 1) * kH * kRow;       // [kOutPad][kRow]
+  static constexpr int kBias = kLast + kOutPad * kRow;                    // [kHidden][64], [kOutPad]
+  static constexpr int kInputs = kBias + kHidden * kH + kOutPad;          // [16][kRow]: the tile's inputs
+  static constexpr int kEnd = kInputs + 16 * kRow;
+};
+template <int kHidden>
+__device__ __forceinline__ void load_weights(const MlpShape& m, const float* __restrict__ params, float* sm) {
+  using T = TileWeights<kHidden>;
+  const int t = threadIdx.x;
+  for (int i = t; i < kH * 16; i += kThreads) {
+    const int j = i >> 4, k = i & 15;
+    sm[T::kFirst + j * kInRow + k] = k < m.n_in ? params[m.off_w[0] + j * m.n_in + k] : 0.0f;
+  }
+#pragma unroll
+  for (int l = 1; l < kHidden; ++l)
+    for (int i = t; i < kH * kH; i += kThreads)
+      sm[T::kMiddle + (l - 1) * kH * kRow + (i >> 6) * kRow + (i & 63)] = params[m.off_w[l] + i];
+  for (int i = t; i < kOutPad * kH; i += kThreads)
+    sm[T::kLast + (i >> 6) * kRow + (i & 63)] = (i >> 6) < m.n_out ? params[m.off_w[kHidden] + i] : 0.0f;
+#pragma unroll
+  for (int l = 0; l < kHidden; ++l)
+    if (t < kH) sm[T::kBias + l * kH + t] = params[m.off_b[l] + t];
+  if (t < kOutPad) sm[T::kBias + kHidden * kH + t] = t < m.n_out ? params[m.off_b[kHidden] + t] : 0.0f;
+  for (int i = t; i < 16 * kRow; i += kThreads) sm[T::kInputs + i] = 0.0f;
+}
+// The tile's inputs, transposed; rows of samples past n zero.
+template <int kHidden>
+__device__ __forceinline__ void load_inputs(const MlpShape& m, const float* __restrict__ inputs, long long base,
+                                            long long n, float* sm) {
+  float* x = sm + TileWeights<kHidden>::kInputs;
+  const long long left = (n - base) * m.n_in;
+  for (int i = threadIdx.x; i < kS * m.n_in; i += kThreads)
+    x[(i % m.n_in) * kRow + i / m.n_in] = i < left ? inputs[base * m.n_in + i] : 0.0f;
+}
+// Pre-activations of hidden layer l from its inputs, from the bias on.
+template <int kHidden>
+__device__ __forceinline__ void hidden_layer(const MlpShape& m, const float* sm, int l, const float* in,
+                                             float (&acc)[4][4]) {
+  using T = TileWeights<kHidden>;
+#pragma unroll
+  for (int r = 0; r < 4; ++r) {
+    const float b = sm[T::kBias + l * kH + group_tall() + 16 * r];
+#pragma unroll
+    for (int c = 0; c < 4; ++c) acc[r][c] = b;
+  }
+  if (l == 0)
+    product_forward(sm + T::kFirst, kInRow, in, (m.n_in + 3) >> 2, acc);
+  else
+    product_forward(sm + T::kMiddle + (l - 1) * kH * kRow, kRow, in, kH / 4, acc);
+}
+// Outputs 2 p and 2 p + 1 of sample s = thread & 63, p = thread >> 6.
+template <int kHidden>
+__device__ __forceinline__ void output_layer(const float* sm, const float* in, float (&y)[2]) {
+  using T = TileWeights<kHidden>;
+  const int s = threadIdx.x & 63, p = threadIdx.x >> 6;
+  const float* w = sm + T::kLast + 2 * p * kRow;
+  y[0] = sm[T::kBias + kHidden * kH + 2 * p];
+  y[1] = sm[T::kBias + kHidden * kH + 2 * p + 1];
+#pragma unroll 4
+  for (int q = 0; q < kH / 4; ++q) {
+    const Vec4 w0 = lds4(w + 4 * q), w1 = lds4(w + kRow + 4 * q);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const float a = in[(4 * q + i) * kRow + s];
+      y[0] = fmaf(w0.v[i], a, y[0]);
+      y[1] = fmaf(w1.v[i], a, y[1]);
     }
   }
 }
 
-// Fused forward + backward over one tile of kS samples; writes this CTA's
-// gradient of the batch loss (every parameter) and its squared-error sum.
-__global__ void __launch_bounds__(kThreads) k_mlp_grad(MlpShape m, const float* __restrict__ params,
-                                                       const float* __restrict__ inputs,
-                                                       const float* __restrict__ targets,
-                                                       const float* __restrict__ weights, long long n,
-                                                       float inv_count, float* __restrict__ grad_partial,
-                                                       float* __restrict__ loss_partial) {
-  extern __shared__ float sm[];
-  const TrainSmem L = train_smem(m);
+template <int kHidden>
+constexpr int train_floats() {  // weights and inputs, A and D of each hidden layer, the outputs' gradients
+  return TileWeights<kHidden>::kEnd + 2 * kHidden * kH * kRow + kOutPad * kRow;
+}
+
+// Fused forward + backward.  Each block stays for the launch: it walks tiles
+// of 64 samples with the gradients of all weights in its threads' registers,
+// and writes them once (its row of grad_partial, and its squared-error sum).
+// A[l] holds layer l's activations, D[l] their derivative and then, in its
+// place, the gradient of its pre-activations.  A step of 16,384 samples (11 ->
+// 4 x 64 -> 6) takes 65 us with its reduction, 178 us when each 64-sample block
+// wrote a gradient row of its own and four launches followed.
+template <int kHidden>
+__global__ void __launch_bounds__(kThreads, 1) k_mlp_grad(MlpShape m, const float* __restrict__ params,
+                                                          const float* __restrict__ inputs,
+                                                          const float* __restrict__ targets,
+                                                          const float* __restrict__ weights, long long n,
+                                                          float inv_count, float* __restrict__ grad_partial,
+                                                          float* __restrict__ loss_partial) {
+  using T = TileWeights<kHidden>;
+  extern __shared__ __align__(16) float sm[];
+  __shared__ float s_red[kThreads / 32];
+  float* A = sm + T::kEnd;
+  float* D = A + kHidden * kH * kRow;
+  float* dY = D + kHidden * kH * kRow;
+  constexpr int kPlane = kH * kRow;
   const int t = threadIdx.x;
-  const long long base = static_cast<long long>(blockIdx.x) * kS;
-  const int L_out = m.n_layers - 1;
-  // weights and biases -> smem (padded rows)
-  for (int l = 0; l < m.n_layers; ++l) {
-    const int in = m.in_dim[l], out = m.out_dim[l];
-    for (int i = t; i < out * in; i += kThreads) sm[L.w[l] + (i / in) * (in + 1) + i % in] = params[m.off_w[l] + i];
-    for (int i = t; i < out; i += kThreads) sm[L.b[l] + i] = params[m.off_b[l] + i];
-  }
-  for (int i = t; i < kS * m.n_in; i += kThreads) {
-    const int s = i / m.n_in, k = i % m.n_in;
-    sm[L.x + s * (m.n_in + 1) + k] = base + s < n ? inputs[(base + s) * m.n_in + k] : 0.0f;
-  }
-  __syncthreads();
-  // forward
-  for (int l = 0; l < m.n_layers; ++l) {
-    const float* in = l == 0 ? sm + L.x : sm + L.a[l - 1];
-    const int in_stride = l == 0 ? m.n_in + 1 : kStride;
-    float* out = l == L_out ? sm + L.y : sm + L.z[l];
-    const int out_stride = l == L_out ? m.n_out + 1 : kStride;
-    dense_forward(in, in_stride, m.in_dim[l], sm + L.w[l], sm + L.b[l], m.out_dim[l], out, out_stride);
+  float gw[kHidden > 1 ? kHidden - 1 : 1][4][4] = {}, gb[kHidden] = {}, g_first[4] = {}, g_last[2] = {}, gb_last = 0.0f;
+  float sq = 0.0f;
+  load_weights<kHidden>(m, params, sm);
+  for (long long base = blockIdx.x * (long long)kS; base < n; base += gridDim.x * (long long)kS) {
+    __syncthreads();  // the weights are in; the tile before is done with its inputs
+    load_inputs<kHidden>(m, inputs, base, n, sm);
     __syncthreads();
-    if (l != L_out) {
-      for (int i = t; i < kS * kH; i += kThreads) {
-        const int s = i / kH, j = i % kH;
-        const float z = sm[L.z[l] + s * kStride + j];
-        sm[L.a[l] + s * kStride + j] = z * sigmoid_fast(z);
+    const int wide = group_wide(), tall = group_tall();
+#pragma unroll
+    for (int l = 0; l < kHidden; ++l) {
+      float acc[4][4];
+      hidden_layer<kHidden>(m, sm, l, l == 0 ? sm + T::kInputs : A + (l - 1) * kPlane, acc);
+#pragma unroll
+      for (int r = 0; r < 4; ++r) {
+        float a[4], d[4];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          const float z = acc[r][c], sg = sigmoid_fast(z);
+          a[c] = z * sg;
+          d[c] = sg * (1.0f + z * (1.0f - sg));
+        }
+        sts4(A + l * kPlane + (tall + 16 * r) * kRow + 4 * wide, a);
+        sts4(D + l * kPlane + (tall + 16 * r) * kRow + 4 * wide, d);
       }
       __syncthreads();
     }
-  }
-  // loss and output gradient (mean over batch x outputs)
-  float sq = 0.0f;
-  for (int i = t; i < kS * m.n_out; i += kThreads) {
-    const int s = i / m.n_out, o = i % m.n_out;
-    float g = 0.0f;
-    if (base + s < n) {
-      const float d = sm[L.y + s * (m.n_out + 1) + o] - targets[(base + s) * m.n_out + o];
-      const float w = weights != nullptr ? weights[(base + s) * m.n_out + o] : 1.0f;
-      sq += w * d * d;
-      g = 2.0f * w * d * inv_count;
-    }
-    sm[L.y + s * (m.n_out + 1) + o] = g;
-  }
-  __syncthreads();
-  // backward: dZ_l lives in place of Z_l (or Y for the output layer)
-  float* gp = grad_partial + static_cast<long long>(blockIdx.x) * m.n_params;
-  for (int l = L_out; l >= 0; --l) {
-    const int in = m.in_dim[l], out = m.out_dim[l];
-    const float* dz = l == L_out ? sm + L.y : sm + L.z[l];
-    const int dz_stride = l == L_out ? m.n_out + 1 : kStride;
-    const float* a_prev = l == 0 ? sm + L.x : sm + L.a[l - 1];
-    const int a_stride = l == 0 ? m.n_in + 1 : kStride;
-    // dW[j][k] = sum_s dz[s][j] a_prev[s][k];  db[j] = sum_s dz[s][j]
-    if (out == kH) {
-      // register tiles: 4 neurons j = 4 (t >> 4) + r by in/16 inputs
-      // k = (t & 15) + 16 c; per sample 8 shared loads feed 16 FMAs
-      const int j0 = (t >> 4) * 4, kk = t & 15;
-      float acc[4][4] = {};
-      float bacc = 0.0f;
-      for (int s = 0; s < kS; ++s) {
-        float dv[4], av[4];
+    // loss and output gradient (mean over batch x outputs)
+    {
+      float y[2];
+      output_layer<kHidden>(sm, A + (kHidden - 1) * kPlane, y);
+      const int s = t & 63, o = 2 * (t >> 6);
 #pragma unroll
-        for (int r = 0; r < 4; ++r) dv[r] = dz[s * dz_stride + j0 + r];
-#pragma unroll
-        for (int c = 0; c < 4; ++c) av[c] = kk + 16 * c < in ? a_prev[s * a_stride + kk + 16 * c] : 0.0f;
-#pragma unroll
-        for (int r = 0; r < 4; ++r)
-#pragma unroll
-          for (int c = 0; c < 4; ++c) acc[r][c] = fmaf(dv[r], av[c], acc[r][c]);
-        bacc += kk == 0 ? dv[0] : kk == 1 ? dv[1] : kk == 2 ? dv[2] : dv[3];  // used by kk < 4
-      }
-#pragma unroll
-      for (int r = 0; r < 4; ++r)
-#pragma unroll
-        for (int c = 0; c < 4; ++c)
-          if (kk + 16 * c < in) gp[m.off_w[l] + (j0 + r) * in + kk + 16 * c] = acc[r][c];
-      if (kk < 4) gp[m.off_b[l] + j0 + kk] = bacc;
-    } else {
-      for (int idx = t; idx < out * in; idx += kThreads) {
-        const int j = idx / in, k = idx % in;
-        float acc = 0.0f;
-        for (int s = 0; s < kS; ++s) acc = fmaf(dz[s * dz_stride + j], a_prev[s * a_stride + k], acc);
-        gp[m.off_w[l] + idx] = acc;
-      }
-      for (int j = t; j < out; j += kThreads) {
-        float acc = 0.0f;
-        for (int s = 0; s < kS; ++s) acc += dz[s * dz_stride + j];
-        gp[m.off_b[l] + j] = acc;
+      for (int i = 0; i < 2; ++i) {
+        float g = 0.0f;
+        if (base + s < n && o + i < m.n_out) {
+          const long long at = (base + s) * m.n_out + o + i;
+          const float d = y[i] - targets[at];
+          const float w = weights != nullptr ? weights[at] : 1.0f;
+          sq += w * d * d;
+          g = 2.0f * w * d * inv_count;
+        }
+        dY[(o + i) * kRow + s] = g;
       }
     }
-    if (l == 0) break;
-    // dZ_{l-1}[s][k] = (sum_j dz[s][j] W[j][k]) * silu'(Z_{l-1}[s][k]), in
-    // place of Z_{l-1} (in == 64 here): register tiles of 4 samples
-    // s = 4 (t >> 4) + r by 4 inputs k = (t & 15) + 16 c
-    const float* W = sm + L.w[l];
-    float* zp = sm + L.z[l - 1];
-    const int s0 = (t >> 4) * 4, kk = t & 15;
-    float acc[4][4] = {};
-    for (int j = 0; j < out; ++j) {
-      float dv[4], wv[4];
-#pragma unroll
-      for (int r = 0; r < 4; ++r) dv[r] = dz[(s0 + r) * dz_stride + j];
-#pragma unroll
-      for (int c = 0; c < 4; ++c) wv[c] = W[j * (in + 1) + kk + 16 * c];
-#pragma unroll
-      for (int r = 0; r < 4; ++r)
-#pragma unroll
-        for (int c = 0; c < 4; ++c) acc[r][c] = fmaf(dv[r], wv[c], acc[r][c]);
-    }
-#pragma unroll
-    for (int r = 0; r < 4; ++r)
-#pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        const float z = zp[(s0 + r) * kStride + kk + 16 * c];
-        const float sg = sigmoid_fast(z);
-        acc[r][c] = acc[r][c] * sg * (1.0f + z * (1.0f - sg));
-      }
-    __syncthreads();  // all reads of Z_{l-1} (and of dZ_l by the dW loop) are done
-#pragma unroll
-    for (int r = 0; r < 4; ++r)
-#pragma unroll
-      for (int c = 0; c < 4; ++c) zp[(s0 + r) * kStride + kk + 16 * c] = acc[r][c];
     __syncthreads();
+    // the output layer's weights (row t >> 5, inputs t & 31 and + 32) and biases
+    {
+      const float* dz = dY + (t >> 5) * kRow;
+      const float* a = A + (kHidden - 1) * kPlane + (t & 31) * kRow;
+#pragma unroll 4
+      for (int q = 0; q < kS / 4; ++q) {
+        const Vec4 d = lds4(dz + 4 * q);
+        g_last[0] = dot4(d, lds4(a + 4 * q), g_last[0]);
+        g_last[1] = dot4(d, lds4(a + 32 * kRow + 4 * q), g_last[1]);
+      }
+      if (t < 4 * kOutPad)
+        for (int q = t & 3; q < kS / 4; q += 4) gb_last += sum4(lds4(dY + (t >> 2) * kRow + 4 * q));
+    }
+#pragma unroll
+    for (int l = kHidden - 1; l >= 0; --l) {
+      // gradient of layer l's pre-activations, in place of its derivative
+      float acc[4][4] = {};
+      if (l == kHidden - 1)
+        product_data(sm + T::kLast, dY, m.n_out, acc);
+      else
+        product_data(sm + T::kMiddle + l * kH * kRow, D + (l + 1) * kPlane, kH, acc);
+#pragma unroll
+      for (int r = 0; r < 4; ++r) {
+        float* d = D + l * kPlane + (4 * tall + r) * kRow + 4 * wide;
+        const Vec4 v = lds4(d);
+        float o[4];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) o[c] = acc[r][c] * v.v[c];
+        sts4(d, o);
+      }
+      __syncthreads();
+      const float* dz = D + l * kPlane;
+      if (l > 0) {
+        product_weights(dz, A + (l - 1) * kPlane, gw[l - 1]);
+      } else {  // inputs (t & 3) + 4 c of neuron t >> 2
+        const float* x = sm + T::kInputs + (t & 3) * kRow;
+#pragma unroll 4
+        for (int q = 0; q < kS / 4; ++q) {
+          const Vec4 d = lds4(dz + (t >> 2) * kRow + 4 * q);
+#pragma unroll
+          for (int c = 0; c < 4; ++c) g_first[c] = dot4(d, lds4(x + 4 * c * kRow + 4 * q), g_first[c]);
+        }
+      }
+      for (int q = t & 3; q < kS / 4; q += 4) gb[l] += sum4(lds4(dz + (t >> 2) * kRow + 4 * q));
+    }
   }
-  // squared-error sum of the tile
-  __shared__ float s_red[kThreads / 32];
+  // this block's gradients
+  float* gp = grad_partial + static_cast<long long>(blockIdx.x) * m.n_params;
+  const int k0 = group_wide(), j0 = group_tall();
+#pragma unroll
+  for (int l = 1; l < kHidden; ++l)
+#pragma unroll
+    for (int r = 0; r < 4; ++r)
+#pragma unroll
+      for (int c = 0; c < 4; ++c) gp[m.off_w[l] + (j0 + 16 * r) * kH + k0 + 16 * c] = gw[l - 1][r][c];
+#pragma unroll
+  for (int c = 0; c < 4; ++c)
+    if ((t & 3) + 4 * c < m.n_in) gp[m.off_w[0] + (t >> 2) * m.n_in + (t & 3) + 4 * c] = g_first[c];
+  if ((t >> 5) < m.n_out) {
+    gp[m.off_w[kHidden] + (t >> 5) * kH + (t & 31)] = g_last[0];
+    gp[m.off_w[kHidden] + (t >> 5) * kH + (t & 31) + 32] = g_last[1];
+  }
+#pragma unroll
+  for (int l = 0; l < kHidden; ++l) {  // four threads a bias
+    gb[l] += __shfl_xor_sync(0xffffffffu, gb[l], 1);
+    gb[l] += __shfl_xor_sync(0xffffffffu, gb[l], 2);
+    if ((t & 3) == 0) gp[m.off_b[l] + (t >> 2)] = gb[l];
+  }
+  gb_last += __shfl_xor_sync(0xffffffffu, gb_last, 1);
+  gb_last += __shfl_xor_sync(0xffffffffu, gb_last, 2);
+  if ((t & 3) == 0 && (t >> 2) < m.n_out) gp[m.off_b[kHidden] + (t >> 2)] = gb_last;
+  // squared-error sum of the block
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o);
   if ((t & 31) == 0) s_red[t >> 5] = sq;
@@ -249,50 +347,94 @@ __global__ void __launch_bounds__(kThreads) k_mlp_grad(MlpShape m, const float* 
   }
 }
 
-// grad[p] = sum over CTAs of grad_partial[cta][p], in CTA order.
-__global__ void k_reduce_partials(const float* __restrict__ partial, int n_ctas, int n_params,
-                                  float* __restrict__ out) {
-  for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < n_params; p += gridDim.x * blockDim.x) {
-    float acc = 0.0f;
-    for (int c = 0; c < n_ctas; ++c) acc += partial[static_cast<long long>(c) * n_params + p];
-    out[p] = acc;
+// Adam's state and rates; params null: the gradient alone.
+struct AdamStep {
+  float *params, *m1, *m2;
+  float lr, b1, b2, eps, c1, c2;
+};
+// grad[p] = sum of the rows of partial in a fixed order, then Adam's update of
+// parameter p; the last block sums the losses (if out).  Eight groups of rows
+// by 32 parameters a block: a serial sum over the rows by one thread a
+// parameter is a chain of their loads.
+constexpr int kReduceGroups = 8;
+__global__ void __launch_bounds__(32 * kReduceGroups) k_reduce_adam(const float* __restrict__ partial, int rows,
+                                                                    int n_params, float* __restrict__ grad,
+                                                                    const float* __restrict__ loss_partial,
+                                                                    float* __restrict__ loss, AdamStep S) {
+  __shared__ float s_sum[kReduceGroups][32];
+  const int lane = threadIdx.x & 31, g = threadIdx.x >> 5;
+  const bool losses = blockIdx.x == gridDim.x - 1;
+  const int p = blockIdx.x * 32 + lane;
+  float acc = 0.0f;
+  if (losses) {
+    if (loss != nullptr)
+      for (int c = threadIdx.x; c < rows; c += 32 * kReduceGroups) acc += loss_partial[c];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+  } else if (p < n_params) {
+#pragma unroll 4
+    for (int c = g; c < rows; c += kReduceGroups) acc += partial[static_cast<long long>(c) * n_params + p];
   }
+  s_sum[g][lane] = acc;
+  __syncthreads();
+  if (g != 0) return;
+  acc = 0.0f;
+#pragma unroll
+  for (int k = 0; k < kReduceGroups; ++k) acc += s_sum[k][lane];
+  if (losses) {
+    if (loss != nullptr && lane == 0) *loss = acc;
+    return;
+  }
+  if (p >= n_params) return;
+  grad[p] = acc;
+  if (S.params == nullptr) return;
+  const float a = S.b1 * S.m1[p] + (1.0f - S.b1) * acc;
+  const float v = S.b2 * S.m2[p] + (1.0f - S.b2) * acc * acc;
+  S.m1[p] = a;
+  S.m2[p] = v;
+  S.params[p] -= S.lr * (a / S.c1) / (sqrtf(v / S.c2) + S.eps);
 }
 
-__global__ void k_adam(float* __restrict__ params, const float* __restrict__ grad, float* __restrict__ m1,
-                       float* __restrict__ m2, int n, float lr, float b1, float b2, float eps, float c1, float c2) {
-  for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < n; p += gridDim.x * blockDim.x) {
-    const float g = grad[p];
-    const float a = b1 * m1[p] + (1.0f - b1) * g;
-    const float v = b2 * m2[p] + (1.0f - b2) * g * g;
-    m1[p] = a;
-    m2[p] = v;
-    params[p] -= lr * (a / c1) / (sqrtf(v / c2) + eps);
-  }
+// FP32 forward (reference path of the BF16 kernels): the same tiles, two
+// blocks an SM; every output is summed in the order of a sample-by-sample
+// forward.  65,536 samples (11 -> 4 x 64 -> 6): 62 us, 440 us at one thread a
+// sample with the weights read through L1.
+template <int kHidden>
+constexpr int forward_floats() {
+  return TileWeights<kHidden>::kEnd + 2 * kH * kRow;
 }
-
-// FP32 forward, one thread per sample (reference path of the BF16 kernel).
-__global__ void __launch_bounds__(128) k_mlp_forward_f32(MlpShape m, const float* __restrict__ params,
-                                                        const float* __restrict__ inputs, float* __restrict__ outputs,
-                                                        long long n) {
-  const long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
-  if (i >= n) return;
-  float a[kH], z[kH];
-  for (int k = 0; k < m.n_in; ++k) a[k] = inputs[i * m.n_in + k];
-  for (int l = 0; l < m.n_layers; ++l) {
-    const float* W = params + m.off_w[l];
-    const float* b = params + m.off_b[l];
-    const int in = m.in_dim[l], out = m.out_dim[l];
-    for (int j = 0; j < out; ++j) {
-      float acc = b[j];
-      for (int k = 0; k < in; ++k) acc = fmaf(a[k], __ldg(W + j * in + k), acc);
-      z[j] = acc;
+template <int kHidden>
+__global__ void __launch_bounds__(kThreads, 2) k_mlp_forward_f32(MlpShape m, const float* __restrict__ params,
+                                                                const float* __restrict__ inputs,
+                                                                float* __restrict__ outputs, long long n) {
+  using T = TileWeights<kHidden>;
+  extern __shared__ __align__(16) float sm[];
+  float* A = sm + T::kEnd;
+  constexpr int kPlane = kH * kRow;
+  load_weights<kHidden>(m, params, sm);
+  for (long long base = blockIdx.x * (long long)kS; base < n; base += gridDim.x * (long long)kS) {
+    __syncthreads();
+    load_inputs<kHidden>(m, inputs, base, n, sm);
+    __syncthreads();
+#pragma unroll
+    for (int l = 0; l < kHidden; ++l) {
+      float acc[4][4];
+      hidden_layer<kHidden>(m, sm, l, l == 0 ? sm + T::kInputs : A + ((l - 1) & 1) * kPlane, acc);
+#pragma unroll
+      for (int r = 0; r < 4; ++r) {
+        float a[4];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) a[c] = acc[r][c] * sigmoid(acc[r][c]);
+        sts4(A + (l & 1) * kPlane + (group_tall() + 16 * r) * kRow + 4 * group_wide(), a);
+      }
+      __syncthreads();
     }
-    if (l + 1 == m.n_layers) {
-      for (int j = 0; j < out; ++j) outputs[i * m.n_out + j] = z[j];
-    } else {
-      for (int j = 0; j < out; ++j) a[j] = z[j] * sigmoid(z[j]);
-    }
+    float y[2];
+    output_layer<kHidden>(sm, A + ((kHidden - 1) & 1) * kPlane, y);
+    const int s = threadIdx.x & 63, o = 2 * (threadIdx.x >> 6);
+    if (base + s < n)
+      for (int i = 0; i < 2; ++i)
+        if (o + i < m.n_out) outputs[(base + s) * m.n_out + o + i] = y[i];
   }
 }
 
@@ -403,13 +545,17 @@ __global__ void __launch_bounds__(128) k_mlp_forward_tc(MlpShape m, const unsign
   if (threadIdx.x < 32) tc::dealloc(s_tmem, 256);
 }
 
+// The weights (whole 16-byte pieces) are copied once a block: few blocks of
+// eight warps, each with several 16-row tiles (65,536 samples: 14 us, 41 us
+// with a copy every 64 rows).
+constexpr int kBf16Threads = 256;
 template <int kHidden>
-__global__ void __launch_bounds__(128) k_mlp_forward_bf16(MlpShape m, const unsigned char* __restrict__ packed,
-                                                          int packed_bytes, const float* __restrict__ inputs,
-                                                          float* __restrict__ outputs, long long n) {
-  extern __shared__ __align__(16) unsigned char smw[];
-  for (int i = threadIdx.x * 4; i < packed_bytes; i += blockDim.x * 4)
-    *reinterpret_cast<uint32_t*>(smw + i) = *reinterpret_cast<const uint32_t*>(packed + i);
+__global__ void __launch_bounds__(kBf16Threads) k_mlp_forward_bf16(MlpShape m, const unsigned char* __restrict__ packed,
+                                                                   int packed_bytes, const float* __restrict__ inputs,
+                                                                   float* __restrict__ outputs, long long n) {
+  extern __shared__ __align__(128) unsigned char smw[];
+  for (int i = threadIdx.x * 16; i < packed_bytes; i += blockDim.x * 16)
+    *reinterpret_cast<uint4*>(smw + i) = *reinterpret_cast<const uint4*>(packed + i);
   __syncthreads();
   const int lane = threadIdx.x & 31;
   const int g = lane >> 2, q = lane & 3;
@@ -455,42 +601,69 @@ MlpShape make_mlp_shape(int n_in, int n_hidden, int n_out) {
   return m;
 }
 
-int mlp_train_ctas(long long n) { return int((n + kS - 1) / kS); }
+// Blocks of a training launch: one an SM, and no more than there are tiles.
+int mlp_train_ctas(long long n, int sm_count) { return int(std::min<long long>((n + kS - 1) / kS, sm_count)); }
 
-size_t mlp_train_smem_bytes(const MlpShape& m) { return size_t(train_smem(m).total) * sizeof(float); }
+namespace {
+// Calls f with the network's hidden-layer count as a constant.
+template <class F>
+cudaError_t with_hidden(const MlpShape& m, F f) {
+  switch (m.n_layers - 1) {
+    case 1: return f(std::integral_constant<int, 1>{});
+    case 2: return f(std::integral_constant<int, 2>{});
+    case 3: return f(std::integral_constant<int, 3>{});
+    case 4: return f(std::integral_constant<int, 4>{});
+    default: return cudaErrorInvalidValue;
+  }
+}
+cudaError_t launch_reduce(const float* partial, int rows, int n_params, float* grad, const float* loss_partial,
+                          float* loss, const AdamStep& step, cudaStream_t s) {
+  k_reduce_adam<<<(n_params + 31) / 32 + 1, 32 * kReduceGroups, 0, s>>>(partial, rows, n_params, grad, loss_partial,
+                                                                       loss, step);
+  return cudaGetLastError();
+}
+}  // namespace
 
 cudaError_t launch_mlp_grad(const MlpShape& m, const float* params, const float* inputs, const float* targets,
-                            const float* weights, long long n, float* grad_partial, float* loss_partial, float* grad,
+                            const float* weights, long long n, float* grad_partial, float* loss_partial, int sm_count,
                             cudaStream_t s) {
-  const size_t smem = mlp_train_smem_bytes(m);
-  cudaError_t e = cudaFuncSetAttribute(k_mlp_grad, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
-  if (e != cudaSuccess) return e;
-  const int ctas = mlp_train_ctas(n);
   const float inv = 1.0f / float(double(n) * m.n_out);
-  k_mlp_grad<<<ctas, kThreads, smem, s>>>(m, params, inputs, targets, weights, n, inv, grad_partial, loss_partial);
-  e = cudaGetLastError();
-  if (e != cudaSuccess) return e;
-  k_reduce_partials<<<(m.n_params + 255) / 256, 256, 0, s>>>(grad_partial, ctas, m.n_params, grad);
-  return cudaGetLastError();
+  return with_hidden(m, [&](auto hidden) {
+    constexpr int kBytes = train_floats<hidden.value>() * int(sizeof(float));
+    cudaError_t e =
+        cudaFuncSetAttribute(k_mlp_grad<hidden.value>, cudaFuncAttributeMaxDynamicSharedMemorySize, kBytes);
+    if (e != cudaSuccess) return e;
+    k_mlp_grad<hidden.value><<<mlp_train_ctas(n, sm_count), kThreads, kBytes, s>>>(
+        m, params, inputs, targets, weights, n, inv, grad_partial, loss_partial);
+    return cudaGetLastError();
+  });
 }
 
-cudaError_t launch_reduce_partials(const float* partial, int rows, int cols, float* out, cudaStream_t s) {
-  k_reduce_partials<<<(cols + 255) / 256, 256, 0, s>>>(partial, rows, cols, out);
-  return cudaGetLastError();
+cudaError_t launch_mlp_reduce(const MlpShape& m, const float* grad_partial, int rows, float* grad,
+                              const float* loss_partial, float* loss, cudaStream_t s) {
+  return launch_reduce(grad_partial, rows, m.n_params, grad, loss_partial, loss, AdamStep{}, s);
 }
 
-cudaError_t launch_adam(float* params, const float* grad, float* m1, float* m2, int n, float lr, float b1, float b2,
-                        float eps, long long step, cudaStream_t s) {
+cudaError_t launch_mlp_adam(const MlpShape& m, const float* grad_partial, int rows, float* grad,
+                            const float* loss_partial, float* loss, float* params, float* m1, float* m2, float lr,
+                            float b1, float b2, float eps, long long step, cudaStream_t s) {
   const float c1 = 1.0f - float(pow(double(b1), double(step)));
   const float c2 = 1.0f - float(pow(double(b2), double(step)));
-  k_adam<<<(n + 255) / 256, 256, 0, s>>>(params, grad, m1, m2, n, lr, b1, b2, eps, c1, c2);
-  return cudaGetLastError();
+  return launch_reduce(grad_partial, rows, m.n_params, grad, loss_partial, loss,
+                       AdamStep{params, m1, m2, lr, b1, b2, eps, c1, c2}, s);
 }
 
 cudaError_t launch_mlp_forward_f32(const MlpShape& m, const float* params, const float* inputs, float* outputs,
-                                   long long n, cudaStream_t s) {
-  k_mlp_forward_f32<<<unsigned((n + 127) / 128), 128, 0, s>>>(m, params, inputs, outputs, n);
-  return cudaGetLastError();
+                                   long long n, int sm_count, cudaStream_t s) {
+  const int blocks = int(std::min<long long>((n + kS - 1) / kS, 2LL * sm_count));
+  return with_hidden(m, [&](auto hidden) {
+    constexpr int kBytes = forward_floats<hidden.value>() * int(sizeof(float));
+    cudaError_t e =
+        cudaFuncSetAttribute(k_mlp_forward_f32<hidden.value>, cudaFuncAttributeMaxDynamicSharedMemorySize, kBytes);
+    if (e != cudaSuccess) return e;
+    k_mlp_forward_f32<hidden.value><<<blocks, kThreads, kBytes, s>>>(m, params, inputs, outputs, n);
+    return cudaGetLastError();
+  });
 }
 
 size_t mlp_tc_bytes(const MlpShape& m) {
@@ -537,13 +710,13 @@ cudaError_t launch_mlp_pack_bf16(const MlpShape& m, const float* params, void* p
 cudaError_t launch_mlp_forward_bf16(const MlpShape& m, const void* packed, const float* inputs, float* outputs,
                                     long long n, int sm_count, cudaStream_t s) {
   const int bytes = int(mlp_bf16_bytes(m));
-  const unsigned blocks = unsigned(std::min<long long>((n + 63) / 64, 8LL * sm_count));
+  const unsigned blocks = unsigned(std::min<long long>((n + 127) / 128, 3LL * sm_count));
   const auto* p = static_cast<const unsigned char*>(packed);
   switch (m.n_layers - 1) {
-    case 1: k_mlp_forward_bf16<1><<<blocks, 128, bytes, s>>>(m, p, bytes, inputs, outputs, n); break;
-    case 2: k_mlp_forward_bf16<2><<<blocks, 128, bytes, s>>>(m, p, bytes, inputs, outputs, n); break;
-    case 3: k_mlp_forward_bf16<3><<<blocks, 128, bytes, s>>>(m, p, bytes, inputs, outputs, n); break;
-    case 4: k_mlp_forward_bf16<4><<<blocks, 128, bytes, s>>>(m, p, bytes, inputs, outputs, n); break;
+    case 1: k_mlp_forward_bf16<1><<<blocks, kBf16Threads, bytes, s>>>(m, p, bytes, inputs, outputs, n); break;
+    case 2: k_mlp_forward_bf16<2><<<blocks, kBf16Threads, bytes, s>>>(m, p, bytes, inputs, outputs, n); break;
+    case 3: k_mlp_forward_bf16<3><<<blocks, kBf16Threads, bytes, s>>>(m, p, bytes, inputs, outputs, n); break;
+    case 4: k_mlp_forward_bf16<4><<<blocks, kBf16Threads, bytes, s>>>(m, p, bytes, inputs, outputs, n); break;
     default: return cudaErrorInvalidValue;
   }
   return cudaGetLastError();
