@@ -25,17 +25,24 @@ struct ImageLayout {
 // a flat 64-bit pixel index costs its kernel two long divisions a pixel.
 constexpr int kRunPixels = 32, kRunRows = 8;
 inline dim3 run_block() { return dim3(kRunPixels, kRunRows); }
+// fast x slow elements; rows of blocks past a grid's 65,535 lie along z.
+inline dim3 run_grid(int fast, int slow) {
+  const unsigned rows = unsigned(slow - 1) / kRunRows + 1, y = rows < 65535u ? rows : 65535u;
+  return dim3(unsigned(fast - 1) / kRunPixels + 1, y, (rows + y - 1) / y);
+}
+__device__ __forceinline__ bool run_element(int fast, int slow, int& f, int& s) {
+  const unsigned uf = blockIdx.x * kRunPixels + threadIdx.x;
+  const unsigned us = (blockIdx.z * gridDim.y + blockIdx.y) * kRunRows + threadIdx.y;
+  f = int(uf);
+  s = int(us);
+  return uf < unsigned(fast) && us < unsigned(slow);
+}
 inline dim3 run_grid(const ImageLayout& L) {
-  const bool y_fast = L.sy <= L.sx;
-  const int fast = y_fast ? L.height : L.width, slow = y_fast ? L.width : L.height;
-  return dim3((fast + kRunPixels - 1) / kRunPixels, (slow + kRunRows - 1) / kRunRows);
+  return L.sy <= L.sx ? run_grid(L.height, L.width) : run_grid(L.width, L.height);
 }
 __device__ __forceinline__ bool run_pixel(const ImageLayout& L, int& x, int& y) {
-  const int fast = blockIdx.x * kRunPixels + threadIdx.x, slow = blockIdx.y * kRunRows + threadIdx.y;
-  const bool y_fast = L.sy <= L.sx;  // the reference's (W, H, 3) layout
-  x = y_fast ? slow : fast;
-  y = y_fast ? fast : slow;
-  return x < L.width && y < L.height;
+  return L.sy <= L.sx ? run_element(L.height, L.width, y, x)  // the reference's (W, H, 3) layout
+                      : run_element(L.width, L.height, x, y);
 }
 
 struct CompositeScalars {

@@ -29,3 +29,56 @@ def test_ocean_at_run_edges_and_each_spectrum_size(width, height, resolution, la
                              a["view_basis"], a["tangent_half_fov"], a["time_seconds"], 0)
     got, _ = _run(inputs, config, a, layout, 3)
     _check(got, ref)
+
+
+# blur strips of 24 (two passes) and 28 (one) half-resolution texels, segments of rows, one texel; odd passes
+@pytest.mark.parametrize("width,height", [(1, 1), (2, 5), (48, 9), (49, 131), (57, 113), (400, 3)])
+@pytest.mark.parametrize("layout", ["wh", "hw"])
+@pytest.mark.parametrize("passes", [1, 2, 3, 8])
+def test_bloom_at_strip_and_segment_edges(width, height, layout, passes):
+    from types import SimpleNamespace
+
+    from oracle import postprocess as op
+    from test_gpu_postprocess import DEFAULTS, DISPLAY_ATOL, _processor
+    from test_gpu_postprocess import _run as _process
+
+    hdr = np.exp(np.random.default_rng(width).normal(0.0, 1.5, (width, height, 3))).astype(np.float32)
+    config = dict(bloom_passes=passes)
+    cfg = SimpleNamespace(**{**DEFAULTS, **config})
+    pp = _processor(width, height, config, layout)
+    got = _process(pp, hdr, 1.0, True, True, layout=layout)
+    a = op.extract(hdr, float(np.float32(2.0)), cfg)
+    for _ in range(passes):
+        a = op.blur_vertical(op.blur_horizontal(a))
+    np.testing.assert_allclose(pp.bloom_plane().cpu().numpy(), a, rtol=2.0 ** -22, atol=0)
+    np.testing.assert_allclose(got, op.process(hdr, 1.0, cfg, bloom=True, tone_map=True), rtol=0, atol=DISPLAY_ATOL)
+    pp.close()
+
+
+def test_display_of_the_largest_values():
+    """The ACES fit's quotient where its terms near and leave float's range: the IEEE quotient's result."""
+
+    from types import SimpleNamespace
+
+    from oracle import postprocess as op
+    from test_gpu_postprocess import DEFAULTS, DISPLAY_ATOL, _processor
+
+    v = np.array([0.0, 1e-30, 1e-3, 0.0031, 1.0, 9e17, 1.1e18, 1.15e19, 1.18e19, 1.3e19, 3e38, np.inf, np.nan, -1.0],
+                 np.float32)
+    hdr = np.repeat(v[:, None, None], 3, 2)
+    cfg = SimpleNamespace(**DEFAULTS)
+    pp = _processor(len(v), 1, {})
+    with np.errstate(all="ignore"):
+        ref = op.process(hdr, 0.0, cfg, bloom=False, tone_map=True)
+    ref = np.where(np.isnan(ref), np.float32(0.0), ref)  # the device's clamps take the bound for a NaN
+    np.testing.assert_allclose(_process_nan(pp, hdr), ref, rtol=0, atol=DISPLAY_ATOL)
+    pp.close()
+
+
+def _process_nan(pp, hdr):
+    import torch
+
+    src = torch.as_tensor(hdr, device="cuda")
+    display = torch.full_like(src, -1.0)
+    pp.process(src, display, 0.0, bloom=False, tone_map=True)
+    return display.cpu().numpy()
