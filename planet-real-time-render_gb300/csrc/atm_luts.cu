@@ -30,7 +30,8 @@ namespace {
 constexpr int kTLanes = 8;
 constexpr long long kWaveThreads = 152LL * 2048;  // resident threads of the whole chip
 
-__global__ void __launch_bounds__(256) k_transmittance(DevParams P, float bottom, float4* __restrict__ out) {
+constexpr int kTBlock = 64;
+__global__ void __launch_bounds__(kTBlock) k_transmittance(DevParams P, float bottom, float4* __restrict__ out) {
   const int gid = blockIdx.x * blockDim.x + threadIdx.x;
   const int texel = gid / kTLanes;
   const int sub = gid % kTLanes;
@@ -66,11 +67,13 @@ __global__ void __launch_bounds__(256) k_transmittance(DevParams P, float bottom
 constexpr int kMaxDirs = 128, kMaxDirectionSteps = 128;  // atm_create's ranges
 
 // kLanes consecutive lanes share a direction's march; kLanes ms_dirs threads
-// (rounded up to whole warps) a texel.  Latency-bound: 32x32 texels of 64
-// directions are 13 warps an SM at one lane a direction (44 us), 54 at four
-// (30 us).
+// (rounded up to whole warps) a texel.  Bound by latency and by the blocks'
+// wait for their longest direction: 32x32 texels of 64 directions take 44 us
+// at one lane a direction (13 warps an SM), 27 us at four (2.3 waves of
+// blocks), 22 us at two, whose 1024 blocks are resident at once at 72
+// registers.
 template <int kLanes>
-__global__ void __launch_bounds__(kMaxDirs* kLanes) k_multi_scattering(DevParams P, Frame F,
+__global__ void __maxnreg__(72) k_multi_scattering(DevParams P, Frame F,
                                                                        float4* __restrict__ out,
                                                                        unsigned long long* counter) {
   __shared__ float s_fraction[kMaxDirectionSteps + 1];
@@ -180,8 +183,11 @@ __global__ void __launch_bounds__(kMaxDirs* kLanes) k_multi_scattering(DevParams
 }
 
 // ---- sky-view (:1208-1302) and aerial perspective (:1304-1420) -----------------
+// A warp a block: 4 lanes of 192x108 texels leave the SMs with 2 or 3
+// blocks of 256 (11.9 us) or with 17 or 18 of 32 (11.0 us).
+constexpr int kSkyBlock = 32;
 template <int kLanes>
-__global__ void __launch_bounds__(256) k_sky_view(DevParams P, Frame F, float cam_alt, float4* __restrict__ out,
+__global__ void __launch_bounds__(kSkyBlock) k_sky_view(DevParams P, Frame F, float cam_alt, float4* __restrict__ out,
                                                   unsigned long long* counter) {
   __shared__ float s_fraction[kMaxSkySteps + 1];
   fill_fractions(s_fraction, P.sv_steps, threadIdx.x, blockDim.x);
@@ -194,7 +200,8 @@ __global__ void __launch_bounds__(256) k_sky_view(DevParams P, Frame F, float ca
   warp_count(samples, counter);
 }
 
-__global__ void __launch_bounds__(256) k_aerial(DevParams P, Frame F, AerialView V, float4* __restrict__ out,
+constexpr int kAerialBlock = 128;
+__global__ void __launch_bounds__(kAerialBlock) k_aerial(DevParams P, Frame F, AerialView V, float4* __restrict__ out,
                                                 unsigned long long* counter) {
   __shared__ float s_fraction[kMaxAerialSteps + 1];
   fill_fractions(s_fraction, P.ap_steps, threadIdx.x, blockDim.x);
@@ -205,24 +212,30 @@ __global__ void __launch_bounds__(256) k_aerial(DevParams P, Frame F, AerialView
   warp_count(samples, counter);
 }
 
-__global__ void k_lut_to_fields(const float4* __restrict__ lut, int w, int h, int d, float* __restrict__ dst) {
-  const size_t n = size_t(w) * h * d;
-  for (size_t i = blockIdx.x * size_t(blockDim.x) + threadIdx.x; i < n; i += size_t(gridDim.x) * blockDim.x) {
-    // dst index (x, y, z) in (W, H, D) order
-    size_t z = i % d, y = (i / d) % h, x = i / (size_t(d) * h);
-    float4 v = lut[(z * h + y) * w + x];
-    dst[i * 3 + 0] = v.x;
-    dst[i * 3 + 1] = v.y;
-    dst[i * 3 + 2] = v.z;
-  }
+// Field element i = (x h + y) d + z of a LUT's w x h x d texels, in 32 bits (a
+// LUT has at most 2^24 texels).  A read is latency alone, and 64-bit divisions
+// were most of that: with launches back to back, 256x64 texels take 1.5 us
+// instead of 2.9.
+__device__ __forceinline__ unsigned lut_index(unsigned i, unsigned w, unsigned h, unsigned d) {
+  const unsigned xy = d == 1 ? i : i / d, z = i - xy * d;
+  const unsigned x = xy / h, y = xy - x * h;
+  return (z * h + y) * w + x;
 }
-
-__global__ void k_fields_to_lut(const float* __restrict__ src, int w, int h, int d, float4* __restrict__ lut) {
-  const size_t n = size_t(w) * h * d;
-  for (size_t i = blockIdx.x * size_t(blockDim.x) + threadIdx.x; i < n; i += size_t(gridDim.x) * blockDim.x) {
-    size_t z = i % d, y = (i / d) % h, x = i / (size_t(d) * h);
-    lut[(z * h + y) * w + x] = make_float4(src[i * 3 + 0], src[i * 3 + 1], src[i * 3 + 2], 0.0f);
-  }
+constexpr int kFieldBlock = 128;
+__global__ void __launch_bounds__(kFieldBlock) k_lut_to_fields(const float4* __restrict__ lut, unsigned w, unsigned h,
+                                                               unsigned d, float* __restrict__ dst) {
+  const unsigned i = blockIdx.x * kFieldBlock + threadIdx.x;
+  if (i >= w * h * d) return;
+  const float4 v = lut[lut_index(i, w, h, d)];
+  dst[i * 3 + 0] = v.x;
+  dst[i * 3 + 1] = v.y;
+  dst[i * 3 + 2] = v.z;
+}
+__global__ void __launch_bounds__(kFieldBlock) k_fields_to_lut(const float* __restrict__ src, unsigned w, unsigned h,
+                                                               unsigned d, float4* __restrict__ lut) {
+  const unsigned i = blockIdx.x * kFieldBlock + threadIdx.x;
+  if (i >= w * h * d) return;
+  lut[lut_index(i, w, h, d)] = make_float4(src[i * 3 + 0], src[i * 3 + 1], src[i * 3 + 2], 0.0f);
 }
 
 inline f3 host3(const float* v) { return {v[0], v[1], v[2]}; }
@@ -230,7 +243,7 @@ inline f3 host3(const float* v) { return {v[0], v[1], v[2]}; }
 }  // namespace
 
 cudaError_t launch_transmittance(const DevParams& P, float bottom, float4* out, cudaStream_t s) {
-  const int threads = 256;
+  const int threads = kTBlock;
   const int total = P.t_w * P.t_h * kTLanes;
   k_transmittance<<<(total + threads - 1) / threads, threads, 0, s>>>(P, bottom, out);
   return cudaGetLastError();
@@ -239,14 +252,17 @@ cudaError_t launch_transmittance(const DevParams& P, float bottom, float4* out, 
 cudaError_t launch_multi_scattering(const DevParams& P, float bottom, const float E[3], float ar,
                                     const float4* tlut, float4* out, unsigned long long* counter, cudaStream_t s) {
   if (P.ms_dirs > kMaxDirs || P.ms_steps > kMaxDirectionSteps) return cudaErrorInvalidValue;
-  // Four lanes a direction while that leaves the launch within one resident
-  // wave of threads, else one: the set-up is then repeated for nothing.
-  const int lanes = 4LL * P.ms_w * P.ms_h * P.ms_dirs <= kWaveThreads ? 4 : 1;
+  // The most lanes a direction that keep the launch within half a wave of the
+  // chip's threads, which is what fits at the kernel's registers.
+  const long long directions = (long long)P.ms_w * P.ms_h * P.ms_dirs;
+  const int lanes = 4 * directions <= kWaveThreads / 2 ? 4 : 2 * directions <= kWaveThreads / 2 ? 2 : 1;
   const int threads = ((lanes * P.ms_dirs + 31) / 32) * 32;
   const int blocks = P.ms_w * P.ms_h;
   const Frame F = make_frame(P, tlut, nullptr, bottom, ar, {0.0f, 1.0f, 0.0f}, host3(E));  // the texel's own sun in it
   if (lanes == 4)
     k_multi_scattering<4><<<blocks, threads, 0, s>>>(P, F, out, counter);
+  else if (lanes == 2)
+    k_multi_scattering<2><<<blocks, threads, 0, s>>>(P, F, out, counter);
   else
     k_multi_scattering<1><<<blocks, threads, 0, s>>>(P, F, out, counter);
   return cudaGetLastError();
@@ -256,7 +272,7 @@ cudaError_t launch_sky_view(const DevParams& P, float bottom, float cam_alt, flo
                             float ar, const float4* tlut, const float4* mslut, float4* out,
                             unsigned long long* counter, cudaStream_t s) {
   if (P.sv_steps > kMaxSkySteps) return cudaErrorInvalidValue;
-  const int threads = 256;
+  const int threads = kSkyBlock;
   const long long texels = (long long)P.sv_w * P.sv_h;
   const auto go = [&](auto kernel, int lanes) {
     kernel<<<unsigned((lanes * texels + threads - 1) / threads), threads, 0, s>>>(
@@ -280,7 +296,7 @@ cudaError_t launch_aerial(const DevParams& P, int width, int height, float botto
                           float tanfov, const float4* tlut, const float4* mslut, float4* out,
                           unsigned long long* counter, cudaStream_t s) {
   if (P.ap_steps > kMaxAerialSteps) return cudaErrorInvalidValue;
-  const int threads = 256;
+  const int threads = kAerialBlock;
   const long long total = 32LL * P.ap_w * P.ap_h;
   const float aspect = float(width) / float(height);
   k_aerial<<<unsigned((total + threads - 1) / threads), threads, 0, s>>>(
@@ -290,18 +306,12 @@ cudaError_t launch_aerial(const DevParams& P, int width, int height, float botto
 }
 
 cudaError_t launch_lut_to_fields(const float4* lut, int w, int h, int d, float* dst, cudaStream_t s) {
-  const size_t n = size_t(w) * h * d;
-  const int threads = 256;
-  const unsigned blocks = unsigned(std::min<size_t>((n + threads - 1) / threads, 4096));
-  k_lut_to_fields<<<blocks, threads, 0, s>>>(lut, w, h, d, dst);
+  k_lut_to_fields<<<(w * h * d - 1) / kFieldBlock + 1, kFieldBlock, 0, s>>>(lut, w, h, d, dst);
   return cudaGetLastError();
 }
 
 cudaError_t launch_fields_to_lut(const float* src, int w, int h, int d, float4* lut, cudaStream_t s) {
-  const size_t n = size_t(w) * h * d;
-  const int threads = 256;
-  const unsigned blocks = unsigned(std::min<size_t>((n + threads - 1) / threads, 4096));
-  k_fields_to_lut<<<blocks, threads, 0, s>>>(src, w, h, d, lut);
+  k_fields_to_lut<<<(w * h * d - 1) / kFieldBlock + 1, kFieldBlock, 0, s>>>(src, w, h, d, lut);
   return cudaGetLastError();
 }
 
