@@ -393,6 +393,30 @@ def check(rc: int) -> None:
     raise AtmError(rc, message)
 
 
+_current_raw_stream = None
+
+
+def stream(device) -> ctypes.c_void_p:
+    """The handle of ``device``'s current torch stream.  The raw handle is
+    0.1 us; ``torch.cuda.current_stream`` forms a Stream object on the way
+    (2 us, a fifth of a small call)."""
+
+    global _current_raw_stream
+    if _current_raw_stream is None:
+        import torch
+
+        torch.cuda.init()
+        _current_raw_stream = torch._C._cuda_getCurrentRawStream
+    if device.type != "cuda":
+        raise ValueError(f"Expected a cuda device, but got: {device}")
+    index = device.index
+    if index is None:
+        import torch
+
+        index = torch.cuda.current_device()
+    return ctypes.c_void_p(_current_raw_stream(index))
+
+
 def d3(values) -> ctypes.Array:
     return c_double3(*[float(v) for v in values])
 

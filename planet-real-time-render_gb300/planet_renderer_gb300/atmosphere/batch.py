@@ -96,7 +96,7 @@ class BatchedLutBuilder:
                                                      self._stream()))
 
     def _stream(self):
-        return ctypes.c_void_p(torch.cuda.current_stream(self.device).cuda_stream)
+        return _native.stream(self.device)
 
     def close(self):
         if getattr(self, "_handle", None) is not None and self._handle.value:

@@ -43,7 +43,7 @@ class Mlp:
         self._packed = False
 
     def _s(self):
-        return ctypes.c_void_p(torch.cuda.current_stream(self.device).cuda_stream)
+        return _native.stream(self.device)
 
     @staticmethod
     def _p(t: torch.Tensor):

@@ -39,10 +39,6 @@ _KINDS = {
 }
 
 
-def _stream_handle(device: torch.device) -> ctypes.c_void_p:
-    return ctypes.c_void_p(torch.cuda.current_stream(device).cuda_stream)
-
-
 class LutField:
     """One LUT of a renderer, readable like the reference's Taichi field."""
 
@@ -66,7 +62,7 @@ class LutField:
         r = self._renderer
         out = torch.empty(self.shape + (3,), dtype=torch.float32, device=r.device)
         _native.check(r._lib.atm_read_lut(r._handle, self.kind, ctypes.c_void_p(out.data_ptr()),
-                                          _stream_handle(r.device)))
+                                          _native.stream(r.device)))
         return out
 
     def to_numpy(self) -> np.ndarray:
@@ -78,7 +74,7 @@ class LutField:
         if tuple(src.shape) != self.shape + (3,):
             raise ValueError(f"expected shape {self.shape + (3,)}, got {tuple(src.shape)}")
         _native.check(r._lib.atm_load_lut(r._handle, self.kind, ctypes.c_void_p(src.data_ptr()),
-                                          _stream_handle(r.device)))
+                                          _native.stream(r.device)))
         torch.cuda.current_stream(r.device).synchronize()
 
     def from_numpy(self, values: np.ndarray) -> None:
@@ -219,7 +215,7 @@ class AtmosphereRenderer:
             sun_local /= max(float(np.linalg.norm(sun_local)), 1.0e-12)
         _native.check(self._lib.atm_update(self._handle, float(planet_radius_m), float(camera_radius_m),
                                            _native.d3(sun_local), _native.d3(solar_irradiance),
-                                           float(sun_angular_radius_degrees), _stream_handle(self.device)))
+                                           float(sun_angular_radius_degrees), _native.stream(self.device)))
 
     def prepare_frame(self, position_view, surface_id, planet_radius_m: float, camera_radius_m: float, sun_local,
                       solar_irradiance, sun_angular_radius_degrees: float, view_basis,
@@ -232,7 +228,7 @@ class AtmosphereRenderer:
             ctypes.byref(img), float(planet_radius_m), float(camera_radius_m), _native.d3(sun_local),
             _native.d3(solar_irradiance), float(sun_angular_radius_degrees), _native.d9(view_basis),
             float(tangent_half_fov), ctypes.c_void_p(self.surface_sun_transmittance.data_ptr()),
-            ctypes.c_void_p(self.surface_sky_radiance.data_ptr()), _stream_handle(self.device)))
+            ctypes.c_void_p(self.surface_sky_radiance.data_ptr()), _native.stream(self.device)))
 
     def composite(self, scene_hdr, space_hdr, surface_id, position_view, hdr, planet_radius_m: float,
                   camera_radius_m: float, sun_local, solar_irradiance, sun_disk_radiance,
@@ -249,7 +245,7 @@ class AtmosphereRenderer:
             _native.d3(sun_local), _native.d3(solar_irradiance), _native.d3(sun_disk_radiance),
             float(sun_angular_radius_degrees), _native.d9(view_basis), float(tangent_half_fov),
             float(star_contrast_start), float(star_contrast_end), int(diagnostic_view),
-            _stream_handle(self.device)))
+            _native.stream(self.device)))
 
     # ---- extensions ------------------------------------------------------------
     def composite_surrogate(self, scene_hdr, space_hdr, surface_id, position_view, hdr, planet_radius_m: float,
@@ -276,7 +272,7 @@ class AtmosphereRenderer:
             ctypes.c_void_p(hdr.data_ptr()), ctypes.byref(img), float(planet_radius_m), float(camera_radius_m),
             _native.d3(sun_local), _native.d3(solar_irradiance), _native.d3(sun_disk_radiance),
             float(sun_angular_radius_degrees), _native.d9(view_basis), float(tangent_half_fov),
-            float(star_contrast_start), float(star_contrast_end), ctypes.byref(sg), _stream_handle(self.device)))
+            float(star_contrast_start), float(star_contrast_end), ctypes.byref(sg), _native.stream(self.device)))
 
     def build_lut(self, kind: str, *, planet_radius_m: float, camera_altitude_m: float = 0.0,
                   sun_zenith_cosine: float = 1.0, sun_local=(0.0, 1.0, 0.0), solar_irradiance=(4.0, 3.9, 3.7),
@@ -295,7 +291,7 @@ class AtmosphereRenderer:
         a.tangent_half_fov = float(tangent_half_fov)
         a.frame_width, a.frame_height = self.width, self.height
         _native.check(self._lib.atm_build_lut(self._handle, _KINDS[kind], ctypes.byref(a),
-                                              _stream_handle(self.device)))
+                                              _native.stream(self.device)))
 
     def render_frame(self, gbuffer: dict, space_hdr, hdr, planet_radius_m: float, camera_radius_m: float,
                      sun_local, solar_irradiance, sun_disk_radiance, sun_angular_radius_degrees: float, view_basis,
@@ -340,7 +336,7 @@ class AtmosphereRenderer:
             _native.d3(sun_local), _native.d3(solar_irradiance), _native.d3(sun_disk_radiance),
             float(sun_angular_radius_degrees), _native.d9(view_basis), float(tangent_half_fov),
             float(star_contrast_start), float(star_contrast_end), None if sg is None else ctypes.byref(sg),
-            _stream_handle(self.device)))
+            _native.stream(self.device)))
 
     def sky_pixels(self, radiance, planet_radius_m: float, camera_radius_m: float, sun_local, solar_irradiance,
                    sun_angular_radius_degrees: float, view_basis, tangent_half_fov: float, mode: str = "plain",
@@ -362,7 +358,7 @@ class AtmosphereRenderer:
             self._handle, code, ctypes.c_void_p(radiance.data_ptr()), ctypes.byref(img), float(planet_radius_m),
             float(camera_radius_m), _native.d3(sun_local), _native.d3(solar_irradiance),
             float(sun_angular_radius_degrees), _native.d9(view_basis), float(tangent_half_fov),
-            None if sg is None else ctypes.byref(sg), _stream_handle(self.device)))
+            None if sg is None else ctypes.byref(sg), _native.stream(self.device)))
 
     def check(self) -> None:
         """Synchronise the stream and raise the device-side errors of earlier
@@ -370,12 +366,12 @@ class AtmosphereRenderer:
         ``composite_surrogate`` gave up: those pixels took the plain
         integrator).  Clears what it reports."""
 
-        _native.check(self._lib.atm_check(self._handle, _stream_handle(self.device)))
+        _native.check(self._lib.atm_check(self._handle, _native.stream(self.device)))
 
     def radiance_samples(self, reset: bool = False) -> int:
         """Radiance samples evaluated by composites (synchronises the stream)."""
 
         out = ctypes.c_uint64()
         _native.check(self._lib.atm_read_sample_counter(self._handle, 1 if reset else 0, ctypes.byref(out),
-                                                        _stream_handle(self.device)))
+                                                        _native.stream(self.device)))
         return int(out.value)

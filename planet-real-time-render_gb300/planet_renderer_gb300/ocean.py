@@ -221,11 +221,11 @@ class OceanRenderer:
                    seabed_albedo, seabed_normal, slope_variance, surface_id, surface_cell_id)
         image = self._image(tensors)
         imgs = _native.AtmOceanImages(*[ctypes.c_void_p(t.data_ptr()) for t in tensors])
-        stream = torch.cuda.current_stream(self.device).cuda_stream
+        stream = _native.stream(self.device)
         _native.check(self._lib.atm_ocean_rasterize(
             self._handle, ctypes.byref(imgs), ctypes.byref(image), float(planet_radius_m), float(camera_altitude_m),
             _native.d9(planet_frame), _native.d9(view_basis), float(tangent_half_fov), float(time_seconds),
-            int(debug_mode), ctypes.c_void_p(stream)))
+            int(debug_mode), stream))
 
     def rasterize_gbuffer(self, gbuffer: dict, *args, **kwargs) -> None:
         """``rasterize`` over a dict holding the images under the names
@@ -264,9 +264,9 @@ class OceanRenderer:
         out = {"height": np.zeros((CASCADES, n, n), np.float32), "gradient": np.zeros((CASCADES, n, n, 2), np.float32),
                "displacement": np.zeros((CASCADES, n, n, 2), np.float32),
                "jacobian": np.zeros((CASCADES, n, n, 4), np.float32)}
-        stream = torch.cuda.current_stream(self.device).cuda_stream
+        stream = _native.stream(self.device)
         _native.check(self._lib.atm_ocean_read_spectrum(self._handle, *(a.ctypes.data for a in out.values()),
-                                                        ctypes.c_void_p(stream)))
+                                                        stream))
         return out
 
     def close(self) -> None:

@@ -120,7 +120,7 @@ class PostProcessor:
         _native.check(self._lib.atm_post_process(
             self._handle, ctypes.c_void_p(hdr.data_ptr()), ctypes.c_void_p(display.data_ptr()), ctypes.byref(image),
             float(exposure_ev), 1 if bloom else 0, 1 if tone_map else 0,
-            ctypes.c_void_p(torch.cuda.current_stream(self.device).cuda_stream)))
+            _native.stream(self.device)))
 
     def bloom_plane(self) -> torch.Tensor:
         """Copy of the half-resolution bloom of the last ``process`` that ran
@@ -130,5 +130,5 @@ class PostProcessor:
         out = torch.empty((self.half_height, self.half_width, 4), dtype=torch.float32, device=self.device)
         dims = (ctypes.c_int32 * 2)()
         _native.check(self._lib.atm_post_read_bloom(self._handle, dims, ctypes.c_void_p(out.data_ptr()),
-                                                    ctypes.c_void_p(torch.cuda.current_stream(self.device).cuda_stream)))
+                                                    _native.stream(self.device)))
         return out[..., :3].permute(1, 0, 2).contiguous()

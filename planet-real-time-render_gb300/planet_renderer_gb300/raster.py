@@ -279,18 +279,18 @@ class TerrainRaster:
         m.n_active = n_active
         outs = _native.AtmRasterOutputs(*[ctypes.c_void_p(gbuffer[n].data_ptr() if n in gbuffer else None)
                                           for n in _native.RASTER_OUTPUTS])
-        stream = torch.cuda.current_stream(self.device).cuda_stream
+        stream = _native.stream(self.device)
         _native.check(self._lib.atm_raster_terrain(self._handle, ctypes.byref(m), float(near), float(tangent_half_fov),
                                                    int(view_mode), ctypes.byref(outs), ctypes.byref(image),
-                                                   ctypes.c_void_p(stream)))
+                                                   stream))
 
     def emitted(self) -> int:
         """Triangles the last frame emitted (``clipped_count``; synchronises
         the current stream).  Above ``capacity`` means some were dropped."""
 
         n = ctypes.c_int64()
-        stream = torch.cuda.current_stream(self.device).cuda_stream
-        _native.check(self._lib.atm_raster_emitted(self._handle, ctypes.byref(n), ctypes.c_void_p(stream)))
+        stream = _native.stream(self.device)
+        _native.check(self._lib.atm_raster_emitted(self._handle, ctypes.byref(n), stream))
         return int(n.value)
 
     def close(self) -> None:

@@ -130,4 +130,4 @@ def shade_surface(gbuffer: dict, sun_transmittance: torch.Tensor, sky_radiance: 
                                      sun_angular_radius, tangent_half_fov, mode, layout, ocean_surface_id)
     lib = _native.library()
     _native.check(lib.atm_shade_surface(ctypes.byref(p), ctypes.byref(ptrs), ctypes.byref(image),
-                                        ctypes.c_void_p(torch.cuda.current_stream(surface_hdr.device).cuda_stream)))
+                                        _native.stream(surface_hdr.device)))
