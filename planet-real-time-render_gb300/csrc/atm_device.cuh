@@ -22,16 +22,16 @@ namespace atm {
 constexpr float kPiF = 3.14159265358979323846f;  // f32(math.pi), renderer.py:12
 constexpr float kLargeF = 1.0e30f;               // _LARGE_DISTANCE, :13
 
-// A 2D LUT's size as its bilinear tap reads it: width and height, the largest
-// texel coordinates, 2^23 plus the last texel that has a right (lower)
-// neighbour, and the row pitch.  LUTs are at least 2 x 2.
+// A 2D LUT's size as its bilinear tap reads it: width and height, 2^23 plus
+// the last texel that has a right (lower) neighbour, and the row pitch.  LUTs
+// are at least 2 x 2.
 struct LutDims {
-  float w, h, x_max, y_max, x_last, y_last;
+  float w, h, x_last, y_last;
   int pitch;
 };
 constexpr float kMagic = 8388608.0f;  // 2^23: adding it leaves floor(x) in the low mantissa bits
 __host__ __device__ inline LutDims lut_dims(int w, int h) {
-  return {float(w), float(h), float(w - 1), float(h - 1), kMagic + float(w - 2), kMagic + float(h - 2), w};
+  return {float(w), float(h), kMagic + float(w - 2), kMagic + float(h - 2), w};
 }
 
 // Parameters rounded to float exactly where the Taichi trace rounds them
@@ -133,19 +133,30 @@ __device__ __forceinline__ Seg seg_then(Seg a, Seg b) { return {a.L + a.T * b.L,
 struct Density {
   float r, m, o;
 };
+// Zero outside the shell: at an infinite altitude the exponentials are 0 and
+// the ozone tent has ended.
 __device__ __forceinline__ Density density(const DevParams& P, float h) {
-  const bool inside = 0.0f <= h && h <= P.top;
+  const float a = 0.0f <= h && h <= P.top ? h : INFINITY;
   Density d;
-  d.r = inside ? fexp2(h * P.exp2_r) : 0.0f;
-  d.m = inside ? fexp2(h * P.exp2_m) : 0.0f;
-  d.o = inside ? mx(1.0f - fabsf(h - P.oz_peak) * P.inv_oz_half, 0.0f) : 0.0f;
+  d.r = fexp2(a * P.exp2_r);
+  d.m = fexp2(a * P.exp2_m);
+  d.o = mx(1.0f - fabsf(a - P.oz_peak) * P.inv_oz_half, 0.0f);
   return d;
+}
+// Extinction and scattering of one density share the Rayleigh products.
+struct Medium {
+  f3 ext, scat;
+};
+__device__ __forceinline__ Medium medium_of(const DevParams& P, Density d) {
+  const f3 r = arr3(P.beta_r) * d.r;
+  Medium m;
+  m.ext = {fmaf(P.beta_o[0], d.o, fmaf(P.beta_me[0], d.m, r.x)), fmaf(P.beta_o[1], d.o, fmaf(P.beta_me[1], d.m, r.y)),
+           fmaf(P.beta_o[2], d.o, fmaf(P.beta_me[2], d.m, r.z))};
+  m.scat = {fmaf(P.beta_ms[0], d.m, r.x), fmaf(P.beta_ms[1], d.m, r.y), fmaf(P.beta_ms[2], d.m, r.z)};
+  return m;
 }
 __device__ __forceinline__ f3 extinction_of(const DevParams& P, Density d) {
   return (arr3(P.beta_r) * d.r + arr3(P.beta_me) * d.m) + arr3(P.beta_o) * d.o;
-}
-__device__ __forceinline__ f3 scattering_of(const DevParams& P, Density d) {
-  return arr3(P.beta_r) * d.r + arr3(P.beta_ms) * d.m;
 }
 
 // ---- shells and intervals (:211-408) ---------------------------------------
@@ -505,10 +516,10 @@ __device__ __forceinline__ float sun_u_to_cosine(float u, float h, float bottom)
   return clampf(c, -1.0f, 1.0f);
 }
 __device__ __forceinline__ float sun_cosine_to_u(float c, float hc) {
-  const bool below = c < hc;
-  const float n = __saturatef(fabsf(c - hc) * frcp(mx(1.0f + (below ? hc : -hc), 1.0e-6f)));
-  const float s = 0.5f * fsqrt(n);
-  return below ? 0.5f - s : 0.5f + s;
+  const float t = c - hc;
+  const float side = copysignf(1.0f, t);  // -1 below the horizon
+  const float n = __saturatef(fabsf(t) * frcp(mx(fmaf(side, -hc, 1.0f), 1.0e-6f)));
+  return fmaf(0.5f * side, fsqrt(n), 0.5f);
 }
 
 // ---- LUT sampling -----------------------------------------------------------
@@ -516,20 +527,19 @@ __device__ __forceinline__ float sun_cosine_to_u(float c, float hc) {
 // (:618-640, :655-683, :1503-1525).  The texel index is formed in float (2^23
 // plus an integer below 2^23 is exact), which keeps the conversions off the
 // XU pipe and the index arithmetic off the ALU, the two pipes a march is
-// short of; the last texel is the right end of the last pair (fx = 1), so
-// the four taps are two addresses apart by constants.
+// short of; past the last texel's centre the last pair's weight saturates at
+// its right end, so the four taps are two addresses apart by constants.
 __device__ __forceinline__ f3 bilinear(const float4* __restrict__ lut, const LutDims& D, float u, float v) {
-  const float x = clampf(fmaf(u, D.w, -0.5f), 0.0f, D.x_max);
-  const float y = clampf(fmaf(v, D.h, -0.5f), 0.0f, D.y_max);
+  const float x = mx(fmaf(u, D.w, -0.5f), 0.0f);
+  const float y = mx(fmaf(v, D.h, -0.5f), 0.0f);
   const float xm = mn(__fadd_rd(x, kMagic), D.x_last);
   const float yf = mn(__fadd_rd(y, kMagic), D.y_last) - kMagic;
-  const float fx = x - (xm - kMagic);
-  const float fy = y - yf;
+  const float fx = __saturatef(x - (xm - kMagic));
+  const float fy = __saturatef(y - yf);
   const float4* t = lut + (__float_as_int(fmaf(yf, D.w, xm)) & 0x7fffff);
   const float4* t1 = t + D.pitch;
   const float4 a = __ldg(t), b = __ldg(t + 1), c = __ldg(t1), d = __ldg(t1 + 1);
-  const float gx = 1.0f - fx, gy = 1.0f - fy;
-  const float wa = gx * gy, wb = fx * gy, wc = gx * fy, wd = fx * fy;
+  const float wd = fx * fy, wc = fy - wd, wb = fx - wd, wa = (1.0f - fx) - wc;
   return {fmaf(d.x, wd, fmaf(c.x, wc, fmaf(b.x, wb, a.x * wa))), fmaf(d.y, wd, fmaf(c.y, wc, fmaf(b.y, wb, a.y * wa))),
           fmaf(d.z, wd, fmaf(c.z, wc, fmaf(b.z, wb, a.z * wa)))};
 }
@@ -576,7 +586,7 @@ inline f3 sky_view_sun(float sun_cos) {
 // zenith angle.  The distance to the shell top is then sqrt(rc^2 + shell2 -
 // rho2) - rc.
 __device__ __forceinline__ f3 sample_t_at(const DevParams& P, const Frame& F, float h, float rho2, float rho, float rc) {
-  const float d = mx(fsqrt(mx(fmaf(rc, rc, F.shell2 - rho2), 0.0f)) - rc, 0.0f);
+  const float d = fsqrt(mx(fmaf(rc, rc, F.shell2 - rho2), 0.0f)) - rc;  // below 0 only above the shell
   const float dmin = P.top - h;
   const float u = __saturatef((d - dmin) * frcp(mx((rho + F.shell_top) - dmin, 1.0e-6f)));
   const float v = __saturatef(rho * F.inv_shell_top);
@@ -669,34 +679,55 @@ __device__ __forceinline__ float mie_phase(const DevParams& P, float c) {
 // f32 when x is small: centimetre segments next to a camera standing on the
 // ground give x ~ 1e-7 and a weight with no significant digit left (its own
 // f32 result is then percents away from its f64 one).  Up to x = 1 both come
-// from phi = (1 - e^-x) / x = e^(-x/2) sinh(x/2) / (x/2), the series in
-// (x/2)^2 cut where it is 1e-8: weight step phi, T = 1 - x phi (step itself
-// at ext = 0, as the reference's ext <= 1e-12 branch).  One exponential, no
-// division and no branch a channel; larger x take 1 - T, which keeps 7 digits.
-__device__ __forceinline__ void segment_thin(float x, float step, float& tr, float& w) {
-  const float z = x * x;
-  const float p = fmaf(z, fmaf(z, fmaf(z, 1.0f / 322560.0f, 1.0f / 1920.0f), 1.0f / 24.0f), 1.0f);
-  const float phi = fexp2(x * -0.72134752044448170f) * p;  // 2^(-x log2(e) / 2)
-  tr = fmaf(-x, phi, 1.0f);
-  w = phi * step;
+// from phi = (1 - e^-x) / x: weight = step phi, T = 1 - ext weight (step
+// itself at ext = 0, as the reference's ext <= 1e-12 branch).  phi is a
+// polynomial, near-minimax with phi(0) = 1: degree 4 up to x = 1/4, which
+// most segments are within, degree 6 up to 1, 2.9e-9 and 2.7e-9 off; a
+// rounding error each in float, 4 and 6 operations a channel, against 7 and
+// 2^x for the form e^(-x/2) sinh(x/2) / (x/2).  Larger x take 1 - T, which
+// keeps 7 digits.
+__device__ __forceinline__ float phi_quarter(float x) {
+  return fmaf(x, fmaf(x, fmaf(x, fmaf(x, 0.007530156057327986f, -0.04150012508034706f), 0.1666528880596161f),
+                      -0.49999964237213135f), 1.0f);
+}
+__device__ __forceinline__ float phi_one(float x) {
+  const float high = fmaf(x, fmaf(x, 0.00012912976671941578f, -0.0013011228293180466f), 0.008276204578578472f);
+  return fmaf(x, fmaf(x, fmaf(x, fmaf(x, high, -0.04164746776223183f), 0.16666366159915924f), -0.49999985098838806f),
+              1.0f);
 }
 __device__ __forceinline__ void segment_any(float ext, float x, float step, float& tr, float& w) {
-  segment_thin(mn(x, 1.0f), step, tr, w);
+  w = phi_one(mn(x, 1.0f)) * step;
+  tr = fmaf(-w, ext, 1.0f);
   if (x > 1.0f) {
     tr = fexp2(mn(x, 80.0f) * -1.4426950408889634f);
     w = (1.0f - tr) * frcp(ext);
   }
 }
-__device__ __forceinline__ void segment_integral(f3 ext, float step, f3& tr, f3& integ) {
+__device__ __forceinline__ void segment_integral(f3 ext, float step, f3& tr, f3& w) {
   const f3 x = ext * step;
-  if (mx(mx(x.x, x.y), x.z) <= 1.0f) {
-    segment_thin(x.x, step, tr.x, integ.x);
-    segment_thin(x.y, step, tr.y, integ.y);
-    segment_thin(x.z, step, tr.z, integ.z);
+  if (mx(mx(x.x, x.y), x.z) <= 0.25f) {
+    w = mk(phi_quarter(x.x), phi_quarter(x.y), phi_quarter(x.z)) * step;
+    tr = {fmaf(-w.x, ext.x, 1.0f), fmaf(-w.y, ext.y, 1.0f), fmaf(-w.z, ext.z, 1.0f)};
   } else {
-    segment_any(ext.x, x.x, step, tr.x, integ.x);
-    segment_any(ext.y, x.y, step, tr.y, integ.y);
-    segment_any(ext.z, x.z, step, tr.z, integ.z);
+    segment_any(ext.x, x.x, step, tr.x, w.x);
+    segment_any(ext.y, x.y, step, tr.y, w.y);
+    segment_any(ext.z, x.z, step, tr.z, w.z);
+  }
+}
+// A segment of extinction ext and source src a metre after what acc holds.
+__device__ __forceinline__ void then_segment(Seg& acc, f3 src, f3 ext, float step) {
+  const f3 x = ext * step;
+  const float thickest = mx(mx(x.x, x.y), x.z);
+  if (thickest <= 1.0f) {
+    const f3 phi = thickest <= 0.25f ? mk(phi_quarter(x.x), phi_quarter(x.y), phi_quarter(x.z))
+                                     : mk(phi_one(x.x), phi_one(x.y), phi_one(x.z));
+    const f3 a = acc.T * (phi * step);
+    acc.L = {fmaf(a.x, src.x, acc.L.x), fmaf(a.y, src.y, acc.L.y), fmaf(a.z, src.z, acc.L.z)};
+    acc.T = {fmaf(-a.x, ext.x, acc.T.x), fmaf(-a.y, ext.y, acc.T.y), fmaf(-a.z, ext.z, acc.T.z)};
+  } else {
+    f3 t, w;
+    segment_integral(ext, step, t, w);
+    acc = seg_then(acc, {src * w, t});
   }
 }
 
@@ -731,7 +762,7 @@ __device__ __forceinline__ RaySource make_ray_source(const DevParams& P, const F
 }
 
 // The medium and the sun at the middle of a segment [start, end] of the ray:
-// density, segment transmittance T and in-scattering weight, finite-disk sun
+// density, extinction and scattering, the segment's length, finite-disk sun
 // transmittance st and disk visibility, altitude h, sun cosine sc, horizon
 // cosine hc.  The sample's radius is bottom + h (its altitude on the ray) and
 // its sun cosine (p(t0) . sun + (t - t0) ray . sun) / radius; the reference
@@ -743,17 +774,18 @@ __device__ __forceinline__ RaySource make_ray_source(const DevParams& P, const F
 // the shell top; 1/r by one rsqrt gives r, both cosines and the horizon's
 // sine.  Altitude and sun cosine keep the operations that decide where the
 // density is cut off (delta's sign).  With the tap and the segment weight
-// above, a 1080p composite from 2 km went from 1369 to 839 us (1.48e9 to
-// 0.92e9 warp instructions).
+// above, a 1080p composite from 2 km went from 1369 to 782 us (1.48e9 to
+// 0.86e9 warp instructions).
 struct MarchSample {
   Density d;
-  f3 T, weight, st;
-  float vis, h, sc, hc;
+  Medium medium;
+  f3 st;
+  float step, vis, h, sc, hc;
 };
 __device__ __forceinline__ MarchSample march_sample(const DevParams& P, const Frame& F, const RaySource& R,
                                                     float start, float end) {
   MarchSample m;
-  const float step = mx(end - start, 0.0f);
+  m.step = mx(end - start, 0.0f);
   const float u = (start + end) * 0.5f - R.t0;
   const float delta = fmaf(u, u, fmaf(R.q1, u, R.q0));
   const float r2 = mx(fmaf(F.bottom, F.bottom, delta), 1.0f);
@@ -761,7 +793,7 @@ __device__ __forceinline__ MarchSample march_sample(const DevParams& P, const Fr
   const float r = r2 * inv_r;
   m.h = delta * frcp(r + F.bottom);
   m.d = density(P, m.h);
-  segment_integral(extinction_of(P, m.d), step, m.T, m.weight);
+  m.medium = medium_of(P, m.d);
   const float rc = fmaf(u, R.r_sun, R.s0);
   m.sc = rc * inv_r;
   const Horizon H = horizon_of(mx(delta, 0.0f), inv_r, F.bottom);
@@ -770,15 +802,16 @@ __device__ __forceinline__ MarchSample march_sample(const DevParams& P, const Fr
   return m;
 }
 
-// One constant-source segment [start, end] of the ray: _scattering_segment
-// :858-899 with _scattering_source :818-856.  Returns (L, T) and the finite
-// disk visibility at the sample.
-__device__ __forceinline__ Seg source_segment(const DevParams& P, const Frame& F, const RaySource& R, float start,
-                                              float end, float& vis) {
+// _scattering_source :818-856 at a sample.
+__device__ __forceinline__ f3 source_of(const DevParams& P, const Frame& F, const RaySource& R, const MarchSample& m) {
+  return m.st * (R.ER * m.d.r + R.EM * m.d.m) + m.medium.scat * sample_ms(P, F, m.h, m.sc, m.hc);
+}
+// One constant-source segment [start, end] of the ray after what acc holds:
+// _scattering_segment :858-899.
+__device__ __forceinline__ void then_source_segment(const DevParams& P, const Frame& F, const RaySource& R,
+                                                    float start, float end, Seg& acc) {
   const MarchSample m = march_sample(P, F, R, start, end);
-  vis = m.vis;
-  const f3 src = m.st * (R.ER * m.d.r + R.EM * m.d.m) + scattering_of(P, m.d) * sample_ms(P, F, m.h, m.sc, m.hc);
-  return {src * m.weight, m.T};
+  then_segment(acc, source_of(P, F, R, m), m.medium.ext, m.step);
 }
 
 // The base intervals [i0, i1) of n of a ray's march: source segments without
@@ -796,8 +829,7 @@ __device__ __forceinline__ Seg march(const DevParams& P, const Frame& F, const R
       half = warp_half(w, true);
     }
     const float d1 = warp_at(half, fraction(i + 1));
-    float vis;
-    acc = seg_then(acc, source_segment(P, F, R, d0, d1, vis));
+    then_source_segment(P, F, R, d0, d1, acc);
     d0 = d1;
   }
   return acc;

@@ -209,17 +209,19 @@ __device__ __forceinline__ DivideFractions divide_fractions(const DevParams& P) 
   return {{float(P.limb_steps)}, {float(P.substeps)}};
 }
 
-// One base interval [d0, d1] with its terminator refinement (:901-1031).
+// One base interval [d0, d1] with its terminator refinement (:901-1031) after
+// what acc holds.
 template <class Fractions>
-__device__ __forceinline__ Seg surface_interval_seg(const DevParams& P, const Frame& F, const SurfaceMarch& M, float d0,
-                                                    float d1, const Fractions& fractions, uint32_t& samples) {
-  float vis;
-  Seg coarse = source_segment(P, F, M.rs, d0, d1, vis);
+__device__ __forceinline__ void then_surface_interval(const DevParams& P, const Frame& F, const SurfaceMarch& M,
+                                                      float d0, float d1, const Fractions& fractions,
+                                                      uint32_t& samples, Seg& acc) {
+  const MarchSample m = march_sample(P, F, M.rs, d0, d1);
+  const f3 src = source_of(P, F, M.rs, m);
   ++samples;
   // _terminator_refinement_weight :901-966; zero unless a shadow-cylinder
   // root exists or the disk is partly hidden at the midpoint
   float w = 0.0f;
-  if ((M.sv0 || M.sv1) || (vis > 0.0f && vis < 1.0f)) {
+  if ((M.sv0 || M.sv1) || (m.vis > 0.0f && m.vis < 1.0f)) {
     float mid = (d0 + d1) * 0.5f;
     float iw = mx(d1 - d0, 1.0e-4f);
     float closest_root = 1.0e30f;
@@ -227,25 +229,24 @@ __device__ __forceinline__ Seg surface_interval_seg(const DevParams& P, const Fr
     if (M.sv1) closest_root = mn(closest_root, fabsf(mid - M.sr1));
     float prox = __saturatef(2.0f - fdiv(closest_root, iw));
     prox = prox * prox * (3.0f - 2.0f * prox);
-    w = mx(prox, 4.0f * vis * (1.0f - vis));
+    w = mx(prox, 4.0f * m.vis * (1.0f - m.vis));
   }
-  Seg interval = coarse;
-  if (w > 0.0f) {
-    // _integrate_adaptive_scattering_interval :998-1031
-    const int nsub = P.substeps;
-    Seg fine = {splat(0.0f), splat(1.0f)};
-    float c0 = d0;
-    for (int k = 0; k < nsub; ++k) {
-      float c1 = fmaf(d1 - d0, fractions.sub(k + 1), d0);
-      float cvis;
-      fine = seg_then(fine, source_segment(P, F, M.rs, c0, c1, cvis));
-      c0 = c1;
-    }
-    samples += nsub;
-    interval.L = coarse.L * (1.0f - w) + fine.L * w;
-    interval.T = coarse.T * (1.0f - w) + fine.T * w;
+  if (!(w > 0.0f)) {
+    then_segment(acc, src, m.medium.ext, m.step);
+    return;
   }
-  return interval;
+  // _integrate_adaptive_scattering_interval :998-1031
+  Seg coarse = {splat(0.0f), splat(1.0f)}, fine = coarse;
+  then_segment(coarse, src, m.medium.ext, m.step);
+  const int nsub = P.substeps;
+  float c0 = d0;
+  for (int k = 0; k < nsub; ++k) {
+    float c1 = fmaf(d1 - d0, fractions.sub(k + 1), d0);
+    then_source_segment(P, F, M.rs, c0, c1, fine);
+    c0 = c1;
+  }
+  samples += nsub;
+  acc = seg_then(acc, {coarse.L * (1.0f - w) + fine.L * w, coarse.T * (1.0f - w) + fine.T * w});
 }
 
 // The base intervals [i0, i1) of a surface march, in ray order.
@@ -263,7 +264,7 @@ __device__ __forceinline__ Seg surface_march(const DevParams& P, const Frame& F,
       half = warp_half(M.rw, true);
     }
     const float d1 = warp_at(half, fractions.limb(i + 1));
-    acc = seg_then(acc, surface_interval_seg(P, F, M, d0, d1, fractions, samples));
+    then_surface_interval(P, F, M, d0, d1, fractions, samples, acc);
     d0 = d1;
   }
   return acc;

@@ -129,10 +129,12 @@ __global__ void __maxnreg__(72) k_multi_scattering(DevParams P, Frame F,
         }
         const float d1 = warp_at(half, s_fraction[i + 1]);
         const MarchSample m = march_sample(P, F, R, d0, d1);
-        const f3 t = pT * m.weight;
-        dL = dL + t * (m.st * (R.ER * m.d.r + R.EM * m.d.m));
-        dF = dF + t * scattering_of(P, m.d);
-        pT = pT * m.T;
+        f3 t, w;
+        segment_integral(m.medium.ext, m.step, t, w);
+        w = pT * w;
+        dL = dL + w * (m.st * (R.ER * m.d.r + R.EM * m.d.m));
+        dF = dF + w * m.medium.scat;
+        pT = pT * t;
         d0 = d1;
       }
       samples = uint32_t(i1 - i0);

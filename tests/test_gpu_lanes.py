@@ -102,6 +102,26 @@ def test_luts_match_oracle_at_each_lane_count(sky, ms, dirs, oracle_f32):
     assert_parity(r.aerial_scattering_lut.to_numpy(), ap, "aerial, three slices a lane")
 
 
+# segments of optical thickness below 1/4, across it, across 1 and beyond: steps of a few to 80 km
+@pytest.mark.parametrize("scale", [0.0, 1.0, 6.0, 40.0, 2000.0])
+def test_segments_of_every_thickness(scale, oracle_f32):
+    from planet_renderer_gb300.atmosphere import AtmosphereRenderer
+    from planet_renderer_gb300.atmosphere.config import earth_baseline
+
+    cfg = earth_baseline()
+    cfg = dataclasses.replace(cfg, sky_view_lut_width=32, sky_view_lut_height=24, sky_view_steps=12,
+                              rayleigh_scattering_per_m=tuple(scale * v for v in cfg.rayleigh_scattering_per_m))
+    r = AtmosphereRenderer(16, 9, cfg)
+    kw = dict(planet_radius_m=R, camera_altitude_m=500.0, sun_zenith_cosine=0.25, sun_local=(0.9682458, 0.25, 0.0))
+    for kind in ("transmittance", "multi_scattering", "sky_view"):
+        r.build_lut(kind, **kw)
+    ar = float(np.float32(np.radians(0.266)))
+    t = oracle_f32.build_transmittance(cfg, R)
+    m = oracle_f32.build_multi_scattering(cfg, R, E, ar, t)
+    assert_parity(r.multi_scattering_lut.to_numpy(), m, "multi-scattering")
+    assert_parity(r.sky_view_lut.to_numpy(), oracle_f32.build_sky_view(cfg, R, 500.0, 0.25, E, ar, t, m), "sky-view")
+
+
 @pytest.mark.parametrize("n_in", [12, 13, 14])
 def test_tcgen05_bias_inputs(n_in):
     """The bias's three inputs beside the network's (13 leave room) and in a step of their own (14 do not)."""
