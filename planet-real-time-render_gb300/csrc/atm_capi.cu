@@ -1497,7 +1497,7 @@ struct AtmRaster {
   int32_t width = 0, height = 0, max_patches = 0, triangles_per_patch = 0;
   atm::RasterTri* tris = nullptr;
   long long capacity = 0;
-  uint32_t* count = nullptr;  // emitted, large, spare
+  uint32_t* count = nullptr;  // emitted, large, a 64-bit ticket, the 64-bit counter of listed triangles
   uint32_t* large = nullptr;
   uint32_t* large_tiles = nullptr;
   unsigned long long* tile_prefix = nullptr;
@@ -1524,7 +1524,7 @@ ATM_API int atm_raster_create(int32_t width, int32_t height, int32_t max_patches
   r->triangles_per_patch = triangles_per_patch;
   r->capacity = capacity;
   cudaError_t e = cudaMalloc(&r->tris, sizeof(atm::RasterTri) * size_t(capacity));
-  if (e == cudaSuccess) e = cudaMalloc(&r->count, 4 * sizeof(uint32_t));
+  if (e == cudaSuccess) e = cudaMalloc(&r->count, 6 * sizeof(uint32_t));
   if (e == cudaSuccess) e = cudaMalloc(&r->large, sizeof(uint32_t) * size_t(capacity));
   if (e == cudaSuccess) e = cudaMalloc(&r->large_tiles, sizeof(uint32_t) * size_t(capacity));
   if (e == cudaSuccess) e = cudaMalloc(&r->tile_prefix, sizeof(unsigned long long) * (size_t(capacity) + 1));
@@ -1588,7 +1588,8 @@ ATM_API int atm_raster_terrain(AtmRaster* r, const AtmRasterMesh* m, double near
                        m->cell,       m->triangles,  m->active_slots, m->skirt_mask,
                        m->slot_level, m->patches,    m->vertices_per_patch, m->triangles_per_patch,
                        m->surface_triangles_per_patch, m->resolution, m->n_active};
-  atm::RasterStream S{r->tris, r->count, r->capacity, r->large, r->large_tiles, r->tile_prefix, r->block_sums};
+  atm::RasterStream S{r->tris, r->count, r->capacity, r->large, r->large_tiles, r->tile_prefix, r->block_sums,
+                      reinterpret_cast<unsigned long long*>(r->count + 4)};
   if (o->terrain_surface_id && (!o->terrain_position || !o->terrain_normal || !o->terrain_albedo))
     return fail(ATM_E_INVALID, "the terrain snapshot needs position, normal and albedo images");
   atm::RasterOutDev O{o->depth,          o->position,        o->normal,           o->albedo,

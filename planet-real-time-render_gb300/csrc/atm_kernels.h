@@ -317,6 +317,7 @@ struct RasterStream {
   uint32_t* large_tiles;           // capacity: their pixel-tile counts
   unsigned long long* tile_prefix; // capacity + 1: exclusive prefix of the tile counts
   unsigned long long* block_sums;  // kRasterScanBlocks + 1: the prefix's per-block partial sums
+  unsigned long long* listed;      // large triangles and their tiles in one counter (k_raster_depth)
 };
 constexpr int kRasterScanBlocks = 256;
 struct RasterMeshDev {

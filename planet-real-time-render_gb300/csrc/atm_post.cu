@@ -169,9 +169,9 @@ __device__ __forceinline__ BlurRow taps_fast(const BlurRow& v, const BlurLane& l
 // One pass: next() gives its output rows one after another from `row` on,
 // pulling the rows of the pass (or the plane) before it as it needs them.
 // Rows past either end of the plane are the end row's again.
+struct BlurPlane;
 template <bool kXFast, class Source>
 struct BlurPass {
-  static constexpr bool kEndless = false;
   Source src;
   BlurLane lane;
   int row, last, rows;  // the next output row, the last row pulled, rows of the plane
@@ -181,7 +181,7 @@ struct BlurPass {
 #pragma unroll
     for (int k = 0; k < 4; ++k) w[k] = w[k + 1];
     w[4] = end;
-    if (Source::kEndless || last < rows - 1) {
+    if (std::is_same_v<Source, BlurPlane> || last < rows - 1) {  // the plane repeats its last row itself
       const BlurRow v = src.next();
       w[4] = kXFast ? taps_fast(v, lane) : v;  // x first, along the fast axis
       ++last;
@@ -205,7 +205,6 @@ struct BlurPass {
 };
 // The rows of the plane, one read ahead; after the last one, it again.
 struct BlurPlane {
-  static constexpr bool kEndless = true;
   const float4 *p, *q;  // of the lane's texels
   size_t pitch;
   int left;  // rows behind p

@@ -9,10 +9,10 @@
 //    plane and the four frustum sides, and the emission (an atomic append)
 //    of each resulting triangle with its screen setup: projection snapped to
 //    1/256 pixel, edge equations, top-left flags, inverse area;
-//  * k_raster_depth (+ k_raster_scan_*, k_raster_depth_tiles): coverage
+//  * k_raster_depth (and k_raster_depth_tiles): coverage
 //    by the edge equations with the top-left rule and a 64-bit atomic
 //    minimum of (depth bits << 32 | triangle) per pixel; small triangles by
-//    one thread, medium ones by a warp, large ones cut into 8 x 32 pixel
+//    eight lanes, medium ones by a warp, large ones cut into 8 x 32 pixel
 //    tiles spread over the whole grid;
 //  * k_raster_resolve: thread per pixel: the winning triangle's
 //    perspective-correct position, normal, material weights and height, the
@@ -262,7 +262,7 @@ __device__ __forceinline__ Box bbox(const RasterSetup& T, const ImageLayout& L) 
   return {max(int(floorf(fmn(fmn(ax, bx), cx))), 0), min(int(ceilf(fmx(fmx(ax, bx), cx))), L.width - 1),
           max(int(floorf(fmn(fmn(ay, by), cy))), 0), min(int(ceilf(fmx(fmx(ay, by), cy))), L.height - 1)};
 }
-constexpr long long kRasterThreadArea = 16;  // bounding boxes up to this many pixels: one thread
+constexpr long long kRasterLanesArea = 16;   // bounding boxes up to this many pixels: kDepthLanes lanes
 constexpr long long kRasterWarpArea = 256;   // up to this: one warp; larger: tiles over the whole grid
 constexpr int kRasterTileW = 256, kRasterTileH = 32;  // a large triangle's work item: 256 columns x 32 rows
 constexpr int kRasterItemsPerTicket = 4;              // work items a warp takes per ticket
@@ -347,53 +347,78 @@ __device__ __forceinline__ void warp_block(const RasterSetup& T, unsigned long l
   }
 }
 
-// Thread per emitted triangle (grid-stride, warp-aligned): small boxes are
-// walked by their own thread, medium ones by the whole warp in turn, large
-// ones are listed for k_raster_depth_tiles.
-__global__ void __launch_bounds__(256) k_raster_depth(RasterStream S, ImageLayout L,
+// Lanes take the pixels of a box of at most 256 in turn: pixel k of it.
+__device__ __forceinline__ void box_pixels(const RasterSetup& T, const Box& b, int first, int stride, int H,
+                                           unsigned long long* __restrict__ depth_key, unsigned long long q) {
+  const int bh = b.y1 - b.y0 + 1, area = (b.x1 - b.x0 + 1) * bh;
+  const unsigned inv = (65535u + unsigned(bh)) / unsigned(bh);  // k inv >> 16 = k / bh for k, bh <= 256
+  for (int k = first; k < area; k += stride) {
+    const int column = int((unsigned(k) * inv) >> 16);
+    depth_pixel(T, b.x0 + column, b.y0 + (k - column * bh), H, depth_key, q);
+  }
+}
+
+// kDepthLanes lanes per emitted triangle (grid-stride, warp-aligned): small
+// boxes are walked by those lanes, medium ones by the whole warp in turn,
+// large ones are listed for k_raster_depth_tiles.  Latency-bound, by the
+// medium boxes that a warp walks one after another: with a lane a triangle,
+// 32 of them a warp, a 1366x767 frame of a terrain of 98,000 triangles took 70
+// us, on 8% of the warps; four a warp take 24.
+//
+// tile_bits > 0: one 64-bit counter holds the listed triangles (high bits) and
+// their tiles (the low tile_bits), so that an entry's index and its tiles'
+// exclusive prefix come from one atomic and the list is sorted by the prefix
+// (the three scans were 13 us).  0: only the tile counts are listed, for the scans below.
+constexpr int kDepthLanes = 8, kDepthTris = 32 / kDepthLanes;
+__global__ void __launch_bounds__(256) k_raster_depth(RasterStream S, ImageLayout L, int tile_bits,
                                                       unsigned long long* __restrict__ depth_key) {
-  const int lane = threadIdx.x & 31;
+  const int lane = threadIdx.x & 31, sub = lane % kDepthLanes;
   const long long n = min((long long)S.count[0], (long long)S.capacity);
-  const long long stride = (long long)gridDim.x * blockDim.x;
-  for (long long base = blockIdx.x * (long long)blockDim.x + (threadIdx.x & ~31); base < n; base += stride) {
-    const long long q = base + lane;
+  const long long warp = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
+  const long long stride = ((long long)gridDim.x * blockDim.x >> 5) * kDepthTris;
+  for (long long base = warp * kDepthTris; base < n; base += stride) {
+    const long long q = base + lane / kDepthLanes;
     bool medium = false;
     if (q < n) {
       const RasterSetup T = load_setup(S.tris + q);
       const Box b = bbox(T, L);
       if (T.inv_area > 0.0f && b.x0 <= b.x1 && b.y0 <= b.y1) {
         const long long area = (long long)(b.x1 - b.x0 + 1) * (b.y1 - b.y0 + 1);
-        if (area <= kRasterThreadArea) {
-          for (int x = b.x0; x <= b.x1; ++x)
-            for (int y = b.y0; y <= b.y1; ++y) depth_pixel(T, x, y, L.height, depth_key, (unsigned long long)q);
+        if (area <= kRasterLanesArea) {
+          box_pixels(T, b, sub, kDepthLanes, L.height, depth_key, (unsigned long long)q);
         } else if (area <= kRasterWarpArea) {
           medium = true;
-        } else {
-          const uint32_t idx = atomicAdd(S.count + 1, 1u);  // at most one entry per stored triangle
-          S.large[idx] = uint32_t(q);
-          S.large_tiles[idx] = uint32_t((b.x1 - b.x0 + kRasterTileW) / kRasterTileW) *
-                               uint32_t((b.y1 - b.y0 + kRasterTileH) / kRasterTileH);
+        } else if (sub == 0) {
+          const uint32_t tiles = uint32_t((b.x1 - b.x0 + kRasterTileW) / kRasterTileW) *
+                                 uint32_t((b.y1 - b.y0 + kRasterTileH) / kRasterTileH);
+          if (tile_bits > 0) {
+            const unsigned long long old = atomicAdd(S.listed, (1ull << tile_bits) + tiles);
+            const uint32_t idx = uint32_t(old >> tile_bits);  // at most one entry per stored triangle
+            S.large[idx] = uint32_t(q);
+            S.tile_prefix[idx] = old & ((1ull << tile_bits) - 1);
+          } else {
+            const uint32_t idx = atomicAdd(S.count + 1, 1u);
+            S.large[idx] = uint32_t(q);
+            S.large_tiles[idx] = tiles;
+          }
         }
       }
     }
-    unsigned m = __ballot_sync(0xffffffffu, medium);
+    unsigned m = __ballot_sync(0xffffffffu, medium && sub == 0);
     while (m) {
       const int leader = __ffs(m) - 1;
       m &= m - 1;
-      const long long ql = base + leader;
+      const long long ql = base + leader / kDepthLanes;
       const RasterSetup T = load_setup(S.tris + ql);
-      const Box b = bbox(T, L);
-      const int bh = b.y1 - b.y0 + 1;
-      const int area = (b.x1 - b.x0 + 1) * bh;  // at most kRasterWarpArea: 8 pixels per lane
-      for (int k = lane; k < area; k += 32)
-        depth_pixel(T, b.x0 + k / bh, b.y0 + k % bh, L.height, depth_key, (unsigned long long)ql);
+      box_pixels(T, bbox(T, L), lane, 32, L.height, depth_key, (unsigned long long)ql);
     }
   }
 }
 
 // The exclusive prefix of the large triangles' tile counts (64-bit) in three
 // launches: per-block sums over kRasterScanBlocks equal ranges, a scan of
-// the sums, then each block's own scan offset by its sum's prefix.
+// the sums, then each block's own scan offset by its sum's prefix.  Only for
+// streams whose list and tiles do not fit one 64-bit counter.
 __device__ __forceinline__ void scan_range(uint32_t n, uint32_t& lo, uint32_t& hi) {
   const uint32_t per = (n + kRasterScanBlocks - 1) / kRasterScanBlocks;
   lo = min(n, blockIdx.x * per);
@@ -454,11 +479,13 @@ __global__ void __launch_bounds__(256) k_raster_scan_apply(RasterStream S) {
 // bounding boxes), taken by warps from a ticket kRasterItemsPerTicket at a
 // time (the first item's triangle by binary search of the prefix, the next
 // ones by walking on); blocks the edge equations reject are skipped.
-__global__ void __launch_bounds__(256) k_raster_depth_tiles(RasterStream S, ImageLayout L,
+__global__ void __launch_bounds__(256) k_raster_depth_tiles(RasterStream S, ImageLayout L, int tile_bits,
                                                             unsigned long long* __restrict__ depth_key) {
-  const uint32_t n = S.count[1];
+  const unsigned long long listed = *S.listed;
+  const uint32_t n = tile_bits > 0 ? uint32_t(listed >> tile_bits) : S.count[1];
   if (n == 0) return;
-  const unsigned long long total = S.tile_prefix[n];
+  const unsigned long long total = tile_bits > 0 ? listed & ((1ull << tile_bits) - 1) : S.tile_prefix[n];
+  const auto prefix_after = [&](uint32_t k) { return k + 1 < n ? S.tile_prefix[k + 1] : total; };
   const int lane = threadIdx.x & 31;
   for (;;) {
     unsigned long long w0 = 0;
@@ -472,12 +499,12 @@ __global__ void __launch_bounds__(256) k_raster_depth_tiles(RasterStream S, Imag
       const uint32_t mid = (k + hi + 1) >> 1;
       if (S.tile_prefix[mid] <= w0) k = mid; else hi = mid - 1;
     }
-    unsigned long long first = S.tile_prefix[k], next = S.tile_prefix[k + 1];
+    unsigned long long first = S.tile_prefix[k], next = prefix_after(k);
     for (unsigned long long w = w0; w < w1; ++w) {
       while (w >= next) {
         ++k;
         first = next;
-        next = S.tile_prefix[k + 1];
+        next = prefix_after(k);
       }
       const uint32_t q = S.large[k];
       const RasterSetup T = load_setup(S.tris + q);
@@ -540,16 +567,8 @@ __global__ void __launch_bounds__(256) k_raster_resolve(RasterStream S, ImageLay
                                                         const unsigned long long* __restrict__ depth_key,
                                                         RasterOutDev O, int mode, int triangles_per_patch,
                                                         const int32_t* __restrict__ slot_level) {
-  const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (i >= (long long)L.width * L.height) return;
   int x, y;
-  if (L.sy <= L.sx) {  // y contiguous: the reference's (W, H, ...) layout
-    x = int(i / L.height);
-    y = int(i % L.height);
-  } else {
-    y = int(i / L.width);
-    x = int(i % L.width);
-  }
+  if (!run_pixel(L, x, y)) return;
   const long long e = (long long)x * L.sx + (long long)y * L.sy;
   const unsigned long long key = depth_key[size_t(x) * L.height + y];
   if (key == kSentinel) {
@@ -599,10 +618,25 @@ __global__ void __launch_bounds__(256) k_raster_resolve(RasterStream S, ImageLay
   }
 }
 
-__global__ void k_raster_clear(unsigned long long* __restrict__ depth_key, long long n, uint32_t* count) {
-  const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (i < 4) count[i] = 0u;
-  if (i < n) depth_key[i] = kSentinel;
+// Two keys a thread, a 16-byte store (the keys' allocation is aligned).
+__global__ void k_raster_clear(unsigned long long* __restrict__ depth_key, long long n, RasterStream S) {
+  const long long i = 2 * (blockIdx.x * (long long)blockDim.x + threadIdx.x);
+  if (i < 4) S.count[i] = S.count[i + 1] = 0u;
+  if (i == 0) *S.listed = 0;
+  if (i + 1 < n)
+    *reinterpret_cast<ulonglong2*>(depth_key + i) = make_ulonglong2(kSentinel, kSentinel);
+  else if (i < n)
+    depth_key[i] = kSentinel;
+}
+
+// Bits of the listed tiles in the 64-bit counter, 0 where a full stream's list
+// and tiles might not fit one.
+int tile_bits_of(const RasterStream& S, const ImageLayout& L) {
+  const long long tiles = ((L.width - 1) / kRasterTileW + 2LL) * ((L.height - 1) / kRasterTileH + 2LL);
+  int list = 1, bits = 1;
+  while ((S.capacity >> list) > 0) ++list;
+  while (bits < 63 && (((unsigned long long)tiles * S.capacity) >> bits) > 0) ++bits;
+  return list + bits <= 64 ? bits : 0;
 }
 
 }  // namespace
@@ -611,7 +645,7 @@ cudaError_t launch_raster(const RasterMeshDev& M, const RasterStream& S, const I
                           unsigned long long* depth_key, const RasterOutDev& O, float near, float tf, int mode,
                           int sm_count, cudaStream_t s) {
   const long long pixels = (long long)L.width * L.height;
-  k_raster_clear<<<unsigned((pixels + 255) / 256), 256, 0, s>>>(depth_key, pixels, S.count);
+  k_raster_clear<<<unsigned((pixels + 511) / 512), 256, 0, s>>>(depth_key, pixels, S);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
   const long long sources = (long long)M.n_active * M.triangles_per_patch;
@@ -620,19 +654,21 @@ cudaError_t launch_raster(const RasterMeshDev& M, const RasterStream& S, const I
     e = cudaGetLastError();
     if (e != cudaSuccess) return e;
   }
-  k_raster_depth<<<unsigned(sm_count * 8), 256, 0, s>>>(S, L, depth_key);
+  const int tile_bits = tile_bits_of(S, L);
+  k_raster_depth<<<unsigned(sm_count * 8), 256, 0, s>>>(S, L, tile_bits, depth_key);
   e = cudaGetLastError();
   if (e != cudaSuccess) return e;
-  k_raster_scan_sums<<<kRasterScanBlocks, 256, 0, s>>>(S);
-  k_raster_scan_top<<<1, 256, 0, s>>>(S);
-  k_raster_scan_apply<<<kRasterScanBlocks, 256, 0, s>>>(S);
+  if (tile_bits == 0) {
+    k_raster_scan_sums<<<kRasterScanBlocks, 256, 0, s>>>(S);
+    k_raster_scan_top<<<1, 256, 0, s>>>(S);
+    k_raster_scan_apply<<<kRasterScanBlocks, 256, 0, s>>>(S);
+    e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+  }
+  k_raster_depth_tiles<<<unsigned(sm_count * 8), 256, 0, s>>>(S, L, tile_bits, depth_key);
   e = cudaGetLastError();
   if (e != cudaSuccess) return e;
-  k_raster_depth_tiles<<<unsigned(sm_count * 8), 256, 0, s>>>(S, L, depth_key);
-  e = cudaGetLastError();
-  if (e != cudaSuccess) return e;
-  k_raster_resolve<<<unsigned((pixels + 255) / 256), 256, 0, s>>>(S, L, depth_key, O, mode, M.triangles_per_patch,
-                                                                  M.slot_level);
+  k_raster_resolve<<<run_grid(L), run_block(), 0, s>>>(S, L, depth_key, O, mode, M.triangles_per_patch, M.slot_level);
   return cudaGetLastError();
 }
 

@@ -82,3 +82,21 @@ def _process_nan(pp, hdr):
     display = torch.full_like(src, -1.0)
     pp.process(src, display, 0.0, bloom=False, tone_map=True)
     return display.cpu().numpy()
+
+
+# an odd number of depth keys; boxes of a few pixels, of a warp, of several tiles; fewer triangles than a warp's
+@pytest.mark.parametrize("width,height,patches,res", [(1, 1, 3, 1), (31, 33, 4, 12), (263, 41, 3, 2), (701, 397, 2, 1)])
+@pytest.mark.parametrize("layout", ["wh", "hw"])
+def test_raster_boxes_of_each_size(width, height, patches, res, layout):
+    from oracle import raster
+    from test_gpu_raster import _compare, _mesh_tensors, _render, _terrain
+
+    view, normal, material, height_m, cell, tris, skirt, level, surface = _terrain(patches, res, 3)
+    active = list(range(patches))
+    ref = raster.render(view, normal, material, height_m, cell, tris, active, 0.5, 0.62, width, height, 0, level,
+                        surface, res, skirt)
+    ref["material_weights"] = ref.pop("material")
+    mesh = _mesh_tensors(view, normal, material, height_m, cell, tris, active, skirt, level, surface, res)
+    got, count = _render(mesh, width, height, 0.5, 0.62, 0, layout)
+    assert count == ref["clipped_count"]
+    _compare(got, ref, ref["ties"])
