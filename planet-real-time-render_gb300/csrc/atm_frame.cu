@@ -24,13 +24,13 @@ namespace atm {
 namespace {
 
 // _prepare_surface_lighting :1422-1472
-__global__ void __launch_bounds__(256) k_prepare_surface(DevParams P, Frame F, ImageLayout L,
+__global__ void __launch_bounds__(kRunPixels * kRunRows) k_prepare_surface(DevParams P, Frame F, ImageLayout L,
                                                          const float* __restrict__ pos,
                                                          const int32_t* __restrict__ sid, float cam_alt, f3 right,
                                                          f3 up, f3 fwd, float* __restrict__ out_t,
                                                          float* __restrict__ out_sky) {
   int x, y;
-  if (!linear_pixel(L, x, y)) return;
+  if (!run_pixel(L, x, y)) return;
   const size_t e = pix_offset(L, x, y);
   const size_t o = e * L.channels;
   f3 st = splat(1.0f), sky = splat(0.0f);
@@ -270,10 +270,9 @@ cudaError_t launch_prepare_surface(const DevParams& P, const ImageLayout& L, con
                                    float bottom, float cam_alt, const float sun[3], float ar, const float right[3],
                                    const float up[3], const float fwd[3], const float4* tlut, const float4* mslut,
                                    float* out_sun_t, float* out_sky, cudaStream_t s) {
-  const unsigned blocks = unsigned((static_cast<long long>(L.width) * L.height + 255) / 256);
   const Frame F = make_frame(P, tlut, mslut, bottom, ar, host3(sun), {0.0f, 0.0f, 0.0f});
-  k_prepare_surface<<<blocks, 256, 0, s>>>(P, F, L, pos, sid, cam_alt, host3(right), host3(up), host3(fwd), out_sun_t,
-                                           out_sky);
+  k_prepare_surface<<<run_grid(L), run_block(), 0, s>>>(P, F, L, pos, sid, cam_alt, host3(right), host3(up),
+                                                        host3(fwd), out_sun_t, out_sky);
   return cudaGetLastError();
 }
 

@@ -40,21 +40,6 @@ __device__ __forceinline__ bool split_pixel(const ImageLayout& L, int& x, int& y
   return px < L.width && py < L.height;
 }
 
-// Pixel of a thread for memory-bound per-pixel kernels: consecutive threads
-// take consecutive elements along the image's contiguous dimension.
-__device__ __forceinline__ bool linear_pixel(const ImageLayout& L, int& x, int& y) {
-  const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (i >= (long long)L.width * L.height) return false;
-  if (L.sy <= L.sx) {  // y contiguous: the reference's (W, H, 3) layout
-    x = int(i / L.height);
-    y = int(i % L.height);
-  } else {
-    y = int(i / L.width);
-    x = int(i % L.width);
-  }
-  return true;
-}
-
 struct PixelRay {
   f3 ray;
   float su, sv;

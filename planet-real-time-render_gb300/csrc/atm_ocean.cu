@@ -261,7 +261,7 @@ __device__ __forceinline__ void st3(float* p, r3 v) {
 
 // _rasterize :517-684
 template <int kLog2N>
-__global__ void __launch_bounds__(256) k_ocean_coverage(OceanSpectrum S, OceanFrame F, ImageLayout L,
+__global__ void __launch_bounds__(kRunPixels * kRunRows) k_ocean_coverage(OceanSpectrum S, OceanFrame F, ImageLayout L,
                                                         OceanImages G) {
   __shared__ OceanAxes s_axes;
   if (threadIdx.x == 0 && threadIdx.y == 0) s_axes = {cosf(F.wind), sinf(F.wind)};

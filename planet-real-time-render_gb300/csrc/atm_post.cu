@@ -75,7 +75,7 @@ __device__ __forceinline__ bool post_element(const PostParams& Q, int width, int
 
 // _extract, postprocess.py:110-119: one thread per half-resolution texel, in
 // storage order.
-__global__ void __launch_bounds__(256) k_post_extract(PostParams Q, ImageLayout L, const float* __restrict__ hdr,
+__global__ void __launch_bounds__(kRunPixels * kRunRows) k_post_extract(PostParams Q, ImageLayout L, const float* __restrict__ hdr,
                                                       float scale, float4* __restrict__ bloom) {
   int x, y;
   if (!post_element(Q, Q.hw, Q.hh, x, y)) return;
@@ -372,14 +372,14 @@ __device__ __forceinline__ float display_channel(float v) {
 // quotients and a flat 64-bit pixel index, 75 us with a pixel a thread, 60 us so.
 constexpr int kResolveRows = 8;
 template <bool kXFast, bool kBloom>
-__global__ void __launch_bounds__(256) k_post_resolve(PostParams Q, ImageLayout L, const float* __restrict__ hdr,
+__global__ void __launch_bounds__(kRunPixels * kRunRows) k_post_resolve(PostParams Q, ImageLayout L, const float* __restrict__ hdr,
                                                       float* __restrict__ display, const float4* __restrict__ bloom,
                                                       float exposure, float strength, int tone_map) {
   const int nf = kXFast ? L.width : L.height, ns = kXFast ? L.height : L.width;
   const int bf = kXFast ? Q.hw : Q.hh, bs = kXFast ? Q.hh : Q.hw;
   int f, group;
   if (!run_element(nf, 0x7fffffff, f, group)) return;
-  // the block's rows lie together: thread row t takes t, t + 8, ...
+  // the block's rows lie together: thread row t takes t, t + kRunRows, ...
   const unsigned s0 = (unsigned(group) - threadIdx.y) * kResolveRows + threadIdx.y;
   const BloomAxis fast = kBloom ? bloom_axis(f, nf, bf) : BloomAxis();
   const int64_t at = (kXFast ? f * L.sx + int64_t(s0) * L.sy : int64_t(s0) * L.sx + f * L.sy) * L.channels;

@@ -563,7 +563,7 @@ __device__ r3 surface_color(float h, const float (&m)[4], int slot, int mode, co
 }
 
 // _resolve_raster :1208-1267
-__global__ void __launch_bounds__(256) k_raster_resolve(RasterStream S, ImageLayout L,
+__global__ void __launch_bounds__(kRunPixels * kRunRows) k_raster_resolve(RasterStream S, ImageLayout L,
                                                         const unsigned long long* __restrict__ depth_key,
                                                         RasterOutDev O, int mode, int triangles_per_patch,
                                                         const int32_t* __restrict__ slot_level) {

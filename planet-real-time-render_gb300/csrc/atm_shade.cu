@@ -23,17 +23,9 @@ namespace {
 
 using namespace shading;
 
-__global__ void __launch_bounds__(256) k_shade_surface(ShadeParams S, ImageLayout L, ShadeImages I) {
-  const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (i >= int64_t(L.width) * L.height) return;
+__global__ void __launch_bounds__(kRunPixels * kRunRows) k_shade_surface(ShadeParams S, ImageLayout L, ShadeImages I) {
   int x, y;
-  if (L.sy <= L.sx) {  // y contiguous: the reference's (W, H, 3) layout
-    x = int(i / L.height);
-    y = int(i % L.height);
-  } else {
-    y = int(i / L.width);
-    x = int(i % L.width);
-  }
+  if (!run_pixel(L, x, y)) return;
   const int64_t e = int64_t(x) * L.sx + int64_t(y) * L.sy;
   const int c = L.channels;
   const int32_t sid = I.surface_id[e];
@@ -52,8 +44,7 @@ __global__ void __launch_bounds__(256) k_shade_surface(ShadeParams S, ImageLayou
 }  // namespace
 
 cudaError_t launch_shade_surface(const ShadeParams& S, const ImageLayout& L, const ShadeImages& I, cudaStream_t s) {
-  const int64_t n = int64_t(L.width) * L.height;
-  k_shade_surface<<<unsigned((n + 255) / 256), 256, 0, s>>>(S, L, I);
+  k_shade_surface<<<run_grid(L), run_block(), 0, s>>>(S, L, I);
   return cudaGetLastError();
 }
 
