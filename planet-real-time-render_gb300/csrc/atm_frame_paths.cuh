@@ -40,14 +40,21 @@ __device__ __forceinline__ bool split_pixel(const ImageLayout& L, int& x, int& y
   return px < L.width && py < L.height;
 }
 
+// (i + 1/2) / n from the rounded reciprocal of n: one residual correction
+// gives the IEEE quotient for every i < n of every n up to 16384, a frame's
+// largest side (each of the 1.3e8 compared).
+__device__ __forceinline__ float pixel_fraction(int i, int n, float inv_n) {
+  const float a = float(i) + 0.5f, q = a * inv_n;
+  return fmaf(fmaf(-q, float(n), a), inv_n, q);
+}
 struct PixelRay {
   f3 ray;
   float su, sv;
 };
 __device__ __forceinline__ PixelRay pixel_ray(const ImageLayout& L, const CompositeScalars& A, int x, int y) {
   PixelRay r;
-  r.su = (float(x) + 0.5f) / float(L.width);
-  r.sv = (float(y) + 0.5f) / float(L.height);
+  r.su = pixel_fraction(x, L.width, A.inv_w);
+  r.sv = pixel_fraction(y, L.height, A.inv_h);
   float sx = (r.su * 2.0f - 1.0f) * A.aspect;
   float sy = r.sv * 2.0f - 1.0f;
   f3 rv = (arr3(A.right) * sx + arr3(A.up) * sy) + arr3(A.fwd_t);

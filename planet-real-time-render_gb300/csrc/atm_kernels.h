@@ -51,8 +51,8 @@ struct CompositeScalars {
   float bottom, cam_alt, sky_alt, ar, tanfov, star_start, star_end;
   float sun[3], E[3], disk[3], right[3], up[3], fwd[3];
   int32_t view;
-  // set by the launch: width / height and fwd / tanfov, of every pixel's ray
-  float aspect, fwd_t[3];
+  // set by the launch: width / height, fwd / tanfov and the sizes' reciprocals, of every pixel's ray
+  float aspect, fwd_t[3], inv_w, inv_h;
 };
 inline Frame frame_of(const DevParams& P, const CompositeScalars& A, const float4* tlut, const float4* mslut) {
   return make_frame(P, tlut, mslut, A.bottom, A.ar, {A.sun[0], A.sun[1], A.sun[2]}, {A.E[0], A.E[1], A.E[2]});
@@ -60,6 +60,8 @@ inline Frame frame_of(const DevParams& P, const CompositeScalars& A, const float
 inline CompositeScalars with_image(CompositeScalars A, const ImageLayout& L) {
   A.aspect = float(L.width) / float(L.height);
   for (int k = 0; k < 3; ++k) A.fwd_t[k] = A.fwd[k] / A.tanfov;
+  A.inv_w = 1.0f / float(L.width);
+  A.inv_h = 1.0f / float(L.height);
   return A;
 }
 

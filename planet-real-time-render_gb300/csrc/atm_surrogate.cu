@@ -39,12 +39,27 @@ constexpr unsigned kAll = 0xffffffffu;
 // root, reciprocal and rsqrt (1-2 ulp).  The sun cosines do not: gates
 // compare them, and a pixel's path hangs on their last bit.
 //
-// Sky-view v of a zenith angle whose cosine is mu, at altitude h
-// (sky_zenith_to_v of sky_horizon_zenith).
-__device__ __forceinline__ float view_feature(float mu, float h, float bottom) {
-  const float z = acosf(clampf(mu, -1.0f, 1.0f));
+// acos by Abramowitz and Stegun 4.4.46, 2e-8 off: a root and eight operations.
+__device__ __forceinline__ float feature_acos(float c) {
+  const float x = fabsf(c);
+  float p = fmaf(x, -0.0012624911f, 0.0066700901f);
+  p = fmaf(x, p, -0.0170881256f);
+  p = fmaf(x, p, 0.0308918810f);
+  p = fmaf(x, p, -0.0501743046f);
+  p = fmaf(x, p, 0.0889789874f);
+  p = fmaf(x, p, -0.2145988016f);
+  p = fmaf(x, p, 1.5707963050f) * fsqrt(__saturatef(1.0f - x));
+  return c < 0.0f ? kPiF - p : p;
+}
+// The horizon's zenith angle at altitude h (sky_horizon_zenith).
+__device__ __forceinline__ float horizon_feature(float h, float bottom) {
   const float a = mx(h, 0.0f);
-  const float hz = kPiF - acosf(clampf(shell_rho(a, bottom) * frcp(mx(bottom + a, 1.0f)), 0.0f, 1.0f));
+  return kPiF - feature_acos(clampf(shell_rho(a, bottom) * frcp(mx(bottom + a, 1.0f)), 0.0f, 1.0f));
+}
+// Sky-view v of a zenith angle whose cosine is mu (sky_zenith_to_v), hz the
+// horizon's.
+__device__ __forceinline__ float view_feature(float mu, float hz) {
+  const float z = feature_acos(clampf(mu, -1.0f, 1.0f));
   const bool above = z < hz;
   const float n = __saturatef(fdiv(above ? z : z - hz, mx(above ? hz : kPiF - hz, 1.0e-6f)));
   return above ? 0.5f * (1.0f - fsqrt(1.0f - n)) : 0.5f + 0.5f * fsqrt(n);
@@ -54,13 +69,34 @@ __device__ __forceinline__ float view_feature(float mu, float h, float bottom) {
 __device__ __forceinline__ float azimuth_cosine(float ab, float aa, float bb) {
   return aa > 1.0e-12f && bb > 1.0e-12f ? ab * frsqrt(aa * bb) : 1.0f;
 }
-// x[0..3]: altitude, view, sun, relative azimuth at the segment's first point.
-__device__ __forceinline__ void geometry_features(const DevParams& P, float bottom, float h, float mu_v, float mu_s,
-                                                  float cos_dphi, float* x) {
-  x[0] = 2.0f * fsqrt(__saturatef(h * P.inv_top)) - 1.0f;
-  x[1] = 2.0f * view_feature(mu_v, h, bottom) - 1.0f;
-  x[2] = 2.0f * sun_cosine_to_u(clampf(mu_s, -1.0f, 1.0f), horizon_cosine(h, bottom)) - 1.0f;
-  x[3] = clampf(cos_dphi, -1.0f, 1.0f);
+// What the features take from the segment's first point alone: up its
+// vertical, the sun's cosine and horizontal part there, x[0] and x[2] (altitude
+// and sun) and the horizon.  For a camera inside the shell that point is the
+// camera and all of it is the frame's: formed once a block.
+struct StartPoint {
+  f3 up, ts;
+  float mu_s, ts2, x0, x2, hz;
+};
+__device__ __forceinline__ float altitude_feature(const DevParams& P, float h) {
+  return 2.0f * fsqrt(__saturatef(h * P.inv_top)) - 1.0f;
+}
+__device__ __forceinline__ float sun_feature(float bottom, float h, float mu_s) {
+  return 2.0f * sun_cosine_to_u(clampf(mu_s, -1.0f, 1.0f), horizon_cosine(h, bottom)) - 1.0f;
+}
+__device__ __forceinline__ StartPoint start_point(const DevParams& P, const Frame& F, float cam_alt, const RayGeom& G,
+                                                  f3 ray, float start) {
+  const float o_y = F.bottom + cam_alt;
+  const float h = altitude_at(G, start, F.bottom);
+  const f3 ps = mk(ray.x * start, o_y + ray.y * start, ray.z * start);
+  StartPoint S;
+  S.up = ps * (1.0f / mx(norm(ps), 1.0f));
+  S.mu_s = dot(F.sun, S.up);
+  S.ts = F.sun - S.up * S.mu_s;
+  S.ts2 = dot(S.ts, S.ts);
+  S.x0 = altitude_feature(P, h);
+  S.x2 = sun_feature(F.bottom, h, S.mu_s);
+  S.hz = horizon_feature(h, F.bottom);
+  return S;
 }
 
 // Sun (multi-scattering u mapping) and altitude features, x[0] and x[1], of
@@ -68,11 +104,14 @@ __device__ __forceinline__ void geometry_features(const DevParams& P, float bott
 // Where a segment's light comes from depends on where it ends and how low it
 // dips as much as on where it starts: with these points given, the sky
 // network's held-out error drops by a quarter and the aerial network's on
-// camera-to-surface segments to a third.  Returns the point's sun cosine.
+// camera-to-surface segments to a third.  Returns the point's sun cosine,
+// exact (kGate) for a gate or as the feature takes it.
+template <bool kGate>
 __device__ __forceinline__ float point_features(const DevParams& P, float bottom, const RayGeom& G, f3 ray, float o_y,
                                                 f3 sun, float t, float* x) {
   const f3 pt = mk(ray.x * t, o_y + ray.y * t, ray.z * t);
-  const float mu = clampf(dot(sun, pt) / mx(norm(pt), 1.0f), -1.0f, 1.0f);
+  const float mu = clampf(kGate ? dot(sun, pt) / mx(norm(pt), 1.0f) : dot(sun, pt) * frsqrt(mx(dot(pt, pt), 1.0f)),
+                          -1.0f, 1.0f);
   const float h = altitude_at(G, t, bottom);
   x[0] = 2.0f * sun_cosine_to_u(mu, horizon_cosine(h, bottom)) - 1.0f;
   x[1] = 2.0f * fsqrt(__saturatef(h * P.inv_top)) - 1.0f;
@@ -84,8 +123,8 @@ __device__ __forceinline__ float point_features(const DevParams& P, float bottom
 __device__ __forceinline__ float segment_features(const DevParams& P, float bottom, const RayGeom& G, f3 ray,
                                                   float o_y, f3 sun, float start, float end, float* x,
                                                   float& mu_end, float& mu_mid) {
-  mu_end = point_features(P, bottom, G, ray, o_y, sun, end, x + 7);
-  mu_mid = point_features(P, bottom, G, ray, o_y, sun, 0.5f * (start + end), x + 9);
+  mu_end = point_features<true>(P, bottom, G, ray, o_y, sun, end, x + 7);
+  mu_mid = point_features<true>(P, bottom, G, ray, o_y, sun, 0.5f * (start + end), x + 9);
   return mn(fabsf(mu_end), fabsf(mu_mid));
 }
 // Sky x[6..9]: the end of the ray's march (the shell top or the ground),
@@ -97,8 +136,8 @@ __device__ __forceinline__ void sky_ray_features(const DevParams& P, float botto
   segment_of(P, G, bottom, start, end, valid, ground);
   if (!valid) start = end = 0.0f;
   const float o_y = bottom + mx(h, 0.0f);
-  point_features(P, bottom, G, ray, o_y, sun, end, x + 6);
-  point_features(P, bottom, G, ray, o_y, sun, clampf(G.tc, start, end), x + 8);
+  point_features<false>(P, bottom, G, ray, o_y, sun, end, x + 6);
+  point_features<false>(P, bottom, G, ray, o_y, sun, clampf(G.tc, start, end), x + 8);
 }
 
 // Counter-based uniform in [0, 1): 64-bit mix of (seed, index, lane).
@@ -154,7 +193,11 @@ __global__ void __launch_bounds__(128) k_gen_samples(const SurrogateSetDev* __re
     const float cphi = x[3], sphi = sqrtf(mx(1.0f - cphi * cphi, 0.0f));
     const f3 ray = mk(sv, mu_v, 0.0f);
     const f3 sun = mk(ss * cphi, mu_s, ss * sphi);
-    geometry_features(P, R, h, mu_v, mu_s, cphi, x);  // rounding-consistent features
+    // rounding-consistent features
+    x[0] = altitude_feature(P, h);
+    x[1] = 2.0f * view_feature(mu_v, horizon_feature(h, R)) - 1.0f;
+    x[2] = sun_feature(R, h, mu_s);
+    x[3] = clampf(cphi, -1.0f, 1.0f);
     x[4] = S.lhr_n;
     x[5] = S.lhm_n;
     Frame F = S.F;
@@ -242,8 +285,9 @@ enum PixelKind : int { kNone = 0, kSurfMlp, kSurfPlain, kSurfEmpty, kSkyMlp, kSk
 // tanh (XU) and the issue of features and outputs around them, at the
 // latency of the five serial layers; five tiles are what 512 tensor-memory
 // columns hold (64 accumulator and 32 activation columns a tile, the bias's 8
-// shared).  A 4K frame takes 0.83 ms, against 0.99 ms with two tiles a block,
-// three blocks an SM and the weights copied by each block.
+// shared).  A 4K frame takes 0.80 ms; 0.83 ms with the start point's features
+// formed by each pixel, 0.99 ms with two tiles a block, three blocks an SM and
+// the weights copied by each block.
 constexpr int kWorkers = 5;
 constexpr uint32_t kWorkerCols = 96, kOnesCol = kWorkers * kWorkerCols, kSurrogateTmemCols = 512;
 
@@ -251,20 +295,41 @@ struct NetBlock {
   uint64_t mbar[kWorkers + 1];  // the tiles' MMA completions, the weights' arrival
   uint32_t tmem;
   float horizon;  // the camera's horizon zenith
+  float limb_low, limb_high;  // no ray whose y is outside is within the limb's angle
+  StartPoint camera;          // of a camera inside the shell
 };
+// Whether a ray lies within limb_rad of the limb.  The bounds decide most rays
+// without the angle; they are a margin of 1e-5 wider than it, in cosines, so
+// that the angle's last bits never matter beyond them.
+__device__ __forceinline__ bool near_limb_of(const NetBlock& B, float y, float limb_rad) {
+  if (y < B.limb_low || y > B.limb_high) return false;
+  return fabsf(acosf(clampf(y, -1.0f, 1.0f)) - B.horizon) < limb_rad;
+}
+// x[0..3] of a sky ray: the camera's horizontal plane and vertical are y = 0 and y.
+__device__ __forceinline__ void sky_start_features(const NetBlock& B, const Frame& F, f3 ray, float* x) {
+  x[0] = B.camera.x0;
+  x[1] = 2.0f * view_feature(ray.y, B.camera.hz) - 1.0f;
+  x[2] = B.camera.x2;
+  x[3] = clampf(azimuth_cosine(ray.x * F.sun.x + ray.z * F.sun.z, ray.x * ray.x + ray.z * ray.z,
+                               F.sun.x * F.sun.x + F.sun.z * F.sun.z), -1.0f, 1.0f);
+}
 // Sets a block up (every thread calls): the weights into smem by bulk copies,
 // tensor memory, barriers.  Returns this thread's tile; `weights` false if the
 // weights did not arrive in time.
 __device__ __forceinline__ TcTile net_block_begin(NetBlock& B, unsigned char* smem, const unsigned char* w0, int n0,
-                                                  const unsigned char* w1, int n1, float horizon_altitude, float bottom,
-                                                  bool& weights) {
+                                                  const unsigned char* w1, int n1, const DevParams& P, const Frame& F,
+                                                  float cam_alt, float limb_rad, bool& weights) {
   if (threadIdx.x == 0) {
     for (int k = 0; k <= kWorkers; ++k) tc::mbar_init(&B.mbar[k], 1);
     tc::mbar_init_fence();
     tc::mbar_arrive_expect_tx(&B.mbar[kWorkers], uint32_t(n0 + n1));
     if (n0 > 0) tc::bulk_g2s(smem, w0, uint32_t(n0), &B.mbar[kWorkers]);
     if (n1 > 0) tc::bulk_g2s(smem + n0, w1, uint32_t(n1), &B.mbar[kWorkers]);
-    B.horizon = sky_horizon_zenith(horizon_altitude, bottom);
+    B.horizon = sky_horizon_zenith(cam_alt, F.bottom);
+    B.limb_low = cosf(mn(B.horizon + limb_rad, kPiF)) - 1.0e-5f;
+    B.limb_high = cosf(mx(B.horizon - limb_rad, 0.0f)) + 1.0e-5f;
+    const f3 zenith = mk(0.0f, 1.0f, 0.0f);
+    B.camera = start_point(P, F, cam_alt, camera_ray_geom(P, F.bottom, cam_alt, zenith), zenith, 0.0f);
   }
   if (threadIdx.x >> 5 == 1) tc::alloc(&B.tmem, kSurrogateTmemCols);
   tc::fence_before_sync();
@@ -324,7 +389,8 @@ __global__ void __launch_bounds__(128 * kWorkers, 1) k_composite_surrogate(
   extern __shared__ __align__(128) unsigned char smem[];  // the aerial network, then the sky network
   __shared__ NetBlock B;
   bool nets_ok;  // tile-uniform: the networks may run
-  TcTile T = net_block_begin(B, smem, nets.ap, nets.ap_bytes, nets.sky, nets.sky_bytes, A.cam_alt, A.bottom, nets_ok);
+  TcTile T = net_block_begin(B, smem, nets.ap, nets.ap_bytes, nets.sky, nets.sky_bytes, P, F, A.cam_alt,
+                             nets.limb_rad, nets_ok);
   const int lane = threadIdx.x & 31;
   for (int t = T.tile * gridDim.x + blockIdx.x; t < N.count; t += kWorkers * gridDim.x) {
     int x, y;
@@ -333,7 +399,7 @@ __global__ void __launch_bounds__(128 * kWorkers, 1) k_composite_surrogate(
     const size_t e = pix_offset(L, cx, cy);
     const size_t o = e * L.channels;
     const f3 ray = pixel_ray(L, A, cx, cy).ray;
-    const bool near_limb = fabsf(acosf(clampf(ray.y, -1.0f, 1.0f)) - B.horizon) < nets.limb_rad;
+    const bool near_limb = near_limb_of(B, ray.y, nets.limb_rad);
 
     int kind = kNone;
     uint32_t xp[8] = {};
@@ -349,13 +415,14 @@ __global__ void __launch_bounds__(128 * kWorkers, 1) k_composite_surrogate(
         } else {
           // features at the segment's first point inside the shell
           const float o_y = A.bottom + A.cam_alt;
-          const float hs = altitude_at(G, start, A.bottom);
-          const f3 ps = mk(ray.x * start, o_y + ray.y * start, ray.z * start);
-          const f3 up = ps * (1.0f / mx(norm(ps), 1.0f));
-          const float mu_v = dot(ray, up), mu_s = dot(F.sun, up);
-          const f3 tv = ray - up * mu_v, ts = F.sun - up * mu_s;
-          const float cphi = azimuth_cosine(dot(tv, ts), dot(tv, tv), dot(ts, ts));
-          geometry_features(P, A.bottom, hs, mu_v, mu_s, cphi, fx);
+          const StartPoint sp = start == 0.0f ? B.camera : start_point(P, F, A.cam_alt, G, ray, start);
+          const float mu_s = sp.mu_s;
+          const float mu_v = dot(ray, sp.up);
+          const f3 tv = ray - sp.up * mu_v;
+          fx[0] = sp.x0;
+          fx[1] = 2.0f * view_feature(mu_v, sp.hz) - 1.0f;
+          fx[2] = sp.x2;
+          fx[3] = clampf(azimuth_cosine(dot(tv, sp.ts), dot(tv, tv), sp.ts2), -1.0f, 1.0f);
           fx[4] = nets.lhr_n;
           fx[5] = nets.lhm_n;
           fx[6] = 2.0f * __logf(clampf(end - start, 1.0f, kSurrogateMaxLength)) / logf(kSurrogateMaxLength) - 1.0f;
@@ -371,9 +438,7 @@ __global__ void __launch_bounds__(128 * kWorkers, 1) k_composite_surrogate(
         }
       } else if (nets.sky != nullptr && A.cam_alt <= P.top && fabsf(F.sun.y) >= nets.sky_twilight_cos && !near_limb) {
         kind = kSkyMlp;
-        const float cphi = azimuth_cosine(ray.x * F.sun.x + ray.z * F.sun.z, ray.x * ray.x + ray.z * ray.z,
-                                          F.sun.x * F.sun.x + F.sun.z * F.sun.z);
-        geometry_features(P, A.bottom, A.cam_alt, ray.y, F.sun.y, cphi, fx);
+        sky_start_features(B, F, ray, fx);
         fx[4] = nets.lhr_n;
         fx[5] = nets.lhm_n;
         sky_ray_features(P, A.bottom, A.cam_alt, ray, F.sun, fx);
@@ -482,8 +547,9 @@ __global__ void __launch_bounds__(128 * kWorkers, 1) k_composite_surrogate(
 // Lanes that share a queued pixel's march: a short queue (the checked 1% of a
 // frame is about one pixel a resident thread) would run as one or two whole
 // marches a thread on part of the warps; a long one would only repeat each
-// pixel's set-up.  4K, 1% checked: 77 us against 111 us at one lane a pixel.
-constexpr int kQueueLanes = 4;
+// pixel's set-up.  4K, 1% checked, three blocks an SM: 67 us (two blocks: 73;
+// 8 lanes: 92; 1 lane: 111).
+constexpr int kQueueLanes = 4, kQueueBlocks = 3;
 __device__ __forceinline__ bool split_queue(uint32_t n) { return n <= 8u * gridDim.x * blockDim.x; }
 
 // Sky radiance along `ray` by kLanes consecutive lanes, as sky_radiance; the
@@ -586,7 +652,7 @@ __device__ __forceinline__ void fallback_queue(const DevParams& P, const Frame& 
   }
 }
 template <bool kShade>
-__global__ void __launch_bounds__(256, 2) k_surrogate_fallback(
+__global__ void __launch_bounds__(256, 3) k_surrogate_fallback(
     DevParams P, Frame F, ImageLayout L, CompositeScalars A, const float* __restrict__ scene,
     const float* __restrict__ space, const float* __restrict__ pos, SurrogateQueue Q, float* __restrict__ hdr,
     unsigned long long* counter, ShadeParams S, ShadeImages I) {
@@ -676,7 +742,7 @@ __global__ void __launch_bounds__(128 * kWorkers, 1) k_sky_pixels_net(DevParams 
   extern __shared__ __align__(128) unsigned char smem[];  // the sky network
   __shared__ NetBlock B;
   bool nets_ok;
-  TcTile T = net_block_begin(B, smem, nets.sky, nets.sky_bytes, nullptr, 0, A.cam_alt, A.bottom, nets_ok);
+  TcTile T = net_block_begin(B, smem, nets.sky, nets.sky_bytes, nullptr, 0, P, F, A.cam_alt, nets.limb_rad, nets_ok);
   const int lane = threadIdx.x & 31;
   uint32_t samples = 0;
   for (int t = T.tile * gridDim.x + blockIdx.x; t < N.count; t += kWorkers * gridDim.x) {
@@ -684,15 +750,13 @@ __global__ void __launch_bounds__(128 * kWorkers, 1) k_sky_pixels_net(DevParams 
     const bool inside = tile_pixel_of(L, N, t, T.row, x, y);
     const int cx = inside ? x : 0, cy = inside ? y : 0;
     const f3 ray = pixel_ray(L, A, cx, cy).ray;
-    const bool near_limb = fabsf(acosf(clampf(ray.y, -1.0f, 1.0f)) - B.horizon) < nets.limb_rad;
+    const bool near_limb = near_limb_of(B, ray.y, nets.limb_rad);
     const bool net = inside && A.cam_alt <= P.top && fabsf(F.sun.y) >= nets.sky_twilight_cos && !near_limb;
     bool plain = !net, checked = false;
     uint32_t xp[8] = {};
     if (net) {
       float fx[16] = {};
-      const float cphi = azimuth_cosine(ray.x * F.sun.x + ray.z * F.sun.z, ray.x * ray.x + ray.z * ray.z,
-                                        F.sun.x * F.sun.x + F.sun.z * F.sun.z);
-      geometry_features(P, A.bottom, A.cam_alt, ray.y, F.sun.y, cphi, fx);
+      sky_start_features(B, F, ray, fx);
       fx[4] = nets.lhr_n;
       fx[5] = nets.lhm_n;
       sky_ray_features(P, A.bottom, A.cam_alt, ray, F.sun, fx);
@@ -828,7 +892,7 @@ cudaError_t launch_sky_pixels(int mode, const DevParams& P, const ImageLayout& L
                                                                                      counter, Q);
   e = cudaGetLastError();
   if (e != cudaSuccess || Q.net_mask == nullptr) return e;
-  k_sky_pixels_check<<<2 * sm_count, 256, 0, s>>>(P, F, L, A, Q, out, counter);
+  k_sky_pixels_check<<<kQueueBlocks * sm_count, 256, 0, s>>>(P, F, L, A, Q, out, counter);
   e = cudaGetLastError();
   if (e != cudaSuccess) return e;
   k_sky_pixels_calibrate<<<run_grid(L), run_block(), 0, s>>>(L, Q, out);
@@ -872,7 +936,7 @@ cudaError_t launch_composite_surrogate(const DevParams& P, const ImageLayout& L,
                                                         hdr, S, I);
     e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    k_surrogate_fallback<true><<<2 * sm_count, 256, 0, s>>>(P, F, L, A, scene, space, pos, Q, hdr, counter, S, I);
+    k_surrogate_fallback<true><<<kQueueBlocks * sm_count, 256, 0, s>>>(P, F, L, A, scene, space, pos, Q, hdr, counter, S, I);
   } else {
     e = cudaFuncSetAttribute(k_composite_surrogate<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return e;
@@ -880,7 +944,7 @@ cudaError_t launch_composite_surrogate(const DevParams& P, const ImageLayout& L,
                                                          Q, hdr, S, I);
     e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    k_surrogate_fallback<false><<<2 * sm_count, 256, 0, s>>>(P, F, L, A, scene, space, pos, Q, hdr, counter, S, I);
+    k_surrogate_fallback<false><<<kQueueBlocks * sm_count, 256, 0, s>>>(P, F, L, A, scene, space, pos, Q, hdr, counter, S, I);
   }
   e = cudaGetLastError();
   if (e != cudaSuccess || Q.lm == nullptr) return e;
