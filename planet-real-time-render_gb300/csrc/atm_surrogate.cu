@@ -547,9 +547,9 @@ __global__ void __launch_bounds__(128 * kWorkers, 1) k_composite_surrogate(
 // Lanes that share a queued pixel's march: a short queue (the checked 1% of a
 // frame is about one pixel a resident thread) would run as one or two whole
 // marches a thread on part of the warps; a long one would only repeat each
-// pixel's set-up.  4K, 1% checked, three blocks an SM: 67 us (two blocks: 73;
-// 8 lanes: 92; 1 lane: 111).
-constexpr int kQueueLanes = 4, kQueueBlocks = 3;
+// pixel's set-up.  4K, 1% checked, three blocks an SM: 63 us (4 lanes: 67, 1
+// lane: 66; two or four blocks an SM: 73, 66).
+constexpr int kQueueLanes = 2, kQueueBlocks = 3;
 __device__ __forceinline__ bool split_queue(uint32_t n) { return n <= 8u * gridDim.x * blockDim.x; }
 
 // Sky radiance along `ray` by kLanes consecutive lanes, as sky_radiance; the
