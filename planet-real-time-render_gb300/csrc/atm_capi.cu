@@ -148,6 +148,7 @@ DevParams make_dev_params(const AtmParams& p) {
   d.t_lut = lut_dims(d.t_w, d.t_h);
   d.ms_lut = lut_dims(d.ms_w, d.ms_h);
   d.sv_lut = lut_dims(d.sv_w, d.sv_h);
+  d.ms_half_w = 0.5f * float(d.ms_w);
   return d;
 }
 

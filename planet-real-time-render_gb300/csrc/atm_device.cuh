@@ -50,6 +50,7 @@ struct DevParams {
   float ray_k;                 // f32(16 pi)
   float exp2_r, exp2_m;        // -log2(e) / scale height: exp(-h / H) = 2^(h exp2)
   float inv_oz_half, inv_top;  // f32 reciprocals of the above
+  float ms_half_w;                // half the multi-scattering LUT's width
   LutDims t_lut, ms_lut, sv_lut;  // of the transmittance, multi-scattering and sky-view LUTs
   int t_w, t_h, ms_w, ms_h, sv_w, sv_h, ap_w, ap_h, ap_d;
   int t_steps, ms_dirs, ms_steps, sv_steps, ap_steps, limb_steps, substeps;
@@ -529,9 +530,9 @@ __device__ __forceinline__ float sun_cosine_to_u(float c, float hc) {
 // XU pipe and the index arithmetic off the ALU, the two pipes a march is
 // short of; past the last texel's centre the last pair's weight saturates at
 // its right end, so the four taps are two addresses apart by constants.
-__device__ __forceinline__ f3 bilinear(const float4* __restrict__ lut, const LutDims& D, float u, float v) {
-  const float x = mx(fmaf(u, D.w, -0.5f), 0.0f);
-  const float y = mx(fmaf(v, D.h, -0.5f), 0.0f);
+__device__ __forceinline__ f3 bilinear_at(const float4* __restrict__ lut, const LutDims& D, float cx, float cy) {
+  const float x = mx(cx, 0.0f);
+  const float y = mx(cy, 0.0f);
   const float xm = mn(__fadd_rd(x, kMagic), D.x_last);
   const float yf = mn(__fadd_rd(y, kMagic), D.y_last) - kMagic;
   const float fx = __saturatef(x - (xm - kMagic));
@@ -542,6 +543,10 @@ __device__ __forceinline__ f3 bilinear(const float4* __restrict__ lut, const Lut
   const float wd = fx * fy, wc = fy - wd, wb = fx - wd, wa = (1.0f - fx) - wc;
   return {fmaf(d.x, wd, fmaf(c.x, wc, fmaf(b.x, wb, a.x * wa))), fmaf(d.y, wd, fmaf(c.y, wc, fmaf(b.y, wb, a.y * wa))),
           fmaf(d.z, wd, fmaf(c.z, wc, fmaf(b.z, wb, a.z * wa)))};
+}
+
+__device__ __forceinline__ f3 bilinear(const float4* __restrict__ lut, const LutDims& D, float u, float v) {
+  return bilinear_at(lut, D, fmaf(u, D.w, -0.5f), fmaf(v, D.h, -0.5f));
 }
 
 // Per-launch geometry shared by every sample of a kernel, formed on the host
@@ -556,8 +561,9 @@ struct Frame {
   float ar;         // sun angular radius (rad)
   f3 sun;
   f3 E;             // solar irradiance
-  float inv_shell_top;
+  float t_rho;           // transmittance LUT rows a metre of rho: its height / shell_top
   float cos_ar, sin_ar;  // of the sun's angular radius: thresholds of the whole-disk tests
+  float bottom_sin_ar;
 };
 inline Frame make_frame(const DevParams& P, const float4* tlut, const float4* mslut, float bottom, float ar, f3 sun,
                         f3 E) {
@@ -571,9 +577,10 @@ inline Frame make_frame(const DevParams& P, const float4* tlut, const float4* ms
   F.ar = ar;
   F.sun = sun;
   F.E = E;
-  F.inv_shell_top = 1.0f / (F.shell_top > 1.0e-6f ? F.shell_top : 1.0e-6f);
+  F.t_rho = P.t_lut.h / (F.shell_top > 1.0e-6f ? F.shell_top : 1.0e-6f);
   F.sin_ar = float(std::sin(double(ar)));
   F.cos_ar = float(std::cos(double(ar)));
+  F.bottom_sin_ar = float(bottom * std::sin(double(ar)));
   return F;
 }
 // Sun of a sky-view LUT: its zenith cosine alone, in the x-y plane.
@@ -589,8 +596,7 @@ __device__ __forceinline__ f3 sample_t_at(const DevParams& P, const Frame& F, fl
   const float d = fsqrt(mx(fmaf(rc, rc, F.shell2 - rho2), 0.0f)) - rc;  // below 0 only above the shell
   const float dmin = P.top - h;
   const float u = __saturatef((d - dmin) * frcp(mx((rho + F.shell_top) - dmin, 1.0e-6f)));
-  const float v = __saturatef(rho * F.inv_shell_top);
-  return bilinear(F.tlut, P.t_lut, u, v);
+  return bilinear_at(F.tlut, P.t_lut, fmaf(u, P.t_lut.w, -0.5f), fmaf(rho, F.t_rho, -0.5f));
 }
 __device__ __forceinline__ f3 sample_t(const DevParams& P, const Frame& F, float h, float cosv) {
   const float a = clampf(h, 0.0f, P.top);
@@ -600,6 +606,15 @@ __device__ __forceinline__ f3 sample_t(const DevParams& P, const Frame& F, float
 // _sample_multi_scattering :642-683
 __device__ __forceinline__ f3 sample_ms(const DevParams& P, const Frame& F, float h, float sc, float hc) {
   return bilinear(F.mslut, P.ms_lut, sun_cosine_to_u(sc, hc), fsqrt(__saturatef(h * P.inv_top)));
+}
+
+// The same at a march's sample: altitude h, radius r, rc = r cos of the sun's
+// zenith angle, rho = -r cos of the horizon's.
+__device__ __forceinline__ f3 sample_ms_at(const DevParams& P, const Frame& F, float h, float r, float rc, float rho) {
+  const float t = rc + rho;
+  const float n = __saturatef(fabsf(t) * frcp(mx(fmaf(copysignf(1.0f, t), rho, r), 1.0e-6f)));
+  return bilinear_at(F.mslut, P.ms_lut, fmaf(copysignf(P.ms_half_w, t), fsqrt(n), P.ms_half_w - 0.5f),
+                     fmaf(fsqrt(__saturatef(h * P.inv_top)), P.ms_lut.h, -0.5f));
 }
 
 // Horizon at one sample altitude: cosine hc = -rho/r of the horizon
@@ -763,24 +778,24 @@ __device__ __forceinline__ RaySource make_ray_source(const DevParams& P, const F
 
 // The medium and the sun at the middle of a segment [start, end] of the ray:
 // density, extinction and scattering, the segment's length, finite-disk sun
-// transmittance st and disk visibility, altitude h, sun cosine sc, horizon
-// cosine hc.  The sample's radius is bottom + h (its altitude on the ray) and
+// transmittance st and disk visibility, altitude h, radius r, rc = r cos of the
+// sun's zenith angle, rho = -r cos of the horizon's.  The sample's radius is bottom + h (its altitude on the ray) and
 // its sun cosine (p(t0) . sun + (t - t0) ray . sun) / radius; the reference
 // forms the point first - same quantities, rounding differs in the last bits.
 //
 // A march is bound by the instructions it issues, the ALU pipe (compares,
 // selects, minima, integers) first.  What a sample shares is formed once:
 // delta = r^2 - R^2 gives the altitude, the horizon's rho and the distance to
-// the shell top; 1/r by one rsqrt gives r, both cosines and the horizon's
-// sine.  Altitude and sun cosine keep the operations that decide where the
-// density is cut off (delta's sign).  With the tap and the segment weight
-// above, a 1080p composite from 2 km went from 1369 to 782 us (1.48e9 to
-// 0.86e9 warp instructions).
+// the shell top; lengths along the vertical (rc, rho) stand for the cosines,
+// which only a partly hidden disk needs.  The altitude keeps the operations
+// that decide where the density is cut off (delta's sign).  With the tap and the segment weight
+// above, a 1080p composite from 2 km went from 1369 to 758 us (1.48e9 to
+// 0.83e9 warp instructions).
 struct MarchSample {
   Density d;
   Medium medium;
   f3 st;
-  float step, vis, h, sc, hc;
+  float step, vis, h, r, rc, rho;
 };
 __device__ __forceinline__ MarchSample march_sample(const DevParams& P, const Frame& F, const RaySource& R,
                                                     float start, float end) {
@@ -788,23 +803,27 @@ __device__ __forceinline__ MarchSample march_sample(const DevParams& P, const Fr
   m.step = mx(end - start, 0.0f);
   const float u = (start + end) * 0.5f - R.t0;
   const float delta = fmaf(u, u, fmaf(R.q1, u, R.q0));
-  const float r2 = mx(fmaf(F.bottom, F.bottom, delta), 1.0f);
-  const float inv_r = frsqrt(r2);
-  const float r = r2 * inv_r;
-  m.h = delta * frcp(r + F.bottom);
+  m.r = fsqrt(mx(fmaf(F.bottom, F.bottom, delta), 1.0f));
+  m.h = delta * frcp(m.r + F.bottom);
   m.d = density(P, m.h);
   m.medium = medium_of(P, m.d);
-  const float rc = fmaf(u, R.r_sun, R.s0);
-  m.sc = rc * inv_r;
-  const Horizon H = horizon_of(mx(delta, 0.0f), inv_r, F.bottom);
-  m.hc = H.hc;
-  m.st = sample_solar_t(P, F, m.h, r, m.sc, rc, H, m.vis);
+  m.rc = fmaf(u, R.r_sun, R.s0);
+  const float rho2 = mx(delta, 0.0f);
+  m.rho = fsqrt(rho2);
+  // the disk wholly above the horizon, sample_solar_t's test times r
+  if (m.rc >= fmaf(-m.rho, F.cos_ar, F.bottom_sin_ar)) {
+    m.vis = 1.0f;
+    m.st = sample_t_at(P, F, m.h, rho2, m.rho, m.rc);
+  } else {
+    const float inv_r = frcp(m.r);
+    m.st = sample_solar_t(P, F, m.h, m.r, m.rc * inv_r, m.rc, horizon_of(rho2, inv_r, F.bottom), m.vis);
+  }
   return m;
 }
 
 // _scattering_source :818-856 at a sample.
 __device__ __forceinline__ f3 source_of(const DevParams& P, const Frame& F, const RaySource& R, const MarchSample& m) {
-  return m.st * (R.ER * m.d.r + R.EM * m.d.m) + m.medium.scat * sample_ms(P, F, m.h, m.sc, m.hc);
+  return m.st * (R.ER * m.d.r + R.EM * m.d.m) + m.medium.scat * sample_ms_at(P, F, m.h, m.r, m.rc, m.rho);
 }
 // One constant-source segment [start, end] of the ray after what acc holds:
 // _scattering_segment :858-899.
@@ -814,24 +833,36 @@ __device__ __forceinline__ void then_source_segment(const DevParams& P, const Fr
   then_segment(acc, source_of(P, F, R, m), m.medium.ext, m.step);
 }
 
-// The base intervals [i0, i1) of n of a ray's march: source segments without
-// refinement, composed in ray order.
+// The intervals [i0, i1) of n of a ray's march in ray order: segment(d0, d1).
+// The two halves of the warp are two runs of one loop, so that an interval
+// costs no look at which half it is in.
+template <class Fraction, class Segment>
+__device__ __forceinline__ void for_intervals(const RayWarp& w, int i0, int i1, int n, Fraction fraction,
+                                              Segment segment) {
+  bool second = warp_second(i0, n);
+  float d0 = warp_at(warp_half(w, second), fraction(i0));
+  int i = i0;
+#pragma unroll 1
+  for (;;) {
+    const WarpHalf half = warp_half(w, second);
+    const int stop = second ? i1 : min(i1, (n - 1) / 2);  // boundary i + 1 is in the first half
+#pragma unroll 1
+    for (; i < stop; ++i) {
+      const float d1 = warp_at(half, fraction(i + 1));
+      segment(d0, d1);
+      d0 = d1;
+    }
+    if (second || i >= i1) return;
+    second = true;
+  }
+}
+// The base intervals without refinement.
 template <class Fraction>
 __device__ __forceinline__ Seg march(const DevParams& P, const Frame& F, const RaySource& R, const RayWarp& w, int i0,
                                      int i1, int n, Fraction fraction) {
   Seg acc = {splat(0.0f), splat(1.0f)};
-  bool second = warp_second(i0, n);
-  WarpHalf half = warp_half(w, second);
-  float d0 = warp_at(half, fraction(i0));
-  for (int i = i0; i < i1; ++i) {
-    if (!second && warp_second(i + 1, n)) {
-      second = true;
-      half = warp_half(w, true);
-    }
-    const float d1 = warp_at(half, fraction(i + 1));
-    then_source_segment(P, F, R, d0, d1, acc);
-    d0 = d1;
-  }
+  for_intervals(w, i0, i1, n, fraction,
+                [&](float d0, float d1) { then_source_segment(P, F, R, d0, d1, acc); });
   return acc;
 }
 

@@ -202,14 +202,13 @@ __device__ __forceinline__ DivideFractions divide_fractions(const DevParams& P) 
 }
 
 // One base interval [d0, d1] with its terminator refinement (:901-1031) after
-// what acc holds.
+// what acc holds; counts the refinement's samples.
 template <class Fractions>
 __device__ __forceinline__ void then_surface_interval(const DevParams& P, const Frame& F, const SurfaceMarch& M,
                                                       float d0, float d1, const Fractions& fractions,
                                                       uint32_t& samples, Seg& acc) {
   const MarchSample m = march_sample(P, F, M.rs, d0, d1);
   const f3 src = source_of(P, F, M.rs, m);
-  ++samples;
   // _terminator_refinement_weight :901-966; zero unless a shadow-cylinder
   // root exists or the disk is partly hidden at the midpoint
   float w = 0.0f;
@@ -245,20 +244,10 @@ __device__ __forceinline__ void then_surface_interval(const DevParams& P, const 
 template <class Fractions>
 __device__ __forceinline__ Seg surface_march(const DevParams& P, const Frame& F, const SurfaceMarch& M, int i0, int i1,
                                              const Fractions& fractions, uint32_t& samples) {
-  const int n = P.limb_steps;
   Seg acc = {splat(0.0f), splat(1.0f)};
-  bool second = warp_second(i0, n);
-  WarpHalf half = warp_half(M.rw, second);
-  float d0 = warp_at(half, fractions.limb(i0));
-  for (int i = i0; i < i1; ++i) {
-    if (!second && warp_second(i + 1, n)) {
-      second = true;
-      half = warp_half(M.rw, true);
-    }
-    const float d1 = warp_at(half, fractions.limb(i + 1));
-    then_surface_interval(P, F, M, d0, d1, fractions, samples, acc);
-    d0 = d1;
-  }
+  samples += i1 - i0;
+  for_intervals(M.rw, i0, i1, P.limb_steps, fractions.limb,
+                [&](float d0, float d1) { then_surface_interval(P, F, M, d0, d1, fractions, samples, acc); });
   return acc;
 }
 // _integrate_surface_scattering :1667-1755 (with :901-1032).  `start`/`end`

@@ -119,24 +119,15 @@ __global__ void __maxnreg__(72) k_multi_scattering(DevParams P, Frame F,
       const int n = P.ms_steps;
       const int per = (n + kLanes - 1) / kLanes;
       const int i0 = min(sub * per, n), i1 = min(i0 + per, n);
-      bool second = warp_second(i0, n);
-      WarpHalf half = warp_half(w, second);
-      float d0 = warp_at(half, s_fraction[i0]);
-      for (int i = i0; i < i1; ++i) {
-        if (!second && warp_second(i + 1, n)) {
-          second = true;
-          half = warp_half(w, true);
-        }
-        const float d1 = warp_at(half, s_fraction[i + 1]);
+      for_intervals(w, i0, i1, n, TableFraction{s_fraction}, [&](float d0, float d1) {
         const MarchSample m = march_sample(P, F, R, d0, d1);
-        f3 t, w;
-        segment_integral(m.medium.ext, m.step, t, w);
-        w = pT * w;
-        dL = dL + w * (m.st * (R.ER * m.d.r + R.EM * m.d.m));
-        dF = dF + w * m.medium.scat;
+        f3 t, weight;
+        segment_integral(m.medium.ext, m.step, t, weight);
+        weight = pT * weight;
+        dL = dL + weight * (m.st * (R.ER * m.d.r + R.EM * m.d.m));
+        dF = dF + weight * m.medium.scat;
         pT = pT * t;
-        d0 = d1;
-      }
+      });
       samples = uint32_t(i1 - i0);
     }
   }
