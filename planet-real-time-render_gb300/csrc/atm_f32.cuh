@@ -31,5 +31,30 @@ __device__ __forceinline__ r3 rnormalized(r3 v) {
   const float inv = dv(1.0f, add(__fsqrt_rn(rdot(v, v)), 0.0f));
   return {mul(inv, v.x), mul(inv, v.y), mul(inv, v.z)};
 }
+
+// Two floats in a 64-bit register: an .f32x2 instruction is the two scalar
+// ones, each with its own rounding.  A product is an fma onto zero (its zeros
+// are positive), since the assembler contracts mul.rn.f32x2 and add.rn.f32x2,
+// unlike the scalar forms, into one rounding.
+typedef unsigned long long Pair;
+__device__ __forceinline__ Pair pair(float a, float b) {
+  Pair r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ void halves(Pair p, float& a, float& b) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(p));
+}
+__device__ __forceinline__ Pair mul(Pair a, Pair b) {
+  Pair r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(pair(0.0f, 0.0f)));
+  return r;
+}
+__device__ __forceinline__ Pair mul(Pair a, float w) { return mul(a, pair(w, w)); }
+__device__ __forceinline__ Pair add(Pair a, Pair b) {
+  Pair r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
 }  // namespace f32
 }  // namespace atm

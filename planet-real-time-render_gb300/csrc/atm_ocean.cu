@@ -121,9 +121,10 @@ __device__ constexpr float period_of(int c) { return c == 0 ? 2048.0f : c == 1 ?
 // 2^kLog2N texels a side.  The size and the periods are powers of two, so the
 // scalings are exact, the wrap is a mask and nothing is divided: integer
 // remainders by a run-time size were most of this kernel (4K G-buffer over a
-// coast, 128 texels: 1016 us with them and flat pixel indices, 498 us without;
-// bound by issue, 1700 instructions a warp).  kTapMagic adds an integer below 2^22 into the low mantissa
-// bits; the mask keeps every index in range whatever the input.
+// coast, 128 texels: 1016 us with them and flat pixel indices, 498 us without,
+// 448 us with two components interpolated in an instruction; bound by issue,
+// 1580 instructions a warp).  kTapMagic adds an integer below 2^22 into the
+// low mantissa bits; the mask keeps every index in range whatever the input.
 struct Taps {
   int i00, i10, i01, i11;
   float fx, fy;
@@ -147,18 +148,34 @@ __device__ __forceinline__ Taps spectrum_taps(float u, float v) {
   t.i11 = x1 + y1;
   return t;
 }
-__device__ __forceinline__ float2 taps_disp(const OceanSpectrum& S, const Taps& t) {
-  const float2 a = __ldg(S.displacement + t.i00), b = __ldg(S.displacement + t.i10), c = __ldg(S.displacement + t.i01),
-               d = __ldg(S.displacement + t.i11);
-  return make_float2(lerp_ref(lerp_ref(a.x, b.x, t.fx), lerp_ref(c.x, d.x, t.fx), t.fy),
-                     lerp_ref(lerp_ref(a.y, b.y, t.fx), lerp_ref(c.y, d.y, t.fx), t.fy));
+// The two fractions of a place for lerps of two components at once.
+struct PairLerp {
+  Pair fx, gx, fy, gy;
+};
+__device__ __forceinline__ PairLerp pair_lerp(const Taps& t) {
+  const float gx = sub(1.0f, t.fx), gy = sub(1.0f, t.fy);
+  return {pair(t.fx, t.fx), pair(gx, gx), pair(t.fy, t.fy), pair(gy, gy)};
 }
-__device__ __forceinline__ float4 lerp4(const float4* p, const Taps& t) {
-  const float4 a = __ldg(p + t.i00), b = __ldg(p + t.i10), c = __ldg(p + t.i01), d = __ldg(p + t.i11);
-  return make_float4(lerp_ref(lerp_ref(a.x, b.x, t.fx), lerp_ref(c.x, d.x, t.fx), t.fy),
-                     lerp_ref(lerp_ref(a.y, b.y, t.fx), lerp_ref(c.y, d.y, t.fx), t.fy),
-                     lerp_ref(lerp_ref(a.z, b.z, t.fx), lerp_ref(c.z, d.z, t.fx), t.fy),
-                     lerp_ref(lerp_ref(a.w, b.w, t.fx), lerp_ref(c.w, d.w, t.fx), t.fy));
+__device__ __forceinline__ Pair bilerp(const PairLerp& w, Pair a, Pair b, Pair c, Pair d) {
+  return add(mul(add(mul(a, w.gx), mul(b, w.fx)), w.gy), mul(add(mul(c, w.gx), mul(d, w.fx)), w.fy));
+}
+__device__ __forceinline__ float2 taps_disp(const OceanSpectrum& S, const Taps& t) {
+  const Pair* p = reinterpret_cast<const Pair*>(S.displacement);
+  float2 r;
+  halves(bilerp(pair_lerp(t), __ldg(p + t.i00), __ldg(p + t.i10), __ldg(p + t.i01), __ldg(p + t.i11)), r.x, r.y);
+  return r;
+}
+__device__ __forceinline__ float lerp_x(const float4* p, const Taps& t) {
+  return lerp_ref(lerp_ref(__ldg(&p[t.i00].x), __ldg(&p[t.i10].x), t.fx),
+                  lerp_ref(__ldg(&p[t.i01].x), __ldg(&p[t.i11].x), t.fx), t.fy);
+}
+__device__ __forceinline__ float4 lerp4(const float4* p, const PairLerp& w, const Taps& t) {
+  const ulonglong2* q = reinterpret_cast<const ulonglong2*>(p);
+  const ulonglong2 a = __ldg(q + t.i00), b = __ldg(q + t.i10), c = __ldg(q + t.i01), d = __ldg(q + t.i11);
+  float4 r;
+  halves(bilerp(w, a.x, b.x, c.x, d.x), r.x, r.y);
+  halves(bilerp(w, a.y, b.y, c.y, d.y), r.z, r.w);
+  return r;
 }
 
 // The undisturbed coordinate of cascade kC under the displaced point: the
@@ -184,9 +201,9 @@ __device__ __forceinline__ Taps inverted_taps(const OceanSpectrum& S, const Ocea
 template <int kLog2N>
 __device__ float wave_height(const OceanSpectrum& S, const OceanFrame& F, r3 goff, OceanAxes A) {
   float height = 0.0f;
-  if (F.geometry_cascades > 0) height = add(height, lerp4(S.height_gradient, inverted_taps<kLog2N, 0>(S, F, goff, A)).x);
-  if (F.geometry_cascades > 1) height = add(height, lerp4(S.height_gradient, inverted_taps<kLog2N, 1>(S, F, goff, A)).x);
-  if (F.geometry_cascades > 2) height = add(height, lerp4(S.height_gradient, inverted_taps<kLog2N, 2>(S, F, goff, A)).x);
+  if (F.geometry_cascades > 0) height = add(height, lerp_x(S.height_gradient, inverted_taps<kLog2N, 0>(S, F, goff, A)));
+  if (F.geometry_cascades > 1) height = add(height, lerp_x(S.height_gradient, inverted_taps<kLog2N, 1>(S, F, goff, A)));
+  if (F.geometry_cascades > 2) height = add(height, lerp_x(S.height_gradient, inverted_taps<kLog2N, 2>(S, F, goff, A)));
   return height;
 }
 
@@ -198,8 +215,9 @@ __device__ __forceinline__ void cascade_slope(const OceanSpectrum& S, const Ocea
   r3 au, av;
   cascade_axes<kC>(A, au, av);
   const Taps t = inverted_taps<kLog2N, kC>(S, F, goff, A);
-  const float4 hg = lerp4(S.height_gradient, t);
-  const float4 j = lerp4(S.jacobian, t);
+  const PairLerp w = pair_lerp(t);
+  const float4 hg = lerp4(S.height_gradient, w, t);
+  const float4 j = lerp4(S.jacobian, w, t);
   constexpr float kMinWavelength = period_of(kC) / 5.5f;
   const float spw = dv(kMinWavelength, fmx(footprint, 0.01f));
   float resolved = fmn(fmx(mul(sub(spw, 2.0f), 0.25f), 0.0f), 1.0f);

@@ -23,15 +23,19 @@
 #include <type_traits>
 #include <utility>
 
+#include "atm_f32.cuh"
 #include "atm_kernels.h"
 
 namespace atm {
 
 namespace {
 
-__device__ __forceinline__ float mul(float a, float b) { return __fmul_rn(a, b); }
-__device__ __forceinline__ float add(float a, float b) { return __fadd_rn(a, b); }
-__device__ __forceinline__ float sub(float a, float b) { return __fsub_rn(a, b); }
+using f32::add;
+using f32::halves;
+using f32::mul;
+using f32::pair;
+using f32::Pair;
+using f32::sub;
 __device__ __forceinline__ float fmaxf_(float a, float b) { return a > b ? a : b; }
 __device__ __forceinline__ float fminf_(float a, float b) { return a < b ? a : b; }
 __device__ __forceinline__ float clampf_(float x, float lo, float hi) { return fminf_(fmaxf_(x, lo), hi); }
@@ -97,27 +101,6 @@ __global__ void __launch_bounds__(kRunPixels * kRunRows) k_post_extract(PostPara
 // strip only feed the others.  Bound by issue.  Two passes over 1920x1080
 // texels: 41 us when a tile and its halo lay in shared memory (five 16-byte
 // reads a tap direction and texel), 38 us with one texel a lane, 21 us so.
-typedef unsigned long long Pair;
-__device__ __forceinline__ Pair pair(float a, float b) {
-  Pair r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
-  return r;
-}
-__device__ __forceinline__ void halves(Pair p, float& a, float& b) {
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(p));
-}
-// The rounded products: as an fma onto zero, since the assembler contracts
-// mul.rn.f32x2 and add.rn.f32x2, unlike the scalar forms, into one rounding.
-__device__ __forceinline__ Pair mul(Pair a, float w) {
-  Pair r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(pair(w, w)), "l"(pair(0.0f, 0.0f)));
-  return r;
-}
-__device__ __forceinline__ Pair add(Pair a, Pair b) {
-  Pair r;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
 struct BlurRow {  // a lane's two texels
   Pair c[3];
 };
