@@ -378,14 +378,28 @@ __device__ __forceinline__ bool tile_pixel_of(const ImageLayout& L, const PixelT
   return x < L.width && y < L.height;
 }
 
-// kShade: the surface colour comes from the fused surface lighting and
-// shading (shaded_scene) instead of the scene image.
-template <bool kShade>
+// The fused frame's surface colours (shaded_scene) into hdr, where the
+// composite takes them from: shading in the composite itself, on a network
+// block's 20 warps an SM, took 1.61 ms a 4K frame, 1.39 ms so.
+__global__ void __launch_bounds__(kRunPixels * kRunRows) k_scene(DevParams P, Frame F, ImageLayout L, CompositeScalars A,
+                                                                 ShadeParams S, ShadeImages I,
+                                                                 float* __restrict__ hdr) {
+  int x, y;
+  if (!run_pixel(L, x, y)) return;
+  const size_t e = pix_offset(L, x, y);
+  const f3 color = shaded_scene(P, F, A, S, L, I, x, y, e, I.surface_id[e]);
+  float* out = hdr + e * L.channels;
+  out[0] = color.x;
+  out[1] = color.y;
+  out[2] = color.z;
+}
+
+// `scene` may be hdr: a pixel's colour is read by the thread that then writes
+// it, and by no other.
 __global__ void __launch_bounds__(128 * kWorkers, 1) k_composite_surrogate(
-    DevParams P, Frame F, ImageLayout L, PixelTiles N, CompositeScalars A, const float* __restrict__ scene,
+    DevParams P, Frame F, ImageLayout L, PixelTiles N, CompositeScalars A, const float* scene,
     const float* __restrict__ space, const int32_t* __restrict__ sid, const float* __restrict__ pos,
-    const float4* __restrict__ svlut, SurrogateNets nets, SurrogateQueue Q, float* __restrict__ hdr, ShadeParams S,
-    ShadeImages I) {
+    const float4* __restrict__ svlut, SurrogateNets nets, SurrogateQueue Q, float* hdr) {
   extern __shared__ __align__(128) unsigned char smem[];  // the aerial network, then the sky network
   __shared__ NetBlock B;
   bool nets_ok;  // tile-uniform: the networks may run
@@ -481,7 +495,7 @@ __global__ void __launch_bounds__(128 * kWorkers, 1) k_composite_surrogate(
     uint32_t qkind = kQueueSurface;
     f3 Lnet = mk(-1.0f, 0.0f, 0.0f);  // the network's in-scattering (x < 0: none)
     if (inside && kind != kSurfPlain) {
-      f3 color = kShade ? shaded_scene(P, F, A, S, L, I, x, y, e, sid[e]) : ld3(scene + o);
+      f3 color = ld3(scene + o);
       if (kind == kSurfMlp) {
         // transmittance: the plain path's own two-tap LUT ratio (:1603-1665);
         // in-scattering: the network, ln(L / E + floor + floor_t T)
@@ -930,22 +944,23 @@ cudaError_t launch_composite_surrogate(const DevParams& P, const ImageLayout& L,
   const ShadeParams S = shade ? *shade : ShadeParams{};
   const ShadeImages I = shade_images ? *shade_images : ShadeImages{};
   if (shade) {
-    e = cudaFuncSetAttribute(k_composite_surrogate<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return e;
-    k_composite_surrogate<true><<<grid, 128 * kWorkers, smem, s>>>(P, F, L, N, A, scene, space, sid, pos, svlut, nets, Q,
-                                                        hdr, S, I);
+    k_scene<<<run_grid(L), run_block(), 0, s>>>(P, F, L, A, S, I, hdr);
     e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    k_surrogate_fallback<true><<<kQueueBlocks * sm_count, 256, 0, s>>>(P, F, L, A, scene, space, pos, Q, hdr, counter, S, I);
-  } else {
-    e = cudaFuncSetAttribute(k_composite_surrogate<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return e;
-    k_composite_surrogate<false><<<grid, 128 * kWorkers, smem, s>>>(P, F, L, N, A, scene, space, sid, pos, svlut, nets,
-                                                         Q, hdr, S, I);
-    e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-    k_surrogate_fallback<false><<<kQueueBlocks * sm_count, 256, 0, s>>>(P, F, L, A, scene, space, pos, Q, hdr, counter, S, I);
+    scene = hdr;
   }
+  e = cudaFuncSetAttribute(k_composite_surrogate, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  if (e != cudaSuccess) return e;
+  k_composite_surrogate<<<grid, 128 * kWorkers, smem, s>>>(P, F, L, N, A, scene, space, sid, pos, svlut, nets, Q, hdr);
+  e = cudaGetLastError();
+  if (e != cudaSuccess) return e;
+  // the queued pixels' colours may be overwritten in hdr by then: the fused frame shades them again
+  if (shade)
+    k_surrogate_fallback<true><<<kQueueBlocks * sm_count, 256, 0, s>>>(P, F, L, A, scene, space, pos, Q, hdr, counter, S,
+                                                                      I);
+  else
+    k_surrogate_fallback<false><<<kQueueBlocks * sm_count, 256, 0, s>>>(P, F, L, A, scene, space, pos, Q, hdr, counter,
+                                                                       S, I);
   e = cudaGetLastError();
   if (e != cudaSuccess || Q.lm == nullptr) return e;
   k_surrogate_calibrate<<<run_grid(L), run_block(), 0, s>>>(L, Q, hdr);
