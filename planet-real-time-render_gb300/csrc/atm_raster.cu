@@ -369,48 +369,67 @@ __device__ __forceinline__ void box_pixels(const RasterSetup& T, const Box& b, i
 // their tiles (the low tile_bits), so that an entry's index and its tiles'
 // exclusive prefix come from one atomic and the list is sorted by the prefix
 // (the three scans were 13 us).  0: only the tile counts are listed, for the scans below.
-constexpr int kDepthLanes = 8, kDepthTris = 32 / kDepthLanes;
+// A block lists its 32 triangles' large ones with one atomic: thousands of them
+// on one address are a queue (71 us for a frame of 55,000 triangles with one
+// each).
+constexpr int kDepthLanes = 8, kDepthTris = 256 / kDepthLanes;  // of a block
 __global__ void __launch_bounds__(256) k_raster_depth(RasterStream S, ImageLayout L, int tile_bits,
                                                       unsigned long long* __restrict__ depth_key) {
-  const int lane = threadIdx.x & 31, sub = lane % kDepthLanes;
+  __shared__ uint32_t s_tiles[kDepthTris];  // of the block's large triangles, 0 for the others
+  static_assert(kDepthTris == 32, "a warp lists a block's triangles");
+  const int lane = threadIdx.x & 31, sub = lane % kDepthLanes, slot = threadIdx.x / kDepthLanes;
   const long long n = min((long long)S.count[0], (long long)S.capacity);
-  const long long warp = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
-  const long long stride = ((long long)gridDim.x * blockDim.x >> 5) * kDepthTris;
-  for (long long base = warp * kDepthTris; base < n; base += stride) {
-    const long long q = base + lane / kDepthLanes;
-    bool medium = false;
+  for (long long block = blockIdx.x * (long long)kDepthTris; block < n; block += (long long)gridDim.x * kDepthTris) {
+    const long long q = block + slot;
+    uint32_t tiles = 0;
+    bool small = false, medium = false;
+    RasterSetup T;
+    Box b = {0, 0, 0, 0};
     if (q < n) {
-      const RasterSetup T = load_setup(S.tris + q);
-      const Box b = bbox(T, L);
+      T = load_setup(S.tris + q);
+      b = bbox(T, L);
       if (T.inv_area > 0.0f && b.x0 <= b.x1 && b.y0 <= b.y1) {
         const long long area = (long long)(b.x1 - b.x0 + 1) * (b.y1 - b.y0 + 1);
-        if (area <= kRasterLanesArea) {
-          box_pixels(T, b, sub, kDepthLanes, L.height, depth_key, (unsigned long long)q);
-        } else if (area <= kRasterWarpArea) {
-          medium = true;
-        } else if (sub == 0) {
-          const uint32_t tiles = uint32_t((b.x1 - b.x0 + kRasterTileW) / kRasterTileW) *
-                                 uint32_t((b.y1 - b.y0 + kRasterTileH) / kRasterTileH);
-          if (tile_bits > 0) {
-            const unsigned long long old = atomicAdd(S.listed, (1ull << tile_bits) + tiles);
-            const uint32_t idx = uint32_t(old >> tile_bits);  // at most one entry per stored triangle
-            S.large[idx] = uint32_t(q);
-            S.tile_prefix[idx] = old & ((1ull << tile_bits) - 1);
-          } else {
-            const uint32_t idx = atomicAdd(S.count + 1, 1u);
-            S.large[idx] = uint32_t(q);
-            S.large_tiles[idx] = tiles;
-          }
-        }
+        small = area <= kRasterLanesArea;
+        medium = !small && area <= kRasterWarpArea;
+        if (!small && !medium)
+          tiles = uint32_t((b.x1 - b.x0 + kRasterTileW) / kRasterTileW) *
+                  uint32_t((b.y1 - b.y0 + kRasterTileH) / kRasterTileH);
       }
     }
+    if (sub == 0) s_tiles[slot] = tiles;
+    if (__syncthreads_or(tiles != 0) && threadIdx.x < 32) {
+      const uint32_t mine = s_tiles[lane];
+      const unsigned large = __ballot_sync(0xffffffffu, mine != 0);
+      unsigned long long incl = mine;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const unsigned long long t = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += t;
+      }
+      const unsigned long long listed = __popc(large);
+      unsigned long long old = 0;
+      if (lane == 31)
+        old = tile_bits > 0 ? atomicAdd(S.listed, (listed << tile_bits) + incl) : atomicAdd(S.count + 1, uint32_t(listed));
+      old = __shfl_sync(0xffffffffu, old, 31);
+      if (mine != 0) {  // at most one entry per stored triangle
+        const uint32_t idx = uint32_t(tile_bits > 0 ? old >> tile_bits : old) + __popc(large & ((1u << lane) - 1u));
+        S.large[idx] = uint32_t(block + lane);
+        if (tile_bits > 0)
+          S.tile_prefix[idx] = (old & ((1ull << tile_bits) - 1)) + incl - mine;
+        else
+          S.large_tiles[idx] = mine;
+      }
+    }
+    __syncthreads();  // s_tiles has been read
+    if (small) box_pixels(T, b, sub, kDepthLanes, L.height, depth_key, (unsigned long long)q);
     unsigned m = __ballot_sync(0xffffffffu, medium && sub == 0);
     while (m) {
       const int leader = __ffs(m) - 1;
       m &= m - 1;
-      const long long ql = base + leader / kDepthLanes;
-      const RasterSetup T = load_setup(S.tris + ql);
-      box_pixels(T, bbox(T, L), lane, 32, L.height, depth_key, (unsigned long long)ql);
+      const long long ql = q - lane / kDepthLanes + leader / kDepthLanes;
+      const RasterSetup U = load_setup(S.tris + ql);
+      box_pixels(U, bbox(U, L), lane, 32, L.height, depth_key, (unsigned long long)ql);
     }
   }
 }
