@@ -60,8 +60,8 @@ COMPOSITE_FLOP_PER_SAMPLE = 406.16
 COMPOSITE_BYTES_PER_PIXEL = 52
 # DRAM bytes (read + write) of one k_composite launch of the 2 km camera at
 # 1920x1080, from `ncu --metrics dram__bytes_read.sum,dram__bytes_write.sum`
-# on `bench.py --profile-case frame1080p` (58,468,352 + 3,072,256)
-COMPOSITE_DRAM_BYTES_1080P = 58_468_352 + 3_072_256
+# on `bench.py --profile-case frame1080p` (58,328,320 + 3,855,360)
+COMPOSITE_DRAM_BYTES_1080P = 58_328_320 + 3_855_360
 MLP_CHECK_FRACTION = 0.01  # share of MLP pixels the plain path re-integrates
 # A step is this many passes of the three cameras' chains (48 frames of
 # 1080p, ~57 ms): with the usual 20 timed steps the timed region lasts over a
