@@ -1453,8 +1453,8 @@ def _profile_batch(args):
 
 def _profile_train(args):
     """MLP training and batch inference of the aerial network (11 -> 4x64 ->
-    6): 8 Adam steps of 16,384 samples (k_mlp_grad, k_reduce_partials,
-    k_adam), then tcgen05 and mma.sync forwards of 2^20 samples."""
+    6): 8 Adam steps of 16,384 samples (k_mlp_grad,
+    k_reduce_adam), then tcgen05 and mma.sync forwards of 2^20 samples."""
 
     import torch
 
