@@ -70,8 +70,7 @@ __device__ __forceinline__ f3 operator/(f3 a, float s) { return {a.x / s, a.y / 
 __device__ __forceinline__ f3 operator/(f3 a, f3 b) { return {a.x / b.x, a.y / b.y, a.z / b.z}; }
 __device__ __forceinline__ float dot(f3 a, f3 b) { return (a.x * b.x + a.y * b.y) + a.z * b.z; }
 __device__ __forceinline__ float norm(f3 a) { return sqrtf(dot(a, a)); }
-// One FMNMX each; for a NaN first argument the second one, as a > b ? a : b
-// gives it (which costs a compare and a select on the same pipe).
+// For a NaN first argument the second one, as a > b ? a : b gives it.
 __device__ __forceinline__ float mx(float a, float b) { return fmaxf(a, b); }
 __device__ __forceinline__ float mn(float a, float b) { return fminf(a, b); }
 __device__ __forceinline__ float clampf(float x, float lo, float hi) { return mn(mx(x, lo), hi); }
@@ -89,9 +88,8 @@ __device__ __forceinline__ f3 arr3(const float (&a)[3]) { return {a[0], a[1], a[
 // root and 2^x.  Differences ~1e-7 relative against the reference's IEEE
 // operations, far below the 1e-3 parity tolerance.  Subtractions of two
 // Earth-scale quantities keep IEEE sqrtf / division (see callers).  The .ftz
-// forms are one instruction: without it each one is wrapped in a compare and
-// two scalings for subnormal operands, of which these paths have none that
-// matters (the smallest, a density, is subnormal past 87 scale heights).
+// forms flush subnormals, of which these paths have none that matters (the
+// smallest, a density, is subnormal past 87 scale heights), and are faster.
 __device__ __forceinline__ float fdiv(float a, float b) { return __fdividef(a, b); }
 __device__ __forceinline__ float frcp(float b) {
   float r;

@@ -29,10 +29,10 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
 }
 // SiLU of two pre-activations given as halves h = z / 2 (the packed hidden
 // layers are halved): z sigmoid(z) = h (1 + tanh h) = h + h tanh(h) in FP32
-// (tanh.approx.f32, one MUFU op each), rounded once into the packed BF16
+// (tanh.approx.f32), rounded once into the packed BF16
 // pair that feeds the next layer.  (A packed tanh.approx.bf16x2 / fma.bf16x2
-// form halves the MUFU work but costs the networks up to 7x their held-out
-// radiance error: the activations would be rounded three times.)
+// form is faster but costs the networks up to 7x their held-out radiance
+// error: the activations would be rounded three times.)
 __device__ __forceinline__ float silu_half(float h) {
   float t;
   asm("tanh.approx.f32 %0, %1;" : "=f"(t) : "f"(h));
