@@ -567,7 +567,8 @@ int atm_shade_surface(const AtmShadeParams* params, const AtmShadeImages* images
  * atm_shade_surface (renderer.py:1277-1575) and the COMPOSITE view of
  * atm_composite (or, with `surrogate`, of atm_composite_surrogate), as the
  * reference's frame calls them in sequence (renderer.py:1671-1727).  Each
- * pixel's lighting and shaded colour stay in registers: the three
+ * pixel's lighting stays in registers and its shaded colour there or, with
+ * `surrogate`, in `hdr` until the composite replaces it: the three
  * full-resolution images the separate calls write and read back
  * (surface_sun_transmittance, surface_sky_radiance, surface_hdr) are not
  * formed, and `images`' sun_transmittance, sky_radiance and surface_hdr may

@@ -380,7 +380,8 @@ __device__ __forceinline__ bool tile_pixel_of(const ImageLayout& L, const PixelT
 
 // The fused frame's surface colours (shaded_scene) into hdr, where the
 // composite takes them from: shading in the composite itself, on a network
-// block's 20 warps an SM, took 1.61 ms a 4K frame, 1.39 ms so.
+// block's 20 warps an SM, takes 1.61 ms a 4K frame, 1.39 ms so.  Not where hdr
+// is also an input (hdr_is_input), which it would overwrite.
 __global__ void __launch_bounds__(kRunPixels * kRunRows) k_scene(DevParams P, Frame F, ImageLayout L, CompositeScalars A,
                                                                  ShadeParams S, ShadeImages I,
                                                                  float* __restrict__ hdr) {
@@ -394,12 +395,14 @@ __global__ void __launch_bounds__(kRunPixels * kRunRows) k_scene(DevParams P, Fr
   out[2] = color.z;
 }
 
-// `scene` may be hdr: a pixel's colour is read by the thread that then writes
-// it, and by no other.
+// The surface colour is `scene`'s or, with kShade, the fused frame's own
+// (shaded_scene).  hdr may be `scene` or any other image: a pixel is read by
+// the thread that then writes it, and by no other.
+template <bool kShade>
 __global__ void __launch_bounds__(128 * kWorkers, 1) k_composite_surrogate(
     DevParams P, Frame F, ImageLayout L, PixelTiles N, CompositeScalars A, const float* scene,
     const float* __restrict__ space, const int32_t* __restrict__ sid, const float* __restrict__ pos,
-    const float4* __restrict__ svlut, SurrogateNets nets, SurrogateQueue Q, float* hdr) {
+    const float4* __restrict__ svlut, SurrogateNets nets, SurrogateQueue Q, float* hdr, ShadeParams S, ShadeImages I) {
   extern __shared__ __align__(128) unsigned char smem[];  // the aerial network, then the sky network
   __shared__ NetBlock B;
   bool nets_ok;  // tile-uniform: the networks may run
@@ -495,7 +498,7 @@ __global__ void __launch_bounds__(128 * kWorkers, 1) k_composite_surrogate(
     uint32_t qkind = kQueueSurface;
     f3 Lnet = mk(-1.0f, 0.0f, 0.0f);  // the network's in-scattering (x < 0: none)
     if (inside && kind != kSurfPlain) {
-      f3 color = ld3(scene + o);
+      f3 color = kShade ? shaded_scene(P, F, A, S, L, I, x, y, e, sid[e]) : ld3(scene + o);
       if (kind == kSurfMlp) {
         // transmittance: the plain path's own two-tap LUT ratio (:1603-1665);
         // in-scattering: the network, ln(L / E + floor + floor_t T)
@@ -921,6 +924,25 @@ cudaError_t launch_gen_samples(const SurrogateSetDev* sets, int n_sets, int kind
   return cudaGetLastError();
 }
 
+namespace {
+// Whether hdr shares memory with the stars or with an image of the G-buffer.
+bool hdr_is_input(const ImageLayout& L, const float* hdr, const float* space, const ShadeImages& I) {
+  const int64_t elements = (L.width - 1) * int64_t(L.sx) + (L.height - 1) * int64_t(L.sy) + 1;
+  const auto meets = [&](const void* image, int channels) {
+    const uintptr_t a = reinterpret_cast<uintptr_t>(hdr), b = reinterpret_cast<uintptr_t>(image);
+    return b != 0 && a < b + uintptr_t(elements) * channels * 4 && b < a + uintptr_t(elements) * L.channels * 4;
+  };
+  const void* const vectors[] = {space,         I.position,         I.normal,         I.albedo,        I.seabed_albedo,
+                                 I.seabed_normal, I.terrain_position, I.terrain_normal, I.terrain_albedo};
+  const void* const scalars[] = {I.water_depth, I.slope_variance, I.surface_id, I.terrain_surface_id};
+  for (const void* p : vectors)
+    if (meets(p, L.channels)) return true;
+  for (const void* p : scalars)
+    if (meets(p, 1)) return true;
+  return false;
+}
+}  // namespace
+
 size_t surrogate_smem_bytes(const SurrogateNets& nets) { return size_t(nets.ap_bytes) + size_t(nets.sky_bytes); }
 
 cudaError_t launch_composite_surrogate(const DevParams& P, const ImageLayout& L, const CompositeScalars& scalars,
@@ -943,15 +965,17 @@ cudaError_t launch_composite_surrogate(const DevParams& P, const ImageLayout& L,
   const int grid = std::min(sm_count, N.count);
   const ShadeParams S = shade ? *shade : ShadeParams{};
   const ShadeImages I = shade_images ? *shade_images : ShadeImages{};
-  if (shade) {
+  const bool in_composite = shade && hdr_is_input(L, hdr, space, I);
+  if (shade && !in_composite) {
     k_scene<<<run_grid(L), run_block(), 0, s>>>(P, F, L, A, S, I, hdr);
     e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     scene = hdr;
   }
-  e = cudaFuncSetAttribute(k_composite_surrogate, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  const auto composite = in_composite ? k_composite_surrogate<true> : k_composite_surrogate<false>;
+  e = cudaFuncSetAttribute(composite, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return e;
-  k_composite_surrogate<<<grid, 128 * kWorkers, smem, s>>>(P, F, L, N, A, scene, space, sid, pos, svlut, nets, Q, hdr);
+  composite<<<grid, 128 * kWorkers, smem, s>>>(P, F, L, N, A, scene, space, sid, pos, svlut, nets, Q, hdr, S, I);
   e = cudaGetLastError();
   if (e != cudaSuccess) return e;
   // the queued pixels' colours may be overwritten in hdr by then: the fused frame shades them again

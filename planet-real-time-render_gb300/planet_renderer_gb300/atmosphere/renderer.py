@@ -300,15 +300,17 @@ class AtmosphereRenderer:
                      ocean_surface_id: int | None = None, surrogate=None, stats: torch.Tensor | None = None,
                      check_fraction: float = 0.01, seed: int = 0) -> None:
         """``prepare_frame`` -> surface shading -> ``composite`` (COMPOSITE
-        view) in one pass over the pixels, the surface lighting and shaded
-        colour of each pixel kept in registers (``atm_render_frame``).
+        view) without the images between them (``atm_render_frame``): one
+        pass over the pixels, with ``surrogate`` two, the shaded colours held
+        in ``hdr`` between them.
         ``gbuffer`` holds the shading's G-buffer and terrain-snapshot images
         (``shading.GBUFFER_IMAGES``; ``position`` and ``surface_id`` are the
         composite's ``position_view`` and ``surface_id``).  ``sun_global`` and
         ``view_basis_global`` default to the local ones (a global frame equal
         to the camera's local frame).  With ``surrogate`` the composite is
-        ``composite_surrogate``'s.  The aerial volume and the public surface
-        lighting images are not updated."""
+        ``composite_surrogate``'s.  ``hdr`` may be an input image too (the
+        frame then shades in the composite).  The aerial volume and the public
+        surface lighting images are not updated."""
 
         from .. import shading
 
