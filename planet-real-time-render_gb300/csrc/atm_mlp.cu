@@ -10,6 +10,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cfloat>
 #include <cmath>
 #include <cstdint>
 #include <type_traits>
@@ -27,10 +28,11 @@ constexpr int kS = 64;        // samples of a tile
 constexpr int kThreads = 256;
 
 // z sigmoid(z), the forward's: the reciprocal is the hardware's with one Newton
-// step, within an ulp of the IEEE quotient; past z = -80, where the denominator
-// would leave float's range, that of -80 (1.8e-35).
+// step, within an ulp of the IEEE quotient; 0 for a denominator past 2^126 (z
+// below -87.3), the infinite one held at the largest float so that the step
+// stays finite.
 __device__ __forceinline__ float silu(float z) {
-  const float d = 1.0f + expf(fminf(-z, 80.0f));
+  const float d = fminf(1.0f + expf(-z), FLT_MAX);
   float r;
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
   return z * fmaf(fmaf(-d, r, 1.0f), r, r);
