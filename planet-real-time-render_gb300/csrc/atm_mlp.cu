@@ -501,7 +501,7 @@ __global__ void k_pack_tc(MlpShape m, const float* __restrict__ params, unsigned
         v = params[m.off_w[l] + n * in + k] * scale;
       } else if (n < out && k >= bk && k < bk + 3) {  // the bias in three BF16 parts
         v = params[m.off_b[l] + n] * scale;
-        for (int part = bk; part < k; ++part) v -= __bfloat162float(__float2bfloat16_rn(v));
+        for (int part = bk; part < k; ++part) v = isinf(v) ? 0.0f : v - __bfloat162float(__float2bfloat16_rn(v));
       }
       *reinterpret_cast<__nv_bfloat16*>(packed + off + tc_w_offset(n, k, np)) = __float2bfloat16_rn(v);
     }

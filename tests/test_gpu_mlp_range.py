@@ -26,3 +26,21 @@ def test_silu_of_large_preactivations(z):
         ref = z / (1.0 + np.exp(np.float64(-z)))
     np.testing.assert_allclose(net.forward(x, "f32").cpu().numpy(), ref, rtol=1e-6, atol=2e-36)
     net.close()
+
+
+@pytest.mark.parametrize("n_in", [11, 16])
+def test_infinite_output_biases_of_the_tensor_core_forward(n_in):
+    """The bias rides in three parts: an infinite one is its first part alone."""
+
+    import torch
+
+    from planet_renderer_gb300.atmosphere.mlp import Mlp
+
+    net = Mlp(n_in, 2, 3, seed=3)
+    p = net.params()
+    p[-3:] = torch.tensor([float("inf"), 0.5, float("-inf")], device="cuda")
+    net.set_params(p)
+    x = torch.as_tensor(np.random.default_rng(2).uniform(-1.0, 1.0, (130, n_in)).astype(np.float32), device="cuda")
+    got = net.forward(x, "bf16_tc")
+    assert torch.isposinf(got[:, 0]).all() and torch.isfinite(got[:, 1]).all() and torch.isneginf(got[:, 2]).all()
+    net.close()
