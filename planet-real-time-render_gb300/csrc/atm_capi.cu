@@ -12,6 +12,7 @@
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
+#include <limits>
 #include <new>
 #include <string>
 #include <vector>
@@ -101,6 +102,12 @@ int validate(const AtmParams& p) {
 // math.radians: x * (pi / 180) in double, then the kernel argument's f32 rounding
 float radians_f32(double degrees) { return float(degrees * (kPi / 180.0)); }
 
+// Factor of the altitude in exp(-h / H) = 2^(h rate); below 0 for every H, so
+// that the infinite altitude of a point outside the shell gives 0.
+float exp2_rate(double scale_height) {
+  return std::min(float(-M_LOG2E / scale_height), -std::numeric_limits<float>::denorm_min());
+}
+
 }  // namespace
 
 namespace atm {
@@ -125,8 +132,8 @@ DevParams make_dev_params(const AtmParams& p) {
   d.mie_k1 = float(3.0 * (1.0 - g * g));
   d.mie_k2 = float(8.0 * kPi * (2.0 + g * g));
   d.ray_k = float(16.0 * kPi);
-  d.exp2_r = float(-M_LOG2E / p.rayleigh_scale_height_m);
-  d.exp2_m = float(-M_LOG2E / p.mie_scale_height_m);
+  d.exp2_r = exp2_rate(p.rayleigh_scale_height_m);
+  d.exp2_m = exp2_rate(p.mie_scale_height_m);
   d.inv_oz_half = float(1.0 / p.absorption_half_width_m);
   d.inv_top = float(1.0 / p.top_altitude_m);
   d.t_w = p.transmittance_lut_width;
