@@ -643,13 +643,14 @@ ATM_API int atm_batch_create(const AtmParams* sets, const double* planet_radius_
 ATM_API int atm_batch_build(AtmBatch* b, const AtmBatchJob* jobs, int32_t n_jobs, void* arena, int64_t arena_texels,
                             const AtmBatchTuning* tuning, void* stream) {
   if (!b || !jobs || !arena || !tuning || n_jobs < 1) return fail(ATM_E_INVALID, "null argument to atm_batch_build");
-  int sv_item = tuning->sky_view_texels_per_item, ap_item = tuning->aerial_columns_per_item;
+  const int sv_item = tuning->sky_view_texels_per_item, ap_item = tuning->aerial_columns_per_item;
   if (sv_item < 1 || sv_item > 4096 || ap_item < 1 || ap_item > 4096 || tuning->blocks_per_sm < 1 ||
       tuning->blocks_per_sm > 8)
     return fail(ATM_E_INVALID, "tuning out of range");
-  // a lane takes a texel or a column: items are whole warps
-  sv_item = (sv_item + 31) / 32 * 32;
-  ap_item = (ap_item + 31) / 32 * 32;
+  long long columns = 0;
+  for (int i = 0; i < n_jobs; ++i)
+    if (jobs[i].kind == ATM_LUT_AERIAL) columns += (long long)jobs[i].width * jobs[i].height;
+  const bool groups = atm::batch_groups(columns, b->sm_count, tuning->blocks_per_sm);
   const size_t jsz = atm::batch_job_size();
   b->h_jobs.assign(size_t(n_jobs) * jsz, 0);
   b->h_prefix.assign(size_t(n_jobs) + 1, 0);
@@ -669,7 +670,7 @@ ATM_API int atm_batch_build(AtmBatch* b, const AtmBatchJob* jobs, int32_t n_jobs
     if (j.param_set < 0 || j.param_set >= int(b->params.size()))
       return fail(ATM_E_INVALID, "job %d: parameter set %d out of range", i, j.param_set);
     long long texels = 0;
-    int units = 0, per = 0;
+    int units = 0, per = 0, lanes = 1;
     if (j.kind == ATM_LUT_SKY_VIEW) {
       if (j.width < 16 || j.width > 2048 || j.height < 16 || j.height > 2048)
         return fail(ATM_E_INVALID, "job %d: sky-view size %dx%d outside 16..2048", i, j.width, j.height);
@@ -686,6 +687,7 @@ ATM_API int atm_batch_build(AtmBatch* b, const AtmBatchJob* jobs, int32_t n_jobs
       texels = (long long)j.width * j.height * j.depth;
       units = j.width * j.height;
       per = ap_item;
+      lanes = atm::batch_column_lanes(groups, j.depth);
     } else {
       return fail(ATM_E_INVALID, "job %d: kind %d is not sky-view or aerial", i, j.kind);
     }
@@ -694,9 +696,11 @@ ATM_API int atm_batch_build(AtmBatch* b, const AtmBatchJob* jobs, int32_t n_jobs
                   (long long)j.output_offset, (long long)(j.output_offset + texels), (long long)arena_texels);
     if (!std::isfinite(j.camera_altitude_m) || !std::isfinite(j.sun_zenith_cosine))
       return fail(ATM_E_INVALID, "job %d: non-finite camera or sun", i);
+    // an item is a multiple of the units that a warp takes at once; of shared columns those alone
+    per = lanes > 1 ? 32 / lanes : (per + 31) / 32 * 32;
     const int p = j.param_set;
     atm::fill_batch_job(*reinterpret_cast<atm::BatchJobDev*>(b->h_jobs.data() + size_t(slot) * jsz), b->dev[p], j,
-                        base, b->tlut[p], b->mslut[p], b->radius[p], b->E, b->ar_rad, per);
+                        base, b->tlut[p], b->mslut[p], b->radius[p], b->E, b->ar_rad, per, lanes);
     b->h_prefix[slot + 1] = b->h_prefix[slot] + (units + per - 1) / per;
   }
   cudaStream_t s = static_cast<cudaStream_t>(stream);
@@ -721,7 +725,7 @@ ATM_API int atm_batch_build(AtmBatch* b, const AtmBatchJob* jobs, int32_t n_jobs
   // the host tables are re-filled by the next call: make sure this one's copies are done
   ATM_CUDA(cudaStreamSynchronize(s), "job upload sync");
   ATM_CUDA(atm::launch_batch(reinterpret_cast<const atm::BatchJobDev*>(b->d_jobs), b->d_prefix, n_jobs,
-                             b->h_prefix[n_jobs], b->d_ticket, b->d_samples, b->sm_count * tuning->blocks_per_sm, s),
+                             b->h_prefix[n_jobs], b->d_ticket, b->d_samples, b->sm_count * tuning->blocks_per_sm, groups, s),
            "batch launch");
   return ATM_OK;
 }

@@ -95,9 +95,14 @@ struct BatchJobDev;
 size_t batch_job_size();
 void fill_batch_job(BatchJobDev& d, const DevParams& set_params, const AtmBatchJob& j, float4* arena,
                     const float4* tlut, const float4* mslut, double radius, const double E[3], double ar_rad,
-                    int per_item);
+                    int per_item, int lanes);
+// Whether the lanes of a warp share the columns of a batch of `columns` in all,
+// and how many share one of a volume `depth` slices deep.
+bool batch_groups(long long columns, int sm_count, int blocks_per_sm);
+int batch_column_lanes(bool groups, int depth);
 cudaError_t launch_batch(const BatchJobDev* jobs, const long long* prefix, int n_jobs, long long n_items,
-                         unsigned long long* ticket, unsigned long long* samples, int blocks, cudaStream_t s);
+                         unsigned long long* ticket, unsigned long long* samples, int blocks, bool groups,
+                         cudaStream_t s);
 
 // MLP surrogates (atm_mlp.cu): n_in -> [64 SiLU] x (n_layers - 1) -> n_out.
 constexpr int kMaxMlpLayers = 5;

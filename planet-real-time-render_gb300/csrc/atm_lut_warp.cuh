@@ -6,9 +6,10 @@
 // A texel's or column's set-up (its ray, the shell intersections, the phases)
 // costs as much as one to two march samples and every lane of its group
 // repeats it, so a group is as small as the launch allows: one lane where a
-// batch fills the machine, more where a single LUT would leave it idle.  A
-// batch of 512 LUTs takes 2.29 ms at one lane a texel or column, 7.8 ms at a
-// warp; a single 192x108 sky-view LUT 15.6 us at four lanes, 26 us at a warp.
+// batch fills the machine, more where a single LUT or a small batch would
+// leave it idle.  A batch of 512 LUTs takes 2.14 ms at one lane a texel or
+// column, 7.8 ms at a warp; a single 192x108 sky-view LUT 11 us at four lanes,
+// 26 us at a warp.
 #pragma once
 
 #include "atm_device.cuh"
@@ -44,17 +45,18 @@ __device__ __forceinline__ Seg group_compose(Seg s) {
   }
   return s;
 }
-// Ordered inclusive scan: lane i receives segment 0 then ... then i.
-__device__ __forceinline__ Seg warp_scan(Seg s) {
-  const int lane = threadIdx.x & 31;
+// Ordered inclusive scan within each group of kLanes consecutive lanes: lane i
+// receives segment 0 then ... then i.  Every lane must call.
+template <int kLanes>
+__device__ __forceinline__ Seg group_scan(Seg s) {
+  const int lane = threadIdx.x & (kLanes - 1);
 #pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
+  for (int o = 1; o < kLanes; o <<= 1) {
     Seg before = shfl_up_seg(s, o);
     if (lane >= o) s = seg_then(before, s);
   }
   return s;
 }
-
 
 // Boundary fractions i / n of a march into t[0..n], by the threads first,
 // first + stride, ...
@@ -189,17 +191,20 @@ __device__ __forceinline__ uint32_t aerial_column_lane(const DevParams& P, const
   return samples;
 }
 
-// One froxel column (x, y) by a warp: lanes take runs of depth slices, an
-// ordered scan of the runs gives each lane what lies before its own.  A run's
-// slices are stored as they are marched and completed in place after the
-// scan.  Returns the samples this lane evaluated.
-__device__ __forceinline__ uint32_t aerial_column_warp(const DevParams& P, const Frame& F, const AerialView& V, int x,
-                                                       int y, TableFraction fraction, float4* __restrict__ out) {
-  const int lane = threadIdx.x & 31;
+// One froxel column (x, y) by kLanes consecutive lanes, which take runs of
+// depth slices; an ordered scan of the runs gives each lane what lies before
+// its own.  A run's slices are stored (if `store`) as they are marched and
+// completed in place after the scan.  Every lane of the warp must call.
+// Returns the samples this lane evaluated.
+template <int kLanes>
+__device__ __forceinline__ uint32_t aerial_column_group(const DevParams& P, const Frame& F, const AerialView& V, int x,
+                                                        int y, bool store, TableFraction fraction,
+                                                        float4* __restrict__ out) {
+  const int lane = threadIdx.x & (kLanes - 1);
   const AerialColumn C = aerial_ray(P, F, V, x, y);
   const int depth = P.ap_d;
-  const int per = (depth + 31) >> 5;
-  const int k0 = min(lane * per, depth), k1 = min(k0 + per, depth);
+  const int per = (depth + kLanes - 1) / kLanes;
+  const int k0 = min(lane * per, depth), k1 = store ? min(k0 + per, depth) : k0;
   const size_t plane = size_t(P.ap_w) * P.ap_h;
   float4* o = out + size_t(y) * P.ap_w + x;
   Seg run = seg_identity();
@@ -211,9 +216,9 @@ __device__ __forceinline__ uint32_t aerial_column_warp(const DevParams& P, const
     if (per > 1) o[k * plane] = to4(run.L);
     prev = target;
   }
-  const Seg incl = warp_scan(run);
+  const Seg incl = group_scan<kLanes>(run);
   if (per == 1) {
-    if (lane < depth) o[lane * plane] = to4(vmax(incl.L, 0.0f));
+    if (k0 < k1) o[k0 * plane] = to4(vmax(incl.L, 0.0f));
     return samples;
   }
   Seg before = shfl_up_seg(incl, 1);

@@ -201,7 +201,7 @@ __global__ void __launch_bounds__(kAerialBlock) k_aerial(DevParams P, Frame F, A
   __syncthreads();
   const int warp_id = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   if (warp_id >= P.ap_w * P.ap_h) return;  // warp-uniform
-  uint32_t samples = aerial_column_warp(P, F, V, warp_id % P.ap_w, warp_id / P.ap_w, {s_fraction}, out);
+  uint32_t samples = aerial_column_group<32>(P, F, V, warp_id % P.ap_w, warp_id / P.ap_w, true, {s_fraction}, out);
   warp_count(samples, counter);
 }
 
