@@ -224,7 +224,11 @@ typedef struct AtmBatchJob {
   double tangent_half_fov;  /* aerial                                            */
 } AtmBatchJob;
 
-/* Work split of a batch launch (chosen by the Python autotuner). */
+/* Work split of a batch launch (chosen by the Python autotuner).  A warp takes
+ * an item at a time, a texel or a column a lane: both sizes are rounded up to a
+ * multiple of 32.  In a batch whose columns are at most a quarter of the
+ * launch's threads several lanes share a column, and an item is the 1 or 4
+ * columns that a warp then holds. */
 typedef struct AtmBatchTuning {
   int32_t sky_view_texels_per_item; /* 1..4096 */
   int32_t aerial_columns_per_item;  /* 1..4096 */

@@ -4,7 +4,8 @@ Times candidate ``Tuning`` values (texels per sky-view work item, columns per
 aerial work item, resident blocks per SM) on a sample of a batch's jobs with
 CUDA events, keeps the fastest and caches it in a JSON file keyed by the GPU,
 the native library build and the batch's job mix, so later runs with the same
-mix skip the search.
+mix skip the search.  The sample is large enough to be split as the whole
+batch is (``AtmBatchTuning``).
 """
 
 from __future__ import annotations
@@ -18,12 +19,13 @@ from pathlib import Path
 import torch
 
 from .. import _native
-from .batch import BatchedLutBuilder, Tuning
+from .batch import AERIAL, BatchedLutBuilder, Tuning
 
+# items are whole warps' units: multiples of 32
 CANDIDATES = [
     Tuning(sv, ap, b)
-    for sv in (4, 16, 64)
-    for ap in (1, 4, 16)
+    for sv in (32, 64, 128)
+    for ap in (32, 64, 128)
     for b in (2, 3)
 ]
 
@@ -45,6 +47,19 @@ def mix_key(jobs, device) -> str:
     mix = Counter((j.kind, j.width, j.height, j.depth) for j in jobs)
     text = json.dumps([props.name, props.multi_processor_count, build, sorted(mix.items())])
     return hashlib.sha256(text.encode()).hexdigest()[:24]
+
+
+def sample(jobs, every: int, sm_count: int):
+    """Every ``every``-th job, or more of them where those are few enough
+    columns for lanes to share one and the whole batch's are not."""
+
+    def few(some):
+        return 4 * sum(j.width * j.height for j in some if j.kind == AERIAL) <= 3 * 256 * sm_count
+
+    every = max(every, 1)
+    while every > 1 and few(jobs[::every]) != few(jobs):
+        every //= 2
+    return jobs[::every]
 
 
 def _time(builder: BatchedLutBuilder, prepared, jobs, tuning: Tuning, arena, reps: int) -> float:
@@ -73,7 +88,7 @@ def tune(builder: BatchedLutBuilder, jobs, sample_every: int = 8, reps: int = 2,
     if use_cache and key in cache:
         t = cache[key]["tuning"]
         return Tuning(**t), {"cached": True, "key": key}
-    subset = jobs[::max(sample_every, 1)]
+    subset = sample(jobs, sample_every, torch.cuda.get_device_properties(builder.device).multi_processor_count)
     prepared = builder.prepare(subset)
     arena = torch.empty((prepared[1], 4), dtype=torch.float32, device=builder.device)
     report = {}

@@ -55,6 +55,10 @@ class BatchJob:
 
 @dataclass
 class Tuning:
+    """Work split of a batch (``AtmBatchTuning``): both item sizes are rounded
+    up to multiples of a warp's 32 units; a batch of few columns splits them
+    by itself."""
+
     sky_view_texels_per_item: int = 16
     aerial_columns_per_item: int = 4
     blocks_per_sm: int = 3
