@@ -349,12 +349,12 @@ __device__ __forceinline__ float display_channel(float v) {
 }
 
 // _resolve, postprocess.py:155-174: runs along the image's contiguous axis
-// (kXFast: x), kResolveRows pixels a thread across it, which share their place
-// on the fast axis.  The ACES quotients, the power and the bloom taps are what
+// (kXFast: x), kRows pixels a thread across it (kResolveRows, in small frames
+// 1), which share their place on the fast axis.  The ACES quotients, the power and the bloom taps are what
 // it executes; 4K with bloom and tone map took 116 us with powf, IEEE
 // quotients and a flat 64-bit pixel index, 75 us with a pixel a thread, 60 us so.
 constexpr int kResolveRows = 8;
-template <bool kXFast, bool kBloom>
+template <bool kXFast, bool kBloom, int kRows>
 __global__ void __launch_bounds__(kRunPixels * kRunRows) k_post_resolve(PostParams Q, ImageLayout L, const float* __restrict__ hdr,
                                                       float* __restrict__ display, const float4* __restrict__ bloom,
                                                       float exposure, float strength, int tone_map) {
@@ -363,14 +363,14 @@ __global__ void __launch_bounds__(kRunPixels * kRunRows) k_post_resolve(PostPara
   int f, group;
   if (!run_element(nf, 0x7fffffff, f, group)) return;
   // the block's rows lie together: thread row t takes t, t + kRunRows, ...
-  const unsigned s0 = (unsigned(group) - threadIdx.y) * kResolveRows + threadIdx.y;
+  const unsigned s0 = (unsigned(group) - threadIdx.y) * kRows + threadIdx.y;
   const BloomAxis fast = kBloom ? bloom_axis(f, nf, bf) : BloomAxis();
   const int64_t at = (kXFast ? f * L.sx + int64_t(s0) * L.sy : int64_t(s0) * L.sx + f * L.sy) * L.channels;
   const int64_t step = (kXFast ? L.sy : L.sx) * kRunRows * L.channels;
   const float* in = hdr + at;
   float* out = display + at;
 #pragma unroll
-  for (int k = 0; k < kResolveRows; ++k) {
+  for (int k = 0; k < kRows; ++k) {
     const unsigned sl = s0 + k * kRunRows;
     if (sl >= unsigned(ns)) return;
     float4 v = scale4(make_float4(in[0], in[1], in[2], 0.0f), exposure);
@@ -389,6 +389,54 @@ __global__ void __launch_bounds__(kRunPixels * kRunRows) k_post_resolve(PostPara
   }
 }
 
+// centre, -1, +1, -2, +2 in the reference's order of summation
+__device__ __forceinline__ float4 taps5(float4 c, float4 m1, float4 p1, float4 m2, float4 p2) {
+  float4 r = scale4(c, kW0);
+  r = add4(r, scale4(m1, kW1));
+  r = add4(r, scale4(p1, kW1));
+  r = add4(r, scale4(m2, kW2));
+  return add4(r, scale4(p2, kW2));
+}
+// One blur pass of a small plane: a tile of kTileS slow rows by kTileF fast
+// texels a block, its neighbourhood loaded once (clamped, which is the edge
+// rule) and both directions' taps taken from shared memory.  A small plane's
+// blur is latency: one load here, a dozen rows one after another in a
+// streaming warp.
+constexpr int kTileF = 32, kTileS = 8, kHalo = 2;
+constexpr int kInF = kTileF + 2 * kHalo, kInS = kTileS + 2 * kHalo;
+template <bool kXFast>
+__global__ void __launch_bounds__(kTileF * kTileS) k_post_blur_tile(PostParams Q, const float4* __restrict__ src,
+                                                                    float4* __restrict__ dst) {
+  __shared__ float4 s_in[kInS][kInF];
+  __shared__ float4 s_mid[kInS][kInF];  // after the x taps
+  const int t = threadIdx.x;
+  const int nf = kXFast ? Q.hw : Q.hh, ns = kXFast ? Q.hh : Q.hw;  // fast / slow extents
+  const int f0 = blockIdx.x * kTileF, s0 = blockIdx.y * kTileS;
+  for (int k = t; k < kInS * kInF; k += kTileF * kTileS) {
+    const int r = k / kInF, c = k % kInF;
+    s_in[r][c] = src[size_t(min(max(s0 - kHalo + r, 0), ns - 1)) * nf + min(max(f0 - kHalo + c, 0), nf - 1)];
+  }
+  __syncthreads();
+  if (kXFast) {  // x along the fast axis, on every slow row
+    for (int k = t; k < kInS * kTileF; k += kTileF * kTileS) {
+      const int r = k / kTileF, c = k % kTileF + kHalo;
+      s_mid[r][c] = taps5(s_in[r][c], s_in[r][c - 1], s_in[r][c + 1], s_in[r][c - 2], s_in[r][c + 2]);
+    }
+  } else {  // x along the slow axis, on every fast column
+    for (int k = t; k < kTileS * kInF; k += kTileF * kTileS) {
+      const int r = k / kInF + kHalo, c = k % kInF;
+      s_mid[r][c] = taps5(s_in[r][c], s_in[r - 1][c], s_in[r + 1][c], s_in[r - 2][c], s_in[r + 2][c]);
+    }
+  }
+  __syncthreads();
+  const int c = t % kTileF + kHalo, r = t / kTileF + kHalo;
+  const int f = f0 + c - kHalo, sl = s0 + r - kHalo;
+  if (f < nf && sl < ns)
+    dst[size_t(sl) * nf + f] =
+        kXFast ? taps5(s_mid[r][c], s_mid[r - 1][c], s_mid[r + 1][c], s_mid[r - 2][c], s_mid[r + 2][c])
+               : taps5(s_mid[r][c], s_mid[r][c - 1], s_mid[r][c + 1], s_mid[r][c - 2], s_mid[r][c + 2]);
+}
+
 // Rows of a blur warp's segment: it first walks 2 kStages rows before and
 // after its own, so segments are long, unless the plane is too small to give
 // every scheduler of the chip four warps that way (two: 8 us more at 1920x1080).
@@ -402,6 +450,19 @@ void blur(const PostParams& Q, const float4* src, float4* dst, cudaStream_t s) {
   k_post_blur<kXFast, kStages><<<grid, 32 * kBlurWarps, 0, s>>>(Q, src, dst, segment);
 }
 
+template <bool kXFast>
+void blur_tiles(const PostParams& Q, const float4* src, float4* dst, cudaStream_t s) {
+  const int nf = kXFast ? Q.hw : Q.hh, ns = kXFast ? Q.hh : Q.hw;
+  k_post_blur_tile<kXFast><<<dim3((nf - 1) / kTileF + 1, (ns - 1) / kTileS + 1), kTileF * kTileS, 0, s>>>(Q, src, dst);
+}
+// Planes up to this take the blur by tiles and the resolve a pixel a thread:
+// their launches wait for a warp's chain of rows, not for the chip.  Frames of
+// 96x54, 640x360 and 960x540 with four passes: 10.9, 14.4 and 19.2 us so, 19.9,
+// 22.7 and 23.9 us streaming; 1366x767 27.1 and 28.7, but with its HDR image
+// just written the two launches fewer weigh more (a whole frame of that size
+// 552 us streaming, 556 so); 1920x1080 45.3 and 41.5.
+constexpr long long kSmallPlane = 3LL << 16;
+
 }  // namespace
 
 bool image_x_fast(const ImageLayout& L) {
@@ -413,6 +474,7 @@ cudaError_t launch_post(const PostParams& Q, const ImageLayout& L, const float* 
                         float4* bloom_b, float exposure, float strength, int passes, bool use_bloom, bool tone_map,
                         const float4** bloom_out, cudaStream_t s) {
   const float4* bloom = bloom_a;
+  const bool small = (long long)Q.hw * Q.hh <= kSmallPlane;
   if (use_bloom) {
     const int nf = Q.x_fast ? Q.hw : Q.hh, ns = Q.x_fast ? Q.hh : Q.hw;
     k_post_extract<<<run_grid(nf, ns), run_block(), 0, s>>>(Q, L, hdr, 0.25f * exposure, bloom_a);  // exact: a power of two
@@ -420,9 +482,11 @@ cudaError_t launch_post(const PostParams& Q, const ImageLayout& L, const float* 
     if (e != cudaSuccess) return e;
     float4* src = bloom_a;
     float4* dst = bloom_b;
-    for (int p = 0; p < passes; p += 2) {
+    for (int p = 0; p < passes; p += small ? 1 : 2) {
       const bool two = p + 1 < passes;
-      if (Q.x_fast)
+      if (small)
+        Q.x_fast ? blur_tiles<true>(Q, src, dst, s) : blur_tiles<false>(Q, src, dst, s);
+      else if (Q.x_fast)
         two ? blur<true, 2>(Q, src, dst, s) : blur<true, 1>(Q, src, dst, s);
       else
         two ? blur<false, 2>(Q, src, dst, s) : blur<false, 1>(Q, src, dst, s);
@@ -436,8 +500,12 @@ cudaError_t launch_post(const PostParams& Q, const ImageLayout& L, const float* 
   const auto resolve = [&](auto x_fast, auto with_bloom) {
     constexpr bool kXFast = decltype(x_fast)::value, kBloom = decltype(with_bloom)::value;
     const int nf = kXFast ? L.width : L.height, ns = kXFast ? L.height : L.width;
-    k_post_resolve<kXFast, kBloom><<<run_grid(nf, (ns - 1) / kResolveRows + 1), run_block(), 0, s>>>(
-        Q, L, hdr, display, bloom, exposure, strength, tone_map ? 1 : 0);
+    const auto go = [&](auto kernel, int rows) {
+      kernel<<<run_grid(nf, (ns - 1) / rows + 1), run_block(), 0, s>>>(Q, L, hdr, display, bloom, exposure, strength,
+                                                                      tone_map ? 1 : 0);
+    };
+    small ? go(k_post_resolve<kXFast, kBloom, 1>, 1)
+          : go(k_post_resolve<kXFast, kBloom, kResolveRows>, kResolveRows);
   };
   if (Q.x_fast)
     use_bloom ? resolve(std::true_type(), std::true_type()) : resolve(std::true_type(), std::false_type());
