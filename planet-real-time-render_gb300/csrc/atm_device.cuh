@@ -695,17 +695,17 @@ __device__ __forceinline__ float mie_phase(const DevParams& P, float c) {
 // from phi = (1 - e^-x) / x: weight = step phi, T = 1 - ext weight (step
 // itself at ext = 0, as the reference's ext <= 1e-12 branch).  phi is a
 // polynomial, near-minimax with phi(0) = 1: degree 4 up to x = 1/4, which
-// most segments are within, degree 6 up to 1, 2.9e-9 and 2.7e-9 off; a
-// rounding error each in float, 4 and 6 operations a channel, against 7 and
-// 2^x for the form e^(-x/2) sinh(x/2) / (x/2).  Larger x take 1 - T, which
+// most segments are within, degree 6 up to 1, both within 3e-9 of phi with
+// their float coefficients; a rounding error each in float, 4 and 6 operations
+// a channel, against 7 and 2^x for the form e^(-x/2) sinh(x/2) / (x/2).  Larger x take 1 - T, which
 // keeps 7 digits.
 __device__ __forceinline__ float phi_quarter(float x) {
   return fmaf(x, fmaf(x, fmaf(x, fmaf(x, 0.007530156057327986f, -0.04150012508034706f), 0.1666528880596161f),
                       -0.49999964237213135f), 1.0f);
 }
 __device__ __forceinline__ float phi_one(float x) {
-  const float high = fmaf(x, fmaf(x, 0.00012912976671941578f, -0.0013011228293180466f), 0.008276204578578472f);
-  return fmaf(x, fmaf(x, fmaf(x, fmaf(x, high, -0.04164746776223183f), 0.16666366159915924f), -0.49999985098838806f),
+  const float high = fmaf(x, fmaf(x, 0.00012931223318446428f, -0.0013017107266932726f), 0.008276925422251225f);
+  return fmaf(x, fmaf(x, fmaf(x, fmaf(x, high, -0.041647881269454956f), 0.1666637659072876f), -0.49999985098838806f),
               1.0f);
 }
 __device__ __forceinline__ void segment_any(float ext, float x, float step, float& tr, float& w) {
