@@ -596,10 +596,14 @@ __device__ __forceinline__ f3 sample_t_at(const DevParams& P, const Frame& F, fl
   const float u = __saturatef((d - dmin) * frcp(mx((rho + F.shell_top) - dmin, 1.0e-6f)));
   return bilinear_at(F.tlut, P.t_lut, fmaf(u, P.t_lut.w, -0.5f), fmaf(rho, F.t_rho, -0.5f));
 }
-__device__ __forceinline__ f3 sample_t(const DevParams& P, const Frame& F, float h, float cosv) {
+// The same from any altitude, with IEEE operations where the march takes the
+// hardware's: once a pixel (camera_t).
+__device__ __forceinline__ f3 sample_t(const DevParams& P, const Frame& F, float h, float rc) {
   const float a = clampf(h, 0.0f, P.top);
-  const float rho2 = a * (2.0f * F.bottom + a);
-  return sample_t_at(P, F, a, rho2, fsqrt(rho2), (F.bottom + a) * cosv);
+  const float rho = sqrtf(a * (2.0f * F.bottom + a)), dmin = P.top - a;
+  const float d = sqrtf(mx(fmaf(rc, rc, dmin * ((2.0f * F.bottom + P.top) + a)), 0.0f)) - rc;
+  const float u = __saturatef((d - dmin) / mx((rho + F.shell_top) - dmin, 1.0e-6f));
+  return bilinear_at(F.tlut, P.t_lut, fmaf(u, P.t_lut.w, -0.5f), fmaf(rho, F.t_rho, -0.5f));
 }
 // _sample_multi_scattering :642-683
 __device__ __forceinline__ f3 sample_ms(const DevParams& P, const Frame& F, float h, float sc, float hc) {

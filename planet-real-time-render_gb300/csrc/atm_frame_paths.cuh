@@ -275,10 +275,10 @@ __device__ __forceinline__ f3 integrate_surface_split(const DevParams& P, const 
   return vmax(group_compose<kLanes>(acc).L, 0.0f);
 }
 
-// The transmittance LUT at distance t along a camera ray, in the direction of
-// the ray (sign 1) or back toward the camera (sign -1): the local vertical's
-// cosine is (t - t_c) / r, so neither the point nor its normal is formed.
-__device__ __forceinline__ f3 ray_t(const DevParams& P, const Frame& F, const RayGeom& G, float t, float sign) {
+// The transmittance LUT at distance t along a camera ray, back toward the
+// camera: the local vertical's cosine is (t - t_c) / r, so neither the point nor
+// its normal is formed.
+__device__ __forceinline__ f3 ray_t(const DevParams& P, const Frame& F, const RayGeom& G, float t) {
   const float u = t - G.t0;
   const float delta = fmaf(u, u, fmaf(G.q1, u, G.q0));
   const float r2 = mx(fmaf(F.bottom, F.bottom, delta), 1.0f);
@@ -286,13 +286,13 @@ __device__ __forceinline__ f3 ray_t(const DevParams& P, const Frame& F, const Ra
   const float h = clampf(delta * frcp(r2 * inv_r + F.bottom), 0.0f, P.top);
   const float rho2 = clampf(delta, 0.0f, F.shell2);
   // clamped with the radius that the clamped altitude has
-  return sample_t_at(P, F, h, rho2, fsqrt(rho2), sign * (t - G.tc) * (inv_r * (F.bottom + h)));
+  return sample_t_at(P, F, h, rho2, fsqrt(rho2), (G.tc - t) * (inv_r * (F.bottom + h)));
 }
 
 // _surface_segment_transmittance :1603-1665 on an already clipped interval.
 __device__ __forceinline__ f3 surface_segment_t(const DevParams& P, const Frame& F, const RayGeom& G, float start,
                                                 float end) {
-  const f3 s2t = ray_t(P, F, G, end, -1.0f), n2t = vmax(ray_t(P, F, G, start, -1.0f), 1.0e-6f);
+  const f3 s2t = ray_t(P, F, G, end), n2t = vmax(ray_t(P, F, G, start), 1.0e-6f);
   return vclamp(mk(fdiv(s2t.x, n2t.x), fdiv(s2t.y, n2t.y), fdiv(s2t.z, n2t.z)), 0.0f, 1.0f);
 }
 
@@ -303,7 +303,8 @@ __device__ __forceinline__ f3 camera_t(const DevParams& P, const Frame& F, const
   segment_of(P, G, F.bottom, s, e, valid, ground);
   if (!valid) return splat(1.0f);
   if (ground) return splat(0.0f);
-  return ray_t(P, F, G, s, 1.0f);
+  // a ray that does not start in the shell enters it at its top
+  return sample_t(P, F, s > 0.0f ? P.top : G.h0, s - G.tc);
 }
 
 // _sample_sky_view :1474-1525
