@@ -35,34 +35,23 @@ namespace {
 constexpr unsigned kAll = 0xffffffffu;
 
 // The features are rounded to BF16, and what they cost is most of what a
-// network pixel executes beside its network: they take the hardware's square
-// root, reciprocal and rsqrt (1-2 ulp).  The sun cosines do not: gates
-// compare them, and a pixel's path hangs on their last bit.
-//
-// acos by Abramowitz and Stegun 4.4.46, 2e-8 off: a root and eight operations.
-__device__ __forceinline__ float feature_acos(float c) {
-  const float x = fabsf(c);
-  float p = fmaf(x, -0.0012624911f, 0.0066700901f);
-  p = fmaf(x, p, -0.0170881256f);
-  p = fmaf(x, p, 0.0308918810f);
-  p = fmaf(x, p, -0.0501743046f);
-  p = fmaf(x, p, 0.0889789874f);
-  p = fmaf(x, p, -0.2145988016f);
-  p = fmaf(x, p, 1.5707963050f) * fsqrt(__saturatef(1.0f - x));
-  return c < 0.0f ? kPiF - p : p;
-}
-// The horizon's zenith angle at altitude h (sky_horizon_zenith).
-__device__ __forceinline__ float horizon_feature(float h, float bottom) {
-  const float a = mx(h, 0.0f);
-  return kPiF - feature_acos(clampf(shell_rho(a, bottom) * frcp(mx(bottom + a, 1.0f)), 0.0f, 1.0f));
-}
+// network pixel executes beside its network: the points along the ray and the
+// azimuth take the hardware's square root and rsqrt (1-2 ulp) there, and IEEE
+// operations in the training samples, whose features are FP32.  The start
+// point's altitude and view, a difference of two angles, and the sun cosines
+// that gates compare keep IEEE operations in both (a 4K frame of two cameras
+// 1.96 ms; 1.94 with hardware functions and a polynomial acos throughout, which
+// left the view feature 4.5e-6 off, rms, instead of 1.7e-6; 2.04 ms with IEEE
+// operations throughout).
+
 // Sky-view v of a zenith angle whose cosine is mu (sky_zenith_to_v), hz the
 // horizon's.
 __device__ __forceinline__ float view_feature(float mu, float hz) {
-  const float z = feature_acos(clampf(mu, -1.0f, 1.0f));
+  const float z = acosf(clampf(mu, -1.0f, 1.0f));
   const bool above = z < hz;
-  const float n = __saturatef(fdiv(above ? z : z - hz, mx(above ? hz : kPiF - hz, 1.0e-6f)));
-  return above ? 0.5f * (1.0f - fsqrt(1.0f - n)) : 0.5f + 0.5f * fsqrt(n);
+  const float n = __saturatef((above ? z : z - hz) / mx(above ? hz : kPiF - hz, 1.0e-6f));
+  const float half_root = 0.5f * sqrtf(above ? 1.0f - n : n);
+  return above ? 0.5f - half_root : 0.5f + half_root;
 }
 // Cosine of the azimuth between two horizontal vectors, from their dot
 // product and squared lengths; 1 where one is shorter than 1e-6.
@@ -78,7 +67,7 @@ struct StartPoint {
   float mu_s, ts2, x0, x2, hz;
 };
 __device__ __forceinline__ float altitude_feature(const DevParams& P, float h) {
-  return 2.0f * fsqrt(__saturatef(h * P.inv_top)) - 1.0f;
+  return 2.0f * sqrtf(__saturatef(h * P.inv_top)) - 1.0f;
 }
 __device__ __forceinline__ float sun_feature(float bottom, float h, float mu_s) {
   return 2.0f * sun_cosine_to_u(clampf(mu_s, -1.0f, 1.0f), horizon_cosine(h, bottom)) - 1.0f;
@@ -95,7 +84,7 @@ __device__ __forceinline__ StartPoint start_point(const DevParams& P, const Fram
   S.ts2 = dot(S.ts, S.ts);
   S.x0 = altitude_feature(P, h);
   S.x2 = sun_feature(F.bottom, h, S.mu_s);
-  S.hz = horizon_feature(h, F.bottom);
+  S.hz = sky_horizon_zenith(h, F.bottom);
   return S;
 }
 
@@ -104,31 +93,33 @@ __device__ __forceinline__ StartPoint start_point(const DevParams& P, const Fram
 // Where a segment's light comes from depends on where it ends and how low it
 // dips as much as on where it starts: with these points given, the sky
 // network's held-out error drops by a quarter and the aerial network's on
-// camera-to-surface segments to a third.  Returns the point's sun cosine,
-// exact (kGate) for a gate or as the feature takes it.
-template <bool kGate>
+// camera-to-surface segments to a third.  Returns the point's sun cosine.
+// kExactSun, kExactAltitude: IEEE operations (a gate, a training sample).
+template <bool kExactSun, bool kExactAltitude>
 __device__ __forceinline__ float point_features(const DevParams& P, float bottom, const RayGeom& G, f3 ray, float o_y,
                                                 f3 sun, float t, float* x) {
   const f3 pt = mk(ray.x * t, o_y + ray.y * t, ray.z * t);
-  const float mu = clampf(kGate ? dot(sun, pt) / mx(norm(pt), 1.0f) : dot(sun, pt) * frsqrt(mx(dot(pt, pt), 1.0f)),
-                          -1.0f, 1.0f);
+  const float mu = clampf(kExactSun ? dot(sun, pt) / mx(norm(pt), 1.0f)
+                                    : dot(sun, pt) * frsqrt(mx(dot(pt, pt), 1.0f)), -1.0f, 1.0f);
   const float h = altitude_at(G, t, bottom);
   x[0] = 2.0f * sun_cosine_to_u(mu, horizon_cosine(h, bottom)) - 1.0f;
-  x[1] = 2.0f * fsqrt(__saturatef(h * P.inv_top)) - 1.0f;
+  x[1] = kExactAltitude ? altitude_feature(P, h) : 2.0f * fsqrt(__saturatef(h * P.inv_top)) - 1.0f;
   return mu;
 }
 // Aerial x[7..10]: the segment's end, then its middle.  Returns the smaller
 // |sun cosine| of the two (the twilight gate); `mu_end`, `mu_mid` receive
-// the cosines themselves.
+// the cosines themselves.  kSample: of a training sample.
+template <bool kSample>
 __device__ __forceinline__ float segment_features(const DevParams& P, float bottom, const RayGeom& G, f3 ray,
                                                   float o_y, f3 sun, float start, float end, float* x,
                                                   float& mu_end, float& mu_mid) {
-  mu_end = point_features<true>(P, bottom, G, ray, o_y, sun, end, x + 7);
-  mu_mid = point_features<true>(P, bottom, G, ray, o_y, sun, 0.5f * (start + end), x + 9);
+  mu_end = point_features<true, kSample>(P, bottom, G, ray, o_y, sun, end, x + 7);
+  mu_mid = point_features<true, kSample>(P, bottom, G, ray, o_y, sun, 0.5f * (start + end), x + 9);
   return mn(fabsf(mu_end), fabsf(mu_mid));
 }
 // Sky x[6..9]: the end of the ray's march (the shell top or the ground),
 // then its lowest point (the closest approach, clamped to the march).
+template <bool kSample>
 __device__ __forceinline__ void sky_ray_features(const DevParams& P, float bottom, float h, f3 ray, f3 sun, float* x) {
   const RayGeom G = camera_ray_geom(P, bottom, h, ray);
   float start, end;
@@ -136,8 +127,8 @@ __device__ __forceinline__ void sky_ray_features(const DevParams& P, float botto
   segment_of(P, G, bottom, start, end, valid, ground);
   if (!valid) start = end = 0.0f;
   const float o_y = bottom + mx(h, 0.0f);
-  point_features<false>(P, bottom, G, ray, o_y, sun, end, x + 6);
-  point_features<false>(P, bottom, G, ray, o_y, sun, clampf(G.tc, start, end), x + 8);
+  point_features<kSample, kSample>(P, bottom, G, ray, o_y, sun, end, x + 6);
+  point_features<kSample, kSample>(P, bottom, G, ray, o_y, sun, clampf(G.tc, start, end), x + 8);
 }
 
 // Counter-based uniform in [0, 1): 64-bit mix of (seed, index, lane).
@@ -195,7 +186,7 @@ __global__ void __launch_bounds__(128) k_gen_samples(const SurrogateSetDev* __re
     const f3 sun = mk(ss * cphi, mu_s, ss * sphi);
     // rounding-consistent features
     x[0] = altitude_feature(P, h);
-    x[1] = 2.0f * view_feature(mu_v, horizon_feature(h, R)) - 1.0f;
+    x[1] = 2.0f * view_feature(mu_v, sky_horizon_zenith(h, R)) - 1.0f;
     x[2] = sun_feature(R, h, mu_s);
     x[3] = clampf(cphi, -1.0f, 1.0f);
     x[4] = S.lhr_n;
@@ -206,7 +197,7 @@ __global__ void __launch_bounds__(128) k_gen_samples(const SurrogateSetDev* __re
     if (kind == 0) {  // sky: 10 features -> log(L/E + floor)
       const f3 L = sky_radiance(P, F, h, ray) * inv_e;
       samples = uint32_t(P.sv_steps);
-      sky_ray_features(P, R, h, ray, sun, x);
+      sky_ray_features<true>(P, R, h, ray, sun, x);
       for (int k = 0; k < kSurrogateSkyIn; ++k) features[i * kSurrogateSkyIn + k] = x[k];
       targets[i * 3 + 0] = logf(L.x + kSurrogateFloor);
       targets[i * 3 + 1] = logf(L.y + kSurrogateFloor);
@@ -236,7 +227,7 @@ __global__ void __launch_bounds__(128) k_gen_samples(const SurrogateSetDev* __re
         start = end = 0.0f;
       }
       float mu_end, mu_mid;
-      segment_features(P, R, G, ray, R + h, sun, start, end, x, mu_end, mu_mid);
+      segment_features<true>(P, R, G, ray, R + h, sun, start, end, x, mu_end, mu_mid);
       for (int k = 0; k < kSurrogateApIn; ++k) features[i * kSurrogateApIn + k] = x[k];
       targets[i * 6 + 0] = logf(L.x + kSurrogateFloor);
       targets[i * 6 + 1] = logf(L.y + kSurrogateFloor);
@@ -447,7 +438,7 @@ __global__ void __launch_bounds__(128 * kWorkers, 1) k_composite_surrogate(
           // of different signs there (the segment crosses the terminator)
           float mu_end, mu_mid;
           const float mu_min =
-              mn(fabsf(mu_s), segment_features(P, A.bottom, G, ray, o_y, F.sun, start, end, fx, mu_end, mu_mid));
+              mn(fabsf(mu_s), segment_features<false>(P, A.bottom, G, ray, o_y, F.sun, start, end, fx, mu_end, mu_mid));
           const bool crosses =
               nets.gate_crossing && ((mu_s > 0.0f) != (mu_end > 0.0f) || (mu_s > 0.0f) != (mu_mid > 0.0f));
           kind = (mu_min < nets.twilight_cos || crosses) ? kSurfPlain : kSurfMlp;
@@ -458,7 +449,7 @@ __global__ void __launch_bounds__(128 * kWorkers, 1) k_composite_surrogate(
         sky_start_features(B, F, ray, fx);
         fx[4] = nets.lhr_n;
         fx[5] = nets.lhm_n;
-        sky_ray_features(P, A.bottom, A.cam_alt, ray, F.sun, fx);
+        sky_ray_features<false>(P, A.bottom, A.cam_alt, ray, F.sun, fx);
         pack_inputs(fx, kSurrogateSkyIn, xp);
       } else {
         kind = kSkyLut;
@@ -776,7 +767,7 @@ __global__ void __launch_bounds__(128 * kWorkers, 1) k_sky_pixels_net(DevParams 
       sky_start_features(B, F, ray, fx);
       fx[4] = nets.lhr_n;
       fx[5] = nets.lhm_n;
-      sky_ray_features(P, A.bottom, A.cam_alt, ray, F.sun, fx);
+      sky_ray_features<false>(P, A.bottom, A.cam_alt, ray, F.sun, fx);
       pack_inputs(fx, kSurrogateSkyIn, xp);
     }
     const bool need = tc::tile_any(T.tile, net);
