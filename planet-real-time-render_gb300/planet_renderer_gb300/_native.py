@@ -396,6 +396,17 @@ def check(rc: int) -> None:
 _current_raw_stream = None
 
 
+def _raw_stream_of():
+    """A function from a device index to its current stream's handle: torch's
+    own, or its public Stream object where a torch does not have it."""
+
+    import torch
+
+    torch.cuda.init()
+    return getattr(torch._C, "_cuda_getCurrentRawStream",
+                   lambda index: torch.cuda.current_stream(index).cuda_stream)
+
+
 def stream(device) -> ctypes.c_void_p:
     """The handle of ``device``'s current torch stream.  The raw handle is
     0.1 us; ``torch.cuda.current_stream`` forms a Stream object on the way
@@ -403,10 +414,7 @@ def stream(device) -> ctypes.c_void_p:
 
     global _current_raw_stream
     if _current_raw_stream is None:
-        import torch
-
-        torch.cuda.init()
-        _current_raw_stream = torch._C._cuda_getCurrentRawStream
+        _current_raw_stream = _raw_stream_of()
     if device.type != "cuda":
         raise ValueError(f"Expected a cuda device, but got: {device}")
     index = device.index
