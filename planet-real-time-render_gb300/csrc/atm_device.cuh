@@ -111,7 +111,6 @@ __device__ __forceinline__ float fexp2(float x) {
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
   return r;
 }
-__device__ __forceinline__ float fnorm(f3 a) { return fsqrt(dot(a, a)); }
 
 // Adds a per-lane count into a device counter: one atomic per warp.  Every
 // lane of the warp must call it (no lane may have exited before).
@@ -256,16 +255,6 @@ __device__ __forceinline__ void segment_vec(const DevParams& P, f3 o, f3 d, floa
     }
   }
 }
-__device__ __forceinline__ void aerial_prefix(const DevParams& P, float h, float cosv, float bottom, float& start,
-                                              float& end, bool& valid) {
-  bool v, g;
-  segment_from_altitude(P, h, cosv, bottom, start, end, v, g);
-  if (v && !g) {
-    float closest = -(bottom + h) * cosv;
-    if (closest > start && closest < end) end = closest;
-  }
-  valid = v && end > start;
-}
 
 // ---- per-ray geometry ---------------------------------------------------------
 // a + b = s + err exactly (Knuth's two-sum; no contraction applies to it).
@@ -340,10 +329,6 @@ __device__ __forceinline__ float altitude_at(const RayGeom& G, float t, float bo
   const float delta = (G.q0 + G.q1 * u) + u * u;
   const float len = fsqrt(mx(bottom * bottom + delta, 0.0f));
   return fdiv(delta, mx(len + bottom, 1.0f));
-}
-// Cosine between the ray and the local vertical at distance t, r = R + h.
-__device__ __forceinline__ float vertical_cosine_at(const RayGeom& G, float t, float radius) {
-  return (t - G.tc) * frcp(mx(radius, 1.0f));
 }
 // Roots of the ray with the sphere of radius bottom + shell.
 __device__ __forceinline__ void shell_roots_g(const RayGeom& G, float shell, float bottom, float& nearv, float& farv,

@@ -136,13 +136,10 @@ __device__ __forceinline__ void st8(uint32_t taddr, const uint32_t (&v)[8]) {
 }
 __device__ __forceinline__ void wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
-// Named barrier over the 128 threads of one tile (ids 1..).
-__device__ __forceinline__ void tile_sync(int tile) {
-  asm volatile("bar.sync %0, 128;" ::"r"(tile + 1) : "memory");
-}
-// The same barrier, returning whether v holds in every thread of the tile:
-// a bounded wait can end true in one thread and false in another, and the
-// tile must take one path afterwards (its barriers stay matched).
+// Named barrier over the 128 threads of one tile (ids 1..), returning whether v
+// holds in every thread of the tile: a bounded wait can end true in one thread
+// and false in another, and the tile must take one path afterwards (its
+// barriers stay matched).
 __device__ __forceinline__ bool tile_all(int tile, bool v) {
   uint32_t r;
   __syncwarp();  // the barrier takes whole warps
