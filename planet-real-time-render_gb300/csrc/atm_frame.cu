@@ -8,7 +8,7 @@
 // lanes in small frames, launch_split); a warp covers an 8x4 pixel tile so
 // that the data-dependent paths (sky vs surface, refined intervals) diverge as
 // little as neighbouring pixels do.  Bound by instruction issue (88% active,
-// about 290 instructions a sample).  The
+// about 266 instructions a sample).  The
 // terminator weight reuses the disk visibility of the interval's coarse
 // sample, which the reference computes twice from identical inputs.
 #include <cuda_runtime.h>

@@ -12,8 +12,8 @@
 //  * k_raster_depth (and k_raster_depth_tiles): coverage
 //    by the edge equations with the top-left rule and a 64-bit atomic
 //    minimum of (depth bits << 32 | triangle) per pixel; small triangles by
-//    eight lanes, medium ones by a warp, large ones cut into 8 x 32 pixel
-//    tiles spread over the whole grid;
+//    eight lanes, medium ones by a warp, large ones cut into 256 x 32 pixel
+//    blocks spread over the whole grid;
 //  * k_raster_resolve: thread per pixel: the winning triangle's
 //    perspective-correct position, normal, material weights and height, the
 //    dominant vertex's cell id and the albedo of the view mode.
