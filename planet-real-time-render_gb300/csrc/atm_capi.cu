@@ -647,9 +647,10 @@ ATM_API int atm_batch_build(AtmBatch* b, const AtmBatchJob* jobs, int32_t n_jobs
   if (sv_item < 1 || sv_item > 4096 || ap_item < 1 || ap_item > 4096 || tuning->blocks_per_sm < 1 ||
       tuning->blocks_per_sm > 8)
     return fail(ATM_E_INVALID, "tuning out of range");
-  long long columns = 0;
+  long long columns = 0;  // of the volumes whose sizes the loop below accepts
   for (int i = 0; i < n_jobs; ++i)
-    if (jobs[i].kind == ATM_LUT_AERIAL) columns += (long long)jobs[i].width * jobs[i].height;
+    if (jobs[i].kind == ATM_LUT_AERIAL && std::max(jobs[i].width, jobs[i].height) <= 256)
+      columns += std::max(jobs[i].width, 0) * std::max(jobs[i].height, 0);
   const bool groups = atm::batch_groups(columns, b->sm_count, tuning->blocks_per_sm);
   const size_t jsz = atm::batch_job_size();
   b->h_jobs.assign(size_t(n_jobs) * jsz, 0);
