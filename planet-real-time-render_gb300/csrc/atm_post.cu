@@ -356,7 +356,7 @@ __device__ __forceinline__ float display_channel(float v) {
 // 1), which share their place on the fast axis.  The ACES quotients, the power
 // and the bloom taps are what it executes; 4K with bloom and tone map took 116
 // us with powf, IEEE quotients and a flat 64-bit pixel index, 75 us with a
-// pixel a thread, 60 us so (64 with the nearer power).
+// pixel a thread, 60 us so and 1.5 more for the nearer power.
 constexpr int kResolveRows = 8;
 template <bool kXFast, bool kBloom, int kRows>
 __global__ void __launch_bounds__(kRunPixels * kRunRows) k_post_resolve(PostParams Q, ImageLayout L, const float* __restrict__ hdr,
